@@ -903,7 +903,7 @@ int vc1cu_lp_analyze(vc1cu_lp* net, const vc1cu_params* p, const vc1cu_lp_pass* 
  *
  * Limits: 1 <= n <= 16 pictures per call and 0 <= range <= 32; larger requests are
  * rejected with VC1CU_ERR_ARG. The search state lives in one fixed device array of
- * 168,192 bytes that every GPU loading this library holds until the process exits. All
+ * 134,784 bytes that every GPU loading this library holds until the process exits. All
  * calls on one device share that array: two calls whose GPU work can overlap (issued on
  * different streams, or from threads that do not order them) race on it and give wrong
  * results; calls issued in order on one stream are safe, and devices are independent.

@@ -42,11 +42,13 @@ cudaError_t launch_subpel_planes(const uint8_t* ref, int pitch, int W, int H, in
                                  uint8_t* out, int opitch, int border, long long stride, cudaStream_t s);
 int warp_bytes_for_host(const WinCfg& wc);
 struct GState;
+struct GIn;
 size_t gstate_bytes();
-int run_global_search(GState* d_states, int n, int R, int W, int H, cudaStream_t stream);
+size_t gin_bytes();
+int run_global_search(GState* d_states, const GIn* d_in, int n, int R, int W, int H, cudaStream_t stream);
 cudaError_t launch_global_fanout(const GlobalCopy* d_copies, int n, cudaStream_t s);
-void init_gstate(GState* h, const DevFrame& cur, const DevFrame& ref, int range, int* out_global,
-                 unsigned long long* out_sad);
+void init_gin(GIn* h, const DevFrame& cur, const DevFrame& ref, int range, int* out_global,
+              unsigned long long* out_sad);
 void launch_mc(const DevParams& P, const DevFrame& ref, const int2* mvs, const int2* bmv, const uint8_t* use4, int mode,
                uint8_t* dy, uint8_t* du, uint8_t* dv, int pitch_y, int pitch_c, cudaStream_t s);
 void launch_xform(const DevParams& P, const DevFrame& src, const DevFrame& pred, int type_mask, double* coeffs,
@@ -783,6 +785,41 @@ int score_common(vc1cu_ctx* c, const DevParams& P, const ScoreArgs& a, const vc1
     return VC1CU_OK;
 }
 
+// A batch of whole-frame searches: their inputs in a staging buffer, and on the device the states
+// followed by the inputs' copy (only the inputs travel; the kernels initialise the states).
+struct GSearches {
+    uint8_t* h = nullptr;
+    uint8_t* d_states = nullptr;
+    uint8_t* d_in = nullptr;
+    int n = 0;
+    GIn* host(int k) const { return reinterpret_cast<GIn*>(h + gin_bytes() * k); }
+    GIn* dev(int k) const { return reinterpret_cast<GIn*>(d_in + gin_bytes() * k); }
+    GState* state(int k) const { return reinterpret_cast<GState*>(d_states + gstate_bytes() * k); }
+};
+
+GSearches global_searches(vc1cu_ctx* c, int n) {
+    if (c->gstates_cap < n) {
+        if (c->d_gstates) cudaFree(c->d_gstates);
+        c->d_gstates = nullptr;
+        c->gstates_cap = 0;
+        void* d = nullptr;
+        ck(cudaMalloc(&d, (gstate_bytes() + gin_bytes()) * n), "cudaMalloc(global search state)");
+        c->d_gstates = static_cast<GState*>(d);
+        c->gstates_cap = n;
+    }
+    GSearches g;
+    g.n = n;
+    g.h = static_cast<uint8_t*>(staging(c, gin_bytes() * n));
+    g.d_states = reinterpret_cast<uint8_t*>(c->d_gstates);
+    g.d_in = g.d_states + gstate_bytes() * c->gstates_cap;
+    return g;
+}
+
+void global_searches_send(vc1cu_ctx* c, const GSearches& g) {
+    ck(cudaMemcpyAsync(g.d_in, g.h, gin_bytes() * g.n, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(global search)");
+    staging_mark(c);
+}
+
 // Launches a batch of independent core passes (global search first for unseeded ones).
 // globals_ready: the unseeded passes' global translation results are already in their slots.
 // Per-pass additions of the learned form (all null for the plain passes): the candidates of a
@@ -932,17 +969,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         }
     if (!globals_ready && !unseeded.empty() && P.range > 0) {
         const int nu = (int)unseeded.size();
-        const size_t gb = gstate_bytes();
-        if (c->gstates_cap < nu) {
-            if (c->d_gstates) cudaFree(c->d_gstates);
-            c->d_gstates = nullptr;
-            c->gstates_cap = 0;
-            void* d = nullptr;
-            ck(cudaMalloc(&d, gb * nu), "cudaMalloc(global search state)");
-            c->d_gstates = static_cast<GState*>(d);
-            c->gstates_cap = nu;
-        }
-        uint8_t* hs = static_cast<uint8_t*>(staging(c, gb * nu));
+        GSearches gs = global_searches(c, nu);
         const int grange = std::min(P.local_range, 32);
         // states in raster-size order, so that every size's searches are one contiguous run
         std::vector<int> order(unseeded);
@@ -951,18 +978,16 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         });
         for (int k = 0; k < nu; ++k) {
             const PassDesc& d = h[order[k]];
-            init_gstate(reinterpret_cast<GState*>(hs + gb * k), d.cur, d.ref, grange, d.out.global, d.out.gsad);
+            init_gin(gs.host(k), d.cur, d.ref, grange, d.out.global, d.out.gsad);
         }
-        ck(cudaMemcpyAsync(c->d_gstates, hs, gb * nu, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(gstate)");
-        staging_mark(c);
+        global_searches_send(c, gs);
         Timer tm(c, kGlobal);
         int launches = 0;
         for (int k0 = 0; k0 < nu;) {
             int k1 = k0 + 1;
             const DevParams& g0 = h[order[k0]].geom;
             while (k1 < nu && h[order[k1]].geom.W == g0.W && h[order[k1]].geom.H == g0.H) ++k1;
-            launches += run_global_search(reinterpret_cast<GState*>(reinterpret_cast<uint8_t*>(c->d_gstates) + gb * k0),
-                                          k1 - k0, grange, g0.W, g0.H, c->stream);
+            launches += run_global_search(gs.state(k0), gs.dev(k0), k1 - k0, grange, g0.W, g0.H, c->stream);
             k0 = k1;
         }
         ck(cudaGetLastError(), "global search launch");
@@ -1256,17 +1281,7 @@ int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
             }
         } else {
             const int nu = (int)un.size();
-            const size_t gb = gstate_bytes();
-            if (c->gstates_cap < nu) {
-                if (c->d_gstates) cudaFree(c->d_gstates);
-                c->d_gstates = nullptr;
-                c->gstates_cap = 0;
-                void* d = nullptr;
-                ck(cudaMalloc(&d, gb * nu), "cudaMalloc(global search state)");
-                c->d_gstates = static_cast<GState*>(d);
-                c->gstates_cap = nu;
-            }
-            uint8_t* hs = static_cast<uint8_t*>(staging(c, gb * nu));
+            GSearches gs = global_searches(c, nu);
             const int grange = std::min(P.local_range, 32);
             for (int k = 0; k < nu; ++k) {
                 const vc1cu_pass& q = passes[un[k]];
@@ -1274,13 +1289,11 @@ int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
                 FrameSlot& fr = frame_slot(c, q.ref_id);
                 if (fc.w != P.W || fc.h != P.H || fr.w != P.W || fr.h != P.H)
                     throw Fail{VC1CU_ERR_ARG, "P-picture reference dimensions do not match the configuration"};
-                init_gstate(reinterpret_cast<GState*>(hs + gb * k), fc.view(), fr.view(), grange, outs[un[k]]->global,
-                            outs[un[k]]->gsad);
+                init_gin(gs.host(k), fc.view(), fr.view(), grange, outs[un[k]]->global, outs[un[k]]->gsad);
             }
-            ck(cudaMemcpyAsync(c->d_gstates, hs, gb * nu, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(gstate)");
-            staging_mark(c);
+            global_searches_send(c, gs);
             Timer tm(c, kGlobal);
-            const int launches = run_global_search(c->d_gstates, nu, grange, P.W, P.H, c->stream);
+            const int launches = run_global_search(gs.state(0), gs.dev(0), nu, grange, P.W, P.H, c->stream);
             ck(cudaGetLastError(), "global search launch");
             tm.stop(launches);
             // the passes that reuse a search take its result, in one launch (not one copy each)
@@ -1697,21 +1710,13 @@ void ic_estimate(vc1cu_ctx* c, const DevParams& P, const std::vector<IcJob>& job
 void global_search_one(vc1cu_ctx* c, const DevFrame& cur, const DevFrame& ref, int range, int W, int H, int slot, int mbs,
                        int* dx, int* dy, uint64_t* sad) {
     ResultSlot& s = result_slot(c, slot, mbs, true);
-    const size_t gb = gstate_bytes();
-    if (c->gstates_cap < 1) {
-        void* d = nullptr;
-        ck(cudaMalloc(&d, gb), "cudaMalloc(global search state)");
-        c->d_gstates = static_cast<GState*>(d);
-        c->gstates_cap = 1;
-    }
-    uint8_t* hs = static_cast<uint8_t*>(staging(c, gb));
+    GSearches gs_in = global_searches(c, 1);
     const int grange = std::min(range, 32);
-    init_gstate(reinterpret_cast<GState*>(hs), cur, ref, grange, s.r.global, s.r.gsad);
-    ck(cudaMemcpyAsync(c->d_gstates, hs, gb, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(gstate)");
-    staging_mark(c);
+    init_gin(gs_in.host(0), cur, ref, grange, s.r.global, s.r.gsad);
+    global_searches_send(c, gs_in);
     {
         Timer tm(c, kGlobal);
-        const int launches = run_global_search(c->d_gstates, 1, grange, W, H, c->stream);
+        const int launches = run_global_search(gs_in.state(0), gs_in.dev(0), 1, grange, W, H, c->stream);
         ck(cudaGetLastError(), "global search launch");
         tm.stop(launches);
     }

@@ -5,8 +5,18 @@
 // with frame_sad (encoder_motion.cpp:1499-1576) and then folded by a sequential rule
 // (top-8 insertion with truncation, first-visit tie breaks). Here every stage is one
 // parallel scoring launch (one block per candidate x row slab, partial sums combined with
-// integer atomics, so the order of summation does not matter) followed by a one-thread
-// replay of the reference's sequential fold over the precomputed costs.
+// integer atomics, so the order of summation does not matter); the last block of a picture to
+// finish folds the stage's costs and plans the next stage, so a search is one planning launch
+// and one launch per stage.
+//
+// The fold is bound by latency, not work (at most 392 costs per stage). Its rules are restated
+// in an order-free form where the reference's result is one: the plain search's top-8 insertion
+// with truncation keeps the eight least of a multiset, found by ranking every cost against every
+// other; its refinement keeps the first-visited least cost, a minimum over (cost, |d|, slot) with
+// the visit order as the slot index. The extended search's list (least cost per vector, sorted
+// only on insertion) does depend on the order and is replayed by one warp, entry per lane.
+// Folding on one thread, with the lists in global memory, took 117 us per stage at range 31
+// (0.46-0.94 ms of a call); this form takes about 4 us.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -16,301 +26,348 @@
 namespace vc1cu {
 
 constexpr int kGMaxCand = 512;  // largest stage: range 31 refine, 8 x 7 x 7 = 392
+constexpr int kGThreads = 256;
+constexpr int kGTop = 8;
 
-struct GCand {
-    int dx, dy, stride;
-};
-
-struct GState {
-    // inputs
+// One search's inputs and output addresses.
+struct GIn {
     DevFrame cur, ref;
     int range;                 // min(local range, 32)
     int* out_global;           // [dx, dy]
     unsigned long long* out_sad;
-    // stage scratch
-    int n;                     // candidates of the current stage
-    GCand cand[kGMaxCand];
-    unsigned long long cost[kGMaxCand];
-    // fold state
-    int top_n;
-    unsigned long long top_cost[9];
-    int top_dx[9], top_dy[9];
-    int best_dx, best_dy;
-    unsigned long long best_cost;
-    int phase;
 };
 
-__device__ __forceinline__ bool gless(unsigned long long ca, int ax, int ay, unsigned long long cb, int bx, int by) {
-    if (ca != cb) return ca < cb;
-    const int am = iabs(ax) + iabs(ay), bm = iabs(bx) + iabs(by);
-    if (am != bm) return am < bm;
-    if (ay != by) return ay < by;
-    return ax < bx;
+struct GState {
+    GIn in;
+    int n;                     // candidate slots of the current stage
+    int arrived;               // blocks of the current stage that have finished
+    int top_n;
+    int sorted;                // extended search: no cost was lowered since the list's last insertion
+    int2 top[kGTop];
+    unsigned long long top_cost[kGTop];
+    int2 cand[kGMaxCand];      // x = INT_MIN: an empty slot
+    unsigned long long cost[kGMaxCand];
+};
+
+constexpr int kGEmpty = -0x7fffffff - 1;
+
+// (cost, |dx| + |dy|, dy, dx) in one comparable key: a frame SAD of at most 16384 x 16384 samples
+// is below 2^37, |d| <= 64 and each component within [-32, 32].
+__device__ __forceinline__ unsigned long long gkey(unsigned long long cost, int2 d) {
+    return (cost << 21) | ((unsigned long long)(iabs(d.x) + iabs(d.y)) << 14) | ((unsigned long long)(d.y + 32) << 7) |
+           (unsigned long long)(d.x + 32);
 }
 
-// frame_sad of every candidate of every state: grid (slab, candidate, state)
-__global__ void gsad_kernel(GState* states, int W, int H, int rows_per_slab) {
+// Sampling stride of a search's stages.
+__host__ __device__ inline int gstage_stride(int R, int stage) {
+    if (R <= 0) return 1;
+    if (R <= 31) return stage == 0 ? 4 : (stage == 1 ? 2 : 1);
+    return stage == 0 ? 16 : (stage == 1 ? 8 : (stage == 2 ? 4 : 1));
+}
+__host__ __device__ inline int gstage_count(int R) { return R <= 0 ? 1 : (R <= 31 ? 3 : 4); }
+__host__ __device__ inline int gcoarse_step(int R) { return R >= 4 ? 4 : (R >= 2 ? 2 : 1); }
+constexpr int kGExtStep = 8;  // the extended search's step (its range is 32 here)
+
+// Candidate slots of a stage (an upper bound where slots may be empty).
+__host__ __device__ inline int gstage_slots(int R, int stage) {
+    if (R <= 0) return 1;
+    if (R <= 31) {
+        const int cs = gcoarse_step(R), L = (2 * R) / cs + 1, w = 2 * cs - 1;
+        return stage == 0 ? L * L + 1 + 2 * L : (stage == 1 ? kGTop * w * w : 1);
+    }
+    const int k = R / kGExtStep, g = (2 * kGExtStep) / 4 + 1;
+    return stage == 0 ? 1 + 12 * k : (stage == 1 ? 4 * g * g : (stage == 2 ? 81 : 9));
+}
+
+// Slot t of a search's first stage: the coarse grid, zero and the far edges (:2110-2124), or the
+// extended search's cross and octagon rings (:2040-2052).
+__device__ __forceinline__ int2 gfirst(int R, int t) {
+    if (R <= 0) return make_int2(0, 0);
+    if (R <= 31) {
+        const int cs = gcoarse_step(R), L = (2 * R) / cs + 1;
+        if (t < L * L) return make_int2(-R + (t % L) * cs, -R + (t / L) * cs);
+        if (t == L * L) return make_int2(0, 0);
+        const int j = t - L * L - 1, d = -R + (j >> 1) * cs;
+        return (j & 1) ? make_int2(d, R) : make_int2(R, d);
+    }
+    if (t == 0) return make_int2(0, 0);
+    const int k = R / kGExtStep;
+    int2 v;
+    if (t <= 4 * k) {
+        const int d = kGExtStep * ((t - 1) / 4 + 1), a = (t - 1) & 3;
+        v = a == 0 ? make_int2(-d, 0) : a == 1 ? make_int2(d, 0) : a == 2 ? make_int2(0, -d) : make_int2(0, d);
+    } else {
+        const int j = t - 1 - 4 * k, r = kGExtStep * (j / 8 + 1), h = (r + 1) / 2, a = j & 7;
+        // (-r,-h) (-r,h) (r,-h) (r,h) (-h,-r) (h,-r) (-h,r) (h,r)
+        v = a < 4 ? make_int2(a < 2 ? -r : r, (a & 1) ? h : -h) : make_int2((a & 1) ? h : -h, a < 6 ? -r : r);
+    }
+    return make_int2(iclamp(v.x, -R, R), iclamp(v.y, -R, R));
+}
+
+// One block per search: takes its inputs (when given) and lays out the first stage.
+__global__ void __launch_bounds__(kGThreads) gplan_kernel(GState* states, const GIn* in) {
+    GState& s = states[blockIdx.x];
+    const int R = in ? in[blockIdx.x].range : s.in.range;
+    const int n = gstage_slots(R, 0);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        s.cand[t] = gfirst(R, t);
+        s.cost[t] = 0;
+    }
+    if (threadIdx.x == 0) {
+        if (in) s.in = in[blockIdx.x];
+        s.n = n;
+        s.arrived = 0;
+        s.top_n = 0;
+        s.sorted = 1;
+    }
+}
+
+// The least `v` of the block, on every thread.
+__device__ unsigned long long block_min(unsigned long long v, unsigned long long* red) {
+    v = warp_min_u64(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = red[w] < v ? red[w] : v;
+    return v;
+}
+
+// `consider` of global_motion_search_extended (:2034-2039) over the stage's costs, by warp 0:
+// lane i holds list entry i (the entry's own vector once, its least cost; sorted by insertion, so
+// a lowered cost stays in place until the next insertion, then the eight least are kept).
+__device__ void gfold_ext(GState& s, const unsigned long long* cost, int n, unsigned long long* red) {
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    int tn = s.top_n;
+    int2 v = lane < tn ? s.top[lane] : make_int2(0, 0);
+    unsigned long long c = lane < tn ? s.top_cost[lane] : 0;
+    bool sorted = s.sorted != 0;
+    for (int k = 0; k < n; ++k) {
+        const int2 q = s.cand[k];
+        const unsigned long long qc = cost[k];
+        const bool hit = lane < tn && v.x == q.x && v.y == q.y;
+        if (__any_sync(0xffffffffu, hit)) {
+            const bool lower = hit && qc < c;
+            if (lower) c = qc;
+            if (__any_sync(0xffffffffu, lower)) sorted = false;
+            continue;
+        }
+        const unsigned long long last = __shfl_sync(0xffffffffu, gkey(c, v), kGTop - 1);
+        if (sorted && tn == kGTop && gkey(qc, q) > last) continue;  // would be inserted last and cut
+        if (lane == tn) {
+            v = q;
+            c = qc;
+        }
+        ++tn;
+        const unsigned long long mine = gkey(c, v);
+        int rank = 0;
+        for (int j = 0; j < tn; ++j) rank += __shfl_sync(0xffffffffu, mine, j) < mine ? 1 : 0;
+        // entries move to their ranks through shared memory
+        if (lane < tn) {
+            red[2 * rank] = c;
+            red[2 * rank + 1] = ((unsigned long long)(uint32_t)v.x << 32) | (uint32_t)v.y;
+        }
+        __syncwarp();
+        if (lane < tn) {
+            c = red[2 * lane];
+            const unsigned long long p = red[2 * lane + 1];
+            v = make_int2((int)(uint32_t)(p >> 32), (int)(uint32_t)p);
+        }
+        __syncwarp();
+        tn = imin(tn, kGTop);
+        sorted = true;
+    }
+    if (lane < tn) {
+        s.top[lane] = v;
+        s.top_cost[lane] = c;
+    }
+    if (lane == 0) {
+        s.top_n = tn;
+        s.sorted = sorted ? 1 : 0;
+    }
+}
+
+// Folds the finished stage's costs and lays out the next stage (or writes the result); one block.
+__device__ void gfold(GState& s, int stage) {
+    __shared__ unsigned long long key[kGMaxCand];
+    __shared__ unsigned long long red[32];
+    const int R = s.in.range, n = s.n, st = gstage_stride(R, stage);
+    const unsigned long long scale = (unsigned long long)(st * st);
+    const bool plain = R <= 31;
+    __syncthreads();
+    if (plain && stage == 0 && R > 0) {
+        // the eight least of (cost, |d|, dy, dx), repeats kept (:2086-2098)
+        for (int t = threadIdx.x; t < n; t += blockDim.x) key[t] = gkey(__ldcg(&s.cost[t]) * scale, s.cand[t]);
+        __syncthreads();
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const unsigned long long k = key[t];
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += (key[j] < k || (key[j] == k && j < t)) ? 1 : 0;
+            if (rank < kGTop) s.top[rank] = s.cand[t];
+        }
+        __syncthreads();
+        // the refinement's visit list (:2129-2140): a window about each entry, first visits only
+        const int cs = gcoarse_step(R), w = 2 * cs - 1, tn = imin(kGTop, n), m = tn * w * w;
+        int2 top[kGTop];
+#pragma unroll
+        for (int k = 0; k < kGTop; ++k) top[k] = k < tn ? s.top[k] : make_int2(0, 0);
+        for (int t = threadIdx.x; t < m; t += blockDim.x) {
+            const int k = t / (w * w), q = t - k * w * w;
+            const int2 c0 = s.top[k];
+            int2 d = make_int2(c0.x - (cs - 1) + q % w, c0.y - (cs - 1) + q / w);
+            bool ok = iabs(d.x) <= R && iabs(d.y) <= R;
+#pragma unroll
+            for (int j = 0; j < kGTop; ++j)
+                if (j < k && iabs(d.x - top[j].x) < cs && iabs(d.y - top[j].y) < cs) ok = false;
+            if (!ok) d.x = kGEmpty;
+            s.cand[t] = d;
+            s.cost[t] = 0;
+        }
+        if (threadIdx.x == 0) s.n = m;
+        return;
+    }
+    if (plain && stage == 1) {
+        // the first-visited least (cost, |d|) (:2129-2140)
+        unsigned long long best = ~0ull;
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const int2 d = s.cand[t];
+            if (d.x == kGEmpty) continue;
+            const unsigned long long k = ((__ldcg(&s.cost[t]) * scale) << 16) |
+                                         ((unsigned long long)(iabs(d.x) + iabs(d.y)) << 9) | (unsigned long long)t;
+            best = k < best ? k : best;
+        }
+        best = block_min(best, red);
+        if (threadIdx.x == 0) {
+            const int2 d = s.cand[(int)(best & 511)];
+            s.cand[0] = d;
+            s.cost[0] = 0;
+            s.n = 1;
+        }
+        return;
+    }
+    if (plain) {
+        // range 0: frame_sad(0, 0, 1) (:2082-2085); else the chosen vector's full frame SAD
+        if (threadIdx.x == 0) {
+            const int2 d = s.cand[0];
+            s.in.out_global[0] = d.x;
+            s.in.out_global[1] = d.y;
+            *s.in.out_sad = __ldcg(&s.cost[0]);
+        }
+        return;
+    }
+    if (stage < 3) {
+        for (int t = threadIdx.x; t < n; t += blockDim.x) key[t] = __ldcg(&s.cost[t]) * scale;
+        __syncthreads();
+        gfold_ext(s, key, n, red);
+        __syncthreads();
+        // stage 1: 5x5 at step 4 about the four best; stages 2 and 3: 9x9 and 3x3 about the best
+        const int g = stage == 0 ? (2 * kGExtStep) / 4 + 1 : (stage == 1 ? 9 : 3);
+        const int step = stage == 0 ? 4 : 1, nc = stage == 0 ? imin(4, s.top_n) : 1, m = nc * g * g;
+        for (int t = threadIdx.x; t < m; t += blockDim.x) {
+            const int2 c0 = s.top[t / (g * g)];
+            const int q = t % (g * g), h = step * (g / 2);
+            s.cand[t] = make_int2(iclamp(c0.x - h + step * (q % g), -R, R), iclamp(c0.y - h + step * (q / g), -R, R));
+            s.cost[t] = 0;
+        }
+        if (threadIdx.x == 0) s.n = m;
+        return;
+    }
+    // the full-resolution 3x3: least by the total order (:2066-2074)
+    unsigned long long best = ~0ull;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const unsigned long long k = gkey(__ldcg(&s.cost[t]), s.cand[t]);
+        best = k < best ? k : best;
+    }
+    best = block_min(best, red);
+    if (threadIdx.x == 0) {
+        s.in.out_global[0] = (int)(best & 127) - 32;
+        s.in.out_global[1] = (int)((best >> 7) & 127) - 32;
+        *s.in.out_sad = best >> 21;
+    }
+}
+
+// 16 bytes at any address as four little-endian words: aligned word loads that each hold at least
+// one of the bytes, and funnel shifts.
+__device__ __forceinline__ void gload16(const uint8_t* p, uint32_t r[4]) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
+    const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
+    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+    const uint32_t w4 = sh ? __ldg(w + 4) : 0u;
+    r[0] = __funnelshift_r(w0, w1, sh);
+    r[1] = __funnelshift_r(w1, w2, sh);
+    r[2] = __funnelshift_r(w2, w3, sh);
+    r[3] = __funnelshift_r(w3, w4, sh);
+}
+
+// The bytes 0, ST, 2 ST .. of 16, packed (four for ST 4, eight for ST 2).
+__device__ __forceinline__ uint32_t gpick4(const uint32_t r[4]) {
+    return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+}
+
+// frame_sad of every candidate of every search: grid (slab, candidate slot, search). A thread takes
+// 16-pixel chunks of the sampled rows with packed byte SADs; chunks that the clamped sampling
+// touches, the ragged last one and the strides above 4 go sample by sample.
+// 1080p, range 31 and up, one search: 4 stages 137 us -> 60 us (the byte-per-thread form loaded
+// one sample per load).
+__global__ void __launch_bounds__(kGThreads) gsad_kernel(GState* states, int W, int H, int rows_per_slab, int stage) {
     GState& s = states[blockIdx.z];
     const int ci = blockIdx.y;
-    if (ci >= s.n) return;
-    const GCand c = s.cand[ci];
-    const int st = c.stride;
-    const int nrows = (H + st - 1) / st;
-    const int r0 = blockIdx.x * rows_per_slab;
-    if (r0 >= nrows) return;
-    const int r1 = imin(nrows, r0 + rows_per_slab);
-    const int ncols = (W + st - 1) / st;
-    uint64_t acc = 0;
-    for (int r = r0; r < r1; ++r) {
-        const int y = r * st;
-        const int sy = iclamp(y + c.dy, 0, H - 1);
-        const uint8_t* cp = s.cur.y + (size_t)y * s.cur.pitch_y;
-        const uint8_t* rp = s.ref.y + (size_t)sy * s.ref.pitch_y;
-        for (int k = threadIdx.x; k < ncols; k += blockDim.x) {
-            const int x = k * st;
-            const int sx = iclamp(x + c.dx, 0, W - 1);
-            acc += (uint64_t)iabs((int)__ldg(cp + x) - (int)__ldg(rp + sx));
+    const int st = gstage_stride(s.in.range, stage);
+    const int nrows = (H + st - 1) / st, r0 = blockIdx.x * rows_per_slab, r1 = imin(nrows, r0 + rows_per_slab);
+    const int2 c = ci < s.n ? s.cand[ci] : make_int2(kGEmpty, 0);
+    if (c.x != kGEmpty && r0 < r1) {
+        const int chunks = (W + 15) >> 4, items = (r1 - r0) * chunks;
+        const DevFrame &cf = s.in.cur, &rf = s.in.ref;
+        uint32_t acc = 0;  // at most (64 rows x 16384 samples / 256 threads) x 255
+        for (int t = threadIdx.x; t < items; t += kGThreads) {
+            const int r = t / chunks, x = (t - r * chunks) << 4, y = (r0 + r) * st;
+            const uint8_t* cp = cf.y + (size_t)y * cf.pitch_y;
+            const uint8_t* rp = rf.y + (size_t)iclamp(y + c.y, 0, H - 1) * rf.pitch_y;
+            if (st <= 4 && x + 16 <= W && x + c.x >= 0 && x + c.x + 16 <= W) {
+                uint32_t a[4], b[4];
+                gload16(cp + x, a);
+                gload16(rp + x + c.x, b);
+                if (st == 4) {
+                    acc += __vsadu4(gpick4(a), gpick4(b));
+                } else if (st == 2) {
+                    acc += __vsadu4(__byte_perm(a[0], a[1], 0x6420), __byte_perm(b[0], b[1], 0x6420)) +
+                           __vsadu4(__byte_perm(a[2], a[3], 0x6420), __byte_perm(b[2], b[3], 0x6420));
+                } else {
+                    acc += __vsadu4(a[0], b[0]) + __vsadu4(a[1], b[1]) + __vsadu4(a[2], b[2]) + __vsadu4(a[3], b[3]);
+                }
+            } else {
+                // x is a multiple of 16, so of every stride: the chunk's samples start at x
+                for (int i = 0; i < 16 && x + i < W; i += st)
+                    acc += (uint32_t)iabs((int)__ldg(cp + x + i) - (int)__ldg(rp + iclamp(x + i + c.x, 0, W - 1)));
+            }
+        }
+        const uint64_t sum = warp_sum_u64(acc);
+        __shared__ unsigned long long part[kGThreads / 32];
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long t = 0;
+            for (int w = 0; w < kGThreads / 32; ++w) t += part[w];
+            atomicAdd(&s.cost[ci], t);
         }
     }
-    acc = warp_sum_u64(acc);
-    __shared__ unsigned long long red[32];
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
+    // the last block of this search to arrive sees every block's cost and folds the stage
+    __shared__ bool last;
     if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        atomicAdd(&s.cost[ci], t);
+        __threadfence();
+        last = atomicAdd(&s.arrived, 1) == (int)(gridDim.x * gridDim.y) - 1;
+        __threadfence();
     }
-}
-
-__device__ unsigned long long scaled(const GState& s, int i) {
-    const int st = s.cand[i].stride;
-    return st > 1 ? s.cost[i] * (unsigned long long)(st * st) : s.cost[i];
-}
-
-// sort-and-truncate insertion of global_motion_search (:2086-2098): multiset top-8
-__device__ void push_plain(GState& s, unsigned long long c, int dx, int dy) {
-    int at = s.top_n;
-    while (at > 0 && gless(c, dx, dy, s.top_cost[at - 1], s.top_dx[at - 1], s.top_dy[at - 1])) --at;
-    for (int j = s.top_n; j > at; --j) {
-        s.top_cost[j] = s.top_cost[j - 1];
-        s.top_dx[j] = s.top_dx[j - 1];
-        s.top_dy[j] = s.top_dy[j - 1];
-    }
-    s.top_cost[at] = c;
-    s.top_dx[at] = dx;
-    s.top_dy[at] = dy;
-    if (++s.top_n > 8) s.top_n = 8;
-}
-
-// `consider` of global_motion_search_extended (:2034-2039): keep-min per vector, sorted, 8
-__device__ void push_ext(GState& s, unsigned long long c, int dx, int dy) {
-    for (int i = 0; i < s.top_n; ++i)
-        if (s.top_dx[i] == dx && s.top_dy[i] == dy) {
-            if (c < s.top_cost[i]) {
-                s.top_cost[i] = c;
-                // re-sort (the reference sorts only on insertion; a lowered cost stays in place
-                // until the next insertion sorts the list, which yields the same order)
-            }
-            return;
-        }
-    // insertion then sort then truncate; sorting an almost-sorted list by insertion
-    s.top_cost[s.top_n] = c;
-    s.top_dx[s.top_n] = dx;
-    s.top_dy[s.top_n] = dy;
-    ++s.top_n;
-    for (int i = 1; i < s.top_n; ++i) {
-        const unsigned long long vc = s.top_cost[i];
-        const int vx = s.top_dx[i], vy = s.top_dy[i];
-        int j = i - 1;
-        while (j >= 0 && gless(vc, vx, vy, s.top_cost[j], s.top_dx[j], s.top_dy[j])) {
-            s.top_cost[j + 1] = s.top_cost[j];
-            s.top_dx[j + 1] = s.top_dx[j];
-            s.top_dy[j + 1] = s.top_dy[j];
-            --j;
-        }
-        s.top_cost[j + 1] = vc;
-        s.top_dx[j + 1] = vx;
-        s.top_dy[j + 1] = vy;
-    }
-    if (s.top_n > 8) s.top_n = 8;
-}
-
-__device__ void add_cand(GState& s, int dx, int dy, int stride) {
-    s.cand[s.n].dx = dx;
-    s.cand[s.n].dy = dy;
-    s.cand[s.n].stride = stride;
-    s.cost[s.n] = 0;
-    ++s.n;
-}
-
-// One thread per state: fold the costs of the finished stage and plan the next one.
-// phase 0: plan the first stage. Returns via s.phase = -1 when the result is written.
-__global__ void gplan_kernel(GState* states, int nstates) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nstates) return;
-    GState& s = states[i];
-    const int R = s.range;
-    if (s.phase < 0) return;
-    if (R <= 0) {
-        // range 0: frame_sad(0,0,1) (:2082-2085)
-        if (s.phase == 0) {
-            s.n = 0;
-            add_cand(s, 0, 0, 1);
-            s.phase = 100;
-        } else {
-            s.out_global[0] = 0;
-            s.out_global[1] = 0;
-            *s.out_sad = s.cost[0];
-            s.phase = -1;
-            s.n = 0;
-        }
-        return;
-    }
-    if (R <= 31) {
-        const int cs = R >= 4 ? 4 : (R >= 2 ? 2 : 1);
-        if (s.phase == 0) {
-            // coarse grid + zero + edges at stride 4 (:2110-2124)
-            s.n = 0;
-            for (int dy = -R; dy <= R; dy += cs)
-                for (int dx = -R; dx <= R; dx += cs) add_cand(s, dx, dy, 4);
-            add_cand(s, 0, 0, 4);
-            for (int d = -R; d <= R; d += cs) {
-                add_cand(s, R, d, 4);
-                add_cand(s, d, R, 4);
-            }
-            s.phase = 1;
-            return;
-        }
-        if (s.phase == 1) {
-            s.top_n = 0;
-            for (int k = 0; k < s.n; ++k) push_plain(s, scaled(s, k), s.cand[k].dx, s.cand[k].dy);
-            // refinement visit list around each top entry at stride 2 (:2129-2140)
-            bool seen[63 * 63];
-            for (int k = 0; k < 63 * 63; ++k) seen[k] = false;
-            const int tn = s.top_n;
-            int tdx[8], tdy[8];
-            for (int k = 0; k < tn; ++k) { tdx[k] = s.top_dx[k]; tdy[k] = s.top_dy[k]; }
-            s.n = 0;
-            for (int k = 0; k < tn; ++k)
-                for (int dy = imax(-R, tdy[k] - cs + 1); dy <= imin(R, tdy[k] + cs - 1); ++dy)
-                    for (int dx = imax(-R, tdx[k] - cs + 1); dx <= imin(R, tdx[k] + cs - 1); ++dx) {
-                        const int key = (dy + 31) * 63 + (dx + 31);
-                        if (seen[key]) continue;
-                        seen[key] = true;
-                        add_cand(s, dx, dy, 2);
-                    }
-            s.phase = 2;
-            return;
-        }
-        if (s.phase == 2) {
-            unsigned long long bc = ~0ull;
-            int bx = 0, by = 0;
-            for (int k = 0; k < s.n; ++k) {
-                const unsigned long long c = scaled(s, k);
-                const int dx = s.cand[k].dx, dy = s.cand[k].dy;
-                const int cm = iabs(dx) + iabs(dy), bm = iabs(bx) + iabs(by);
-                if (c < bc || (c == bc && cm < bm)) { bc = c; bx = dx; by = dy; }
-            }
-            s.best_dx = bx;
-            s.best_dy = by;
-            s.n = 0;
-            add_cand(s, bx, by, 1);
-            s.phase = 3;
-            return;
-        }
-        s.out_global[0] = s.best_dx;
-        s.out_global[1] = s.best_dy;
-        *s.out_sad = s.cost[0];
-        s.phase = -1;
-        s.n = 0;
-        return;
-    }
-    // extended search (range 32 after the min(range, 32) clamp), :2025-2074
-    const int step = R >= 160 ? 16 : 8;
-    if (s.phase == 0) {
-        s.n = 0;
-        add_cand(s, 0, 0, 16);
-        for (int d = step; d <= R; d += step) {
-            add_cand(s, iclamp(-d, -R, R), 0, 16);
-            add_cand(s, iclamp(d, -R, R), 0, 16);
-            add_cand(s, 0, iclamp(-d, -R, R), 16);
-            add_cand(s, 0, iclamp(d, -R, R), 16);
-        }
-        for (int r = step; r <= R; r += step) {
-            const int h = (r + 1) / 2;
-            const int xs[8] = {-r, -r, r, r, -h, h, -h, h}, ys[8] = {-h, h, -h, h, -r, -r, r, r};
-            for (int k = 0; k < 8; ++k) add_cand(s, iclamp(xs[k], -R, R), iclamp(ys[k], -R, R), 16);
-        }
-        s.top_n = 0;
-        s.phase = 1;
-        return;
-    }
-    if (s.phase == 1) {
-        for (int k = 0; k < s.n; ++k) push_ext(s, scaled(s, k), s.cand[k].dx, s.cand[k].dy);
-        const int nc = imin(4, s.top_n);
-        int cx[4], cy[4];
-        for (int k = 0; k < nc; ++k) { cx[k] = s.top_dx[k]; cy[k] = s.top_dy[k]; }
-        s.n = 0;
-        for (int k = 0; k < nc; ++k)
-            for (int oy = -step; oy <= step; oy += 4)
-                for (int ox = -step; ox <= step; ox += 4)
-                    add_cand(s, iclamp(cx[k] + ox, -R, R), iclamp(cy[k] + oy, -R, R), 8);
-        s.phase = 2;
-        return;
-    }
-    if (s.phase == 2) {
-        for (int k = 0; k < s.n; ++k) push_ext(s, scaled(s, k), s.cand[k].dx, s.cand[k].dy);
-        if (s.top_n == 0) {  // (:2059) unreachable with a non-empty coarse stage
-            s.n = 0;
-            add_cand(s, 0, 0, 8);
-            s.phase = 20;
-            return;
-        }
-        const int mdx = s.top_dx[0], mdy = s.top_dy[0];
-        s.n = 0;
-        for (int oy = -4; oy <= 4; ++oy)
-            for (int ox = -4; ox <= 4; ++ox) add_cand(s, iclamp(mdx + ox, -R, R), iclamp(mdy + oy, -R, R), 4);
-        s.phase = 3;
-        return;
-    }
-    if (s.phase == 20) {
-        push_ext(s, scaled(s, 0), 0, 0);
-        const int mdx = s.top_dx[0], mdy = s.top_dy[0];
-        s.n = 0;
-        for (int oy = -4; oy <= 4; ++oy)
-            for (int ox = -4; ox <= 4; ++ox) add_cand(s, iclamp(mdx + ox, -R, R), iclamp(mdy + oy, -R, R), 4);
-        s.phase = 3;
-        return;
-    }
-    if (s.phase == 3) {
-        for (int k = 0; k < s.n; ++k) push_ext(s, scaled(s, k), s.cand[k].dx, s.cand[k].dy);
-        const int fdx = s.top_dx[0], fdy = s.top_dy[0];
-        s.n = 0;
-        for (int oy = -1; oy <= 1; ++oy)
-            for (int ox = -1; ox <= 1; ++ox) add_cand(s, iclamp(fdx + ox, -R, R), iclamp(fdy + oy, -R, R), 1);
-        s.phase = 4;
-        return;
-    }
-    // phase 4: full 3x3, min by the total order
-    unsigned long long bc = ~0ull;
-    int bx = 0, by = 0;
-    for (int k = 0; k < s.n; ++k) {
-        const unsigned long long c = s.cost[k];
-        if (gless(c, s.cand[k].dx, s.cand[k].dy, bc, bx, by)) { bc = c; bx = s.cand[k].dx; by = s.cand[k].dy; }
-    }
-    s.out_global[0] = bx;
-    s.out_global[1] = by;
-    *s.out_sad = bc;
-    s.phase = -1;
-    s.n = 0;
+    __syncthreads();
+    if (!last) return;
+    gfold(s, stage);
+    if (threadIdx.x == 0) s.arrived = 0;
 }
 
 size_t gstate_bytes() { return sizeof(GState); }
+size_t gin_bytes() { return sizeof(GIn); }
 
-// Host driver: runs the staged search for n states already initialised in device memory
-// (cur, ref, range, outputs, phase = 0). Every stage is one scoring launch sized to the
-// stage's largest candidate list and sampling stride, bracketed by plan/fold launches.
 // Passes that share one search take its result: one thread per copy (dx, dy and the SAD).
 __global__ void global_fanout_kernel(const GlobalCopy* copies, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -326,50 +383,29 @@ cudaError_t launch_global_fanout(const GlobalCopy* d_copies, int n, cudaStream_t
     return cudaGetLastError();
 }
 
-int run_global_search(GState* d_states, int n, int R, int W, int H, cudaStream_t stream) {
-    struct Stage { int maxc, stride; };
-    Stage st[4];
-    int ns = 0;
-    if (R <= 0) {
-        st[ns++] = {1, 1};
-    } else if (R <= 31) {
-        const int cs = R >= 4 ? 4 : (R >= 2 ? 2 : 1);
-        const int L = (2 * R) / cs + 1;
-        st[ns++] = {L * L + 1 + 2 * L, 4};
-        st[ns++] = {imin(kGMaxCand, 8 * (2 * cs - 1) * (2 * cs - 1)), 2};
-        st[ns++] = {1, 1};
-    } else {
-        const int step = R >= 160 ? 16 : 8;
-        const int k = R / step;
-        const int g = (2 * step) / 4 + 1;
-        st[ns++] = {1 + 4 * k + 8 * k, 16};
-        st[ns++] = {4 * g * g, 8};
-        st[ns++] = {81, 4};
-        st[ns++] = {9, 1};
-    }
+// Host driver: runs the staged search for n searches whose inputs are in device memory (d_in; or
+// already in the states when d_in is null): a planning launch, then one launch per stage, sized
+// to the stage's candidate slots and sampling stride. Returns the launches.
+int run_global_search(GState* d_states, const GIn* d_in, int n, int R, int W, int H, cudaStream_t stream) {
     const int rows_per_slab = 64;
-    gplan_kernel<<<(n + 63) / 64, 64, 0, stream>>>(d_states, n);
+    gplan_kernel<<<n, kGThreads, 0, stream>>>(d_states, d_in);
+    const int ns = gstage_count(R);
     for (int i = 0; i < ns; ++i) {
-        const int rows = (H + st[i].stride - 1) / st[i].stride;
-        dim3 grid((rows + rows_per_slab - 1) / rows_per_slab, st[i].maxc, n);
-        gsad_kernel<<<grid, 256, 0, stream>>>(d_states, W, H, rows_per_slab);
-        gplan_kernel<<<(n + 63) / 64, 64, 0, stream>>>(d_states, n);
+        const int st = gstage_stride(R, i), rows = (H + st - 1) / st;
+        const dim3 grid((rows + rows_per_slab - 1) / rows_per_slab, gstage_slots(R, i), n);
+        gsad_kernel<<<grid, kGThreads, 0, stream>>>(d_states, W, H, rows_per_slab, i);
     }
-    return 1 + 2 * ns;
+    return 1 + ns;
 }
 
-void init_gstate(GState* h, const DevFrame& cur, const DevFrame& ref, int range, int* out_global,
-                 unsigned long long* out_sad) {
+void init_gin(GIn* h, const DevFrame& cur, const DevFrame& ref, int range, int* out_global,
+              unsigned long long* out_sad) {
     h->cur = cur;
     h->ref = ref;
     h->range = range;
     h->out_global = out_global;
     h->out_sad = out_sad;
-    h->n = 0;
-    h->top_n = 0;
-    h->phase = 0;
 }
-
 
 // ---- allocation-free form (vc1cu_global_motion_noalloc) ---------------------------------
 //
@@ -377,11 +413,11 @@ void init_gstate(GState* h, const DevFrame& cur, const DevFrame& ref, int range,
 // of a fixed device-memory budget, or code that runs where a cudaMalloc would synchronise
 // the device or is not permitted. For them the search state of up to
 // kNoAllocMaxPictures pictures lives in this fixed array, which every GPU that loads the
-// library holds until the process exits (16 states of 10,512 bytes: 168,192 bytes).
+// library holds until the process exits (16 states of 8,424 bytes: 134,784 bytes).
 // Every call shares it.
 constexpr int kNoAllocMaxPictures = 16;
 static __device__ __align__(256) GState g_noalloc_states[kNoAllocMaxPictures];
-static_assert(sizeof(GState) * kNoAllocMaxPictures <= 192 * 1024, "no-alloc scratch stays modest");
+static_assert(sizeof(GState) * kNoAllocMaxPictures == 134784, "the size the interface documents");
 
 struct NoAllocInit {
     DevFrame cur[kNoAllocMaxPictures], ref[kNoAllocMaxPictures];
@@ -390,22 +426,17 @@ struct NoAllocInit {
     int range, n;
 };
 
-// Resets the fields the staged search reads before it writes them (the planner zeroes each
-// stage's costs itself), so a call never sees the previous call's state.
+// Writes each search's inputs; the planning launch that follows resets all that a search reads,
+// so a call never sees the previous call's state.
 __global__ void noalloc_init_kernel(GState* states, const __grid_constant__ NoAllocInit a) {
     const int i = threadIdx.x;
     if (i >= a.n) return;
-    GState& s = states[i];
+    GIn& s = states[i].in;
     s.cur = a.cur[i];
     s.ref = a.ref[i];
     s.range = a.range;
     s.out_global = a.out_global + 2 * i;
     s.out_sad = a.out_sad + i;
-    s.n = 0;
-    s.top_n = 0;
-    s.best_dx = s.best_dy = 0;
-    s.best_cost = 0;
-    s.phase = 0;
 }
 
 }  // namespace vc1cu
@@ -458,7 +489,7 @@ extern "C" int vc1cu_global_motion_noalloc(const uint8_t* const* cur_y, const ui
     noalloc_init_kernel<<<1, 32, 0, s>>>(states, a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
-    run_global_search(states, n, range, width, height, s);
+    run_global_search(states, nullptr, n, range, width, height, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
     return VC1CU_OK;
