@@ -128,6 +128,7 @@ constexpr size_t kMaxBatch = 64u * 65535u;   // VulkanComputeContext's candidate
 #define VC1CU_SEEDED_MIXED_RW 8
 #endif
 constexpr int kSeededMixedRw = VC1CU_SEEDED_MIXED_RW;  // window radius of seeded Mixed-MV launches
+constexpr int kMaxLocalRange = 190;  // the largest local range this interface takes
 constexpr int kMinUnseededRw = 24;  // smallest window radius a tuned unseeded launch shrinks to
 #ifndef VC1CU_WINDOW_TMA
 #define VC1CU_WINDOW_TMA 1
@@ -558,18 +559,6 @@ const uint32_t* work_items(vc1cu_ctx* c, const std::vector<int>& mbw, const std:
     nitems = (unsigned)items.size();
     c->items[key] = {static_cast<uint32_t*>(d), nitems};
     return static_cast<uint32_t*>(d);
-}
-
-int stage_max(int R) {
-    int m = 32;
-    const int L = (2 * R) / 8 + 1;
-    if (R >= 8) m = std::max(m, L * L + 2 * L);
-    const int cs = R >= 96 ? 8 : (R >= 32 ? 4 : 2);
-    const int vlimit = std::min(R, std::max(8, R / 2));
-    m = std::max(m, 2 * (R / cs) + 2 * (vlimit / cs));
-    const int hs = R >= 96 ? 8 : (R >= 24 ? 4 : 2);
-    m = std::max(m, 6 * (R / hs));
-    return m;
 }
 
 FrameSlot& frame_slot(vc1cu_ctx* c, int id) {
@@ -1015,23 +1004,16 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     WinCfg wc;
     if (learned) {
         wc.rw = kLearnRw;
-        wc.seen_r = 0;
-        wc.seen_words = 1;
-        wc.keys_cap = 32;
     } else if (any_unseeded) {
+        if (P.local_range > kMaxLocalRange)
+            throw Fail{VC1CU_ERR_UNSUPPORTED, "search window does not fit in shared memory (local range too large)"};
         wc.rw = P.local_range + 1;
-        wc.seen_r = P.local_range;
-        wc.seen_words = ((2 * P.local_range + 1) * (2 * P.local_range + 1) + 31) / 32;
-        wc.keys_cap = std::max(stage_max(P.local_range), 32);  // >= one warp of staged long-range keys
     } else {
         // seeded refinement stays within 3 quarter-pels of the seed; the Mixed-MV block seeds
         // add up to 8 more and their refinement 3 (samples outside the window read HBM)
         bool any_mixed = false;
         for (int i = 0; i < n; ++i) any_mixed |= passes[i].mode == VC1CU_MV_MIXED;
         wc.rw = any_mixed ? kSeededMixedRw : 4;
-        wc.seen_r = 0;
-        wc.seen_words = 1;
-        wc.keys_cap = 32;
     }
     wc.wh = 16 + 2 * wc.rw + 3;
     wc.wp = (wc.wh + 15 + 15) & ~15;
@@ -1100,9 +1082,9 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     }
     // Sub-pel prediction planes, one set per (reference, rounding, filter) of the launch, built
     // before it on the context stream: every candidate's interpolated rows are then read, not
-    // recomputed per candidate and macroblock (the phases each set needs: all 15 for the bicubic
-    // modes, whose SAD batches may score odd seeds; the three half-pel ones for the bilinear mode,
-    // which rejects odd vectors).
+    // recomputed per candidate and macroblock (the phases each set needs: all 16 for the bicubic
+    // modes, whose SAD batches may score odd seeds; the integer and the three half-pel ones for the
+    // bilinear mode, which rejects odd vectors).
     if (VC1CU_SUBPEL_PLANES && P.subpel) {
         struct Key {
             const uint8_t* ref;
@@ -1115,7 +1097,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         std::vector<int> key_of(n);
         for (int i = 0; i < n; ++i) {
             const int bil = h[i].mode == VC1CU_MV_HPEL_BILINEAR ? 1 : 0;
-            const uint32_t mask = bil ? 0x504u : 0xFFFEu;
+            const uint32_t mask = bil ? 0x505u : 0xFFFFu;
             int k = 0;
             while (k < (int)keys.size() && !(keys[k].ref == h[i].ref.y && keys[k].rnd == h[i].geom.rnd && keys[k].bil == bil))
                 ++k;

@@ -62,8 +62,6 @@ extern __shared__ __align__(16) uint32_t g_smem32[];  // the same memory, 32-bit
 enum IndexSite : int {
     kSiteWorkItem = 1,   // work item: pass index < npass, macroblock < the pass's raster
     kSiteWindow = 2,     // search-window read (x, y) inside the staged window
-    kSiteKeys = 3,       // a stage's key slot < the key array's capacity
-    kSiteSeen = 4,       // first-visit bitset: (dx, dy) inside the bitset's square
     kSiteNeighbour = 5,  // neighbour macroblock inside the raster
     kSiteCands = 6,      // learned candidate of a macroblock inside the raster
     kSiteSignature = 7,  // long-range signature cell inside the reference's lattice
@@ -106,21 +104,14 @@ struct SpecBlk;
 struct WarpMem {
     SPtr<uint8_t> cur;          // 16x16 current MB (zero outside the visible raster)
     SPtr<uint8_t> win;          // reference window
-    SPtr<uint32_t> seen;        // first-visit bitset of the sampled UMH stages
-    SPtr<uint32_t> seen_full;   // first-visit bitset of the full-resolution stages
-    SPtr<uint64_t> keys;        // per-stage candidate keys
-    SPtr<int2> list_mv;         // staged-refinement candidate list
-    SPtr<uint64_t> list_sad;
-    SPtr<uint64_t> list_satd;
-    SPtr<uint32_t> list_rate;
-    SPtr<unsigned __int128> list_key;
+    SPtr<uint64_t> keys;        // staged long-range cells of one warp step
+    SPtr<uint64_t> list_sad;    // the long-range search's nearest cells
+    SPtr<uint64_t> list_satd;   // SATD of the shortlist
     SPtr<int2> batch;           // scratch MV batch
     SPtr<uint64_t> batch_cost;
-    SPtr<int2> stencil;         // sub-pel stencil MVs of the current refinement stage
-    SPtr<uint64_t> top;         // sorted top-8 keys of the UMH search
+    SPtr<uint64_t> top;         // the lattice's four least keys
     SPtr<uint32_t> cur2;        // current MB, even columns packed 4 per word: [row][2]
     SPtr<uint32_t> cur4;        // current MB, every 4th column packed: [row]
-    SPtr<int> misc;             // small scalars: [0] top count, [1] compaction count
     SPtr<int2> cur_bmv;         // the current MB's four block MVs while it is searched
     SPtr<int2> nb_mv;           // 1-MV field of the left, top-left, top, top-right neighbours
     SPtr<int2> nb_bmv;          // their block MVs [4][4]
@@ -144,9 +135,6 @@ struct Mb {
     GlobSampler gref;
     uint32_t tma_phase;    // parity of the window mbarrier's next phase
     bool tma_pending;      // a TMA window copy is in flight
-#ifdef VC1CU_INDEX_CHECK
-    int keys_cap;  // capacity of m.sm.keys
-#endif
 };
 
 __device__ __forceinline__ bool win_inside(const Mb& m, int xa, int ya, int xb, int yb) {
@@ -439,21 +427,43 @@ struct MbCtx {
     int subpel, fast_subpel, subpel_range, me_quality, mvrange, mant_bits, lam_s;
     uint64_t lam_m;
     uint32_t batch, cost, satd;  // the warp's shortlist buffers
-    const uint8_t* sp;           // the pass's sub-pel prediction planes (nullptr: none)
+    const uint8_t* sp;           // the pass's prediction planes (nullptr: none)
     int sp_pitch, sp_border;
     long long sp_stride;
+    int xl, yl;                  // an integer vector (dx, dy) is legal when dx <= xl and dy <= yl
 };
-constexpr int kMbCtxBytes = 192;
+constexpr int kMbCtxBytes = 208;
 static_assert(sizeof(MbCtx) <= kMbCtxBytes, "MbCtx layout");
 
 __device__ __forceinline__ const MbCtx& mbctx(uint32_t off) { return *reinterpret_cast<const MbCtx*>(g_smem + off); }
 
+// The largest integer (dx, dy) of the 16x16 MB at (x0, y0) that hidden_padding (with its chroma
+// test) allows: an integer vector reads no fractional neighbour, so each of its tests bounds one
+// component from above (luma: x0 + aw - 1 + dx < vw; chroma, at half the vector rounded up:
+// dx <= 2 (cvw - cx - caw)).
+__device__ __forceinline__ int2 integer_limits(const DevParams& P, int x0, int y0) {
+    int2 l = make_int2(0x7fffffff, 0x7fffffff);
+    const int aw = imax(0, imin(16, P.vw - x0)), ah = imax(0, imin(16, P.vh - y0));
+    if (aw && ah) {
+        if (P.right_pad) l.x = P.vw - x0 - aw;
+        if (P.bottom_pad) l.y = P.vh - y0 - ah;
+    }
+    const int cx = x0 / 2, cy = y0 / 2;
+    const int caw = imax(0, imin(8, P.cvw - cx)), cah = imax(0, imin(8, P.cvh - cy));
+    if (caw && cah) {
+        if (P.cright_pad) l.x = imin(l.x, 2 * (P.cvw - cx - caw));
+        if (P.cbottom_pad) l.y = imin(l.y, 2 * (P.cvh - cy - cah));
+    }
+    return l;
+}
+
 // mb_sad at integer offset (dx, dy) and sampling stride 1/2/4 (encoder_motion.cpp:2197-2285);
-// one out-of-line copy serves every search stage.
+// one out-of-line copy for the searches that score a few candidates and for the UMH search's
+// partial macroblocks and candidates outside the window.
 __device__ __noinline__ uint64_t mb_sad_core(uint32_t ctx, int dx, int dy, int stride) {
     const MbCtx& c = mbctx(ctx);
+    if (dx > c.xl || dy > c.yl) return kBad;
     const DevParams P = geo_params(c.g);
-    if (hidden_padding(P, c.x0, c.y0, 16, 16, dx * 4, dy * 4, VC1CU_MV_QPEL, true)) return kBad;
     uint32_t s;
     const int xa = c.x0 + dx, ya = c.y0 + dy;
     const bool fast = xa >= c.wx0 && ya >= c.wy0 && xa + 15 < c.wx0 + c.wp && ya + 15 < c.wy0 + c.wh;
@@ -496,140 +506,232 @@ __device__ __forceinline__ bool ctx_inside(const MbCtx& c, int xa, int ya, int x
     return xa >= c.wx0 && ya >= c.wy0 && xb < c.wx0 + c.wp && yb < c.wy0 + c.wh;
 }
 
-// The sub-pel plane row of phase (hm, vm) at integer origin (sx, sy), when its n samples lie in
-// the planes (nullptr otherwise).
-__device__ __forceinline__ const uint8_t* sp_row(const MbCtx& c, int hm, int vm, int sx, int sy, int n) {
-    if (!c.sp || !(hm | vm)) return nullptr;
-    const int b = c.sp_border;
-    if (sx < -b || sx + n > c.g.W + b || sy < -b || sy >= c.g.H + b) return nullptr;
-    return c.sp + (long long)(vm * 4 + hm) * c.sp_stride + (long long)(sy + b) * c.sp_pitch + (sx + b);
-}
-
 // n <= 8 bytes of a plane row as two little-endian words (aligned loads and funnel shifts; the
-// row continues at least 3 bytes past any origin sp_row accepts)
+// row continues at least 3 bytes past any origin plane_offset accepts)
 __device__ __forceinline__ void sp_load8(const uint8_t* p, uint32_t& lo, uint32_t& hi) {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
     const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
-    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = sh ? __ldg(w + 2) : 0u;
+    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
     lo = __funnelshift_r(w0, w1, sh);
     hi = __funnelshift_r(w1, w2, sh);
 }
+__device__ __forceinline__ uint32_t sp_load4(const uint8_t* p) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
+    return __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8);
+}
 
-// SAD of n candidates of block (bx,by,bw,bh) (bw,bh in {8,16}) under the CPU law, written
-// to out[]. Each candidate's block is split into 8-pixel row segments over bh*bw/8 lanes.
-// One out-of-line copy serves every call site. Sub-pel rows come from the pass's prediction
-// planes where they cover them, else are interpolated from the window or the frame.
+// Offset in the pass's prediction planes of vector mv's prediction of the bw x bh block at
+// (bx, by), or -1 where the planes do not hold all of it.
+__device__ __forceinline__ long long plane_offset(const MbCtx& c, int2 mv, int bx, int by, int bw, int bh) {
+    const int ix = floor_div4(mv.x), iy = floor_div4(mv.y), hm = mv.x - 4 * ix, vm = mv.y - 4 * iy;
+    const int b = c.sp_border, sx = bx + ix, sy = by + iy;
+    if (!c.sp || sx < -b || sx + bw > c.g.W + b || sy < -b || sy + bh > c.g.H + b) return -1;
+    return (long long)(vm * 4 + hm) * c.sp_stride + (long long)(sy + b) * c.sp_pitch + (sx + b);
+}
+
+// The bytes of an 8-byte (4-byte) group of which the first n are visible (n <= 0: none).
+__device__ __forceinline__ uint32_t vis_mask(int n) { return n >= 4 ? 0xffffffffu : (n <= 0 ? 0u : (1u << (8 * n)) - 1u); }
+
+// One candidate's block SAD where the planes do not hold it: row segments interpolated from the
+// window or the frame (the summed value on every lane that holds a segment).
+__device__ __noinline__ uint32_t sad_interpolated(uint32_t ctx, int mvx, int mvy, int bx, int by, int bw, int bh, int mode) {
+    const MbCtx& c = mbctx(ctx);
+    const int lane = threadIdx.x & 31;
+    const int spr = bw >> 3, segs = bh * spr;
+    const int aw = imax(0, imin(bw, c.g.W - bx)), ah = imax(0, imin(bh, c.g.H - by));
+    const bool bil = mode_bilinear(mode);
+    const int r = lane / spr, c0 = (lane % spr) * 8;
+    uint32_t part = 0;
+    if (lane < segs && r < ah && c0 < aw) {
+        const int ix = floor_div4(mvx), iy = floor_div4(mvy);
+        const uint32_t cp = c.cur_off + (uint32_t)((by - c.y0 + r) * 16 + bx - c.x0 + c0);
+        const int nvis = imin(8, aw - c0);
+        if (ctx_inside(c, bx + ix - 1, by + iy - 1, bx + ix + bw + 1, by + iy + bh + 1)) {
+            part = sad_row8(WinSampler{c.win_off, c.wp, c.wx0, c.wy0, c.wh}, bil, c.g.rnd, mvx, mvy, bx + c0, by + r, cp, nvis);
+        } else {
+            const PredRow<8> g8 = predict_row_glob<8>(c.gref, c.gpitch, c.g.W, c.g.H, bil, c.g.rnd, mvx, mvy, bx + c0, by + r);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < nvis) part += (uint32_t)iabs((int)g_smem[cp + i] - g8.v[i]);
+        }
+    }
+    return __reduce_add_sync(FULL, part);
+}
+
+// SAD of n <= 32 candidates of block (bx,by,bw,bh) (bw = bh in {8,16}) under the CPU law, written
+// to out[]. One out-of-line copy serves every call site. Lane i works out candidate i's legality
+// and address once; the block's 8-pixel row segments lie across 32 (16x16) or 8 (8x8) lanes, whose
+// current pixels stay in registers, and the segments of several candidates are loaded from the
+// prediction planes before any is summed: the routine is bound by the latency of those loads, not
+// by their number. Two SADs share a word in the warp sum (a 16x16 SAD is below 2^16). With the
+// keyed list and the word-wise minima below, a refinement takes 16 K clocks against 43 K for one
+// candidate at a time and selections by shuffles of whole structures (CIF, one macroblock alone).
+constexpr int kSadGroup = 5;  // candidates whose rows are in flight together (registers bound it)
 __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int n, int bx, int by,
                                             int bw, int bh, int mode, uint32_t out_off) {
     const MbCtx& c = mbctx(ctx);
     const int lane = threadIdx.x & 31;
-    const DevParams P = geo_params(c.g);
     const int2* mvs = reinterpret_cast<const int2*>(g_smem + mvs_off);
     uint64_t* out = reinterpret_cast<uint64_t*>(g_smem + out_off);
-    const int spr = bw >> 3;
-    const int segs = bh * spr;  // 32 (16x16) or 8 (8x8)
-    const int per_iter = 32 / segs;
-    const int aw = imax(0, imin(bw, P.W - bx)), ah = imax(0, imin(bh, P.H - by));
-    const bool bil = mode_bilinear(mode);
-    const bool cg = chroma_gate(bx, by, bw, bh);
+    const int aw = imax(0, imin(bw, c.g.W - bx)), ah = imax(0, imin(bh, c.g.H - by));
+    const int2 mv = lane < n ? mvs[lane] : make_int2(0, 0);
+    bool bad = false;
+    long long off = -1;
+    if (lane < n) {
+        const DevParams P = geo_params(c.g);
+        bad = hidden_padding(P, bx, by, bw, bh, mv.x, mv.y, mode, chroma_gate(bx, by, bw, bh)) ||
+              (mode_bilinear(mode) && ((mv.x | mv.y) & 1));
+        if (!bad) off = plane_offset(c, mv, bx, by, bw, bh);
+    }
+    const unsigned planes = __ballot_sync(FULL, off >= 0);
     const int cx = bx - c.x0, cy = by - c.y0;
-    for (int base = 0; base < n; base += per_iter) {
-        const int ci = base + lane / segs;
-        const int sidx = lane % segs;
-        const int r = sidx / spr, c0 = (sidx % spr) * 8;
-        const bool valid = ci < n;
-        const int2 mv = valid ? mvs[ci] : make_int2(0, 0);
-        bool bad = false;
-        uint32_t part = 0;
-        if (valid) {
-            bad = hidden_padding(P, bx, by, bw, bh, mv.x, mv.y, mode, cg) || (bil && ((mv.x & 1) || (mv.y & 1)));
-            if (!bad && r < ah && c0 < aw) {
-                const int ix = floor_div4(mv.x), iy = floor_div4(mv.y);
-                const uint32_t cp = c.cur_off + (uint32_t)((cy + r) * 16 + cx + c0);
-                const int nvis = imin(8, aw - c0);
-                const uint8_t* pr = nvis == 8 ? sp_row(c, mv.x - 4 * ix, mv.y - 4 * iy, bx + c0 + ix, by + r + iy, 8) : nullptr;
-                if (pr) {
-                    uint32_t lo, hi;
-                    sp_load8(pr, lo, hi);
-                    part = __vsadu4(lo, g_smem32[cp >> 2]) + __vsadu4(hi, g_smem32[(cp >> 2) + 1]);
-                } else if (ctx_inside(c, bx + ix - 1, by + iy - 1, bx + ix + bw + 1, by + iy + bh + 1)) {
-                    part = sad_row8(WinSampler{c.win_off, c.wp, c.wx0, c.wy0, c.wh}, bil, P.rnd, mv.x, mv.y, bx + c0, by + r, cp, nvis);
-                } else {
-                    const PredRow<8> g8 = predict_row_glob<8>(c.gref, c.gpitch, P.W, P.H, bil, P.rnd, mv.x, mv.y, bx + c0, by + r);
+    uint32_t mine = 0;  // lane i: candidate i's SAD
+    if (bw == 16) {
+        const int r = lane >> 1, c0 = (lane & 1) * 8, vis = r < ah ? aw - c0 : 0;
+        const uint32_t m0 = vis_mask(vis), m1 = vis_mask(vis - 4);
+        const uint32_t cw = (c.cur_off + (uint32_t)((cy + r) * 16 + cx + c0)) >> 2;
+        const uint32_t a0 = g_smem32[cw] & m0, a1 = g_smem32[cw + 1] & m1;
+        const uint8_t* seg = c.sp + (long long)r * c.sp_pitch + c0;
+#pragma unroll 1
+        for (int base = 0; base < n; base += kSadGroup) {
+            uint32_t part[kSadGroup + 1];
+            part[kSadGroup] = 0;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (i < nvis) part += (uint32_t)iabs((int)g_smem[cp + i] - g8.v[i]);
+            for (int u = 0; u < kSadGroup; ++u) {
+                part[u] = 0;
+                const long long o = __shfl_sync(FULL, off, (base + u) & 31);
+                if (base + u < n && o >= 0) {
+                    uint32_t lo, hi;
+                    sp_load8(seg + o, lo, hi);
+                    part[u] = __vsadu4(lo & m0, a0) + __vsadu4(hi & m1, a1);
                 }
             }
+#pragma unroll
+            for (int u = 0; u < kSadGroup; u += 2) {
+                const uint32_t two = __reduce_add_sync(FULL, part[u] | (part[u + 1] << 16));
+                if (lane == base + u) mine = two & 0xffffu;
+                if (u + 1 < kSadGroup && lane == base + u + 1) mine = two >> 16;
+            }
         }
-        for (int o = segs >> 1; o; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
-        if (valid && sidx == 0) out[ci] = bad ? kBad : (uint64_t)part;
+    } else {
+        const int r = lane & 7, g = lane >> 3, vis = r < ah ? aw : 0;
+        const uint32_t m0 = vis_mask(vis), m1 = vis_mask(vis - 4);
+        const uint32_t cw = (c.cur_off + (uint32_t)((cy + r) * 16 + cx)) >> 2;
+        const uint32_t a0 = g_smem32[cw] & m0, a1 = g_smem32[cw + 1] & m1;
+        const uint8_t* seg = c.sp + (long long)r * c.sp_pitch;
+#pragma unroll 1
+        for (int base = 0; base < n; base += 12) {
+            uint32_t part[4];
+            part[3] = 0;
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                part[u] = 0;
+                const int ci = base + 4 * u + g;
+                const long long o = __shfl_sync(FULL, off, ci & 31);
+                if (ci < n && o >= 0) {
+                    uint32_t lo, hi;
+                    sp_load8(seg + o, lo, hi);
+                    part[u] = __vsadu4(lo & m0, a0) + __vsadu4(hi & m1, a1);
+                }
+            }
+            uint32_t s0 = part[0] | (part[1] << 16), s1 = part[2];
+#pragma unroll
+            for (int o = 4; o; o >>= 1) {
+                s0 += __shfl_xor_sync(FULL, s0, o);
+                s1 += __shfl_xor_sync(FULL, s1, o);
+            }
+            // lane base + 4 u + g takes group g's sum of round u
+            const int k = lane - base;
+            const uint32_t t0 = __shfl_sync(FULL, s0, (k & 3) * 8), t1 = __shfl_sync(FULL, s1, (k & 3) * 8);
+            if (k >= 0 && k < 12) mine = k < 4 ? (t0 & 0xffffu) : (k < 8 ? (t0 >> 16) : t1);
+        }
     }
+    // the candidates beyond the planes
+    unsigned rest = __ballot_sync(FULL, lane < n && !bad) & ~planes;
+    while (rest) {
+        const int i = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const uint32_t v = sad_interpolated(ctx, __shfl_sync(FULL, mv.x, i), __shfl_sync(FULL, mv.y, i), bx, by, bw, bh, mode);
+        if (lane == i) mine = v;
+    }
+    if (lane < n) out[lane] = bad ? kBad : (uint64_t)mine;
     __syncwarp();
 }
 
+// Four rows of a 4x4 tile's prediction as words, where the planes do not hold the block.
+__device__ __noinline__ uint4 tile_interpolated(uint32_t ctx, int mvx, int mvy, int tx, int ty, int mode, bool fast) {
+    const MbCtx& c = mbctx(ctx);
+    const bool bil = mode_bilinear(mode);
+    uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+#pragma unroll 1
+    for (int yy = 0; yy < 4; ++yy) {
+        int4 w;
+        if (fast) {
+            w = pred_row4(WinSampler{c.win_off, c.wp, c.wx0, c.wy0, c.wh}, bil, c.g.rnd, mvx, mvy, tx, ty + yy);
+        } else {
+            const PredRow<4> g4 = predict_row_glob<4>(c.gref, c.gpitch, c.g.W, c.g.H, bil, c.g.rnd, mvx, mvy, tx, ty + yy);
+            w = make_int4(g4.v[0], g4.v[1], g4.v[2], g4.v[3]);
+        }
+        q0 = q1;
+        q1 = q2;
+        q2 = q3;
+        q3 = (uint32_t)w.x | ((uint32_t)w.y << 8) | ((uint32_t)w.z << 16) | ((uint32_t)w.w << 24);
+    }
+    return make_uint4(q0, q1, q2, q3);
+}
+
+// SATD of n <= 32 candidates, one 4x4 tile per lane and candidate, written to out[]. The four plane
+// rows of a tile are loaded together and its current pixels stay in registers across candidates.
 __device__ __noinline__ void satd_batch_core(uint32_t ctx, uint32_t mvs_off, int n, int bx, int by,
                                              int bw, int bh, int mode, uint32_t out_off) {
     const MbCtx& c = mbctx(ctx);
     const int lane = threadIdx.x & 31;
-    const DevParams P = geo_params(c.g);
     const int2* mvs = reinterpret_cast<const int2*>(g_smem + mvs_off);
     uint64_t* out = reinterpret_cast<uint64_t*>(g_smem + out_off);
     const int tpr = bw >> 2;
     const int tiles = tpr * (bh >> 2);  // 16 or 4
     const int per_iter = 32 / tiles;
-    const int aw = imax(0, imin(bw, P.W - bx)), ah = imax(0, imin(bh, P.H - by));
-    const bool bil = mode_bilinear(mode);
-    const int cx = bx - c.x0, cy = by - c.y0;
+    const int aw = imax(0, imin(bw, c.g.W - bx)), ah = imax(0, imin(bh, c.g.H - by));
+    const int t = lane % tiles, tx = (t % tpr) * 4, ty = (t / tpr) * 4;
+    const int tw = imax(0, imin(4, aw - tx)), th = imax(0, imin(4, ah - ty));
+    const uint32_t cw = (c.cur_off + (uint32_t)((by - c.y0 + ty) * 16 + bx - c.x0 + tx)) >> 2;
+    uint32_t m[4], a[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        m[y] = y < th ? vis_mask(tw) : 0u;
+        a[y] = g_smem32[cw + 4 * y] & m[y];
+    }
+#pragma unroll 1
     for (int base = 0; base < n; base += per_iter) {
         const int ci = base + lane / tiles;
-        const int t = lane % tiles;
-        const int tx = (t % tpr) * 4, ty = (t / tpr) * 4;
         const bool valid = ci < n;
         const int2 mv = valid ? mvs[ci] : make_int2(0, 0);
         const bool bad = valid && mode_halfpel(mode) && ((mv.x & 1) || (mv.y & 1));
         uint32_t part = 0;
-        const int tw = imax(0, imin(4, aw - tx)), th = imax(0, imin(4, ah - ty));
         if (valid && !bad && tw && th) {
-            const int ix = floor_div4(mv.x), iy = floor_div4(mv.y);
-            const bool fast = ctx_inside(c, bx + ix - 1, by + iy - 1, bx + ix + bw + 1, by + iy + bh + 1);
-            // rows one at a time (one copy of the interpolation code), row-transformed and
-            // rotated through four registers for the column stage
-            int4 r0 = make_int4(0, 0, 0, 0), r1 = r0, r2 = r0, r3 = r0;
-            const uint8_t* pr = sp_row(c, mv.x - 4 * ix, mv.y - 4 * iy, bx + tx + ix, by + ty + iy, 4);
-            if (pr && !sp_row(c, mv.x - 4 * ix, mv.y - 4 * iy, bx + tx + ix, by + ty + iy + 3, 4)) pr = nullptr;
-#pragma unroll 1
-            for (int yy = 0; yy < 4; ++yy) {
-                int pred[4];
-                if (pr) {
-                    uint32_t lo, hi;
-                    sp_load8(pr + (long long)yy * c.sp_pitch, lo, hi);
-                    pred[0] = lo & 255;
-                    pred[1] = (lo >> 8) & 255;
-                    pred[2] = (lo >> 16) & 255;
-                    pred[3] = lo >> 24;
-                } else if (fast) {
-                    const int4 w4 = pred_row4(WinSampler{c.win_off, c.wp, c.wx0, c.wy0, c.wh}, bil, P.rnd, mv.x, mv.y, bx + tx, by + ty + yy);
-                    pred[0] = w4.x;
-                    pred[1] = w4.y;
-                    pred[2] = w4.z;
-                    pred[3] = w4.w;
-                } else {
-                    const PredRow<4> g4 = predict_row_glob<4>(c.gref, c.gpitch, P.W, P.H, bil, P.rnd, mv.x, mv.y, bx + tx,
-                                                              by + ty + yy);
+            uint32_t p[4];
+            const long long off = plane_offset(c, mv, bx, by, bw, bh);
+            if (off >= 0) {
+                const uint8_t* row = c.sp + off + (long long)ty * c.sp_pitch + tx;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) pred[i] = g4.v[i];
-                }
-                int d[4];
-                const uint32_t crow = c.cur_off + (uint32_t)((cy + ty + yy) * 16 + cx + tx);
-#pragma unroll
-                for (int xx = 0; xx < 4; ++xx) d[xx] = (xx < tw && yy < th) ? (int)g_smem[crow + xx] - pred[xx] : 0;
-                r0 = r1;
-                r1 = r2;
-                r2 = r3;
-                r3 = hadamard_row(d[0], d[1], d[2], d[3]);
+                for (int y = 0; y < 4; ++y) p[y] = sp_load4(row + (long long)y * c.sp_pitch);
+            } else {
+                const int ix = floor_div4(mv.x), iy = floor_div4(mv.y);
+                const bool fast = ctx_inside(c, bx + ix - 1, by + iy - 1, bx + ix + bw + 1, by + iy + bh + 1);
+                const uint4 q = tile_interpolated(ctx, mv.x, mv.y, bx + tx, by + ty, mode, fast);
+                p[0] = q.x;
+                p[1] = q.y;
+                p[2] = q.z;
+                p[3] = q.w;
             }
-            part = hadamard_cols(r0, r1, r2, r3);
+            int4 h[4];
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const uint32_t q = p[y] & m[y];
+                h[y] = hadamard_row((int)(a[y] & 255) - (int)(q & 255), (int)((a[y] >> 8) & 255) - (int)((q >> 8) & 255),
+                                    (int)((a[y] >> 16) & 255) - (int)((q >> 16) & 255), (int)(a[y] >> 24) - (int)(q >> 24));
+            }
+            part = hadamard_cols(h[0], h[1], h[2], h[3]);
         }
         for (int o = tiles >> 1; o; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
         if (valid && t == 0) out[ci] = (!aw || !ah) ? 0 : (bad ? kBad : (uint64_t)part);
@@ -648,124 +750,181 @@ __device__ __forceinline__ void satd_batch(const DevParams& P, const Mb& m, cons
     satd_batch_core(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
 }
 
-// ---- first-visit bitsets ----------------------------------------------------------------
+// ---- integer UMH (encoder_motion.cpp:1781-2023) -----------------------------------------
+//
+// The reference keeps the eight least distinct candidates of its sampled stages, but only the
+// least (every stage's centre) and the four least (the finalists) are ever read, and the four
+// least of a union do not depend on what stood behind them. So the search keeps four keys,
+// identical on every lane. A key holds its vector, so a candidate scored again equals its own
+// entry or falls behind the fourth: no first-visit record is needed, and the full-resolution
+// stages, plain minima, need none either. The macroblock's wavefront neighbours wait for this
+// search, so it is written for its latency: stages of few candidates spread each one's rows over
+// several lanes, and the neighbour-independent lattice is scored before the wait (umh_lattice).
+// A CIF picture alone (clocks per macroblock after the wait): 28 K with the stages' candidates one
+// per lane, first-visit bitsets and a top-8 list in shared memory, 16 K now (and 6 K before the
+// wait for the lattice); a 720p B picture's two passes at range 64, 9.3 -> 4.5 ms with the
+// refinement below.
 
-__device__ __forceinline__ bool seen_test_set(uint32_t* bits, int r, int dx, int dy) {
-    const int side = 2 * r + 1;
-    if (!IDX_OK(dx >= -r && dx <= r && dy >= -r && dy <= r, kSiteSeen, (long long)dy * 65536 + dx)) return true;
-    const int bit = (dy + r) * side + (dx + r);
-    const uint32_t mask = 1u << (bit & 31);
-    return (atomicOr(&bits[bit >> 5], mask) & mask) != 0;
+// The least key of the warp, on every lane.
+__device__ __forceinline__ uint64_t warp_min_key(uint64_t k) {
+    const uint32_t h = __reduce_min_sync(FULL, (uint32_t)(k >> 32));
+    const uint32_t l = __reduce_min_sync(FULL, (uint32_t)(k >> 32) == h ? (uint32_t)k : 0xffffffffu);
+    return ((uint64_t)h << 32) | l;
 }
 
-// ---- integer UMH (encoder_motion.cpp:1781-2023) -----------------------------------------
+struct Top4 {
+    uint64_t a, b, c, d;  // ascending; UINT64_MAX: none
+};
 
-// Merges the n keys of m.sm.keys (UINT64_MAX = skipped) into the sorted top-8 list
-// m.sm.top / m.sm.misc[0]. Keys below the current 8th entry are compacted with a ballot
-// first; the few survivors are ranked and merged on every lane identically.
-__device__ __noinline__ void top8_merge_core(int lane, uint32_t keys_off, uint32_t top_off, uint32_t misc_off,
-                                             uint32_t out8_off, int n) {
-    uint64_t* keys = reinterpret_cast<uint64_t*>(g_smem + keys_off);
-    uint64_t* top = reinterpret_cast<uint64_t*>(g_smem + top_off);
-    int* misc = reinterpret_cast<int*>(g_smem + misc_off);
-    const int tn = misc[0];
-    const uint64_t bound = tn == 8 ? top[7] : UINT64_MAX;
-    int cnt = 0;
+__device__ __forceinline__ void top4_insert(Top4& t, uint64_t k) {
+    if (k >= t.d || k == t.a || k == t.b || k == t.c) return;
+    t.d = k;
+    if (t.d < t.c) { t.d = t.c; t.c = k; }
+    if (t.c < t.b) { t.c = t.b; t.b = k; }
+    if (t.b < t.a) { t.b = t.a; t.a = k; }
+}
+
+// Merges one key per lane (UINT64_MAX: none) into the four least.
+__device__ __forceinline__ void top4_merge(Top4& t, uint64_t key) {
+    while (__any_sync(FULL, key < t.d)) {
+        const uint64_t k = warp_min_key(key);
+        if (key == k) key = UINT64_MAX;
+        top4_insert(t, k);
+    }
+}
+
+// What scoring the macroblock's integer candidates reads, in registers.
+struct SearchGeo {
+    uint32_t win, cur, cur2, cur4;
+    int wp, wx0, wy0, wh, x0, y0, xl, yl;
+    bool whole;  // all 16x16 pixels inside the raster
+    __device__ __forceinline__ explicit SearchGeo(uint32_t ctx) {
+        const MbCtx& c = mbctx(ctx);
+        win = c.win_off;
+        cur = c.cur_off >> 2;
+        cur2 = c.cur2_off >> 2;
+        cur4 = c.cur4_off >> 2;
+        wp = c.wp;
+        wx0 = c.wx0;
+        wy0 = c.wy0;
+        wh = c.wh;
+        x0 = c.x0;
+        y0 = c.y0;
+        xl = c.xl;
+        yl = c.yl;
+        whole = c.aw == 16 && c.ah == 16;
+    }
+    // the candidate's block lies in the window
+    __device__ __forceinline__ bool staged(int dx, int dy) const {
+        const int rx = x0 + dx - wx0, ry = y0 + dy - wy0;
+        return whole && rx >= 0 && ry >= 0 && rx + 16 <= wp && ry + 16 <= wh;
+    }
+    __device__ __forceinline__ uint32_t base(int dx, int dy) const {
+        return win + (uint32_t)((y0 + dy - wy0) * wp + (x0 + dx - wx0));
+    }
+};
+
+// Packed SAD of sampled rows r0 .. r0 + nr - 1 (nr even, or one row at stride 4) of a staged candidate.
+template <int STRIDE>
+__device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, int r0, int nr) {
+    uint32_t acc = 0;
+#pragma unroll 2
+    for (int r = r0; r < r0 + nr; ++r) {
+        uint32_t v[4];
+        win_load16(base + (uint32_t)(r * STRIDE * g.wp), v);
+        if (STRIDE == 1) {
+            acc += __vsadu4(v[0], g_smem32[g.cur + r * 4]) + __vsadu4(v[1], g_smem32[g.cur + r * 4 + 1]) +
+                   __vsadu4(v[2], g_smem32[g.cur + r * 4 + 2]) + __vsadu4(v[3], g_smem32[g.cur + r * 4 + 3]);
+        } else if (STRIDE == 2) {
+            acc += __vsadu4(__byte_perm(v[0], v[1], 0x6420), g_smem32[g.cur2 + r * 4]) +
+                   __vsadu4(__byte_perm(v[2], v[3], 0x6420), g_smem32[g.cur2 + r * 4 + 1]);
+        } else {
+            const uint32_t e = __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
+            acc += __vsadu4(e, g_smem32[g.cur4 + 4 * r]);
+        }
+    }
+    return acc;
+}
+
+// Key of the candidate that 2^sh neighbouring lanes share (each scores its part of the rows): the
+// mb_sad at the given stride. Every lane calls it with its candidate; !on scores nothing.
+template <int STRIDE>
+__device__ __forceinline__ uint64_t shared_key(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
+    const int part = (threadIdx.x & 31) & ((1 << sh) - 1), nr = (16 / STRIDE) >> sh;
+    const bool legal = dx <= g.xl && dy <= g.yl, in = g.staged(dx, dy);
+    uint32_t s = 0;
+    if (on && legal) {
+        if (in) s = sad_rows<STRIDE>(g, g.base(dx, dy), part * nr, nr) * (STRIDE * STRIDE);
+        else if (part == 0) s = (uint32_t)mb_sad_core(ctx, dx, dy, STRIDE);
+    }
+    if (sh > 0) s += __shfl_xor_sync(FULL, s, 1);
+    if (sh > 1) s += __shfl_xor_sync(FULL, s, 2);
+    if (sh > 2) s += __shfl_xor_sync(FULL, s, 4);
+    return on ? int_key(legal ? (uint64_t)s : kBad, dx, dy) : UINT64_MAX;
+}
+
+// The four least keys of the sparse lattice over the whole window (:1865-1870, range >= 8), which
+// depends on no neighbour: scored before the wavefront wait, one candidate per lane, into top[0..3].
+__device__ __noinline__ void umh_lattice(uint32_t ctx, uint32_t top_off, int range) {
+    const SearchGeo g(ctx);
+    const int lane = threadIdx.x & 31;
+    const int L = (2 * range) / 8 + 1;
+    // the far edges repeat the lattice's last row and column when its step divides the window
+    const int n = L * L + ((2 * range) % 8 ? 2 * L : 0);
+    Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
+#pragma unroll 1
     for (int base = 0; base < n; base += 32) {
         const int i = base + lane;
-        const uint64_t k = i < n ? keys[i] : UINT64_MAX;
-        const bool take = k < bound;
-        const unsigned b = __ballot_sync(FULL, take);
-        if (take) keys[cnt + __popc(b & ((1u << lane) - 1))] = k;
-        cnt += __popc(b);
-        __syncwarp();
-    }
-    if (!cnt) return;
-    const uint64_t* sel;
-    int ns = 0;
-    if (cnt <= 32) {
-        // rank of each survivor (keys are distinct), the 8 lowest ranks in order
-        const uint64_t k = lane < cnt ? keys[lane] : UINT64_MAX;
-        int rank = 0;
-        for (int j = 0; j < cnt; ++j) rank += keys[j] < k;
-        __syncwarp();
-        if (lane < cnt && rank < 8) keys[rank] = k;
-        __syncwarp();
-        ns = cnt < 8 ? cnt : 8;
-        sel = keys;
-    } else {
-        uint64_t* out8 = reinterpret_cast<uint64_t*>(g_smem + out8_off);  // idle during the integer search
-        for (int r = 0; r < 8; ++r) {
-            uint64_t lm = UINT64_MAX;
-            for (int i = lane; i < cnt; i += 32) lm = keys[i] < lm ? keys[i] : lm;
-            const uint64_t g = warp_min_u64(lm);
-            if (lane == 0) out8[r] = g;
-            for (int i = lane; i < cnt; i += 32)
-                if (keys[i] == g) keys[i] = UINT64_MAX;
-            __syncwarp();
+        int dx, dy;
+        if (i < L * L) {
+            dy = i / L;
+            dx = -range + (i - dy * L) * 8;
+            dy = -range + dy * 8;
+        } else {
+            const int j = i - L * L, d = -range + (j >> 1) * 8;
+            dx = (j & 1) ? d : range;
+            dy = (j & 1) ? range : d;
         }
-        ns = 8;
-        sel = out8;
+        top4_merge(t, shared_key<2>(ctx, g, i < n, dx, dy, 0));
     }
-    uint64_t out[8];
-    int a = 0, b = 0, o = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        if (a < tn || b < ns) {
-            const uint64_t ta = a < tn ? top[a] : UINT64_MAX, tb = b < ns ? sel[b] : UINT64_MAX;
-            if (ta < tb) { out[q] = ta; ++a; } else { out[q] = tb; ++b; }
-            ++o;
-        }
+    if (lane == 0) {
+        uint64_t* top = reinterpret_cast<uint64_t*>(g_smem + top_off);
+        top[0] = t.a;
+        top[1] = t.b;
+        top[2] = t.c;
+        top[3] = t.d;
     }
-    __syncwarp();
-    if (lane < o) {
-        uint64_t v = out[0];
-#pragma unroll
-        for (int q = 1; q < 8; ++q) if (lane == q) v = out[q];
-        top[lane] = v;
-    }
-    if (lane == 0) misc[0] = o;
     __syncwarp();
 }
 
-__device__ __forceinline__ void top8_merge(const Mb& m, int n) {
-    top8_merge_core(m.lane, m.sm.keys.off, m.sm.top.off, m.sm.misc.off, m.sm.list_sad.off, n);
-}
-
-// Scores the candidates produced by gen(i) for i < n at sampled stride 2 (the UMH
-// `consider` lambda, encoder_motion.cpp:1821-1839) and merges them into top.
-template <class Gen>
-__device__ void umh_stage(const DevParams& P, const Mb& m, int n, int range, Gen gen) {
-    for (int i = m.lane; i < n; i += 32) {
-        int2 c = gen(i);
-        c.x = iclamp(c.x, -range, range);
-        c.y = iclamp(c.y, -range, range);
-        uint64_t key = UINT64_MAX;
-        if (!seen_test_set(m.sm.seen, range, c.x, c.y)) key = int_key(mb_sad(P, m, c.x, c.y, 2), c.x, c.y);
-        if (IDX_OK(i < m.keys_cap, kSiteKeys, i)) m.sm.keys[i] = key;
-    }
-    __syncwarp();
-    top8_merge(m, n);
-}
-
-// Minimum key over full-resolution candidates (no top list), optional first-visit filter.
-template <class Gen>
-__device__ uint64_t full_stage(const DevParams& P, const Mb& m, int n, int range, int stride, bool use_seen, Gen gen) {
+// Least key over the box [x0, x0 + (nx - 1) step] x [y0, ..] (and, with edges, the window's far
+// column and row at +range): the full_resolution / stride-2 / stride-4 scans of the rescue.
+__device__ __noinline__ uint64_t box_min(uint32_t ctx, int bx, int by, int nx, int ny, int step, int stride, int range,
+                                         bool edges) {
+    const SearchGeo g(ctx);
+    const int lane = threadIdx.x & 31;
+    const int n0 = nx * ny, n = n0 + (edges ? 2 * nx : 0);
     uint64_t best = UINT64_MAX;
-    for (int i = m.lane; i < n; i += 32) {
-        bool ok;
-        int2 c = gen(i, ok);
-        if (!ok) continue;
-        if (use_seen && seen_test_set(m.sm.seen_full, range, c.x, c.y)) continue;
-        const uint64_t k = int_key(mb_sad(P, m, c.x, c.y, stride), c.x, c.y);
+#pragma unroll 1
+    for (int base = 0; base < n; base += 32) {
+        const int i = base + lane;
+        int dx, dy;
+        if (i < n0) {
+            dy = i / nx;
+            dx = bx + (i - dy * nx) * step;
+            dy = by + dy * step;
+        } else {
+            const int j = i - n0, d = bx + (j >> 1) * step;
+            dx = (j & 1) ? d : range;
+            dy = (j & 1) ? range : d;
+        }
+        uint64_t k;
+        if (stride == 1) k = shared_key<1>(ctx, g, i < n, dx, dy, 0);
+        else if (stride == 2) k = shared_key<2>(ctx, g, i < n, dx, dy, 0);
+        else k = shared_key<4>(ctx, g, i < n, dx, dy, 0);
         best = k < best ? k : best;
     }
-    return warp_min_u64(best);
-}
-
-__device__ __forceinline__ bool match_good(const DevParams& P, uint64_t sad, uint64_t pixels) {
-    if (!pixels || sad >= UINT64_MAX / 8) return false;
-    return sad <= pixels * 6u;
+    return warp_min_key(best);
 }
 
 struct IntRes {
@@ -773,150 +932,111 @@ struct IntRes {
     uint64_t cost;
 };
 
-__device__ IntRes umh(const DevParams& P, const Mb& m, const PInfo& pi, int gdx, int gdy, int range, uint64_t pixels) {
-    // clear bitsets
-    const int words = ((2 * range + 1) * (2 * range + 1) + 31) >> 5;
-    for (int i = m.lane; i < words; i += 32) {
-        m.sm.seen[i] = 0;
-        m.sm.seen_full[i] = 0;
-    }
-    if (m.lane == 0) m.sm.misc[0] = 0;
-    __syncwarp();
-    const uint64_t* top = m.sm.top;
-    // predictor seeds (:1843-1850)
-    {
-        // predictor, zero, global, then A and C where they exist
-        const int2 sp = make_int2(iclamp(round_qpel_to_pixel(pi.pre.x), -range, range),
-                                  iclamp(round_qpel_to_pixel(pi.pre.y), -range, range));
-        const int2 sa = make_int2(round_qpel_to_pixel(pi.a.x), round_qpel_to_pixel(pi.a.y));
-        const int2 sc = make_int2(round_qpel_to_pixel(pi.c.x), round_qpel_to_pixel(pi.c.y));
-        const int ns = 3 + (pi.a_valid ? 1 : 0) + (pi.c_valid ? 1 : 0);
-        umh_stage(P, m, ns, range, [&](int i) {
-            return i == 0 ? sp : i == 1 ? make_int2(0, 0) : i == 2 ? make_int2(gdx, gdy) : (i == 3 && pi.a_valid) ? sa : sc;
-        });
-    }
-    // 5x5 around best (:1855-1859)
-    {
-        const int cx = key_dx(top[0]), cy = key_dy(top[0]);
-        umh_stage(P, m, 25, range, [&](int i) { return make_int2(cx + i % 5 - 2, cy + i / 5 - 2); });
-    }
-    // sparse lattice over the whole window (:1865-1870)
-    if (range >= 8) {
-        const int L = (2 * range) / 8 + 1;
-        umh_stage(P, m, L * L + 2 * L, range, [&](int i) {
-            if (i < L * L) return make_int2(-range + (i % L) * 8, -range + (i / L) * 8);
-            const int j = i - L * L;
-            const int d = -range + (j >> 1) * 8;
-            return (j & 1) ? make_int2(d, range) : make_int2(range, d);
-        });
-    }
-    // uneven cross (:1875-1884)
-    {
-        const int cs = range >= 96 ? 8 : (range >= 32 ? 4 : 2);
-        const int cx = key_dx(top[0]), cy = key_dy(top[0]);
-        const int vlimit = imin(range, imax(8, range / 2));
-        const int nh = range / cs, nv = vlimit / cs;
-        umh_stage(P, m, 2 * nh + 2 * nv, range, [&](int i) {
-            if (i < 2 * nh) {
-                const int d = cs * (i / 2 + 1);
-                return (i & 1) ? make_int2(cx + d, cy) : make_int2(cx - d, cy);
+// The search after the wavefront wait: seeds in seeds[0..ns), the lattice's four least in
+// top[0..3] (range >= 8). The result's key.
+__device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint32_t top_off, int ns, int range, int pixels) {
+    const SearchGeo g(ctx);
+    const int lane = threadIdx.x & 31;
+    const int2* seeds = reinterpret_cast<const int2*>(g_smem + seeds_off);
+    Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
+    const int cs = range >= 96 ? 8 : (range >= 32 ? 4 : 2);
+    const int nh = range / cs, nv = imin(range, imax(8, range / 2)) / cs;
+    const int hs = range >= 96 ? 8 : (range >= 24 ? 4 : 2);
+    enum { kSeeds, kSquare, kCross, kRings, kHexagon, kDiamond, kDone };
+    int stage = kSeeds, iter = 0;
+#pragma unroll 1
+    while (stage != kDone) {
+        // the stage's centre is the least candidate before it
+        const int cx = key_dx(t.a), cy = key_dy(t.a);
+        const int n = stage == kSeeds ? ns : stage == kSquare ? 25 : stage == kCross ? 2 * (nh + nv)
+                    : stage == kRings ? 6 * (range / hs) : stage == kHexagon ? 6 : 4;
+#pragma unroll 1
+        for (int base = 0; base < n;) {
+            const int rem = n - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : 2);
+            const int i = base + (lane >> sh);
+            int dx = cx, dy = cy;
+            if (stage == kSeeds) {  // predictor, zero, global, then A and C where they exist (:1843-1850)
+                const int2 v = seeds[imin(i, ns - 1)];
+                dx = v.x;
+                dy = v.y;
+            } else if (stage == kSquare) {  // 5x5 around the best (:1855-1859)
+                dx += i % 5 - 2;
+                dy += i / 5 - 2;
+            } else if (stage == kCross) {  // uneven cross (:1875-1884)
+                const int j = i < 2 * nh ? i : i - 2 * nh, d = cs * (j / 2 + 1);
+                if (i < 2 * nh) dx += (j & 1) ? d : -d;
+                else dy += (j & 1) ? d : -d;
+            } else if (stage == kRings) {  // multi-hexagon rings (:1889-1897)
+                const int r = hs * (i / 6 + 1), h = (r + 1) / 2, q = i % 6;
+                dx += q < 2 ? (q ? r : -r) : ((q & 1) ? h : -h);
+                dy += q < 2 ? 0 : (q < 4 ? -r : r);
+            } else if (stage == kHexagon) {  // small hexagon, repeated (:1902-1908)
+                dx += i < 2 ? (i ? 2 : -2) : ((i & 1) ? 1 : -1);
+                dy += i < 2 ? 0 : (i < 4 ? -2 : 2);
+            } else {  // closing diamond (:1909-1913)
+                dx += i < 2 ? (i ? 1 : -1) : 0;
+                dy += i < 2 ? 0 : (i == 3 ? 1 : -1);
             }
-            const int j = i - 2 * nh;
-            const int d = cs * (j / 2 + 1);
-            return (j & 1) ? make_int2(cx, cy + d) : make_int2(cx, cy - d);
-        });
+            dx = iclamp(dx, -range, range);
+            dy = iclamp(dy, -range, range);
+            top4_merge(t, shared_key<2>(ctx, g, i < n, dx, dy, sh));
+            base += 32 >> sh;
+        }
+        if (stage == kSquare && range >= 8) {
+            const uint64_t* top = reinterpret_cast<const uint64_t*>(g_smem + top_off);
+            const uint64_t l0 = top[0], l1 = top[1], l2 = top[2], l3 = top[3];
+            top4_insert(t, l0);
+            top4_insert(t, l1);
+            top4_insert(t, l2);
+            top4_insert(t, l3);
+        }
+        if (stage != kHexagon || ++iter == 32 || (key_dx(t.a) == cx && key_dy(t.a) == cy)) ++stage;
     }
-    // multi-hexagon rings (:1889-1897)
-    {
-        const int hs = range >= 96 ? 8 : (range >= 24 ? 4 : 2);
-        const int hx = key_dx(top[0]), hy = key_dy(top[0]);
-        const int nr = range / hs;
-        umh_stage(P, m, 6 * nr, range, [&](int i) {
-            const int r = hs * (i / 6 + 1), h = (r + 1) / 2;
-            switch (i % 6) {
-                case 0: return make_int2(hx - r, hy);
-                case 1: return make_int2(hx + r, hy);
-                case 2: return make_int2(hx - h, hy - r);
-                case 3: return make_int2(hx + h, hy - r);
-                case 4: return make_int2(hx - h, hy + r);
-                default: return make_int2(hx + h, hy + r);
-            }
-        });
+    // full-resolution 3x3 about the four finalists (:1929-1952)
+    uint64_t fk = UINT64_MAX;
+    const int nf = 9 * ((t.a != UINT64_MAX) + (t.b != UINT64_MAX) + (t.c != UINT64_MAX) + (t.d != UINT64_MAX));
+#pragma unroll 1
+    for (int base = 0; base < nf;) {
+        const int rem = nf - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : (rem > 4 ? 2 : 3));
+        const int i = base + (lane >> sh), f = i / 9, q = i % 9;
+        const uint64_t c = f == 0 ? t.a : (f == 1 ? t.b : (f == 2 ? t.c : t.d));
+        const uint64_t k = shared_key<1>(ctx, g, i < nf, iclamp(key_dx(c) + q % 3 - 1, -range, range),
+                                         iclamp(key_dy(c) + q / 3 - 1, -range, range), sh);
+        fk = k < fk ? k : fk;
+        base += 32 >> sh;
     }
-    // iterative small hexagon (:1902-1908)
-    for (int iter = 0; iter < 32; ++iter) {
-        const uint64_t before = top[0];
-        const int ox = key_dx(before), oy = key_dy(before);
-        umh_stage(P, m, 6, range, [&](int i) {
-            // (-2,0) (2,0) (-1,-2) (1,-2) (-1,2) (1,2)
-            return i < 2 ? make_int2(ox + (i ? 2 : -2), oy) : make_int2(ox + ((i & 1) ? 1 : -1), oy + (i < 4 ? -2 : 2));
-        });
-        if (key_dx(top[0]) == ox && key_dy(top[0]) == oy) break;
-    }
-    // closing diamond (:1909-1913)
-    {
-        const int ox = key_dx(top[0]), oy = key_dy(top[0]);
-        umh_stage(P, m, 4, range, [&](int i) {
-            // (-1,0) (1,0) (0,-1) (0,1)
-            return i < 2 ? make_int2(ox + (i ? 1 : -1), oy) : make_int2(ox, oy + (i == 3 ? 1 : -1));
-        });
-    }
-    // full-resolution finalists (:1929-1952)
-    const int nf = imin(4, m.sm.misc[0]);
-    uint64_t fk = full_stage(P, m, nf * 9, range, 1, true, [&](int i, bool& ok) {
-        ok = true;
-        const uint64_t t = top[i / 9];
-        return make_int2(iclamp(key_dx(t) + (i % 9) % 3 - 1, -range, range),
-                         iclamp(key_dy(t) + (i % 9) / 3 - 1, -range, range));
-    });
-    IntRes full{key_dx(fk), key_dy(fk), key_cost(fk)};
-    if (fk == UINT64_MAX) {  // unreachable in practice (:1948-1951)
-        full.dx = key_dx(top[0]);
-        full.dy = key_dy(top[0]);
-        full.cost = mb_sad(P, m, full.dx, full.dy, 1);
-        fk = int_key(full.cost, full.dx, full.dy);
-    }
+    fk = warp_min_key(fk);
     // bounded rescue on a poor match (:1958-2020)
-    if (range > 0 && !match_good(P, full.cost, pixels)) {
+    const uint64_t px = (uint64_t)pixels;
+    auto good = [&](uint64_t cost) { return px && cost < UINT64_MAX / 8 && cost <= px * 6u; };
+    if (range > 0 && !good(key_cost(fk))) {
         const int step = range >= 8 ? 4 : (range >= 3 ? 2 : 1);
         const int L = (2 * range) / step + 1;
-        const uint64_t ck = full_stage(P, m, L * L + 2 * L, range, 4, false, [&](int i, bool& ok) {
-            ok = true;
-            if (i < L * L) return make_int2(-range + (i % L) * step, -range + (i / L) * step);
-            const int j = i - L * L;
-            const int d = -range + (j >> 1) * step;
-            return (j & 1) ? make_int2(d, range) : make_int2(range, d);
-        });
-        const int cdx = key_dx(ck), cdy = key_dy(ck);
+        const uint64_t ck = box_min(ctx, -range, -range, L, L, step, 4, range, (2 * range) % step != 0);
         const int rr = imax(1, step - 1);
-        const int ylo = imax(-range, cdy - rr), yhi = imin(range, cdy + rr);
-        const int xlo = imax(-range, cdx - rr), xhi = imin(range, cdx + rr);
-        const int nx = xhi - xlo + 1, ny = yhi - ylo + 1;
-        const uint64_t rk = full_stage(P, m, nx * ny, range, 1, true, [&](int i, bool& ok) {
-            ok = true;
-            return make_int2(xlo + i % nx, ylo + i / nx);
-        });
-        if (rk < fk) fk = rk;
-        full = IntRes{key_dx(fk), key_dy(fk), key_cost(fk)};
-        if (pixels && full.cost > pixels * 24u && range <= 32) {
-            const int Ld = range + 1;  // -range..range step 2
-            const uint64_t dk = full_stage(P, m, Ld * Ld, range, 2, false, [&](int i, bool& ok) {
-                ok = true;
-                return make_int2(-range + (i % Ld) * 2, -range + (i / Ld) * 2);
-            });
-            const int ddx = key_dx(dk), ddy = key_dy(dk);
-            const int y0 = imax(-range, ddy - 2), y1 = imin(range, ddy + 2);
-            const int x0 = imax(-range, ddx - 2), x1 = imin(range, ddx + 2);
-            const int mx = x1 - x0 + 1, my = y1 - y0 + 1;
-            const uint64_t dfk = full_stage(P, m, mx * my, range, 1, true, [&](int i, bool& ok) {
-                ok = true;
-                return make_int2(x0 + i % mx, y0 + i / mx);
-            });
-            if (dfk < fk) fk = dfk;
-            full = IntRes{key_dx(fk), key_dy(fk), key_cost(fk)};
-        }
+        auto around = [&](uint64_t k, int r) {
+            const int xlo = imax(-range, key_dx(k) - r), xhi = imin(range, key_dx(k) + r);
+            const int ylo = imax(-range, key_dy(k) - r), yhi = imin(range, key_dy(k) + r);
+            const uint64_t m = box_min(ctx, xlo, ylo, xhi - xlo + 1, yhi - ylo + 1, 1, 1, range, false);
+            if (m < fk) fk = m;
+        };
+        around(ck, rr);
+        if (px && key_cost(fk) > px * 24u && range <= 32)
+            around(box_min(ctx, -range, -range, range + 1, range + 1, 2, 2, range, false), 2);
     }
-    return full;
+    return fk;
+}
+
+__device__ IntRes umh(const DevParams& P, const Mb& m, const PInfo& pi, int gdx, int gdy, int range, uint64_t pixels) {
+    const int ns = 3 + (pi.a_valid ? 1 : 0) + (pi.c_valid ? 1 : 0);
+    if (m.lane < ns) {
+        const int2 v = m.lane == 0 ? pi.pre : ((m.lane == 3 && pi.a_valid) ? pi.a : pi.c);
+        m.sm.batch[m.lane] = m.lane == 1 ? make_int2(0, 0) : m.lane == 2 ? make_int2(gdx, gdy)
+                                         : make_int2(round_qpel_to_pixel(v.x), round_qpel_to_pixel(v.y));
+    }
+    __syncwarp();
+    const uint64_t fk = umh_core(m.sm.ctx.off, soff(m.sm.batch), soff(m.sm.top), ns, range, (int)pixels);
+    return IntRes{key_dx(fk), key_dy(fk), key_cost(fk)};
 }
 
 // integer_motion_diamond, encoder_motion_diamond.cpp:13-73
@@ -1327,92 +1447,74 @@ __device__ __forceinline__ int make_even(int v) { return !(v & 1) ? v : (v > 0 ?
 
 // ---- the refinement's candidate list, held across the warp's lanes -------------------------
 //
-// Lane j < n holds list entry j (vector, CPU-law SAD). Entries are distinct vectors; their
-// order is immaterial because every selection over them uses a total order, so membership
-// tests, minima and ranks are warp votes and shuffles instead of serial scans.
+// Lane j < n holds list entry j as one key: (SAD, |x| + |y|, y, x), the reference's (sad, tie_less)
+// order, with the vector recoverable from it. Entries are distinct vectors; their order is
+// immaterial because every selection over them uses a total order, so membership tests are warp
+// votes and minima two 32-bit warp reductions. A SAD is below 2^16 or kBad (the largest code);
+// components lie within +-4096 and +-1024.
+constexpr uint32_t kSadBadCode = 0x1FFFF;
+
+__device__ __forceinline__ uint32_t mv_id(int2 v) { return ((uint32_t)(v.y + 2048) << 14) | (uint32_t)(v.x + 8192); }
+__device__ __forceinline__ int2 id_mv(uint32_t id) { return make_int2((int)(id & 0x3FFF) - 8192, (int)((id >> 14) & 0xFFF) - 2048); }
+__device__ __forceinline__ uint64_t sad_key(uint64_t sad, int2 v) {
+    const uint64_t c = sad >= kBad ? kSadBadCode : (uint32_t)sad;
+    return (c << 40) | ((uint64_t)(iabs(v.x) + iabs(v.y)) << 26) | mv_id(v);
+}
+__device__ __forceinline__ uint64_t key_sad(uint64_t k) {
+    const uint32_t c = (uint32_t)(k >> 40);
+    return c == kSadBadCode ? kBad : c;
+}
+__device__ __forceinline__ int2 sad_key_mv(uint64_t k) { return id_mv((uint32_t)k & 0x3FFFFFFu); }
+
 struct RegList {
-    int n;  // warp-uniform entry count (<= 32)
-    int2 mv;
-    uint64_t sad;
+    int n;         // warp-uniform entry count (<= 32)
+    uint64_t key;  // this lane's entry (UINT64_MAX: none)
 };
 
-__device__ __forceinline__ bool sad_tie_less(uint64_t sa, int2 a, uint64_t sb, int2 b) {
-    if (sa != sb) return sa < sb;
-    return tie_less(a, b);
-}
-
-// Minimum over the lanes with `valid` of (s, v) under (sad, tie_less); the result on every lane.
-__device__ __forceinline__ void warp_argmin_sad(bool& valid, uint64_t& s, int2& v) {
-#pragma unroll 1
-    for (int o = 16; o; o >>= 1) {
-        const bool ov = __shfl_xor_sync(FULL, valid, o);
-        const uint64_t os = __shfl_xor_sync(FULL, s, o);
-        const int ox = __shfl_xor_sync(FULL, v.x, o), oy = __shfl_xor_sync(FULL, v.y, o);
-        if (ov && (!valid || sad_tie_less(os, make_int2(ox, oy), s, v))) {
-            valid = true;
-            s = os;
-            v = make_int2(ox, oy);
-        }
-    }
-}
-
 // Adds the candidates that lanes i < nb hold in `c` and the list lacks, in lane order, and
-// scores the new ones with the CPU law in one batch (the `add` lambda, :3324-3337).
-__device__ __forceinline__ void reg_add(const DevParams& P, const Mb& m, RegList& L, int2 c, int nb, int bx, int by,
+// scores the new ones with the CPU law in one batch (the `add` lambda, :3324-3337). Returns whether
+// this lane's entry is one of the nb candidates.
+__device__ __forceinline__ bool reg_add(const DevParams& P, const Mb& m, RegList& L, int2 c, int nb, int bx, int by,
                                         int bw, int bh, int mode) {
     const bool act = m.lane < nb;
-    bool listed = false;
-#pragma unroll 1
+    const uint32_t id = mv_id(c), own = m.lane < L.n ? (uint32_t)L.key & 0x3FFFFFFu : 0xffffffffu;
+    bool listed = false, among = false;
+#pragma unroll 3
     for (int i = 0; i < nb; ++i) {
-        const int cx = __shfl_sync(FULL, c.x, i), cy = __shfl_sync(FULL, c.y, i);
-        const bool hit = __any_sync(FULL, m.lane < L.n && L.mv.x == cx && L.mv.y == cy);
+        const bool same = own == __shfl_sync(FULL, id, i);
+        const bool hit = __any_sync(FULL, same);
+        among |= same;
         if (m.lane == i) listed = hit;
     }
+    const unsigned amask = (nb >= 32) ? FULL : ((1u << nb) - 1);
     bool first = false;
-    const unsigned amask = __ballot_sync(FULL, act);
-    if (act) {
-        const unsigned long long key = ((unsigned long long)(uint32_t)c.x << 32) | (uint32_t)c.y;
-        first = (__ffs(__match_any_sync(amask, key)) - 1) == m.lane;
-    }
+    if (act) first = (__ffs(__match_any_sync(amask, id)) - 1) == m.lane;
     const bool fresh = act && !listed && first;
     const unsigned fm = __ballot_sync(FULL, fresh);
     const int nn = __popc(fm);
-    if (!nn) return;
+    if (!nn) return among;
     if (fresh) m.sm.batch[__popc(fm & ((1u << m.lane) - 1))] = c;
     __syncwarp();
     sad_batch(P, m, m.sm.batch, nn, bx, by, bw, bh, mode, m.sm.batch_cost);  // hidden padding costs BAD
     if (m.lane >= L.n && m.lane < L.n + nn) {
-        L.mv = m.sm.batch[m.lane - L.n];
-        L.sad = m.sm.batch_cost[m.lane - L.n];
+        L.key = sad_key(m.sm.batch_cost[m.lane - L.n], m.sm.batch[m.lane - L.n]);
+        among = true;
     }
     L.n += nn;
     __syncwarp();
+    return among;
 }
 
-// The entry equal to the stencil vectors of lanes i < nb with the least (sad, tie_less),
-// folded into (best, best_sad) by the same order (every stencil vector is in the list).
-__device__ __forceinline__ void reg_update_min(const Mb& m, const RegList& L, int2 c, int nb, int2& best,
-                                               uint64_t& best_sad) {
-    bool in_st = false;
-#pragma unroll 1
-    for (int i = 0; i < nb; ++i) {
-        const int cx = __shfl_sync(FULL, c.x, i), cy = __shfl_sync(FULL, c.y, i);
-        in_st |= m.lane < L.n && L.mv.x == cx && L.mv.y == cy;
-    }
-    bool valid = in_st;
-    uint64_t s = L.sad;
-    int2 v = L.mv;
-    warp_argmin_sad(valid, s, v);
-    if (valid && sad_tie_less(s, v, best_sad, best)) {
-        best = v;
-        best_sad = s;
-    }
+// The least entry among the lanes with `in`, folded into `best` by the same order.
+__device__ __forceinline__ void reg_update_min(const RegList& L, bool in, uint64_t& best) {
+    const uint64_t k = warp_min_key(in ? L.key : UINT64_MAX);
+    if (k < best) best = k;
 }
 
-// SAD of the listed vector v (warp-uniform; it must be listed).
+// Key of the listed vector v (warp-uniform; it must be listed).
 __device__ __forceinline__ uint64_t reg_find(const RegList& L, int lane, int2 v) {
-    const unsigned hit = __ballot_sync(FULL, lane < L.n && L.mv.x == v.x && L.mv.y == v.y);
-    return __shfl_sync(FULL, L.sad, __ffs(hit) - 1);
+    const unsigned hit = __ballot_sync(FULL, lane < L.n && ((uint32_t)L.key & 0x3FFFFFFu) == mv_id(v));
+    return __shfl_sync(FULL, L.key, __ffs(hit) - 1);
 }
 
 // refine_motion_integer_only, encoder_motion.cpp:3247-3269
@@ -1456,16 +1558,15 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
         seed = make_int2(0, 0);
         known = UINT64_MAX;
     }
-    RegList L{0, make_int2(0, 0), 0};
+    RegList L{0, UINT64_MAX};
     if (known != UINT64_MAX) {
         L.n = 1;
-        L.mv = seed;
-        L.sad = known;
+        if (m.lane == 0) L.key = sad_key(known, seed);
     } else {
         reg_add(P, m, L, seed, 1, bx, by, bw, bh, emode);
     }
+    uint64_t best_key = __shfl_sync(FULL, L.key, 0);
     int2 best = seed;
-    uint64_t cost = __shfl_sync(FULL, L.sad, 0);
     auto fix = [&](int2 v) {
         v.x = iclamp(v.x, xmin, xmax);
         v.y = iclamp(v.y, ymin, ymax);
@@ -1475,8 +1576,8 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
     // one stencil stage: gen(i) for i < np, clamped, scored and folded into (cost, best)
     auto stage = [&](int np, auto gen) {
         const int2 c = m.lane < np ? fix(gen(m.lane)) : make_int2(0, 0);
-        reg_add(P, m, L, c, np, bx, by, bw, bh, emode);
-        reg_update_min(m, L, c, np, best, cost);
+        reg_update_min(L, reg_add(P, m, L, c, np, bx, by, bw, bh, emode), best_key);
+        best = sad_key_mv(best_key);
     };
     // the two candidates beside an axis move: (c.x, c.y -/+ d) or (c.x -/+ d, c.y)
     auto side = [](int2 c, int d, bool vertical) {
@@ -1489,7 +1590,7 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
         };
     };
     if (P.fast_subpel) {
-        if (cost == 0 && best.x == 0 && best.y == 0) return RefineOut{best, 0};
+        if (key_sad(best_key) == 0 && best.x == 0 && best.y == 0) return RefineOut{best, 0};
         stage(4, cross(seed, 2));
         const int2 axis = best;
         const int dx = axis.x - seed.x, dy = axis.y - seed.y;
@@ -1511,7 +1612,7 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
             stage(9, [=](int i) { return make_int2(half.x + i % 3 - 1, half.y + i / 3 - 1); });
         }
     }
-    return RefineOut{best, cost};
+    return RefineOut{best, key_sad(best_key)};
 }
 
 // The SAD shortlist of one staged refinement, kept in the warp's shared memory between the
@@ -1551,17 +1652,18 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
     seed.x = iclamp(seed.x, xmin, xmax);
     seed.y = iclamp(seed.y, ymin, ymax);
     if (hp) { seed.x = make_even(seed.x); seed.y = make_even(seed.y); }
-    RegList L{0, seed, 0};
+    RegList L{0, UINT64_MAX};
+    const bool seed_hidden = hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, mode, cg);
     // add(seed, known)
     if (known != UINT64_MAX) {
         L.n = 1;
-        L.sad = hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, mode, cg) ? kBad : known;
+        if (m.lane == 0) L.key = sad_key(seed_hidden ? kBad : known, seed);
     } else {
         reg_add(P, m, L, seed, 1, bx, by, bw, bh, mode);
     }
-    if (hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, mode, cg)) reg_add(P, m, L, make_int2(0, 0), 1, bx, by, bw, bh, mode);
+    if (seed_hidden) reg_add(P, m, L, make_int2(0, 0), 1, bx, by, bw, bh, mode);
+    uint64_t half_key = __shfl_sync(FULL, L.key, 0);
     int2 half_best = seed;
-    uint64_t half_sad = __shfl_sync(FULL, L.sad, 0);
     const bool fast = P.fast_subpel;
     auto clampmv = [&](int x, int y) {
         int2 v = make_int2(iclamp(x, xmin, xmax), iclamp(y, ymin, ymax));
@@ -1574,8 +1676,8 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
         const int2 c = fast ? (i == 0 ? seed : i == 1 ? clampmv(seed.x - 2, seed.y) : i == 2 ? clampmv(seed.x + 2, seed.y)
                                              : i == 3 ? clampmv(seed.x, seed.y - 2) : clampmv(seed.x, seed.y + 2))
                             : clampmv(seed.x + (i % 3 - 1) * 2, seed.y + (i / 3 - 1) * 2);
-        reg_add(P, m, L, c, nb, bx, by, bw, bh, mode);
-        reg_update_min(m, L, c, nb, half_best, half_sad);
+        reg_update_min(L, reg_add(P, m, L, c, nb, bx, by, bw, bh, mode), half_key);
+        half_best = sad_key_mv(half_key);
     }
     if (fast && !(half_best.x == seed.x && half_best.y == seed.y)) {
         const int dx = half_best.x - seed.x, dy = half_best.y - seed.y;
@@ -1591,8 +1693,8 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
         }
         if (hp) { c.x = make_even(c.x); c.y = make_even(c.y); }
         if (nd) {
-            reg_add(P, m, L, c, nd, bx, by, bw, bh, mode);
-            reg_update_min(m, L, c, nd, half_best, half_sad);
+            reg_update_min(L, reg_add(P, m, L, c, nd, bx, by, bw, bh, mode), half_key);
+            half_best = sad_key_mv(half_key);
         }
     }
     if (!hp) {
@@ -1602,10 +1704,10 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
                          : i == 2 ? make_int2(iclamp(qc.x + 1, xmin, xmax), qc.y)
                          : i == 3 ? make_int2(qc.x, iclamp(qc.y - 1, ymin, ymax))
                                   : make_int2(qc.x, iclamp(qc.y + 1, ymin, ymax));
-            reg_add(P, m, L, c, 5, bx, by, bw, bh, mode);
-            uint64_t qcost = reg_find(L, m.lane, qc);
-            int2 qbmv = qc;
-            reg_update_min(m, L, c, 5, qbmv, qcost);
+            const bool in = reg_add(P, m, L, c, 5, bx, by, bw, bh, mode);
+            uint64_t qkey = reg_find(L, m.lane, qc);
+            reg_update_min(L, in, qkey);
+            const int2 qbmv = sad_key_mv(qkey);
             const int dx = qbmv.x - qc.x, dy = qbmv.y - qc.y;
             if (dx && !dy) {
                 reg_add(P, m, L, make_int2(qbmv.x, iclamp(qc.y + (i ? 1 : -1), ymin, ymax)), 2, bx, by, bw, bh, mode);
@@ -1618,20 +1720,20 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
                     bx, by, bw, bh, mode);
         }
     }
-    // sort by (sad, tie_less), keep 8 / 4 (:3445-3456): rank of each entry by shuffles
+    // sort by (sad, tie_less), keep 8 / 4 (:3445-3456): each entry ranks itself among all, read
+    // from shared memory (broadcast loads)
     const int keep = fast ? 4 : 8;
+    m.sm.batch_cost[m.lane] = L.key;
+    __syncwarp();
     int rank = 0;
-#pragma unroll 1
-    for (int k = 0; k < L.n; ++k) {
-        const uint64_t sk = __shfl_sync(FULL, L.sad, k);
-        const int kx = __shfl_sync(FULL, L.mv.x, k), ky = __shfl_sync(FULL, L.mv.y, k);
-        rank += sad_tie_less(sk, make_int2(kx, ky), L.sad, L.mv) ? 1 : 0;
-    }
-    const uint64_t screen = warp_min_u64(m.lane < L.n ? L.sad : UINT64_MAX);
+#pragma unroll 4
+    for (int k = 0; k < L.n; ++k) rank += m.sm.batch_cost[k] < L.key ? 1 : 0;
+    const uint64_t screen = key_sad(warp_min_key(L.key));
     const int nk = imin(L.n, keep);
+    __syncwarp();
     if (m.lane < L.n && rank < nk) {
-        m.sm.batch[rank] = L.mv;
-        m.sm.batch_cost[rank] = L.sad;
+        m.sm.batch[rank] = sad_key_mv(L.key);
+        m.sm.batch_cost[rank] = key_sad(L.key);
     }
     __syncwarp();
     sl.direct = 0;
@@ -1647,63 +1749,17 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
     return sl;
 }
 
-// 128-bit value exchanged with the lane `o` positions away (xor).
-__device__ __forceinline__ unsigned __int128 shfl_xor_u128(unsigned __int128 x, int o) {
-    const uint64_t lo = __shfl_xor_sync(FULL, (uint64_t)x, o), hi = __shfl_xor_sync(FULL, (uint64_t)(x >> 64), o);
-    return ((unsigned __int128)hi << 64) | lo;
-}
-
-// One shortlisted candidate in a lane's registers during the final selection.
-struct SelCand {
-    bool valid, elig;
-    unsigned __int128 key;
-    uint64_t satd, sad;
-    int2 mv;
-};
-
-__device__ __forceinline__ SelCand shfl_xor_cand(const SelCand& c, int o) {
-    SelCand r;
-    r.valid = __shfl_xor_sync(FULL, c.valid, o);
-    r.elig = __shfl_xor_sync(FULL, c.elig, o);
-    r.key = shfl_xor_u128(c.key, o);
-    r.satd = __shfl_xor_sync(FULL, c.satd, o);
-    r.sad = __shfl_xor_sync(FULL, c.sad, o);
-    r.mv = make_int2(__shfl_xor_sync(FULL, c.mv.x, o), __shfl_xor_sync(FULL, c.mv.y, o));
-    return r;
-}
-
-// Rate winner order (:3477-3488): (score, sad, tie_less).
-__device__ __forceinline__ bool rate_less(const SelCand& a, const SelCand& b) {
-    if (a.valid != b.valid) return a.valid;
-    if (a.key != b.key) return a.key < b.key;
-    return sad_tie_less(a.sad, a.mv, b.sad, b.mv);
-}
-
-// Final order (:3526-3531): eligible first, then (score, satd, sad, tie_less).
-__device__ __forceinline__ bool final_less(const SelCand& a, const SelCand& b) {
-    if (a.valid != b.valid) return a.valid;
-    if (a.elig != b.elig) return a.elig;
-    if (a.key != b.key) return a.key < b.key;
-    if (a.satd != b.satd) return a.satd < b.satd;
-    return sad_tie_less(a.sad, a.mv, b.sad, b.mv);
-}
-
-// Least candidate of lanes 0..7 under `less`, on every lane.
-template <class Less>
-__device__ __forceinline__ SelCand warp_min8(SelCand c, Less less) {
-#pragma unroll 1
-    for (int o = 4; o; o >>= 1) {
-        const SelCand d = shfl_xor_cand(c, o);
-        if (less(d, c)) c = d;
+// The lane of the least (key, order) among the lanes with `in` (at least one): warp minima of the
+// key's four words and the order's two, most significant first, each over the lanes still tied.
+__device__ __forceinline__ int warp_argmin(bool in, unsigned __int128 key, uint64_t order) {
+    const uint32_t w[6] = {(uint32_t)(key >> 96), (uint32_t)(key >> 64), (uint32_t)(key >> 32), (uint32_t)key,
+                           (uint32_t)(order >> 32), (uint32_t)order};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const uint32_t least = __reduce_min_sync(FULL, in ? w[i] : 0xffffffffu);
+        in = in && w[i] == least;
     }
-    SelCand r;
-    r.valid = __shfl_sync(FULL, c.valid, 0);
-    r.elig = __shfl_sync(FULL, c.elig, 0);
-    r.key = ((unsigned __int128)__shfl_sync(FULL, (uint64_t)(c.key >> 64), 0) << 64) | __shfl_sync(FULL, (uint64_t)c.key, 0);
-    r.satd = __shfl_sync(FULL, c.satd, 0);
-    r.sad = __shfl_sync(FULL, c.sad, 0);
-    r.mv = make_int2(__shfl_sync(FULL, c.mv.x, 0), __shfl_sync(FULL, c.mv.y, 0));
-    return r;
+    return __ffs(__ballot_sync(FULL, in)) - 1;
 }
 
 // The rest of refine_motion_block_staged (encoder_motion.cpp:3458-3535) given the predictor.
@@ -1712,50 +1768,58 @@ __device__ RefineOut refine_select(const DevParams& P, const Mb& m, const Shortl
                                    int mode, const PInfo& pi, bool more) {
     if (sl.direct) return sl.out;
     const int nk = sl.nk;  // <= 8
-    SelCand c;
-    c.valid = m.lane < nk;
-    c.elig = false;
-    c.mv = c.valid ? m.sm.batch[m.lane] : make_int2(0, 0);
-    c.sad = c.valid ? m.sm.batch_cost[m.lane] : UINT64_MAX;
-    c.satd = kBad;
+    const bool valid = m.lane < nk;
+    const int2 mv = valid ? m.sm.batch[m.lane] : make_int2(0, 0);
+    const uint64_t sad = valid ? m.sm.batch_cost[m.lane] : UINT64_MAX;
+    const uint64_t order = valid ? sad_key(sad, mv) : UINT64_MAX;  // (sad, tie_less)
     uint32_t rate = 0;
-    c.key = 0;
-    if (c.valid) {
+    unsigned __int128 key = 0;
+    if (valid) {
         // rate + score (:3458-3476)
         int2 pred = pi.pre;
         if (pi.hybrid) {
-            pred = modular_mv_distance(P, c.mv, pi.a) <= modular_mv_distance(P, c.mv, pi.c) ? pi.a : pi.c;
+            pred = modular_mv_distance(P, mv, pi.a) <= modular_mv_distance(P, mv, pi.c) ? pi.a : pi.c;
             ++rate;
         }
-        rate += mv_rate_bits(P, c.mv, pred, mode, more);
-        c.key = score_key(P, m.lam_m, m.lam_s, c.sad, rate);
+        rate += mv_rate_bits(P, mv, pred, mode, more);
+        key = score_key(P, m.lam_m, m.lam_s, sad, rate);
     }
-    const SelCand rw = warp_min8(c, rate_less);
+    const int rw = warp_argmin(valid, key, order);  // the rate winner (:3477-3488)
     if (P.me_quality == 1) {
         __syncwarp();
-        return RefineOut{rw.mv, sl.screen};
+        return RefineOut{make_int2(__shfl_sync(FULL, mv.x, rw), __shfl_sync(FULL, mv.y, rw)), sl.screen};
     }
-    const uint64_t rws = rw.sad;
+    const uint64_t rws = __shfl_sync(FULL, sad, rw);
     const uint64_t pct3 = (rws / 100) * 3 + (((rws % 100) * 3 + 99) / 100);
     const uint64_t slack = pct3 > 4 ? pct3 : 4;
     const uint64_t limit = rws > UINT64_MAX - slack ? UINT64_MAX : rws + slack;
-    c.elig = c.valid && c.sad < UINT64_MAX / 8 && c.sad <= limit;
+    const bool elig = valid && sad < UINT64_MAX / 8 && sad <= limit;
+    uint64_t satd = kBad;
     // SATD of the eligible shortlist (:3507-3524), unless already known for every entry
+    const unsigned em = __ballot_sync(FULL, elig);
     if (sl.satd_done) {
-        if (c.elig) c.satd = m.sm.list_satd[m.lane];
+        if (elig) satd = m.sm.list_satd[m.lane];
     } else {
-        const unsigned em = __ballot_sync(FULL, c.elig);
         const int pos = __popc(em & ((1u << m.lane) - 1));
         int2* el = m.sm.batch + 16;
-        if (c.elig) el[pos] = c.mv;
+        if (elig) el[pos] = mv;
         __syncwarp();
         satd_batch(P, m, el, __popc(em), bx, by, bw, bh, mode, m.sm.list_satd + 8);
-        if (c.elig) c.satd = m.sm.list_satd[8 + pos];
+        if (elig) satd = m.sm.list_satd[8 + pos];
     }
-    if (c.valid) c.key = score_key(P, m.lam_m, m.lam_s, c.satd, rate);
-    const SelCand best = warp_min8(c, final_less);
+    // the final order (:3526-3531): eligible first, then (score, satd, sad, tie_less); of equal
+    // scores the lesser SATD is found first
+    if (valid) key = score_key(P, m.lam_m, m.lam_s, satd, rate);
+    const bool in = em ? elig : valid;
+    const uint32_t sc = satd >= kBad ? 0xffffffffu : (uint32_t)satd;
+    int best = warp_argmin(in, key, ((uint64_t)sc << 32));
+    // entries that tie in score and SATD: the least (sad, tie_less) of them
+    const uint64_t khi = __shfl_sync(FULL, (uint64_t)(key >> 64), best), klo = __shfl_sync(FULL, (uint64_t)key, best);
+    const uint32_t bsc = __shfl_sync(FULL, sc, best);
+    const bool tied = in && (uint64_t)(key >> 64) == khi && (uint64_t)key == klo && sc == bsc;
+    if (__popc(__ballot_sync(FULL, tied)) > 1) best = warp_argmin(tied, 0, order);
     __syncwarp();
-    return RefineOut{best.mv, sl.screen};
+    return RefineOut{make_int2(__shfl_sync(FULL, mv.x, best), __shfl_sync(FULL, mv.y, best)), sl.screen};
 }
 
 // ---- out-of-line refinement ---------------------------------------------------------------
@@ -1799,6 +1863,9 @@ __device__ void publish_ctx(const DevParams& P, const Mb& m) {
         r.sp_pitch = m.d->sp_pitch;
         r.sp_border = m.d->sp_border;
         r.sp_stride = m.d->sp_stride;
+        const int2 lim = integer_limits(P, m.x0, m.y0);
+        r.xl = lim.x;
+        r.yl = lim.y;
     }
     __syncwarp();
 }
@@ -2186,19 +2253,14 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
         p += (bytes + 15) & ~15u;
         return q;
     };
-    s.list_key.off = take(sizeof(unsigned __int128) * kListCap);
     s.list_sad.off = take(8 * kListCap);
     s.list_satd.off = take(8 * kListCap);
     s.batch_cost.off = take(8 * 32);
-    s.keys.off = take(8 * (uint32_t)wc.keys_cap);
+    s.keys.off = take(8 * 32);
     s.top.off = take(8 * 8);
-    s.list_mv.off = take(8 * kListCap);
     s.batch.off = take(8 * 32);
-    s.stencil.off = take(8 * 16);
-    s.list_rate.off = take(4 * kListCap);
     s.cur2.off = take(4 * 32);
     s.cur4.off = take(4 * 16);
-    s.misc.off = take(4 * 16);
     s.cur_bmv.off = take(8 * 4);
     s.nb_mv.off = take(8 * 4);
     s.nb_bmv.off = take(8 * 16);
@@ -2208,8 +2270,6 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
     s.spec_satd.off = take(8 * 40);
     s.spec_blk.off = take(kSpecBlkBytes * 5);
     s.ctx.off = take(kMbCtxBytes);
-    s.seen.off = take(4 * (uint32_t)wc.seen_words);
-    s.seen_full.off = take(4 * (uint32_t)wc.seen_words);
     s.cur.off = take(256);
     s.tma_bar.off = take(8);
     // the window starts on a 128-byte boundary of the shared address space (a TMA destination)
@@ -2220,10 +2280,8 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
 
 __host__ __device__ inline int warp_bytes_for(const WinCfg& wc) {
     auto r = [](int b) { return (b + 15) & ~15; };
-    return r(16 * kListCap) + r(8 * kListCap) * 2 + r(8 * 32) + r(8 * wc.keys_cap) + r(64) + r(8 * kListCap) +
-           r(8 * 32) + r(128) + r(4 * kListCap) + r(128) + r(64) + r(64) + r(32) + r(32) + r(128) + r(16) +
-           3 * r(8 * 40) + r(kSpecBlkBytes * 5) + r(kMbCtxBytes) +
-           2 * r(4 * wc.seen_words) + r(256) + r(8) + 128 +
+    return r(8 * kListCap) * 2 + r(8 * 32) + r(8 * 32) + r(64) + r(8 * 32) + r(128) + r(64) + r(32) + r(32) +
+           r(128) + r(16) + 3 * r(8 * 40) + r(kSpecBlkBytes * 5) + r(kMbCtxBytes) + r(256) + r(8) + 128 +
            r(wc.wp * wc.wh + 32);
 }
 
@@ -2413,9 +2471,6 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
     m.lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     carve(m.sm, (uint32_t)(warp * wc.warp_bytes), wc);
-#ifdef VC1CU_INDEX_CHECK
-    m.keys_cap = wc.keys_cap;
-#endif
     m.tma_phase = 0;
     m.tma_pending = false;
     if (wc.tma && m.lane == 0) tma_bar_init(sh_addr(m.sm.tma_bar.get()));
@@ -2565,6 +2620,11 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 load_window(P, m, d.ref, 0, 0, wc);
                 publish_ctx(P, m);
                 PHASE_MARK(2);
+                if ((kUmhOnly || P.me_algorithm != 1) && local_range >= 8) {
+                    window_wait(m, st, code, P.wait_log2);
+                    umh_lattice(m.sm.ctx.off, m.sm.top.off, local_range);
+                }
+                PHASE_MARK(3);
             }
             if (allow_intra) intra_sad = intra_proxy(P, m);
             PHASE_MARK(4);
@@ -2923,7 +2983,7 @@ __global__ void subpel_plane_kernel(const uint8_t* ref, int pitch, int W, int H,
     }
     uint8_t* o = out + (long long)py * opitch + px;
 #pragma unroll
-    for (int ph = 1; ph < 16; ++ph) {
+    for (int ph = 0; ph < 16; ++ph) {
         if (!((phase_mask >> ph) & 1)) continue;
         int v[1];
         predict_row<1>(n, BILINEAR, rnd, ph & 3, ph >> 2, x, y, v);

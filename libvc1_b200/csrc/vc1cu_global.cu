@@ -15,8 +15,8 @@
 // other; its refinement keeps the first-visited least cost, a minimum over (cost, |d|, slot) with
 // the visit order as the slot index. The extended search's list (least cost per vector, sorted
 // only on insertion) does depend on the order and is replayed by one warp, entry per lane.
-// Folding on one thread, with the lists in global memory, took 117 us per stage at range 31
-// (0.46-0.94 ms of a call); this form takes about 4 us.
+// Folding on one thread, with the lists in global memory, took 0.87 ms of a CIF search, 2.3 ms of two
+// at 1080p; folded here it is within the scoring launches' time.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -308,8 +308,8 @@ __device__ __forceinline__ uint32_t gpick4(const uint32_t r[4]) {
 // frame_sad of every candidate of every search: grid (slab, candidate slot, search). A thread takes
 // 16-pixel chunks of the sampled rows with packed byte SADs; chunks that the clamped sampling
 // touches, the ragged last one and the strides above 4 go sample by sample.
-// 1080p, range 31 and up, one search: 4 stages 137 us -> 60 us (the byte-per-thread form loaded
-// one sample per load).
+// Two 1080p searches at range 32 (8 launches, the folds included): 277 us, against 363 us for the
+// scoring alone with one sample per load.
 __global__ void __launch_bounds__(kGThreads) gsad_kernel(GState* states, int W, int H, int rows_per_slab, int stage) {
     GState& s = states[blockIdx.z];
     const int ci = blockIdx.y;
