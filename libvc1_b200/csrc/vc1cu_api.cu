@@ -3285,7 +3285,7 @@ static int loop_filter_p(vc1cu_ctx* c, const vc1cu_params* p, int frame_id, cons
                                 reinterpret_cast<const int2*>(d), d + al, d + al + 6 * mbs, d + al + 12 * mbs, c->stream,
                                 main_profile),
            "loop filter launch");
-        tm.stop(2);
+        tm.stop(4);
         // the metadata copies read the caller's pageable arrays; finish before returning
         ck(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
         return VC1CU_OK;

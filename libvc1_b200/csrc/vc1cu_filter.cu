@@ -3,17 +3,20 @@
 // P-picture filter of the coded blocks (apply_p_loop_filter, :610-738).
 //
 // Each edge filter works on groups of four lines across the edge (the third line decides for
-// its group) and only reads and writes along its lines, so the groups of one edge are
-// independent. The reference walks the picture in raster order (per macroblock row, the
-// horizontal edges of MB x before the vertical edges of MB x-1). That order is equivalent to:
-// every horizontal edge first, each 4-column strip walked top to bottom (a strip's edges read
-// rows the edge above it wrote), then every vertical edge, each 4-row strip walked left to right
-// (an inner 4x4 edge reads the column the block's left neighbour's border wrote); strips of one
-// phase touch disjoint pixels. So one thread owns one strip:
-//   lfp_h_kernel  one thread per 4-column strip of a plane: the horizontal edges, top to bottom;
-//   lfp_v_kernel  one thread per 4-row strip: the vertical edges, left to right.
-// The I-like filter has no order between its edges of one direction (8 pixels apart, each reads
-// 4 on either side and writes 1): one thread per 4-line group of every edge.
+// its group); a line reads four samples on either side of the edge and writes the one next to it
+// on each side. The reference walks the picture in raster order (per macroblock row, the
+// horizontal edges of MB x before the vertical edges of MB x-1; per block its border, then its
+// inner edge). That order is equivalent to four independent stages:
+//   1. every horizontal block border (row 8k: reads 8k-4..8k+3, writes 8k-1 and 8k), which never
+//      reads what an inner edge has written by then (its rows 8k-4 and 8k+3 are written by the
+//      inner edges at 8k-4 and 8k+4, both after it) nor what another border writes;
+//   2. every inner horizontal edge (row 8k+4: reads 8k..8k+7, writes 8k+3 and 8k+4), after the
+//      borders above and below it, disjoint from every other inner edge;
+//   3. and 4. the vertical borders and the inner vertical edges, by the same argument.
+// So one thread filters one 4-line group of one edge, one launch per stage, reading the group's
+// eight samples per line as words. The walk of whole strips by one thread each (960 + 540
+// threads at 1080p, every edge behind the one before it) took 3.28 ms per 1080p picture.
+// The I-like filter has only borders: stages 1 and 3.
 //
 // Overlap smoothing (apply_overlap_plane_signed, :217-243) of a signed reconstruction: each
 // edge filter reads and writes the 2 samples on either side along one line, so the lines of
@@ -31,47 +34,87 @@ struct LfPlane {
     int pitch, w, h;
 };
 
-// Vc1Encoder::loop_filter_line (encoder_filter.cpp:366-395): the line across the edge between
-// (x - cross) and (x, y); false when ineligible.
-__device__ bool lf_line(const LfPlane& pl, int x, int y, int cdx, int cdy, int pq) {
-    if (x - 4 * cdx < 0 || y - 4 * cdy < 0 || x + 3 * cdx >= pl.w || y + 3 * cdy >= pl.h || x < 0 || y < 0 ||
-        x >= pl.w || y >= pl.h)
-        return false;
-    const int step = cdy * pl.pitch + cdx;
-    uint8_t* c = pl.p + (size_t)y * pl.pitch + x;
-    auto S = [&](int k) { return (int)c[k * step]; };
-    int a0 = arshift(2 * (S(-2) - S(1)) - 5 * (S(-1) - S(0)) + 4, 3);
+// Vc1Encoder::loop_filter_line (encoder_filter.cpp:366-395) of the eight samples s across the edge
+// (between s[3] and s[4]); false when ineligible.
+__device__ __forceinline__ bool lf_line(int (&s)[8], int pq) {
+    int a0 = arshift(2 * (s[2] - s[5]) - 5 * (s[3] - s[4]) + 4, 3);
     const bool a0_neg = a0 < 0;
     a0 = iabs(a0);
     if (a0 >= pq) return false;
-    const int a1 = iabs(arshift(2 * (S(-4) - S(-1)) - 5 * (S(-3) - S(-2)) + 4, 3));
-    const int a2 = iabs(arshift(2 * (S(0) - S(3)) - 5 * (S(1) - S(2)) + 4, 3));
+    const int a1 = iabs(arshift(2 * (s[0] - s[3]) - 5 * (s[1] - s[2]) + 4, 3));
+    const int a2 = iabs(arshift(2 * (s[4] - s[7]) - 5 * (s[5] - s[6]) + 4, 3));
     if (!(a1 < a0 || a2 < a0)) return false;
-    const int edge = S(-1) - S(0);
+    const int edge = s[3] - s[4];
     const int limit = iabs(edge) >> 1;
     if (!limit) return false;
     int delta = (5 * (a0 - imin(a1, a2))) >> 3;
     if (a0_neg != (edge < 0)) {
         delta = imin(delta, limit);
         if (edge < 0) delta = -delta;
-        c[-step] = (uint8_t)iclamp(S(-1) - delta, 0, 255);
-        c[0] = (uint8_t)iclamp(S(0) + delta, 0, 255);
+        s[3] = iclamp(s[3] - delta, 0, 255);
+        s[4] = iclamp(s[4] + delta, 0, 255);
     }
     return true;
 }
 
-// One 4-line group of loop_filter_edge (:397-416) starting at (x, y) along (adx, ady).
-__device__ void lf_group(const LfPlane& pl, int x, int y, int adx, int ady, int cdx, int cdy, int pq) {
-    if (!lf_line(pl, x + 2 * adx, y + 2 * ady, cdx, cdy, pq)) return;
-    lf_line(pl, x, y, cdx, cdy, pq);
-    lf_line(pl, x + adx, y + ady, cdx, cdy, pq);
-    lf_line(pl, x + 3 * adx, y + 3 * ady, cdx, cdy, pq);
+// The 4-line group of loop_filter_edge (:397-416) of the horizontal edge above row y, columns
+// x..x+3 (x a multiple of 4, so each of its eight rows is one aligned word of the padded pitch).
+__device__ __forceinline__ void lf_hgroup(const LfPlane& pl, int x, int y, int pq) {
+    if (y < 4 || y + 3 >= pl.h || x + 2 >= pl.w) return;  // the third line decides for the group
+    uint8_t* c = pl.p + (size_t)(y - 4) * pl.pitch + x;
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) w[k] = *reinterpret_cast<const uint32_t*>(c + (size_t)k * pl.pitch);
+    uint32_t up = w[3], dn = w[4];
+    auto line = [&](int j) {
+        int s[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] = (int)((w[k] >> (8 * j)) & 255);
+        if (!lf_line(s, pq)) return false;
+        up = (up & ~(255u << (8 * j))) | ((uint32_t)s[3] << (8 * j));
+        dn = (dn & ~(255u << (8 * j))) | ((uint32_t)s[4] << (8 * j));
+        return true;
+    };
+    if (!line(2)) return;
+    line(0);
+    line(1);
+    if (x + 3 < pl.w) line(3);
+    if (up != w[3]) *reinterpret_cast<uint32_t*>(c + 3 * (size_t)pl.pitch) = up;
+    if (dn != w[4]) *reinterpret_cast<uint32_t*>(c + 4 * (size_t)pl.pitch) = dn;
 }
-// the group of a horizontal edge (columns x..x+3, edge above row y) / of a vertical edge
-__device__ __forceinline__ void lf_hgroup(const LfPlane& pl, int x, int y, int pq) { lf_group(pl, x, y, 1, 0, 0, 1, pq); }
-__device__ __forceinline__ void lf_vgroup(const LfPlane& pl, int x, int y, int pq) { lf_group(pl, x, y, 0, 1, 1, 0, pq); }
 
-// The three planes of a frame slot; strip index -> (plane, strip within it).
+// The group of the vertical edge left of column x (a multiple of 4), rows y..y+3.
+__device__ __forceinline__ void lf_vgroup(const LfPlane& pl, int x, int y, int pq) {
+    if (x < 4 || x + 3 >= pl.w || y + 2 >= pl.h) return;
+    uint8_t* c = pl.p + (size_t)y * pl.pitch + x - 4;
+    const int n = imin(4, pl.h - y);
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < n) {
+            lo[j] = *reinterpret_cast<const uint32_t*>(c + (size_t)j * pl.pitch);
+            hi[j] = *reinterpret_cast<const uint32_t*>(c + (size_t)j * pl.pitch + 4);
+        }
+    auto line = [&](int j) {
+        int s[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            s[k] = (int)((lo[j] >> (8 * k)) & 255);
+            s[k + 4] = (int)((hi[j] >> (8 * k)) & 255);
+        }
+        if (!lf_line(s, pq)) return false;
+        uint8_t* q = c + (size_t)j * pl.pitch;
+        q[3] = (uint8_t)s[3];
+        q[4] = (uint8_t)s[4];
+        return true;
+    };
+    if (!line(2)) return;
+    line(0);
+    line(1);
+    if (n > 3) line(3);
+}
+
+// The three planes of a frame slot.
 struct LfFrame {
     LfPlane pl[3];
 };
@@ -97,7 +140,7 @@ __global__ void lfi_v_kernel(LfFrame f, int pq) {
         const LfPlane& pl = f.pl[k];
         const int gy = (pl.h + 3) / 4, ex = (pl.w - 1) / 8;
         if (idx < gy * ex) {
-            lf_vgroup(pl, (idx / gy + 1) * 8, (idx % gy) * 4, pq);
+            lf_vgroup(pl, (idx % ex + 1) * 8, (idx / ex) * 4, pq);
             return;
         }
         idx -= gy * ex;
@@ -165,75 +208,73 @@ __device__ LfBlock lf_block(const LfMeta& m, int k, int bx, int by) {
     return b;
 }
 
-// Horizontal edges of one 4-column strip, top to bottom (process_v_parent, :654-676): each
-// block's bottom border, then its inner 4-row edge.
-__global__ void lfp_h_kernel(LfFrame f, LfMeta m, int pq) {
+// One stage of the P filter: thread = (4-line group along the picture, block across it) of a plane.
+// VERTICAL: the vertical edges (process_h_parent, :677-699) of 4-row groups, else the horizontal
+// edges (process_v_parent, :654-676) of 4-column groups; INNER: the block's inner 4-sample edge,
+// else its border with the next block.
+template <bool VERTICAL, bool INNER>
+__global__ void __launch_bounds__(128) lfp_kernel(LfFrame f, LfMeta m, int pq) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     for (int k = 0; k < 3; ++k) {
         const LfPlane& pl = f.pl[k];
-        const int gx = (pl.w + 3) / 4;
-        if (idx >= gx) {
-            idx -= gx;
+        // groups along the edges; blocks of the macroblock grid across them. Consecutive threads take
+        // consecutive columns, so that a warp's words are neighbours.
+        const int grid_w = k == 0 ? m.mbw * 2 : m.mbw, grid_h = k == 0 ? m.mbh * 2 : m.mbh;
+        const int nx = VERTICAL ? grid_w : (pl.w + 3) / 4, ny = VERTICAL ? (pl.h + 3) / 4 : grid_h;
+        if (idx >= nx * ny) {
+            idx -= nx * ny;
             continue;
         }
-        const int cx = idx * 4, bx = cx >> 3, half = (cx >> 2) & 1;
-        const int grid_h = k == 0 ? m.mbh * 2 : m.mbh;
-        for (int by = 0; by < grid_h; ++by) {
-            const int x0 = bx * 8, y0 = by * 8;
-            if (x0 >= pl.w || y0 >= pl.h) break;
-            const LfBlock b = lf_block(m, k, bx, by);
-            if (by + 1 < grid_h && y0 + 8 < pl.h) {
-                const LfBlock n = lf_block(m, k, bx, by + 1);
+        const int ix = idx % nx, iy = idx / nx;
+        const int bx = VERTICAL ? ix : ix >> 1, by = VERTICAL ? iy >> 1 : iy;
+        const int half = (VERTICAL ? iy : ix) & 1, x0 = bx * 8, y0 = by * 8;
+        if (x0 >= pl.w || y0 >= pl.h) return;
+        if constexpr (!VERTICAL) {
+            const int cx = ix * 4;
+            if constexpr (!INNER) {
+                if (by + 1 >= grid_h || y0 + 8 >= pl.h) return;
+                const LfBlock b = lf_block(m, k, bx, by), n = lf_block(m, k, bx, by + 1);
                 // Main Profile exceptions 1 (block 0 of the first MB intra: every inter MB's top
                 // border filtered whole) and 3 (a 4x4-transformed side: the whole border, :547-553)
                 const bool ex = m.main_profile && (((m.intra[0] & 1) && !n.mb_intra) || b.tt == 7 || n.tt == 7);
+                bool on;
                 if (ex || b.intra || n.intra || b.mv.x != n.mv.x || b.mv.y != n.mv.y) {
-                    if (half * 4 < imin(8, pl.w - x0)) lf_hgroup(pl, cx, y0 + 8, pq);
+                    on = half * 4 < imin(8, pl.w - x0);
                 } else {
                     const int mask = (b.cbp | (n.cbp >> 2)) & 3;
-                    if (half == 0 ? (mask & 2) != 0 : ((mask & 1) && x0 + 4 < pl.w)) lf_hgroup(pl, cx, y0 + 8, pq);
+                    on = half == 0 ? (mask & 2) != 0 : ((mask & 1) && x0 + 4 < pl.w);
                 }
+                if (on) lf_hgroup(pl, cx, y0 + 8, pq);
+            } else {
+                const int mb = (k == 0 ? by >> 1 : by) * m.mbw + (k == 0 ? bx >> 1 : bx);
+                const int bk = mb * 6 + (k == 0 ? (((by & 1) << 1) | (bx & 1)) : 3 + k);
+                const int tt = m.tt[bk], cbp = m.cbp[bk];
+                if ((tt == 7 || tt == 3) && y0 + 4 < pl.h && (half == 0 ? (cbp & 10) != 0 : ((cbp & 5) && x0 + 4 < pl.w)))
+                    lf_hgroup(pl, cx, y0 + 4, pq);
             }
-            if ((b.tt == 7 || b.tt == 3) && y0 + 4 < pl.h) {
-                if (half == 0 ? (b.cbp & 10) != 0 : ((b.cbp & 5) && x0 + 4 < pl.w)) lf_hgroup(pl, cx, y0 + 4, pq);
-            }
-        }
-        return;
-    }
-}
-
-// Vertical edges of one 4-row strip, left to right (process_h_parent, :677-699): each block's
-// right border, then its inner 4-column edge.
-__global__ void lfp_v_kernel(LfFrame f, LfMeta m, int pq) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int k = 0; k < 3; ++k) {
-        const LfPlane& pl = f.pl[k];
-        const int gy = (pl.h + 3) / 4;
-        if (idx >= gy) {
-            idx -= gy;
-            continue;
-        }
-        const int ry = idx * 4, by = ry >> 3, half = (ry >> 2) & 1;
-        const int grid_w = k == 0 ? m.mbw * 2 : m.mbw;
-        for (int bx = 0; bx < grid_w; ++bx) {
-            const int x0 = bx * 8, y0 = by * 8;
-            if (x0 >= pl.w || y0 >= pl.h) break;
-            const LfBlock b = lf_block(m, k, bx, by);
-            if (bx + 1 < grid_w && x0 + 8 < pl.w) {
-                const LfBlock n = lf_block(m, k, bx + 1, by);
+        } else {
+            const int ry = iy * 4;
+            if constexpr (!INNER) {
+                if (bx + 1 >= grid_w || x0 + 8 >= pl.w) return;
+                const LfBlock b = lf_block(m, k, bx, by), n = lf_block(m, k, bx + 1, by);
                 // Main Profile exceptions 1 and 3, and 2: the luma edge between blocks 2 and 3
                 // decides with block 1's pattern and kind on its left (:563-581)
                 const LfBlock d = (m.main_profile && k == 0 && !(bx & 1) && (by & 1)) ? lf_block(m, k, bx + 1, by - 1) : b;
                 const bool ex = m.main_profile && (((m.intra[0] & 1) && !n.mb_intra) || d.tt == 7 || n.tt == 7);
+                bool on;
                 if (ex || b.intra || n.intra || b.mv.x != n.mv.x || b.mv.y != n.mv.y) {
-                    if (half * 4 < imin(8, pl.h - y0)) lf_vgroup(pl, x0 + 8, ry, pq);
+                    on = half * 4 < imin(8, pl.h - y0);
                 } else {
                     const int mask = (d.cbp | (n.cbp >> 1)) & 5;
-                    if (half == 0 ? (mask & 4) != 0 : ((mask & 1) && y0 + 4 < pl.h)) lf_vgroup(pl, x0 + 8, ry, pq);
+                    on = half == 0 ? (mask & 4) != 0 : ((mask & 1) && y0 + 4 < pl.h);
                 }
-            }
-            if ((b.tt == 7 || b.tt == 6) && x0 + 4 < pl.w) {
-                if (half == 0 ? (b.cbp & 12) != 0 : ((b.cbp & 3) && y0 + 4 < pl.h)) lf_vgroup(pl, x0 + 4, ry, pq);
+                if (on) lf_vgroup(pl, x0 + 8, ry, pq);
+            } else {
+                const int mb = (k == 0 ? by >> 1 : by) * m.mbw + (k == 0 ? bx >> 1 : bx);
+                const int bk = mb * 6 + (k == 0 ? (((by & 1) << 1) | (bx & 1)) : 3 + k);
+                const int tt = m.tt[bk], cbp = m.cbp[bk];
+                if ((tt == 7 || tt == 6) && x0 + 4 < pl.w && (half == 0 ? (cbp & 12) != 0 : ((cbp & 3) && y0 + 4 < pl.h)))
+                    lf_vgroup(pl, x0 + 4, ry, pq);
             }
         }
         return;
@@ -267,9 +308,17 @@ cudaError_t launch_loop_filter_p(uint8_t* y, uint8_t* u, uint8_t* v, int pitch_y
                                  cudaStream_t s, int main_profile) {
     const LfFrame f = lf_frame(y, u, v, pitch_y, pitch_c, W, H);
     const LfMeta m{bmv, cbp, tt, intra, (W + 15) / 16, (H + 15) / 16, main_profile};
-    const int nh = (W + 3) / 4 + 2 * ((W / 2 + 3) / 4), nv = (H + 3) / 4 + 2 * ((H / 2 + 3) / 4);
-    lfp_h_kernel<<<(unsigned)((nh + 63) / 64), 64, 0, s>>>(f, m, pq);
-    lfp_v_kernel<<<(unsigned)((nv + 63) / 64), 64, 0, s>>>(f, m, pq);
+    int nh = 0, nv = 0;
+    for (int k = 0; k < 3; ++k) {
+        const LfPlane& pl = f.pl[k];
+        nh += ((pl.w + 3) / 4) * (k ? m.mbh : 2 * m.mbh);
+        nv += ((pl.h + 3) / 4) * (k ? m.mbw : 2 * m.mbw);
+    }
+    const unsigned gh = (unsigned)((nh + 127) / 128), gv = (unsigned)((nv + 127) / 128);
+    lfp_kernel<false, false><<<gh, 128, 0, s>>>(f, m, pq);
+    lfp_kernel<false, true><<<gh, 128, 0, s>>>(f, m, pq);
+    lfp_kernel<true, false><<<gv, 128, 0, s>>>(f, m, pq);
+    lfp_kernel<true, true><<<gv, 128, 0, s>>>(f, m, pq);
     return cudaGetLastError();
 }
 
