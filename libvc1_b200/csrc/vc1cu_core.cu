@@ -104,12 +104,10 @@ struct SpecBlk;
 struct WarpMem {
     SPtr<uint8_t> cur;          // 16x16 current MB (zero outside the visible raster)
     SPtr<uint8_t> win;          // reference window
-    SPtr<uint64_t> keys;        // staged long-range cells of one warp step
-    SPtr<uint64_t> list_sad;    // the long-range search's nearest cells
     SPtr<uint64_t> list_satd;   // SATD of the shortlist
     SPtr<int2> batch;           // scratch MV batch
     SPtr<uint64_t> batch_cost;
-    SPtr<uint64_t> top;         // the lattice's four least keys
+    SPtr<uint64_t> top;         // umh_early's results
     SPtr<uint32_t> cur2;        // current MB, even columns packed 4 per word: [row][2]
     SPtr<uint32_t> cur4;        // current MB, every 4th column packed: [row]
     SPtr<int2> cur_bmv;         // the current MB's four block MVs while it is searched
@@ -796,7 +794,8 @@ __device__ __forceinline__ void top4_merge(Top4& t, uint64_t key) {
 // What scoring the macroblock's integer candidates reads, in registers.
 struct SearchGeo {
     uint32_t win, cur, cur2, cur4;
-    int wp, wx0, wy0, wh, x0, y0, xl, yl;
+    int wp, wx0, wy0, wh, x0, y0, xl, yl, W, H, gpitch;
+    const uint8_t* gref;
     bool whole;  // all 16x16 pixels inside the raster
     __device__ __forceinline__ explicit SearchGeo(uint32_t ctx) {
         const MbCtx& c = mbctx(ctx);
@@ -812,6 +811,10 @@ struct SearchGeo {
         y0 = c.y0;
         xl = c.xl;
         yl = c.yl;
+        W = c.g.W;
+        H = c.g.H;
+        gref = c.gref;
+        gpitch = c.gpitch;
         whole = c.aw == 16 && c.ah == 16;
     }
     // the candidate's block lies in the window
@@ -819,19 +822,26 @@ struct SearchGeo {
         const int rx = x0 + dx - wx0, ry = y0 + dy - wy0;
         return whole && rx >= 0 && ry >= 0 && rx + 16 <= wp && ry + 16 <= wh;
     }
+    // the candidate's block lies in the frame
+    __device__ __forceinline__ bool inside(int dx, int dy) const {
+        const int x = x0 + dx, y = y0 + dy;
+        return whole && x >= 0 && y >= 0 && x + 16 <= W && y + 16 <= H;
+    }
     __device__ __forceinline__ uint32_t base(int dx, int dy) const {
         return win + (uint32_t)((y0 + dy - wy0) * wp + (x0 + dx - wx0));
     }
 };
 
-// Packed SAD of sampled rows r0 .. r0 + nr - 1 (nr even, or one row at stride 4) of a staged candidate.
-template <int STRIDE>
-__device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, int r0, int nr) {
+// Packed SAD of the sampled rows r0 .. r0 + nr - 1 of a candidate, its rows staged in the window
+// (at shared offset base) or, GLOBAL, read from the frame (at ref).
+template <int STRIDE, bool GLOBAL>
+__device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, const uint8_t* ref, int r0, int nr) {
     uint32_t acc = 0;
 #pragma unroll 2
     for (int r = r0; r < r0 + nr; ++r) {
         uint32_t v[4];
-        win_load16(base + (uint32_t)(r * STRIDE * g.wp), v);
+        if (GLOBAL) glob_load16(ref + (size_t)(r * STRIDE) * g.gpitch, v);
+        else win_load16(base + (uint32_t)(r * STRIDE * g.wp), v);
         if (STRIDE == 1) {
             acc += __vsadu4(v[0], g_smem32[g.cur + r * 4]) + __vsadu4(v[1], g_smem32[g.cur + r * 4 + 1]) +
                    __vsadu4(v[2], g_smem32[g.cur + r * 4 + 2]) + __vsadu4(v[3], g_smem32[g.cur + r * 4 + 3]);
@@ -846,27 +856,39 @@ __device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, 
     return acc;
 }
 
-// Key of the candidate that 2^sh neighbouring lanes share (each scores its part of the rows): the
-// mb_sad at the given stride. Every lane calls it with its candidate; !on scores nothing.
-template <int STRIDE>
-__device__ __forceinline__ uint64_t shared_key(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
+// Cost (mb_sad at the given stride; kIllegal for kBad) of the candidate that 2^sh neighbouring
+// lanes share, each scoring its part of the rows. Every lane calls it with its candidate; !on
+// scores nothing. FAR: candidates may lie beyond the window (long-range vectors), where blocks
+// inside the frame are scored from it.
+constexpr uint32_t kIllegal = 0xFFFFF;
+template <int STRIDE, bool FAR = false>
+__device__ __forceinline__ uint32_t shared_cost(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
     const int part = (threadIdx.x & 31) & ((1 << sh) - 1), nr = (16 / STRIDE) >> sh;
-    const bool legal = dx <= g.xl && dy <= g.yl, in = g.staged(dx, dy);
+    const bool legal = dx <= g.xl && dy <= g.yl;
     uint32_t s = 0;
     if (on && legal) {
-        if (in) s = sad_rows<STRIDE>(g, g.base(dx, dy), part * nr, nr) * (STRIDE * STRIDE);
-        else if (part == 0) s = (uint32_t)mb_sad_core(ctx, dx, dy, STRIDE);
+        if (!FAR && g.staged(dx, dy))
+            s = sad_rows<STRIDE, false>(g, g.base(dx, dy), nullptr, part * nr, nr) * (STRIDE * STRIDE);
+        else if (FAR && g.inside(dx, dy))
+            s = sad_rows<STRIDE, true>(g, 0, g.gref + (size_t)(g.y0 + dy) * g.gpitch + g.x0 + dx, part * nr, nr) * (STRIDE * STRIDE);
+        else if (part == 0)
+            s = (uint32_t)mb_sad_core(ctx, dx, dy, STRIDE);
     }
     if (sh > 0) s += __shfl_xor_sync(FULL, s, 1);
     if (sh > 1) s += __shfl_xor_sync(FULL, s, 2);
     if (sh > 2) s += __shfl_xor_sync(FULL, s, 4);
-    return on ? int_key(legal ? (uint64_t)s : kBad, dx, dy) : UINT64_MAX;
+    return legal ? s : kIllegal;
+}
+// int_key of it; UINT64_MAX where !on.
+template <int STRIDE>
+__device__ __forceinline__ uint64_t shared_key(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
+    const uint32_t c = shared_cost<STRIDE>(ctx, g, on, dx, dy, sh);
+    return on ? int_key(c, dx, dy) : UINT64_MAX;
 }
 
-// The four least keys of the sparse lattice over the whole window (:1865-1870, range >= 8), which
-// depends on no neighbour: scored before the wavefront wait, one candidate per lane, into top[0..3].
-__device__ __noinline__ void umh_lattice(uint32_t ctx, uint32_t top_off, int range) {
-    const SearchGeo g(ctx);
+// The four least keys of the sparse lattice over the whole window (:1865-1870, range >= 8), one
+// candidate per lane.
+__device__ __forceinline__ Top4 umh_lattice(uint32_t ctx, const SearchGeo& g, int range) {
     const int lane = threadIdx.x & 31;
     const int L = (2 * range) / 8 + 1;
     // the far edges repeat the lattice's last row and column when its step divides the window
@@ -887,14 +909,7 @@ __device__ __noinline__ void umh_lattice(uint32_t ctx, uint32_t top_off, int ran
         }
         top4_merge(t, shared_key<2>(ctx, g, i < n, dx, dy, 0));
     }
-    if (lane == 0) {
-        uint64_t* top = reinterpret_cast<uint64_t*>(g_smem + top_off);
-        top[0] = t.a;
-        top[1] = t.b;
-        top[2] = t.c;
-        top[3] = t.d;
-    }
-    __syncwarp();
+    return t;
 }
 
 // Least key over the box [x0, x0 + (nx - 1) step] x [y0, ..] (and, with edges, the window's far
@@ -932,8 +947,69 @@ struct IntRes {
     uint64_t cost;
 };
 
-// The search after the wavefront wait: seeds in seeds[0..ns), the lattice's four least in
-// top[0..3] (range >= 8). The result's key.
+__device__ __forceinline__ bool match_good(uint64_t sad, uint64_t pixels) {
+    return pixels && sad < UINT64_MAX / 8 && sad <= pixels * 6u;
+}
+
+// The bounded rescue of a poor match (:1958-2020), two scans that depend on no neighbour: the
+// stride-4 grid and the square about its best; and, on a very poor match (local ranges up to 32),
+// the stride-2 grid and the square about its best. Their least full-resolution keys.
+__device__ __forceinline__ uint64_t rescue_around(uint32_t ctx, uint64_t k, int r, int range) {
+    const int xlo = imax(-range, key_dx(k) - r), xhi = imin(range, key_dx(k) + r);
+    const int ylo = imax(-range, key_dy(k) - r), yhi = imin(range, key_dy(k) + r);
+    return box_min(ctx, xlo, ylo, xhi - xlo + 1, yhi - ylo + 1, 1, 1, range, false);
+}
+__device__ __noinline__ uint64_t rescue_coarse(uint32_t ctx, int range) {
+    const int step = range >= 8 ? 4 : (range >= 3 ? 2 : 1), L = (2 * range) / step + 1;
+    const uint64_t ck = box_min(ctx, -range, -range, L, L, step, 4, range, (2 * range) % step != 0);
+    return rescue_around(ctx, ck, imax(1, step - 1), range);
+}
+__device__ __noinline__ uint64_t rescue_dense(uint32_t ctx, int range) {
+    return rescue_around(ctx, box_min(ctx, -range, -range, range + 1, range + 1, 2, 2, range, false), 2, range);
+}
+__device__ __forceinline__ bool dense_wanted(uint64_t cost, uint64_t pixels, int range) {
+    return pixels && cost > pixels * 24u && range <= 32;
+}
+
+// What of the UMH search depends on no neighbour, done before the wavefront wait, into top[]: the
+// lattice's four least keys ([0..3], range >= 8) and, where zero, the global vector and the
+// lattice's best all match poorly, the rescue's two results ([4], [5]; UINT64_MAX where not
+// computed). Most macroblocks that match poorly there match poorly after the whole search too,
+// and then find the rescue done; the others have spent idle time on it. Returns the least full
+// resolution cost seen.
+__device__ __noinline__ uint64_t umh_early(uint32_t ctx, uint32_t top_off, int gdx, int gdy, int range, int pixels) {
+    const SearchGeo g(ctx);
+    const int lane = threadIdx.x & 31;
+    Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
+    if (range >= 8) t = umh_lattice(ctx, g, range);
+    const int i = lane >> 3;
+    const int dx = i == 1 ? iclamp(gdx, -range, range) : (i == 2 && range >= 8 ? key_dx(t.a) : 0);
+    const int dy = i == 1 ? iclamp(gdy, -range, range) : (i == 2 && range >= 8 ? key_dy(t.a) : 0);
+    uint64_t best = warp_min_key(shared_key<1>(ctx, g, i < 3, dx, dy, 3));
+    uint64_t coarse = UINT64_MAX, dense = UINT64_MAX;
+    if (!match_good(key_cost(best), (uint64_t)pixels)) {
+        coarse = rescue_coarse(ctx, range);
+        if (coarse < best) best = coarse;
+        if (dense_wanted(key_cost(best), (uint64_t)pixels, range)) {
+            dense = rescue_dense(ctx, range);
+            if (dense < best) best = dense;
+        }
+    }
+    if (lane == 0) {
+        uint64_t* top = reinterpret_cast<uint64_t*>(g_smem + top_off);
+        top[0] = t.a;
+        top[1] = t.b;
+        top[2] = t.c;
+        top[3] = t.d;
+        top[4] = coarse;
+        top[5] = dense;
+    }
+    __syncwarp();
+    return key_cost(best);
+}
+
+// The search after the wavefront wait: seeds in seeds[0..ns), umh_early's results in top[]. The
+// result's key.
 __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint32_t top_off, int ns, int range, int pixels) {
     const SearchGeo g(ctx);
     const int lane = threadIdx.x & 31;
@@ -1008,21 +1084,16 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
     fk = warp_min_key(fk);
     // bounded rescue on a poor match (:1958-2020)
     const uint64_t px = (uint64_t)pixels;
-    auto good = [&](uint64_t cost) { return px && cost < UINT64_MAX / 8 && cost <= px * 6u; };
-    if (range > 0 && !good(key_cost(fk))) {
-        const int step = range >= 8 ? 4 : (range >= 3 ? 2 : 1);
-        const int L = (2 * range) / step + 1;
-        const uint64_t ck = box_min(ctx, -range, -range, L, L, step, 4, range, (2 * range) % step != 0);
-        const int rr = imax(1, step - 1);
-        auto around = [&](uint64_t k, int r) {
-            const int xlo = imax(-range, key_dx(k) - r), xhi = imin(range, key_dx(k) + r);
-            const int ylo = imax(-range, key_dy(k) - r), yhi = imin(range, key_dy(k) + r);
-            const uint64_t m = box_min(ctx, xlo, ylo, xhi - xlo + 1, yhi - ylo + 1, 1, 1, range, false);
-            if (m < fk) fk = m;
-        };
-        around(ck, rr);
-        if (px && key_cost(fk) > px * 24u && range <= 32)
-            around(box_min(ctx, -range, -range, range + 1, range + 1, 2, 2, range, false), 2);
+    if (range > 0 && !match_good(key_cost(fk), px)) {
+        const uint64_t* top = reinterpret_cast<const uint64_t*>(g_smem + top_off);
+        uint64_t k = top[4];
+        if (k == UINT64_MAX) k = rescue_coarse(ctx, range);
+        if (k < fk) fk = k;
+        if (dense_wanted(key_cost(fk), px, range)) {
+            k = top[5];
+            if (k == UINT64_MAX) k = rescue_dense(ctx, range);
+            if (k < fk) fk = k;
+        }
     }
     return fk;
 }
@@ -1089,8 +1160,7 @@ __device__ IntRes diamond(const DevParams& P, const Mb& m, const PInfo& pi, int 
 
 // motion_match_good, encoder_motion.cpp:1627-1635
 __device__ __forceinline__ bool match_good(const Mb& m, uint64_t sad) {
-    const uint64_t px = (uint64_t)m.aw * (uint64_t)m.ah;
-    return px && sad < UINT64_MAX / 8 && sad <= px * 6u;
+    return match_good(sad, (uint64_t)m.aw * (uint64_t)m.ah);
 }
 
 // sad > px * mae, exactly: the reference compares in long double, where the product of a
@@ -1123,29 +1193,6 @@ __device__ int distant_decision(const DevParams& P, const Mb& m, uint64_t cand, 
     return cand * 4u <= local * 3u ? 3 : 1;
 }
 
-// Least (sad, |dx|+|dy|, lane) over the lanes with `valid`, on every lane.
-__device__ void warp_argmin_int(bool& valid, uint64_t& sad, int& dx, int& dy, int& idx) {
-#pragma unroll 1
-    for (int o = 16; o; o >>= 1) {
-        const bool ov = __shfl_xor_sync(FULL, valid, o);
-        const uint64_t os = __shfl_xor_sync(FULL, sad, o);
-        const int ox = __shfl_xor_sync(FULL, dx, o), oy = __shfl_xor_sync(FULL, dy, o);
-        const int oi = __shfl_xor_sync(FULL, idx, o);
-        bool take = ov && !valid;
-        if (ov && valid) {
-            const int l1 = iabs(ox) + iabs(oy), l0 = iabs(dx) + iabs(dy);
-            take = os != sad ? os < sad : (l1 != l0 ? l1 < l0 : oi < idx);
-        }
-        if (take) {
-            valid = true;
-            sad = os;
-            dx = ox;
-            dy = oy;
-            idx = oi;
-        }
-    }
-}
-
 // The 13 offsets of propagated_long_range_motion (:1671-1673), by lane.
 __device__ __forceinline__ int2 lr_prop_offset(int l) {
     if (l == 0) return make_int2(0, 0);
@@ -1163,6 +1210,7 @@ __device__ __forceinline__ int2 lr_prop_offset(int l) {
 __device__ IntRes lr_propagated(const DevParams& P, const Mb& m, const DevResult& o, int range) {
     IntRes best{0, 0, UINT64_MAX};
     const Bounds b = bounds_px(range);
+    const SearchGeo g(m.sm.ctx.off);
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
         const int nx = m.mx + (k == 0 || k == 2 ? -1 : (k == 3 ? 1 : 0)), ny = m.my - (k == 0 ? 0 : 1);
@@ -1171,16 +1219,17 @@ __device__ IntRes lr_propagated(const DevParams& P, const Mb& m, const DevResult
         if (!(__ldcg(&o.flags[pos]) & 4)) continue;
         const int2 f = __ldcg(&o.mvs[pos]);
         const int cx = round_qpel_to_pixel(f.x), cy = round_qpel_to_pixel(f.y);
-        bool valid = m.lane < 13;
-        uint64_t sad = UINT64_MAX;
-        int dx = 0, dy = 0, idx = m.lane;
-        if (valid) {
-            const int2 of = lr_prop_offset(m.lane);
-            dx = iclamp(cx + of.x, b.xmin, b.xmax);
-            dy = iclamp(cy + of.y, b.ymin, b.ymax);
-            sad = mb_sad(P, m, dx, dy, 1);
-        }
-        warp_argmin_int(valid, sad, dx, dy, idx);
+        // two lanes per offset; the least (sad, |d|, offset index)
+        const int i = m.lane >> 1;
+        const int2 of = lr_prop_offset(imin(i, 12));
+        int dx = iclamp(cx + of.x, b.xmin, b.xmax), dy = iclamp(cy + of.y, b.ymin, b.ymax);
+        const uint32_t c = shared_cost<1, true>(m.sm.ctx.off, g, i < 13, dx, dy, 1);
+        const uint64_t key = i < 13 ? ((uint64_t)c << 32) | ((uint64_t)(iabs(dx) + iabs(dy)) << 5) | (uint64_t)i : UINT64_MAX;
+        const uint64_t least = warp_min_key(key);
+        const int src = 2 * (int)(least & 31);
+        dx = __shfl_sync(FULL, dx, src);
+        dy = __shfl_sync(FULL, dy, src);
+        const uint64_t sad = (least >> 32) == kIllegal ? kBad : least >> 32;
         if (sad < best.cost || (sad == best.cost && iabs(dx) + iabs(dy) < iabs(best.dx) + iabs(best.dy))) {
             best.cost = sad;
             best.dx = dx;
@@ -1221,109 +1270,97 @@ __device__ uint64_t warp_signature(const DevFrame& f, int W, int H, int x0, int 
     return s;
 }
 
-// long_range_signature_distance (:1605-1614)
+// long_range_signature_distance (:1605-1614): the four luma means weigh 2, the chroma means 3.
 __device__ __forceinline__ uint32_t sig_distance(uint64_t a, uint64_t b) {
-    uint32_t d = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d += (uint32_t)iabs((int)((a >> (8 * i)) & 255) - (int)((b >> (8 * i)) & 255)) * 2u;
-    d += (uint32_t)iabs((int)((a >> 32) & 255) - (int)((b >> 32) & 255)) * 3u;
-    d += (uint32_t)iabs((int)((a >> 40) & 255) - (int)((b >> 40) & 255)) * 3u;
-    return d;
+    return 2u * __vsadu4((uint32_t)a, (uint32_t)b) + 3u * __vsadu4((uint32_t)(a >> 32), (uint32_t)(b >> 32));
 }
 
-// Vc1Encoder::extended_content_motion, encoder_motion.cpp:1696-1779: the 16 lattice cells
-// whose signature is nearest the macroblock's (order (distance, |d|, dy, dx), cells within
-// 32 pixels excluded), each refined by a 5x5 grid of step 4 at stride 2 and a 5x5 full
-// search; `local` stands unless the best is both cheaper and a good enough distant match.
-__device__ IntRes lr_extended(const DevParams& P, const Mb& m, const PassDesc& d, int range, const IntRes& local,
-                              uint64_t& cand_sad, int& decision) {
+// The neighbour-independent part of Vc1Encoder::extended_content_motion,
+// encoder_motion.cpp:1696-1779: the 16 lattice cells whose signature is nearest the macroblock's
+// (order (distance, |d|, dy, dx), cells within 32 pixels excluded), each refined by a 5x5 grid of
+// step 4 at stride 2 and a 5x5 full search, until one is a good match. Bound by the latency of the
+// signature loads (up to 32,400 cells at 1080p) and of the candidates' rows, which come from L2:
+// four signatures per lane are in flight, the sixteen least stand one per lane, and the kernel runs
+// it before the wavefront wait wherever umh_early's matches are poor. With one signature in flight,
+// a serial list and the whole search after the wait, a 1080p pan (range 1024) waited 0.5 ms per
+// wavefront step for macroblocks whose content entered the picture.
+__device__ __noinline__ IntRes lr_nearest(uint32_t ctx, const PassDesc* dp, int W, int H, int range, uint64_t pixels) {
+    const PassDesc& d = *dp;
+    const SearchGeo g(ctx);
+    const int lane = threadIdx.x & 31;
     const Bounds b = bounds_px(range);
-    const uint64_t want = warp_signature(d.cur, P.W, P.H, m.x0, m.y0, m.lane);
-    uint64_t* top = m.sm.list_sad;  // 16 sorted keys (idle after the integer search)
-    uint64_t* stage = m.sm.keys;
-    int tn = 0;
-    const int n = d.lr_nx * d.lr_ny;
+    const uint64_t want = warp_signature(d.cur, W, H, g.x0, g.y0, lane);
+    // the cells whose offset lies within the bounds
+    const int c0 = imax(0, (g.x0 + b.xmin + 7) >> 3), c1 = imin(d.lr_nx - 1, (g.x0 + b.xmax) >> 3);
+    const int r0 = imax(0, (g.y0 + b.ymin + 7) >> 3), r1 = imin(d.lr_ny - 1, (g.y0 + b.ymax) >> 3);
+    const int nc = c1 - c0 + 1;
+    uint64_t top = UINT64_MAX, bound = UINT64_MAX;  // lane j < 16: the j-th least key
+    int cx = c0 + lane, cy = r0;
 #pragma unroll 1
-    for (int base = 0; base < n; base += 32) {
-        const int i = base + m.lane;
-        uint64_t key = UINT64_MAX;
-        if (i < n) {
-            const int dx = (i % d.lr_nx) * 8 - m.x0, dy = (i / d.lr_nx) * 8 - m.y0;
-            if (dx >= b.xmin && dx <= b.xmax && dy >= b.ymin && dy <= b.ymax && !(iabs(dx) <= 32 && iabs(dy) <= 32) &&
-                IDX_OK(d.lr_sig != nullptr, kSiteSignature, i)) {
-                const uint64_t dist = sig_distance(want, __ldg(&d.lr_sig[i]));
-                key = (dist << 36) | ((uint64_t)(iabs(dx) + iabs(dy)) << 24) | ((uint64_t)(dy + 2048) << 12) |
-                      (uint64_t)(dx + 2048);
+    while (nc > 0 && __any_sync(FULL, cy <= r1)) {
+        uint64_t key[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            while (cx > c1) {
+                cx -= nc;
+                ++cy;
+            }
+            key[u] = UINT64_MAX;
+            if (cy <= r1) {
+                const int dx = cx * 8 - g.x0, dy = cy * 8 - g.y0, i = cy * d.lr_nx + cx;
+                if (!(iabs(dx) <= 32 && iabs(dy) <= 32) && IDX_OK(d.lr_sig != nullptr, kSiteSignature, i))
+                    key[u] = ((uint64_t)sig_distance(want, __ldg(&d.lr_sig[i])) << 36) |
+                             ((uint64_t)(iabs(dx) + iabs(dy)) << 24) | ((uint64_t)(dy + 2048) << 12) | (uint64_t)(dx + 2048);
+            }
+            cx += 32;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            unsigned take = __ballot_sync(FULL, key[u] < bound);
+            while (take) {
+                const uint64_t k = __shfl_sync(FULL, key[u], __ffs(take) - 1);
+                take &= take - 1;
+                if (k >= bound) continue;
+                const int rank = __popc(__ballot_sync(FULL, lane < 16 && top < k));
+                const uint64_t up = __shfl_up_sync(FULL, top, 1);
+                if (lane < 16 && lane >= rank) top = lane == rank ? k : up;
+                bound = __shfl_sync(FULL, top, 15);
             }
         }
-        const uint64_t bound = tn == 16 ? top[15] : UINT64_MAX;
-        const bool take = key < bound;
-        const unsigned tm = __ballot_sync(FULL, take);
-        if (!tm) continue;
-        if (take) stage[__popc(tm & ((1u << m.lane) - 1))] = key;
-        __syncwarp();
-        if (m.lane == 0) {
-            const int cnt = __popc(tm);
-            for (int j = 0; j < cnt; ++j) {
-                const uint64_t k = stage[j];
-                if (tn == 16 && k >= top[15]) continue;
-                int at = tn < 16 ? tn : 15;
-                while (at > 0 && top[at - 1] > k) {
-                    top[at] = top[at - 1];
-                    --at;
-                }
-                top[at] = k;
-                if (tn < 16) ++tn;
-            }
-        }
-        tn = __shfl_sync(FULL, tn, 0);
-        __syncwarp();
     }
     IntRes best{0, 0, UINT64_MAX};
 #pragma unroll 1
-    for (int t = 0; t < tn; ++t) {
-        const uint64_t key = top[t];
+    for (int t = 0; t < 16; ++t) {
+        const uint64_t key = __shfl_sync(FULL, top, t);
+        if (key == UINT64_MAX) break;
         const int cdx = (int)(key & 0xFFF) - 2048, cdy = (int)((key >> 12) & 0xFFF) - 2048;
+        const bool on = lane < 25;
         // 5x5 at step 4, stride 2: the first least SAD in scan order
-        bool valid = m.lane < 25;
-        uint64_t sad = UINT64_MAX;
-        int dx = 0, dy = 0, idx = m.lane;
-        if (valid) {
-            dx = iclamp(cdx - 8 + 4 * (m.lane % 5), b.xmin, b.xmax);
-            dy = iclamp(cdy - 8 + 4 * (m.lane / 5), b.ymin, b.ymax);
-            sad = mb_sad(P, m, dx, dy, 2);
-        }
-        {
-            uint64_t s = sad;
-            const uint64_t mn = warp_min_u64(valid ? s : UINT64_MAX);
-            const unsigned at = __ballot_sync(FULL, valid && s == mn);
-            const int src = __ffs(at) - 1;
-            dx = __shfl_sync(FULL, dx, src);
-            dy = __shfl_sync(FULL, dy, src);
-        }
-        const int sx = dx, sy = dy;
+        int dx = iclamp(cdx - 8 + 4 * (lane % 5), b.xmin, b.xmax), dy = iclamp(cdy - 8 + 4 * (lane / 5), b.ymin, b.ymax);
+        uint32_t c = shared_cost<2, true>(ctx, g, on, dx, dy, 0);
+        uint64_t least = warp_min_key(on ? ((uint64_t)c << 32) | (uint64_t)lane : UINT64_MAX);
+        const int sx = __shfl_sync(FULL, dx, (int)(least & 31)), sy = __shfl_sync(FULL, dy, (int)(least & 31));
         // 5x5 full search around it: least (sad, |d|), first in scan order
-        valid = m.lane < 25;
-        sad = UINT64_MAX;
-        idx = m.lane;
-        if (valid) {
-            dx = iclamp(sx + m.lane % 5 - 2, b.xmin, b.xmax);
-            dy = iclamp(sy + m.lane / 5 - 2, b.ymin, b.ymax);
-            sad = mb_sad(P, m, dx, dy, 1);
-        }
-        warp_argmin_int(valid, sad, dx, dy, idx);
-        if (sad < best.cost) {
-            best.cost = sad;
-            best.dx = dx;
-            best.dy = dy;
-        }
-        if (match_good(m, best.cost)) break;
+        dx = iclamp(sx + lane % 5 - 2, b.xmin, b.xmax);
+        dy = iclamp(sy + lane / 5 - 2, b.ymin, b.ymax);
+        c = shared_cost<1, true>(ctx, g, on, dx, dy, 0);
+        least = warp_min_key(on ? ((uint64_t)c << 32) | ((uint64_t)(iabs(dx) + iabs(dy)) << 5) | (uint64_t)lane : UINT64_MAX);
+        dx = __shfl_sync(FULL, dx, (int)(least & 31));
+        dy = __shfl_sync(FULL, dy, (int)(least & 31));
+        const uint64_t sad = (least >> 32) == kIllegal ? kBad : least >> 32;
+        if (sad < best.cost) best = IntRes{dx, dy, sad};
+        if (match_good(best.cost, pixels)) break;
     }
+    return best;
+}
+
+// extended_content_motion's decision on it: `local` stands unless the best is both cheaper and a
+// good enough distant match.
+__device__ __forceinline__ IntRes lr_extended(const DevParams& P, const Mb& m, const IntRes& best, const IntRes& local,
+                                              uint64_t& cand_sad, int& decision) {
     cand_sad = best.cost;
     decision = best.cost < UINT64_MAX / 8 ? distant_decision(P, m, best.cost, local.cost) : 0;
-    __syncwarp();
-    if (best.cost >= local.cost || decision < 2) return local;
-    return best;
+    return (best.cost >= local.cost || decision < 2) ? local : best;
 }
 
 // ---- learned passes: candidates and a short integer descent ----------------------------
@@ -2253,10 +2290,8 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
         p += (bytes + 15) & ~15u;
         return q;
     };
-    s.list_sad.off = take(8 * kListCap);
     s.list_satd.off = take(8 * kListCap);
     s.batch_cost.off = take(8 * 32);
-    s.keys.off = take(8 * 32);
     s.top.off = take(8 * 8);
     s.batch.off = take(8 * 32);
     s.cur2.off = take(4 * 32);
@@ -2280,7 +2315,7 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
 
 __host__ __device__ inline int warp_bytes_for(const WinCfg& wc) {
     auto r = [](int b) { return (b + 15) & ~15; };
-    return r(8 * kListCap) * 2 + r(8 * 32) + r(8 * 32) + r(64) + r(8 * 32) + r(128) + r(64) + r(32) + r(32) +
+    return r(8 * kListCap) + r(8 * 32) + r(64) + r(8 * 32) + r(128) + r(64) + r(32) + r(32) +
            r(128) + r(16) + 3 * r(8 * 40) + r(kSpecBlkBytes * 5) + r(kMbCtxBytes) + r(256) + r(8) + 128 +
            r(wc.wp * wc.wh + 32);
 }
@@ -2555,6 +2590,8 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
         const bool spec4 = allow_4mv && spec;
         int2 one_g = make_int2(0, 0);
         IntRes learned{0, 0, UINT64_MAX};  // learned passes: the integer vector before refinement
+        IntRes ext_best{0, 0, UINT64_MAX};  // the content-signature search, where it ran before the wait
+        bool ext_known = false;
         if (ok) {
             if (seeded) {
                 int2 seed = __ldcg(&d.seed_mvs[m.pos]);
@@ -2620,9 +2657,15 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 load_window(P, m, d.ref, 0, 0, wc);
                 publish_ctx(P, m);
                 PHASE_MARK(2);
-                if ((kUmhOnly || P.me_algorithm != 1) && local_range >= 8) {
+                if (kUmhOnly || P.me_algorithm != 1) {
                     window_wait(m, st, code, P.wait_log2);
-                    umh_lattice(m.sm.ctx.off, m.sm.top.off, local_range);
+                    const int px = m.aw * m.ah;
+                    const uint64_t seen = umh_early(m.sm.ctx.off, m.sm.top.off, __ldcg(&o.global[0]), __ldcg(&o.global[1]),
+                                                    local_range, px);
+                    if (!kUmhOnly && range > local_range && !match_good(seen, (uint64_t)px)) {
+                        ext_best = lr_nearest(m.sm.ctx.off, &d, P.W, P.H, range, (uint64_t)px);
+                        ext_known = true;
+                    }
                 }
                 PHASE_MARK(3);
             }
@@ -2714,7 +2757,8 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                     // content-signature search (:201-225)
                     uint64_t ext_sad = UINT64_MAX;
                     int ext_decision = 0;
-                    const IntRes ext = lr_extended(P, m, d, range, im, ext_sad, ext_decision);
+                    if (!ext_known) ext_best = lr_nearest(m.sm.ctx.off, &d, P.W, P.H, range, pixels);
+                    const IntRes ext = lr_extended(P, m, ext_best, im, ext_sad, ext_decision);
                     if (P.long_range_mode != 2) record(ext_sad, ext_decision);
                     if (ext.dx != im.dx || ext.dy != im.dy) {
                         im = ext;
