@@ -128,6 +128,9 @@ constexpr size_t kMaxBatch = 64u * 65535u;   // VulkanComputeContext's candidate
 #define VC1CU_SEEDED_MIXED_RW 8
 #endif
 constexpr int kSeededMixedRw = VC1CU_SEEDED_MIXED_RW;  // window radius of seeded Mixed-MV launches
+#ifndef VC1CU_MERGE_FRONT
+#define VC1CU_MERGE_FRONT 8
+#endif
 constexpr int kMaxLocalRange = 190;  // the largest local range this interface takes
 constexpr int kMinUnseededRw = 24;  // smallest window radius a tuned unseeded launch shrinks to
 #ifndef VC1CU_WINDOW_TMA
@@ -384,7 +387,7 @@ struct vc1cu_ctx {
     std::vector<Timed> pending;
     std::vector<cudaEvent_t> event_pool;
     vc1cu_timing tsum{};
-    // work-queue tables per launch shape (raster, pass levels)
+    // work-queue tables per launch shape (the passes' rasters)
     std::map<std::vector<int>, std::pair<uint32_t*, unsigned>> items;
 };
 
@@ -506,27 +509,21 @@ void set_lambda(PassDesc& d, int pq) {
 }
 
 // Work-queue table of a launch: (pass << 20) | macroblock. Inside a pass the macroblocks
-// follow the wavefront order (t = x + 2y, then y); a pass at seed level L (seeded by a pass
-// of the same launch at level L-1) is delayed by L * lag positions, so each item follows all
-// of its dependencies. Cached per (raster, pass levels).
-const uint32_t* work_items(vc1cu_ctx* c, const std::vector<int>& mbw, const std::vector<int>& mbh,
-                           const std::vector<int>& level, unsigned& nitems) {
-    const int n = (int)level.size();
+// follow the wavefront order (t = x + 2y, then y), so each item follows all of its dependencies.
+// Cached per the passes' rasters.
+const uint32_t* work_items(vc1cu_ctx* c, const std::vector<int>& mbw, const std::vector<int>& mbh, unsigned& nitems) {
+    const int n = (int)mbw.size();
     std::vector<int> key;
     for (int p = 0; p < n; ++p) {
         key.push_back(mbw[p]);
         key.push_back(mbh[p]);
-        key.push_back(level[p]);
     }
     auto it = c->items.find(key);
     if (it != c->items.end()) {
         nitems = it->second.second;
         return it->second.first;
     }
-    // Each pass's macroblocks in its own wavefront order (t = x + 2y, then y); a seeded pass runs
-    // about two wavefront steps (one raster row of macroblocks) behind its seed pass. The passes'
-    // lists are merged by that step, so every item's dependencies (its neighbours and its seed)
-    // are handed out before it, whatever the passes' raster sizes.
+    // the passes' lists merged step by step, whatever their raster sizes
     std::vector<std::vector<int>> order(n);
     long steps = 0;
     for (int p = 0; p < n; ++p) {
@@ -537,17 +534,15 @@ const uint32_t* work_items(vc1cu_ctx* c, const std::vector<int>& mbw, const std:
                 const int x = t - 2 * y;
                 if (x >= 0 && x < w) order[p].push_back(y * w + x);
             }
-        steps = std::max(steps, (long)w * hh + (long)w * level[p]);
+        steps = std::max(steps, (long)w * hh);
     }
     if (c->capturing)
         throw Fail{VC1CU_ERR_STATE, "run a launch of this shape once before capturing it (its work-item table is "
                                     "built and uploaded outside the capture)"};
     std::vector<uint32_t> items;
     for (long sstep = 0; sstep < steps; ++sstep)
-        for (int p = 0; p < n; ++p) {
-            const long j = sstep - (long)mbw[p] * level[p];
-            if (j >= 0 && j < (long)order[p].size()) items.push_back(((uint32_t)p << 20) | (uint32_t)order[p][j]);
-        }
+        for (int p = 0; p < n; ++p)
+            if (sstep < (long)order[p].size()) items.push_back(((uint32_t)p << 20) | (uint32_t)order[p][sstep]);
     void* d = nullptr;
     ck(cudaMalloc(&d, items.size() * sizeof(uint32_t)), "cudaMalloc(work items)");
     // Ordered on the context stream, which does not synchronise with the legacy default stream:
@@ -809,8 +804,8 @@ void global_searches_send(vc1cu_ctx* c, const GSearches& g) {
     staging_mark(c);
 }
 
-// Launches a batch of independent core passes (global search first for unseeded ones).
-// globals_ready: the unseeded passes' global translation results are already in their slots.
+// Launches a batch of independent core passes, all seeded or all unseeded (global search first
+// for unseeded ones). globals_ready: the unseeded passes' global translation results are already in their slots.
 // Per-pass additions of the learned form (all null for the plain passes): the candidates of a
 // learned pass and where it flags its fallback macroblocks, or the flags a fallback pass
 // computes (only those macroblocks), and the translation hint that replaces the global search.
@@ -875,10 +870,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         if (q.pqindex < 0 || q.pqindex > 31) throw Fail{VC1CU_ERR_ARG, "pass pqindex must be 0 (params) or 1..31"};
         set_lambda(d, q.pqindex ? q.pqindex : d.geom.pq);
         d.seeded = q.seed_slot >= 0;
-        d.seed_pass = -1;
-        for (int j = 0; j < n; ++j)
-            if (q.seed_slot >= 0 && passes[j].out_slot == q.seed_slot) d.seed_pass = j;
-        if (d.seeded && d.seed_pass < 0) {
+        if (d.seeded) {
             ResultSlot& s = result_slot(c, q.seed_slot, mbs, false);
             d.seed_mvs = s.r.mvs;
             d.seed_bmv = s.r.bmv;
@@ -886,8 +878,6 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
             d.seed_dl = s.r.dl;
             d.seed_dc = s.r.dc;
             d.seed_dd = s.r.dd;
-        } else if (d.seeded) {
-            d.seed_mvs = nullptr;  // bound to the seeding pass's result below
         } else {
             d.seed_mvs = nullptr;
             d.seed_dl = d.seed_dc = nullptr;
@@ -930,25 +920,6 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
                     ck(cudaMemsetAsync(h[i].out.gsad, 0, 8, c->stream), "cudaMemsetAsync(hint sad)");
             }
         if (any_hint) globals_ready = true;
-    }
-    // seed levels of in-launch seeds (a chain, never a cycle)
-    std::vector<int> level(n, 0);
-    for (int i = 0; i < n; ++i) {
-        int l = 0, j = i;
-        while (h[j].seed_pass >= 0) {
-            j = h[j].seed_pass;
-            if (++l > n) throw Fail{VC1CU_ERR_ARG, "passes of one launch seed each other in a cycle"};
-        }
-        level[i] = l;
-        if (h[i].seed_pass >= 0) {
-            const DevResult& so = h[h[i].seed_pass].out;
-            h[i].seed_mvs = so.mvs;
-            h[i].seed_bmv = so.bmv;
-            h[i].seed_intra = so.intra;
-            h[i].seed_dl = so.dl;
-            h[i].seed_dc = so.dc;
-            h[i].seed_dd = so.dd;
-        }
     }
     // global translation search of the unseeded passes (none at --search-range 0)
     if (!globals_ready && !unseeded.empty() && P.range == 0)
@@ -1026,13 +997,8 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     // the instantiation: the code this launch's passes can reach (the kCore* flags)
     bool any_mixed_pass = false;
     for (int i = 0; i < n; ++i) any_mixed_pass |= passes[i].mode == VC1CU_MV_MIXED;
-    int kind = kCoreAny;
-    if (!any_unseeded) {
-        kind = kCoreSeededOnly;
-    } else if ((int)unseeded.size() == n) {
-        kind = kCoreUnseededOnly;
-        if (P.me_algorithm == 0 && P.range == P.local_range) kind |= kCoreUmhLocal;
-    }
+    int kind = any_unseeded ? kCoreUnseededOnly : kCoreSeededOnly;
+    if (any_unseeded && P.me_algorithm == 0 && P.range == P.local_range) kind |= kCoreUmhLocal;
     if (!any_mixed_pass && (kind & (kCoreSeededOnly | kCoreUmhLocal))) kind |= kCoreNoMixed;
     if (P.me_quality == 2 && !P.fast_subpel && (kind & (kCoreSeededOnly | kCoreUmhLocal))) kind |= kCoreDefaultRefine;
     bool any_intra_pass = false;
@@ -1041,7 +1007,14 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     if (learned)
         kind = kCoreUnseededOnly | kCoreLearned | kCoreNoMixed | kCoreNoIntra |
                ((P.me_quality == 2 && !P.fast_subpel) ? kCoreDefaultRefine : 0);
-    if (multi) kind = kCoreMulti;
+    if (multi) {
+        // the uneven-size builds: the default search's unseeded and seeded launches, and one general
+        // build of each
+        constexpr int umh = kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed | kCoreDefaultRefine | kCoreNoIntra;
+        if (any_unseeded) kind = kind == umh ? kind : kCoreUnseededOnly;
+        else kind &= ~kCoreNoMixed;
+        kind |= kCoreMulti;
+    }
     // windows so large that a second 4-warp block cannot fit: the wide-register build costs no occupancy
     if (!(kind & kCoreSeededOnly) && 2 * 4 * (size_t)wc.warp_bytes > (size_t)c->max_smem_sm) kind |= kCoreWide;
     const void* kern = core_kernel(kind);
@@ -1182,7 +1155,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
             mbw[i] = h[i].geom.mbw;
             mbh[i] = h[i].geom.mbh;
         }
-        const uint32_t* items = work_items(c, mbw, mbh, level, nitems);
+        const uint32_t* items = work_items(c, mbw, mbh, nitems);
         P.wait_log2 = c->wait_log2;
         P.withhold = c->withhold_next;
         c->withhold_next = 0xFFFFFFFFu;
@@ -1203,31 +1176,109 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     return VC1CU_OK;
 }
 
-// Launches a batch of core passes. Passes of different kinds (seeded or not, MV mode, P-intra)
-// run as separate launches in the order the kinds first appear: each launch then executes
-// one code path, whose instructions stay in the SMs' instruction caches. A batch in which a
-// pass is seeded by another pass of the same batch runs as one launch.
-int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, int n) {
-    bool chained = false;
+// Every check of a call's passes, before any of them is launched.
+void check_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, int n, const vc1cu_params* per_pass) {
+    std::vector<DevParams> geom(n);
+    std::string why;
     for (int i = 0; i < n; ++i) {
-        for (int j = 0; j < n; ++j) {
-            if (j < i && passes[j].out_slot == passes[i].out_slot)
-                throw Fail{VC1CU_ERR_ARG, "two passes write one result slot"};
-            if (passes[i].seed_slot >= 0 && passes[j].out_slot == passes[i].seed_slot) chained = true;
+        const vc1cu_pass& q = passes[i];
+        const int rc = make_dev_params(per_pass ? per_pass + i : p, geom[i], why);
+        if (rc) throw Fail{rc, why};
+        if (q.mode < 0 || q.mode > 3) throw Fail{VC1CU_ERR_ARG, "invalid MV mode"};
+        if (q.out_slot < 0 || q.out_slot > kInternalLast || q.seed_slot == q.out_slot)
+            throw Fail{VC1CU_ERR_ARG, "invalid result slot"};
+        if (q.pqindex < 0 || q.pqindex > 31) throw Fail{VC1CU_ERR_ARG, "pass pqindex must be 0 (params) or 1..31"};
+        if (i > 0) same_search_config(geom[0], geom[i]);
+        const FrameSlot &fc = frame_slot(c, q.cur_id), &fr = frame_slot(c, q.ref_id);
+        if (fc.w != geom[i].W || fc.h != geom[i].H || fr.w != geom[i].W || fr.h != geom[i].H)
+            throw Fail{VC1CU_ERR_ARG, "P-picture reference dimensions do not match the configuration"};
+        for (int j = 0; j < i; ++j)
+            if (passes[j].out_slot == q.out_slot) throw Fail{VC1CU_ERR_ARG, "two passes write one result slot"};
+    }
+    for (int i = 0; i < n; ++i) {
+        if (passes[i].seed_slot < 0) continue;
+        int s = -1;
+        for (int j = 0; j < n; ++j)
+            if (passes[j].out_slot == passes[i].seed_slot) s = j;
+        if (s < 0) result_slot(c, passes[i].seed_slot, geom[i].mbw * geom[i].mbh, false);
+        else if (geom[s].mbw != geom[i].mbw || geom[s].mbh != geom[i].mbh)
+            throw Fail{VC1CU_ERR_ARG, "a pass's seed is a pass over another raster"};
+    }
+}
+
+// Wavefront fronts (macroblocks of one step, at most) of up to this many macroblocks per SM run
+// seeded passes of different modes as one launch. A seeded launch holds 16 warps per SM and every
+// step of its chain waits for one macroblock's latency: passes that leave warps idle cost one chain
+// together instead of one each, and more of them pay for the larger code of several modes.
+constexpr int kMergeFront = VC1CU_MERGE_FRONT;
+
+// The launches of a call's passes, in order, as index lists. A pass seeded by another pass of the
+// call follows it, one launch later (so that its speculation can read the whole seed field); the
+// passes of one step are split by kind (seeded or not, MV mode, P-intra): each launch then executes
+// one code path, whose instructions stay in the SMs' instruction caches. Seeded passes of a step
+// share a launch where their fronts together leave warps idle (kMergeFront), and always in the
+// uneven-size form (per_pass), which is one launch per step for its passes' sake.
+std::vector<std::vector<int>> plan_launches(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, int n,
+                                            const vc1cu_params* per_pass) {
+    std::vector<int> level(n, 0);
+    int top = 0;
+    for (int i = 0; i < n; ++i) {
+        int j = i;
+        for (;;) {
+            int s = -1;
+            for (int k = 0; k < n && passes[j].seed_slot >= 0; ++k)
+                if (passes[k].out_slot == passes[j].seed_slot) s = k;
+            if (s < 0) break;
+            if (++level[i] > n) throw Fail{VC1CU_ERR_ARG, "passes of one call seed each other in a cycle"};
+            j = s;
+        }
+        top = std::max(top, level[i]);
+    }
+    std::vector<std::vector<int>> out;
+    for (int l = 0; l <= top; ++l) {
+        long front = 0;
+        for (int i = 0; i < n; ++i)
+            if (level[i] == l && passes[i].seed_slot >= 0) {
+                const vc1cu_params& g = per_pass ? per_pass[i] : *p;
+                front += std::min(((g.width + 15) / 16 + 1) / 2, (g.height + 15) / 16);
+            }
+        const bool merge = per_pass || front <= (long)kMergeFront * c->sm_count;
+        std::vector<int> keys;
+        const size_t first = out.size();
+        for (int i = 0; i < n; ++i) {
+            if (level[i] != l) continue;
+            const bool seeded = passes[i].seed_slot >= 0;
+            const int kind = 2 * passes[i].mode + (passes[i].allow_intra ? 1 : 0);
+            const int key = seeded ? 8 + (merge ? (passes[i].allow_intra ? 1 : 0) : kind) : (per_pass ? 0 : kind);
+            size_t g = 0;
+            while (g < keys.size() && keys[g] != key) ++g;
+            if (g == keys.size()) {
+                keys.push_back(key);
+                out.emplace_back();
+            }
+            out[first + g].push_back(i);
         }
     }
-    if (n <= 1 || chained) return launch_group(c, p, passes, n);
-    std::vector<int> keys;
-    std::vector<std::vector<vc1cu_pass>> groups;
-    for (int i = 0; i < n; ++i) {
-        const int key = (passes[i].seed_slot >= 0 ? 8 : 0) + 2 * passes[i].mode + (passes[i].allow_intra ? 1 : 0);
-        size_t g = 0;
-        while (g < keys.size() && keys[g] != key) ++g;
-        if (g == keys.size()) {
-            keys.push_back(key);
-            groups.emplace_back();
+    return out;
+}
+
+// Launches a call's core passes: plan_launches' launches in order.
+int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, int n,
+                  const vc1cu_params* per_pass = nullptr) {
+    check_passes(c, p, passes, n, per_pass);
+    const std::vector<std::vector<int>> plan = plan_launches(c, p, passes, n, per_pass);
+    auto run = [&](const std::vector<int>& g, bool globals_ready) {
+        std::vector<vc1cu_pass> q;
+        std::vector<vc1cu_params> pp;
+        for (int i : g) {
+            q.push_back(passes[i]);
+            if (per_pass) pp.push_back(per_pass[i]);
         }
-        groups[g].push_back(passes[i]);
+        launch_group(c, p, q.data(), (int)q.size(), globals_ready, nullptr, per_pass ? pp.data() : nullptr);
+    };
+    if (plan.size() == 1 || per_pass) {
+        for (const auto& g : plan) run(g, false);
+        return VC1CU_OK;
     }
     // The global translation search depends only on (cur, ref) at the call's range, so passes of
     // one picture pair in different groups (a B picture's quarter-pel and bilinear passes) share
@@ -1298,7 +1349,7 @@ int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
             }
         }
     }
-    for (const auto& g : groups) launch_group(c, p, g.data(), (int)g.size(), true);
+    for (const auto& g : plan) run(g, true);
     return VC1CU_OK;
 }
 
@@ -2161,10 +2212,8 @@ int vc1cu_core_passes_multi(vc1cu_ctx* c, const vc1cu_params* params, const vc1c
         for (int i = 0; i < n; ++i) {
             if (passes[i].out_slot < 0 || passes[i].out_slot >= kMaxSlot || passes[i].seed_slot >= kMaxSlot)
                 throw Fail{VC1CU_ERR_ARG, "result slot out of range"};
-            for (int j = 0; j < i; ++j)
-                if (passes[j].out_slot == passes[i].out_slot) throw Fail{VC1CU_ERR_ARG, "two passes write one result slot"};
         }
-        return launch_group(c, params, passes, n, false, nullptr, params);
+        return launch_passes(c, params, passes, n, params);
     });
 }
 
@@ -2247,49 +2296,70 @@ int vc1cu_autotune(vc1cu_ctx* c, const vc1cu_params* params, const vc1cu_pass* p
         if (n <= 0 || !passes || !params) throw Fail{VC1CU_ERR_ARG, "invalid pass list"};
         if (c->capturing) throw Fail{VC1CU_ERR_STATE, "cannot tune during a capture"};
         const vc1cu_params* pp = per_pass_params ? params : nullptr;
-        auto run = [&]() { launch_group(c, params, passes, n, false, nullptr, pp); };
+        check_passes(c, params, passes, n, pp);
         cudaEvent_t a = take_event(c), b = take_event(c);
-        double best = -1.0;
-        std::pair<int, int> best_shape{0, 0};
-        std::vector<int> key;
-        // warps (macroblocks) per block and blocks per SM (0: as many as fit); shapes that do not fit
-        // the launch's instantiation or shared memory are skipped
-        const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
-                                              {5, 1}, {6, 1}, {7, 1}, {8, 1}};
-        for (const auto& s : shapes) {
-            c->tune_force = s;
-            try {
-                run();  // warm-up (and the shape's work-item table)
-                ck(cudaEventRecord(a, c->stream), "cudaEventRecord");
-                run();
-                run();
-                ck(cudaEventRecord(b, c->stream), "cudaEventRecord");
-                check_status(c);
-            } catch (const Fail& f) {
-                if (f.code != VC1CU_ERR_ARG) {  // a shape that does not fit is skipped, anything else fails
-                    c->tune_force = {0, 0};
-                    c->event_pool.push_back(a);
-                    c->event_pool.push_back(b);
-                    throw;
-                }
-                continue;
+        double total = 0.0, longest = -1.0;
+        std::pair<int, int> shown{0, 0};
+        // each of the call's launches in turn (a later one reads the seeds an earlier one leaves)
+        for (const std::vector<int>& g : plan_launches(c, params, passes, n, pp)) {
+            std::vector<vc1cu_pass> q;
+            std::vector<vc1cu_params> gp;
+            for (int i : g) {
+                q.push_back(passes[i]);
+                if (pp) gp.push_back(pp[i]);
             }
-            float ms = 0.f;
-            ck(cudaEventElapsedTime(&ms, a, b), "cudaEventElapsedTime");
-            key = c->last_tune_key;
-            if (best < 0.0 || ms < best) {
-                best = ms;
-                best_shape = s;
+            auto run = [&]() { launch_group(c, params, q.data(), (int)q.size(), false, nullptr, pp ? gp.data() : nullptr); };
+            double best = -1.0;
+            std::pair<int, int> best_shape{0, 0};
+            std::vector<int> key;
+            // warps (macroblocks) per block and blocks per SM (0: as many as fit); shapes that do not fit
+            // the launch's instantiation or shared memory are skipped
+            const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
+                                                  {5, 1}, {6, 1}, {7, 1}, {8, 1}};
+            for (const auto& s : shapes) {
+                c->tune_force = s;
+                try {
+                    run();  // warm-up (and the shape's work-item table)
+                    ck(cudaEventRecord(a, c->stream), "cudaEventRecord");
+                    run();
+                    run();
+                    ck(cudaEventRecord(b, c->stream), "cudaEventRecord");
+                    check_status(c);
+                } catch (const Fail& f) {
+                    if (f.code != VC1CU_ERR_ARG) {  // a shape that does not fit is skipped, anything else fails
+                        c->tune_force = {0, 0};
+                        c->event_pool.push_back(a);
+                        c->event_pool.push_back(b);
+                        throw;
+                    }
+                    continue;
+                }
+                float ms = 0.f;
+                ck(cudaEventElapsedTime(&ms, a, b), "cudaEventElapsedTime");
+                key = c->last_tune_key;
+                if (best < 0.0 || ms < best) {
+                    best = ms;
+                    best_shape = s;
+                }
+            }
+            c->tune_force = {0, 0};
+            if (best < 0.0) {
+                c->event_pool.push_back(a);
+                c->event_pool.push_back(b);
+                throw Fail{VC1CU_ERR_UNSUPPORTED, "no launch shape fits"};
+            }
+            c->tuned[key] = best_shape;
+            total += best / 2.0;
+            if (best > longest) {
+                longest = best;
+                shown = best_shape;
             }
         }
-        c->tune_force = {0, 0};
         c->event_pool.push_back(a);
         c->event_pool.push_back(b);
-        if (best < 0.0) throw Fail{VC1CU_ERR_UNSUPPORTED, "no launch shape fits"};
-        c->tuned[key] = best_shape;
-        if (warps_out) *warps_out = best_shape.first;
-        if (blocks_out) *blocks_out = best_shape.second;
-        if (ms_out) *ms_out = best / 2.0;
+        if (warps_out) *warps_out = shown.first;
+        if (blocks_out) *blocks_out = shown.second;
+        if (ms_out) *ms_out = total;
         return VC1CU_OK;
     });
 }

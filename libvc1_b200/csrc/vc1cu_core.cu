@@ -131,6 +131,7 @@ struct Mb {
     WarpMem sm;
     int wx0, wy0, wp, wh;  // window origin (wx0 a multiple of 16), row pitch = width, height
     GlobSampler gref;
+    bool wide;             // the build has registers for the larger SAD groups (a constant where known)
     uint32_t tma_phase;    // parity of the window mbarrier's next phase
     bool tma_pending;      // a TMA window copy is in flight
 };
@@ -305,13 +306,15 @@ __device__ __forceinline__ void win_load16(uint32_t off, uint32_t r[4]) {
     r[3] = __funnelshift_r(w3, w4, sh);
 }
 
-// mb_sad of a full 16x16 MB from the window with packed byte SADs (__vsadu4), strides 1/2/4.
+// mb_sad from the window with packed byte SADs (__vsadu4), strides 1/2/4: the first ah rows, whose
+// 16 columns are all visible.
 template <int STRIDE>
-__device__ __forceinline__ uint32_t sad_packed(uint32_t cur_off, uint32_t cur2_off, uint32_t cur4_off, int wp, uint32_t base) {
+__device__ __forceinline__ uint32_t sad_packed(uint32_t cur_off, uint32_t cur2_off, uint32_t cur4_off, int wp, uint32_t base,
+                                               int ah) {
     uint32_t acc = 0;
     const uint32_t c = cur_off >> 2, c2 = cur2_off >> 2, c4 = cur4_off >> 2;
 #pragma unroll 4
-    for (int y = 0; y < 16; y += STRIDE) {
+    for (int y = 0; y < ah; y += STRIDE) {
         uint32_t r[4];
         win_load16(base + (uint32_t)(y * wp), r);
         if (STRIDE == 1) {
@@ -343,15 +346,14 @@ __device__ __forceinline__ void glob_load16(const uint8_t* p, uint32_t r[4]) {
     r[3] = __funnelshift_r(w3, w4, sh);
 }
 
-// mb_sad of a full 16x16 MB whose reference block lies inside the frame, read from global
-// memory (the frames stay in L2) with the same packed byte SADs as sad_packed.
+// The same of a block inside the frame, read from global memory (the frames stay in L2).
 template <int STRIDE>
 __device__ __forceinline__ uint32_t sad_packed_glob(uint32_t cur_off, uint32_t cur2_off, uint32_t cur4_off,
-                                                    const uint8_t* ref, int pitch) {
+                                                    const uint8_t* ref, int pitch, int ah) {
     uint32_t acc = 0;
     const uint32_t c = cur_off >> 2, c2 = cur2_off >> 2, c4 = cur4_off >> 2;
 #pragma unroll 4
-    for (int y = 0; y < 16; y += STRIDE) {
+    for (int y = 0; y < ah; y += STRIDE) {
         uint32_t r[4];
         glob_load16(ref + (size_t)y * pitch, r);
         if (STRIDE == 1) {
@@ -465,22 +467,22 @@ __device__ __noinline__ uint64_t mb_sad_core(uint32_t ctx, int dx, int dy, int s
     uint32_t s;
     const int xa = c.x0 + dx, ya = c.y0 + dy;
     const bool fast = xa >= c.wx0 && ya >= c.wy0 && xa + 15 < c.wx0 + c.wp && ya + 15 < c.wy0 + c.wh;
-    if (fast && c.aw == 16 && c.ah == 16) {
+    if (fast && c.aw == 16) {
         const uint32_t base = c.win_off + (uint32_t)((ya - c.wy0) * c.wp + (xa - c.wx0));
-        if (stride == 1) s = sad_packed<1>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base);
-        else if (stride == 2) s = sad_packed<2>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base);
-        else s = sad_packed<4>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base);
+        if (stride == 1) s = sad_packed<1>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base, c.ah);
+        else if (stride == 2) s = sad_packed<2>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base, c.ah);
+        else s = sad_packed<4>(c.cur_off, c.cur2_off, c.cur4_off, c.wp, base, c.ah);
     } else if (fast) {
         const WinSampler ws{c.win_off, c.wp, c.wx0, c.wy0, c.wh};
         if (stride == 1) s = sad_int_loop<1>(ws, c.cur_off, c.x0, c.y0, dx, dy, c.aw, c.ah);
         else if (stride == 2) s = sad_int_loop<2>(ws, c.cur_off, c.x0, c.y0, dx, dy, c.aw, c.ah);
         else s = sad_int_loop<4>(ws, c.cur_off, c.x0, c.y0, dx, dy, c.aw, c.ah);
-    } else if (c.aw == 16 && c.ah == 16 && xa >= 0 && ya >= 0 && xa + 16 <= P.W && ya + 16 <= P.H) {
+    } else if (c.aw == 16 && xa >= 0 && ya >= 0 && xa + 16 <= P.W && ya + c.ah <= P.H) {
         // outside the staged window but inside the frame: no clamping, packed rows from L2
         const uint8_t* base = c.gref + (size_t)ya * c.gpitch + xa;
-        if (stride == 1) s = sad_packed_glob<1>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch);
-        else if (stride == 2) s = sad_packed_glob<2>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch);
-        else s = sad_packed_glob<4>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch);
+        if (stride == 1) s = sad_packed_glob<1>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch, c.ah);
+        else if (stride == 2) s = sad_packed_glob<2>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch, c.ah);
+        else s = sad_packed_glob<4>(c.cur_off, c.cur2_off, c.cur4_off, base, c.gpitch, c.ah);
     } else {
         const GlobSampler gs{c.gref, c.gpitch, P.W, P.H};
         if (stride == 1) s = sad_int_loop<1>(gs, c.cur_off, c.x0, c.y0, dx, dy, c.aw, c.ah);
@@ -564,7 +566,9 @@ __device__ __noinline__ uint32_t sad_interpolated(uint32_t ctx, int mvx, int mvy
 // by their number. Two SADs share a word in the warp sum (a 16x16 SAD is below 2^16). With the
 // keyed list and the word-wise minima below, a refinement takes 16 K clocks against 43 K for one
 // candidate at a time and selections by shuffles of whole structures (CIF, one macroblock alone).
-constexpr int kSadGroup = 5;  // candidates whose rows are in flight together (registers bound it)
+// GROUP: the 16x16 candidates whose rows are in flight together (registers bound it: nine, a whole
+// stencil, in the wide-register builds; five under the seeded builds' 128 registers).
+template <int GROUP>
 __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int n, int bx, int by,
                                             int bw, int bh, int mode, uint32_t out_off) {
     const MbCtx& c = mbctx(ctx);
@@ -591,11 +595,11 @@ __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int 
         const uint32_t a0 = g_smem32[cw] & m0, a1 = g_smem32[cw + 1] & m1;
         const uint8_t* seg = c.sp + (long long)r * c.sp_pitch + c0;
 #pragma unroll 1
-        for (int base = 0; base < n; base += kSadGroup) {
-            uint32_t part[kSadGroup + 1];
-            part[kSadGroup] = 0;
+        for (int base = 0; base < n; base += GROUP) {
+            uint32_t part[GROUP + 1];
+            part[GROUP] = 0;
 #pragma unroll
-            for (int u = 0; u < kSadGroup; ++u) {
+            for (int u = 0; u < GROUP; ++u) {
                 part[u] = 0;
                 const long long o = __shfl_sync(FULL, off, (base + u) & 31);
                 if (base + u < n && o >= 0) {
@@ -605,10 +609,10 @@ __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int 
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kSadGroup; u += 2) {
+            for (int u = 0; u < GROUP; u += 2) {
                 const uint32_t two = __reduce_add_sync(FULL, part[u] | (part[u + 1] << 16));
                 if (lane == base + u) mine = two & 0xffffu;
-                if (u + 1 < kSadGroup && lane == base + u + 1) mine = two >> 16;
+                if (u + 1 < GROUP && lane == base + u + 1) mine = two >> 16;
             }
         }
     } else {
@@ -740,7 +744,8 @@ __device__ __noinline__ void satd_batch_core(uint32_t ctx, uint32_t mvs_off, int
 // mvs and out point into the warp's shared-memory buffers.
 __device__ __forceinline__ void sad_batch(const DevParams& P, const Mb& m, const int2* mvs, int n, int bx, int by, int bw,
                                           int bh, int mode, uint64_t* out) {
-    sad_batch_core(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
+    if (m.wide) sad_batch_core<9>(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
+    else sad_batch_core<5>(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
 }
 
 __device__ __forceinline__ void satd_batch(const DevParams& P, const Mb& m, const int2* mvs, int n, int bx, int by, int bw,
@@ -782,6 +787,22 @@ __device__ __forceinline__ void top4_insert(Top4& t, uint64_t k) {
     if (t.b < t.a) { t.b = t.a; t.a = k; }
 }
 
+// The four least distinct keys among every lane's four, on every lane.
+__device__ __forceinline__ Top4 top4_gather(Top4 own) {
+    uint64_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        r[i] = warp_min_key(own.a);
+        if (own.a == r[i]) {
+            own.a = own.b;
+            own.b = own.c;
+            own.c = own.d;
+            own.d = UINT64_MAX;
+        }
+    }
+    return Top4{r[0], r[1], r[2], r[3]};
+}
+
 // Merges one key per lane (UINT64_MAX: none) into the four least.
 __device__ __forceinline__ void top4_merge(Top4& t, uint64_t key) {
     while (__any_sync(FULL, key < t.d)) {
@@ -796,7 +817,7 @@ struct SearchGeo {
     uint32_t win, cur, cur2, cur4;
     int wp, wx0, wy0, wh, x0, y0, xl, yl, W, H, gpitch;
     const uint8_t* gref;
-    bool whole;  // all 16x16 pixels inside the raster
+    int aw, ah;  // the columns and rows inside the raster
     __device__ __forceinline__ explicit SearchGeo(uint32_t ctx) {
         const MbCtx& c = mbctx(ctx);
         win = c.win_off;
@@ -815,33 +836,43 @@ struct SearchGeo {
         H = c.g.H;
         gref = c.gref;
         gpitch = c.gpitch;
-        whole = c.aw == 16 && c.ah == 16;
+        aw = c.aw;
+        ah = c.ah;
     }
     // the candidate's block lies in the window
     __device__ __forceinline__ bool staged(int dx, int dy) const {
         const int rx = x0 + dx - wx0, ry = y0 + dy - wy0;
-        return whole && rx >= 0 && ry >= 0 && rx + 16 <= wp && ry + 16 <= wh;
+        return rx >= 0 && ry >= 0 && rx + 16 <= wp && ry + 16 <= wh;
     }
     // the candidate's block lies in the frame
     __device__ __forceinline__ bool inside(int dx, int dy) const {
         const int x = x0 + dx, y = y0 + dy;
-        return whole && x >= 0 && y >= 0 && x + 16 <= W && y + 16 <= H;
+        return aw == 16 && x >= 0 && y >= 0 && x + 16 <= W && y + ah <= H;
     }
     __device__ __forceinline__ uint32_t base(int dx, int dy) const {
         return win + (uint32_t)((y0 + dy - wy0) * wp + (x0 + dx - wx0));
     }
 };
 
-// Packed SAD of the sampled rows r0 .. r0 + nr - 1 of a candidate, its rows staged in the window
-// (at shared offset base) or, GLOBAL, read from the frame (at ref).
+// Packed SAD of the sampled rows r0 .. r0 + nr - 1 (those inside the raster) of a candidate, its
+// rows staged in the window (at shared offset base) or, GLOBAL, read from the frame (at ref). The
+// current macroblock is zero outside the raster, so its columns there only need the reference's
+// bytes masked away: a bottom row of half macroblocks (1080 lines) runs like any other, where byte
+// loops made it the tail of every 1080p wavefront (120 macroblocks one behind the other).
 template <int STRIDE, bool GLOBAL>
 __device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, const uint8_t* ref, int r0, int nr) {
     uint32_t acc = 0;
+    const int end = imin(r0 + nr, (g.ah + STRIDE - 1) / STRIDE);
+    const bool ragged = g.aw < 16;
 #pragma unroll 2
-    for (int r = r0; r < r0 + nr; ++r) {
+    for (int r = r0; r < end; ++r) {
         uint32_t v[4];
         if (GLOBAL) glob_load16(ref + (size_t)(r * STRIDE) * g.gpitch, v);
         else win_load16(base + (uint32_t)(r * STRIDE * g.wp), v);
+        if (ragged) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] &= vis_mask(g.aw - 4 * i);
+        }
         if (STRIDE == 1) {
             acc += __vsadu4(v[0], g_smem32[g.cur + r * 4]) + __vsadu4(v[1], g_smem32[g.cur + r * 4 + 1]) +
                    __vsadu4(v[2], g_smem32[g.cur + r * 4 + 2]) + __vsadu4(v[3], g_smem32[g.cur + r * 4 + 3]);
@@ -1014,7 +1045,9 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
     const SearchGeo g(ctx);
     const int lane = threadIdx.x & 31;
     const int2* seeds = reinterpret_cast<const int2*>(g_smem + seeds_off);
-    Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
+    // Each lane keeps the four least of the keys it scored; a stage only needs the least of all.
+    Top4 own{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
+    uint64_t best = UINT64_MAX;
     const int cs = range >= 96 ? 8 : (range >= 32 ? 4 : 2);
     const int nh = range / cs, nv = imin(range, imax(8, range / 2)) / cs;
     const int hs = range >= 96 ? 8 : (range >= 24 ? 4 : 2);
@@ -1023,7 +1056,8 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
 #pragma unroll 1
     while (stage != kDone) {
         // the stage's centre is the least candidate before it
-        const int cx = key_dx(t.a), cy = key_dy(t.a);
+        const int cx = key_dx(best), cy = key_dy(best);
+        uint64_t least = UINT64_MAX;
         const int n = stage == kSeeds ? ns : stage == kSquare ? 25 : stage == kCross ? 2 * (nh + nv)
                     : stage == kRings ? 6 * (range / hs) : stage == kHexagon ? 6 : 4;
 #pragma unroll 1
@@ -1055,19 +1089,21 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
             }
             dx = iclamp(dx, -range, range);
             dy = iclamp(dy, -range, range);
-            top4_merge(t, shared_key<2>(ctx, g, i < n, dx, dy, sh));
+            const uint64_t k = shared_key<2>(ctx, g, i < n, dx, dy, sh);
+            least = k < least ? k : least;
+            top4_insert(own, k);
             base += 32 >> sh;
         }
-        if (stage == kSquare && range >= 8) {
-            const uint64_t* top = reinterpret_cast<const uint64_t*>(g_smem + top_off);
-            const uint64_t l0 = top[0], l1 = top[1], l2 = top[2], l3 = top[3];
-            top4_insert(t, l0);
-            top4_insert(t, l1);
-            top4_insert(t, l2);
-            top4_insert(t, l3);
+        if (stage == kSquare && range >= 8 && lane < 4) {  // the lattice comes after the square
+            const uint64_t k = reinterpret_cast<const uint64_t*>(g_smem + top_off)[lane];
+            least = k < least ? k : least;
+            top4_insert(own, k);
         }
-        if (stage != kHexagon || ++iter == 32 || (key_dx(t.a) == cx && key_dy(t.a) == cy)) ++stage;
+        least = warp_min_key(least);
+        if (least < best) best = least;
+        if (stage != kHexagon || ++iter == 32 || (key_dx(best) == cx && key_dy(best) == cy)) ++stage;
     }
+    const Top4 t = top4_gather(own);
     // full-resolution 3x3 about the four finalists (:1929-1952)
     uint64_t fk = UINT64_MAX;
     const int nf = 9 * ((t.a != UINT64_MAX) + (t.b != UINT64_MAX) + (t.c != UINT64_MAX) + (t.d != UINT64_MAX));
@@ -1918,6 +1954,7 @@ __device__ __forceinline__ void ref_unpack(uint32_t ctx, DevParams& P, Mb& m) {
     P.mvrange = r.mvrange;
     P.mant_bits = r.mant_bits;
     m.lane = threadIdx.x & 31;
+    m.wide = false;
     m.lam_m = r.lam_m;
     m.lam_s = r.lam_s;
     m.x0 = r.x0;
@@ -1969,12 +2006,21 @@ __device__ __noinline__ RefineOut refine_select_ool(uint32_t ctx, const Shortlis
     return refine_select(P, m, sl, bx, by, bw, bh, mode, pi, more);
 }
 
-template <bool DR>
-__device__ __forceinline__ RefineOut refine_staged(const DevParams& P, const Mb& m, int bx, int by, int bw, int bh, int2 seed,
+// INLINE: the launch refines at this one place (unseeded passes without Mixed-MV blocks), so both
+// halves are compiled into it: no parameter block is rebuilt and no shortlist passes through the stack.
+template <bool DR, bool INLINE>
+__device__ __forceinline__ RefineOut refine_staged(const DevParams& P0, const Mb& m, int bx, int by, int bw, int bh, int2 seed,
                                                    int range, int mode, const PInfo& pi, bool more, uint64_t known) {
-    const uint32_t r = m.sm.ctx.off;
-    const Shortlist sl = refine_prepare_ool<DR>(r, bx, by, bw, bh, seed, range, mode, known, false);
-    return refine_select_ool<DR>(r, sl, bx, by, bw, bh, mode, pi, more);
+    if constexpr (INLINE) {
+        DevParams P = P0;
+        refine_defaults<DR>(P);
+        const Shortlist sl = refine_prepare(P, m, bx, by, bw, bh, seed, range, mode, known, false);
+        return refine_select(P, m, sl, bx, by, bw, bh, mode, pi, more);
+    } else {
+        const uint32_t r = m.sm.ctx.off;
+        const Shortlist sl = refine_prepare_ool<DR>(r, bx, by, bw, bh, seed, range, mode, known, false);
+        return refine_select_ool<DR>(r, sl, bx, by, bw, bh, mode, pi, more);
+    }
 }
 
 // ---- shortlists parked across the wavefront wait -----------------------------------------
@@ -2480,13 +2526,12 @@ __device__ uint64_t intra_proxy(const DevParams& P, const Mb& m) {
 }
 
 // items[k] = (pass << 20) | macroblock: the launch's work queue. Inside one pass the
-// macroblocks come in wavefront order (t = x + 2y, then y), so every same-pass dependency
-// (left, top-left, top, top-right) of an item precedes it and the items of one t are
-// independent; a pass seeded by another pass of the launch is delayed behind it, so its
-// seed macroblock precedes it too. Items are handed out in order, hence no wait can
-// depend on an item that no running warp holds.
-// Instantiations (the kCore* flags): kCoreAny runs any mix of passes; the flags compile out what
-// a launch's passes cannot reach (seeded-only launches also need fewer registers and hold more
+// macroblocks come in wavefront order (t = x + 2y, then y), so every dependency (left, top-left,
+// top, top-right) of an item precedes it and the items of one t are independent. Items are handed
+// out in order, hence no wait can depend on an item that no running warp holds. A pass's seed
+// comes from an earlier launch.
+// Instantiations (the kCore* flags): a launch's passes are all seeded or all unseeded; the flags
+// compile out what they cannot reach (seeded-only launches also need fewer registers and hold more
 // resident warps). Four warps per block; at most 65536 / (128 * min blocks) registers per thread.
 #ifndef VC1CU_CORE_MIN_BLOCKS
 #define VC1CU_CORE_MIN_BLOCKS 3
@@ -2538,17 +2583,17 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
         const DevResult& o = d.out;
         constexpr bool kUmhOnly = (KIND & kCoreUmhLocal) != 0;
         constexpr bool kDR = (KIND & kCoreDefaultRefine) != 0;
+        constexpr bool kInline = (KIND & kCoreUnseededOnly) != 0 && (KIND & kCoreNoMixed) != 0;
+        m.wide = kInline;
         const int mode = d.mode,
-                  seeded = (KIND & kCoreSeededOnly) ? 1 : ((KIND & kCoreUnseededOnly) ? 0 : d.seeded);
+                  seeded = (KIND & kCoreSeededOnly) ? 1 : 0;
         const bool allow_intra = !(KIND & kCoreNoIntra) && d.allow_intra && !P.disable_p_intra;
         const bool allow_4mv = !(KIND & kCoreNoMixed) && mode == VC1CU_MV_MIXED;
         const int one_mode = allow_4mv ? VC1CU_MV_QPEL : mode;
         PHASE_START((seeded ? 1 : 0) + (allow_4mv ? 2 : 0));
         bool ok = !*(volatile int*)&st->abort;
+        bool published = false;
         if (d.only && !__ldcg(&d.only[mbi])) ok = false;  // keeps the slot's result, publishes at once
-        // a seed produced by another pass of this launch
-        if (ok && d.seed_pass >= 0)
-            ok = wait_flags(m.lane == 0 ? &passes[d.seed_pass].out.done[mbi] : nullptr, epoch, st, code, P.wait_log2);
         PHASE_MARK(0);
         if (ok) load_cur(P, m, d.cur);
         PHASE_MARK(1);
@@ -2580,14 +2625,10 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
         double dl = -1.0, dc = -1.0;
         uint8_t dd = 0;
         uint64_t intra_sad = 0;
-        // Mixed-MV speculation: the 4MV block work for a guessed 1-MV vector runs before the
-        // wait and is kept when the vector chosen after it matches (seeds from earlier launches)
-        // Speculation: with the seed pass's neighbourhood standing in for this pass's, the
-        // refinements (and for Mixed-MV every block's) run before the wait; after it each
-        // result is kept where the real predictor equals the guessed one (seeds produced by
-        // earlier launches only)
-        const bool spec = seeded && d.seed_pass < 0;
-        const bool spec4 = allow_4mv && spec;
+        // Speculation of seeded passes: with the seed pass's neighbourhood standing in for this
+        // pass's, the refinements (and for Mixed-MV every block's) run before the wait; after it each
+        // result is kept where the real predictor equals the guessed one
+        const bool spec4 = allow_4mv && seeded;
         int2 one_g = make_int2(0, 0);
         IntRes learned{0, 0, UINT64_MAX};  // learned passes: the integer vector before refinement
         IntRes ext_best{0, 0, UINT64_MAX};  // the content-signature search, where it ran before the wait
@@ -2607,42 +2648,40 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 dl = __ldcg(&d.seed_dl[m.pos]);
                 dc = __ldcg(&d.seed_dc[m.pos]);
                 dd = __ldcg(&d.seed_dd[m.pos]);
-                if (spec) {
-                    guess_neighbours(P, m, d);
-                    int2* cur4g = m.sm.cur_bmv;
-                    const Field fg{cur4g, m.sm.nb_bmv, m.sm.nb_intra, P.mbw, P.mbh, m.mx, m.my};
-                    const PInfo pig = predictor_mixed_1mv(P, fg, m.mx, m.my);
-                    shortlist_save(m, 0, sl, seed, 0, 0);
-                    const RefineOut og = refine_select_ool<kDR>(m.sm.ctx.off, sl, m.x0, m.y0, 16, 16, one_mode, pig, true);
-                    spec_result_save(m, 0, pig, og);
-                    one_g = og.mv;
-                    if (hidden_padding(P, m.x0, m.y0, 16, 16, one_g.x, one_g.y, one_mode, true)) one_g = make_int2(0, 0);
-                    if (spec4) {
-                        if (m.lane < 4) cur4g[m.lane] = one_g;
-                        __syncwarp();
-                        for (int k = 0; k < 4; ++k) {
-                            const int bx = m.x0 + (k & 1) * 8, by = m.y0 + ((k >> 1) & 1) * 8;
-                            const PInfo pi4g = predictor_4mv(P, fg, m.mx, m.my, k);
-                            put_4mv_seeds(P, m, one_g, pi4g.pre, qb);
-                            sad_batch(P, m, m.sm.batch, 11, bx, by, 8, 8, VC1CU_MV_QPEL, m.sm.batch_cost);
-                            const SeedPick b10 = pick_4mv_seed(m, true);
-                            const SeedPick bf = pick_4mv_seed(m, false);
-                            const uint32_t rc = m.sm.ctx.off;
-                            const Shortlist sk = refine_prepare_ool<kDR>(rc, bx, by, 8, 8, bf.v, range, VC1CU_MV_MIXED, bf.cost, true);
-                            shortlist_save(m, k + 1, sk, bf.v, bf.cost, bf.slot);
-                            const RefineOut rk = refine_select_ool<kDR>(rc, sk, bx, by, 8, 8, VC1CU_MV_MIXED, pi4g, true);
-                            if (m.lane == 0) {
-                                SpecBlk& sb = m.sm.spec_blk[k + 1];
-                                sb.b10 = b10.v;
-                                sb.b10_cost = b10.cost;
-                                sb.b10_slot = b10.slot;
-                                cur4g[k] = rk.mv;
-                            }
-                            spec_result_save(m, k + 1, pi4g, rk);
+                guess_neighbours(P, m, d);
+                int2* cur4g = m.sm.cur_bmv;
+                const Field fg{cur4g, m.sm.nb_bmv, m.sm.nb_intra, P.mbw, P.mbh, m.mx, m.my};
+                const PInfo pig = predictor_mixed_1mv(P, fg, m.mx, m.my);
+                shortlist_save(m, 0, sl, seed, 0, 0);
+                const RefineOut og = refine_select_ool<kDR>(m.sm.ctx.off, sl, m.x0, m.y0, 16, 16, one_mode, pig, true);
+                spec_result_save(m, 0, pig, og);
+                one_g = og.mv;
+                if (hidden_padding(P, m.x0, m.y0, 16, 16, one_g.x, one_g.y, one_mode, true)) one_g = make_int2(0, 0);
+                if (spec4) {
+                    if (m.lane < 4) cur4g[m.lane] = one_g;
+                    __syncwarp();
+                    for (int k = 0; k < 4; ++k) {
+                        const int bx = m.x0 + (k & 1) * 8, by = m.y0 + ((k >> 1) & 1) * 8;
+                        const PInfo pi4g = predictor_4mv(P, fg, m.mx, m.my, k);
+                        put_4mv_seeds(P, m, one_g, pi4g.pre, qb);
+                        sad_batch(P, m, m.sm.batch, 11, bx, by, 8, 8, VC1CU_MV_QPEL, m.sm.batch_cost);
+                        const SeedPick b10 = pick_4mv_seed(m, true);
+                        const SeedPick bf = pick_4mv_seed(m, false);
+                        const uint32_t rc = m.sm.ctx.off;
+                        const Shortlist sk = refine_prepare_ool<kDR>(rc, bx, by, 8, 8, bf.v, range, VC1CU_MV_MIXED, bf.cost, true);
+                        shortlist_save(m, k + 1, sk, bf.v, bf.cost, bf.slot);
+                        const RefineOut rk = refine_select_ool<kDR>(rc, sk, bx, by, 8, 8, VC1CU_MV_MIXED, pi4g, true);
+                        if (m.lane == 0) {
+                            SpecBlk& sb = m.sm.spec_blk[k + 1];
+                            sb.b10 = b10.v;
+                            sb.b10_cost = b10.cost;
+                            sb.b10_slot = b10.slot;
+                            cur4g[k] = rk.mv;
                         }
+                        spec_result_save(m, k + 1, pi4g, rk);
                     }
-                    PHASE_MARK(12);
                 }
+                PHASE_MARK(12);
             } else if constexpr ((KIND & kCoreLearned) != 0) {
                 // the candidates' exact costs on the full-resolution picture, then a short descent
                 // in a small window about the best (neighbour-independent, before the wait)
@@ -2692,16 +2731,16 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
             bool distant = false;  // the integer vector came from a long-range search
             PHASE_MARK(6);
             if (seeded) {
-                if (spec && pinfo_equal(rate_pi, m.sm.spec_blk[0].pi)) {
+                if (pinfo_equal(rate_pi, m.sm.spec_blk[0].pi)) {
                     one = m.sm.spec_blk[0].res;
                 } else {
-                    if (spec) shortlist_restore(m, 0);
+                    shortlist_restore(m, 0);
                     one = refine_select_ool<kDR>(m.sm.ctx.off, sl, m.x0, m.y0, 16, 16, one_mode, rate_pi, true);
                 }
             } else if constexpr ((KIND & kCoreLearned) != 0) {
                 if (pixels) dl = (double)learned.cost / (double)pixels;
                 PHASE_MARK(7);
-                one = refine_staged<kDR>(P, m, m.x0, m.y0, 16, 16, make_int2(learned.dx * 4, learned.dy * 4), range,
+                one = refine_staged<kDR, kInline>(P, m, m.x0, m.y0, 16, 16, make_int2(learned.dx * 4, learned.dy * 4), range,
                                          one_mode, rate_pi, true, learned.cost);
             } else {
                 const PInfo pi = predictor_info(P, m);
@@ -2766,7 +2805,7 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                     }
                 }
                 PHASE_MARK(7);
-                one = refine_staged<kDR>(P, m, m.x0, m.y0, 16, 16, make_int2(im.dx * 4, im.dy * 4), range, one_mode, rate_pi,
+                one = refine_staged<kDR, kInline>(P, m, m.x0, m.y0, 16, 16, make_int2(im.dx * 4, im.dy * 4), range, one_mode, rate_pi,
                                     true, im.cost);
             }
             PHASE_MARK(8);
@@ -2830,7 +2869,7 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                         seed_cost = b.cost;
                     }
                     PHASE_MARK(9);
-                    if (!have) r = refine_staged<kDR>(P, m, bx, by, 8, 8, best_seed, range, VC1CU_MV_MIXED, pi4, true, seed_cost);
+                    if (!have) r = refine_staged<kDR, kInline>(P, m, bx, by, 8, 8, best_seed, range, VC1CU_MV_MIXED, pi4, true, seed_cost);
                     PHASE_MARK(10);
                     four_screen += r.screen_sad;
                     if (m.lane == 0) cur4[k] = r.mv;
@@ -2885,11 +2924,16 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 moved |= out4[k].x != 0 || out4[k].y != 0;
                 frac |= (out4[k].x % 8) != 0 || (out4[k].y % 8) != 0;
             }
+            // what the neighbours read, then the flag, then the rest (which only later launches read)
             if (m.lane == 0) {
                 o.mvs[m.pos] = out_mv;
-                for (int k = 0; k < 4; ++k) o.bmv[m.pos * 4 + k] = out4[k];
-                o.use4[m.pos] = use4;
                 o.intra[m.pos] = intra;
+                o.flags[m.pos] = (uint8_t)((moved ? 1 : 0) | (frac ? 2 : 0) | (distant ? 4 : 0) | (chose4 ? 8 : 0));
+                int4* b4 = reinterpret_cast<int4*>(&o.bmv[m.pos * 4]);
+                b4[0] = make_int4(out4[0].x, out4[0].y, out4[1].x, out4[1].y);
+                b4[1] = make_int4(out4[2].x, out4[2].y, out4[3].x, out4[3].y);
+                if (code != P.withhold) st_release(&o.done[m.pos], epoch);
+                o.use4[m.pos] = use4;
                 o.screen[m.pos] = temporal_screen;
                 o.ratio[m.pos] = ratio;
                 o.dl[m.pos] = dl;
@@ -2897,14 +2941,11 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 o.dd[m.pos] = dd;
                 o.chosen[m.pos] = chosen;
                 o.temporal[m.pos] = temporal;
-                o.flags[m.pos] = (uint8_t)((moved ? 1 : 0) | (frac ? 2 : 0) | (distant ? 4 : 0) | (chose4 ? 8 : 0));
             }
+            published = true;
         }
-        __syncwarp();
-        if (m.lane == 0 && code != P.withhold) {
-            __threadfence();
-            st_release(&o.done[m.pos], epoch);
-        }
+        // macroblocks that took no part in the analysis (range 0, not flagged, an aborted launch)
+        if (!published && m.lane == 0 && code != P.withhold) st_release(&o.done[m.pos], epoch);
         __syncwarp();
         PHASE_MARK(11);
     }
@@ -2951,7 +2992,7 @@ cudaError_t launch_lr_index(const DevFrame& ref, int W, int H, uint64_t* out, cu
 // Host-side handles of the instantiations (attributes, occupancy, launch): the flag sets the
 // host selects.
 #define VC1CU_CORE_KINDS(X)                                                                      \
-    X(kCoreAny) X(kCoreAny | kCoreWide) X(kCoreSeededOnly) X(kCoreSeededOnly | kCoreNoMixed)     \
+    X(kCoreSeededOnly) X(kCoreSeededOnly | kCoreNoMixed)                                               \
     X(kCoreUnseededOnly) X(kCoreUnseededOnly | kCoreWide) X(kCoreUnseededOnly | kCoreUmhLocal)   \
     X(kCoreUnseededOnly | kCoreUmhLocal | kCoreWide) X(kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed) \
     X(kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed | kCoreWide)                                \
@@ -2968,7 +3009,12 @@ cudaError_t launch_lr_index(const DevFrame& ref, int W, int H, uint64_t* out, cu
     X(kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed | kCoreWide | kCoreDefaultRefine | kCoreNoIntra)    \
     X(kCoreUnseededOnly | kCoreLearned | kCoreNoMixed | kCoreNoIntra)                                   \
     X(kCoreUnseededOnly | kCoreLearned | kCoreNoMixed | kCoreNoIntra | kCoreDefaultRefine)                 \
-    X(kCoreMulti) X(kCoreMulti | kCoreWide)
+    X(kCoreMulti | kCoreUnseededOnly) X(kCoreMulti | kCoreUnseededOnly | kCoreWide)                     \
+    X(kCoreMulti | kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed | kCoreDefaultRefine | kCoreNoIntra)   \
+    X(kCoreMulti | kCoreUnseededOnly | kCoreUmhLocal | kCoreNoMixed | kCoreWide | kCoreDefaultRefine |     \
+      kCoreNoIntra)                                                                                      \
+    X(kCoreMulti | kCoreSeededOnly) X(kCoreMulti | kCoreSeededOnly | kCoreDefaultRefine)                 \
+    X(kCoreMulti | kCoreSeededOnly | kCoreDefaultRefine | kCoreNoIntra)
 
 const void* core_kernel(int kind) {
     switch (kind) {

@@ -55,7 +55,6 @@ struct alignas(64) PassDesc {
     uint64_t lam_m;        // lambda = lam_m * 2^-lam_s exactly
     int lam_s;
     int seeded;            // 1: seed fields below are valid
-    int seed_pass;         // index of the seeding pass in the same launch, -1 if produced earlier
     const int2* seed_mvs;
     const int2* seed_bmv;        // the seed pass's block vectors and P-intra flags (only used to
     const uint8_t* seed_intra;   // guess this pass's predictors before the wavefront wait)
@@ -94,8 +93,6 @@ constexpr int kCoreLearned = 128;       // (with kCoreUnseededOnly) the integer 
                                         // candidates' exact costs and a short descent about the best
 constexpr int kCoreMulti = 256;         // passes of pictures of different sizes in one launch: each
                                         // work item takes its pass's own geometry
-constexpr int kCoreAny = 0;
-constexpr int kCoreSeeded = kCoreSeededOnly;
 
 // Shared-memory window geometry for one launch.
 struct WinCfg {
