@@ -9,6 +9,7 @@
 // operations with __dmul_rn/__dadd_rn), then scalar_quantize_level (:1067-1085).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstring>
 
@@ -404,11 +405,14 @@ void launch_xform(const DevParams& P, const DevFrame& src, const DevFrame& pred,
 
 // ---- transform RD of the default presets (choose_transform_mb, encoder_transform.cpp:1605-1780) ----
 //
-// One warp per macroblock. The lanes evaluate the candidate types' 24 (type, parent) pairs at
-// once (forward transform, scalar or trellis quantisation, inverse transform, reconstruction SSE,
-// bit estimate); lane 0 then takes the macroblock- and block-level decisions in the reference's
-// order; the trellis re-evaluation of the winners is again one parent per lane. Every double
-// operation is the reference's, in its order (this file is compiled without contraction).
+// One block of 128 threads per macroblock, its blocks, coefficients and levels in shared memory.
+// Every stage spreads over the threads what is independent in it: one partition row per thread in
+// the forward transforms, one coefficient in the quantiser, eight threads per parent block in the
+// inverse transform, the SSE and the bit estimate, sixteen (32 at beam 8) per partition in the
+// trellis. Every double operation is the reference's, in its order (this file is compiled without
+// contraction); the statistics are integer sums. The work is latency (a trellis is a chain of up to
+// 64 sorted steps) and FP64. With one lane per parent block and its arrays in local memory, a
+// 1080p picture took 13.6 ms and the 32 sampled macroblocks of a mode decision 0.58 ms.
 
 namespace {
 
@@ -417,6 +421,9 @@ struct TrdTables {
     uint8_t ac_bits[8][2][64][64];  // direct AC code length (0: no direct code) [set][last][run][level]
     uint8_t max_level[8][2][64];    // max_direct_level
     int8_t max_run[8][2][64];       // max_direct_run (-1: none)
+    // trellis_rate_bits: the family's least rate, [intra][PQINDEX < 8][last][run][level]. No set codes a
+    // level of 127 or more but by Escape 3, so the last entry stands for every larger level.
+    uint8_t family[2][2][2][64][128];
 };
 
 struct TrdArgs {
@@ -473,108 +480,63 @@ __device__ __forceinline__ void part_geometry(int t, int part, int& ox, int& oy,
 }
 __device__ __forceinline__ int part_count(int t) { return t == 1 ? 1 : (t == 4 ? 4 : 2); }
 
-// forward_transform_residual_part (:935-1045) into a partition-local 8-stride array: 8x8 output
-// transposed, rectangles row-major; samples outside the visible w x h are zero.
-__device__ void trd_forward(const uint8_t* sp, int spitch, const uint8_t* pp, int ppitch, int w, int h, int x0, int y0,
-                            int bw, int bh, double* c) {
-    double r[8][8];
-    for (int y = 0; y < bh; ++y)
-        for (int x = 0; x < bw; ++x) {
-            const int sx = x0 + x, sy = y0 + y;
-            r[y][x] = (sx < 0 || sy < 0 || sx >= w || sy >= h)
-                          ? 0.0
-                          : (double)((int)__ldg(sp + (size_t)sy * spitch + sx) - (int)__ldg(pp + (size_t)sy * ppitch + sx));
-        }
-    double tmp[8][8];
-    for (int a = 0; a < bh; ++a)
-        for (int x = 0; x < bw; ++x) {
-            double acc = 0.0;
-            for (int y = 0; y < bh; ++y) acc = __dadd_rn(acc, __dmul_rn(bh == 8 ? c_k8[a][y] : c_k4[a][y], r[y][x]));
-            tmp[a][x] = acc;
-        }
-    for (int i = 0; i < 64; ++i) c[i] = 0.0;
-    for (int a = 0; a < bh; ++a)
-        for (int b = 0; b < bw; ++b) {
-            double acc = 0.0;
-            for (int x = 0; x < bw; ++x) acc = __dadd_rn(acc, __dmul_rn(tmp[a][x], bw == 8 ? c_k8[b][x] : c_k4[b][x]));
-            const double v = __dmul_rn(1024.0, acc);
-            if (bw == 8 && bh == 8) c[b * 8 + a] = v;
-            else c[a * 8 + b] = v;
-        }
-}
-
-// inverse_partition (:1173-1274) of partition-local levels q into residuals a (8-stride)
-__device__ void trd_inverse(const DevParams& P, int t, const int* q, int mquant, bool derived, int* a) {
-    int bw, bh, ox, oy;
-    part_geometry(t, 0, ox, oy, bw, bh);
-    int nonzero = 0;
-    for (int y = 0; y < bh; ++y)
-        for (int x = 0; x < bw; ++x) nonzero += q[y * 8 + x] != 0;
-    for (int i = 0; i < 64; ++i) a[i] = 0;
-    for (int y = 0; y < bh; ++y)
-        for (int x = 0; x < bw; ++x) a[y * 8 + x] = trd_dequant(P, q[y * 8 + x], mquant, derived);
-    if (nonzero == 1 && q[0] != 0) {
-        int dc = a[0];
-        if (t == 1) { dc = arshift(3 * dc + 1, 1); dc = arshift(3 * dc + 16, 5); }
-        else if (t == 2) { dc = arshift(3 * dc + 1, 1); dc = arshift(17 * dc + 64, 7); }
-        else if (t == 3) { dc = arshift(17 * dc + 4, 3); dc = arshift(12 * dc + 64, 7); }
-        else { dc = arshift(17 * dc + 4, 3); dc = arshift(17 * dc + 64, 7); }
-        for (int i = 0; i < 64; ++i) a[i] = 0;
-        for (int y = 0; y < bh; ++y)
-            for (int x = 0; x < bw; ++x) a[y * 8 + x] = dc;
-        return;
-    }
-    int tmp[64];
-    for (int i = 0; i < 64; ++i) tmp[i] = 0;
-    if (t == 1) {
-        for (int col = 0; col < 8; ++col) inv8(a + col, 8, tmp + col * 8, 1, 4, 3, 0);
-        for (int col = 0; col < 8; ++col) inv8(tmp + col, 8, a + col, 8, 64, 7, 1);
-    } else if (t == 2) {
-        for (int y = 0; y < 4; ++y) inv8(a + y * 8, 1, tmp + y * 8, 1, 4, 3, 0);
-        for (int x = 0; x < 8; ++x) inv4(tmp + x, 8, a + x, 8, 64, 7);
-    } else if (t == 3) {
-        for (int y = 0; y < 8; ++y) inv4(a + y * 8, 1, tmp + y * 8, 1, 4, 3);
-        for (int x = 0; x < 4; ++x) inv8(tmp + x, 8, a + x, 8, 64, 7, 1);
-    } else {
-        for (int y = 0; y < 4; ++y) inv4(a + y * 8, 1, tmp + y * 8, 1, 4, 3);
-        for (int x = 0; x < 4; ++x) inv4(tmp + x, 8, a + x, 8, 64, 7);
-    }
-}
-
 // ---- the perceptual lambda scale (perceptual_lambda_scale, encoder_aq.cpp:405-653) ----------
+
+// The G neighbouring lanes that share one task; lane: this thread's place among them.
+struct Team {
+    unsigned mask;
+    int lane, size;
+    __device__ __forceinline__ uint32_t sum(uint32_t v) const { return __reduce_add_sync(mask, v); }
+    __device__ __forceinline__ int low(int v) const { return __reduce_min_sync(mask, v); }
+    __device__ __forceinline__ int high(int v) const { return __reduce_max_sync(mask, v); }
+};
 
 struct AqStats {
     double mean = 128.0, grad_avg = 0.0, residual_avg = 0.0;
     int mn = 255, mx = 0, edges = 0, n = 0;
+    uint32_t dark_grad = 0;  // the gradients of samples in [2, 112] (luma blocks)
+    int dark_n = 0;
 };
 
-__device__ AqStats aq_stats(const uint8_t* plane, int pitch, int pw, int ph, int sx, int sy, int sw, int sh,
+__device__ AqStats aq_stats(const Team& g, const uint8_t* plane, int pitch, int pw, int ph, int sx, int sy, int sw, int sh,
                             const uint8_t* pp, int ppitch) {
     AqStats st;
-    unsigned long long sum = 0, grad = 0, residual = 0;
-    int grad_n = 0;
-    for (int y = 0; y < sh && sy + y < ph; ++y)
-        for (int x = 0; x < sw && sx + x < pw; ++x) {
-            const int px = sx + x, py = sy + y;
-            const int v = __ldg(plane + (size_t)py * pitch + px);
-            sum += (unsigned long long)v;
-            st.mn = imin(st.mn, v);
-            st.mx = imax(st.mx, v);
-            ++st.n;
-            if (pp) residual += (unsigned long long)iabs(v - (int)__ldg(pp + (size_t)py * ppitch + px));
-            if (x > 0) {
-                const int d = iabs(v - (int)__ldg(plane + (size_t)py * pitch + px - 1));
-                grad += (unsigned long long)d;
-                ++grad_n;
-                if (d >= 96) ++st.edges;
+    uint32_t sum = 0, grad = 0, residual = 0, dark = 0;
+    int grad_n = 0, n = 0, edges = 0, dark_n = 0, mn = 255, mx = 0;
+    const int cw = imin(sw, pw - sx), chh = imin(sh, ph - sy);
+    for (int i = g.lane; i < sw * sh; i += g.size) {
+        const int x = i % sw, y = i / sw;
+        if (x >= cw || y >= chh) continue;
+        const uint8_t* at = plane + (size_t)(sy + y) * pitch + sx + x;
+        const int v = __ldg(at);
+        sum += (uint32_t)v;
+        mn = imin(mn, v);
+        mx = imax(mx, v);
+        ++n;
+        if (pp) residual += (uint32_t)iabs(v - (int)__ldg(pp + (size_t)(sy + y) * ppitch + sx + x));
+        const bool dk = v >= 2 && v <= 112;
+        auto edge = [&](int d) {
+            grad += (uint32_t)d;
+            ++grad_n;
+            if (d >= 96) ++edges;
+            if (dk) {
+                dark += (uint32_t)d;
+                ++dark_n;
             }
-            if (y > 0) {
-                const int d = iabs(v - (int)__ldg(plane + (size_t)(py - 1) * pitch + px));
-                grad += (unsigned long long)d;
-                ++grad_n;
-                if (d >= 96) ++st.edges;
-            }
-        }
+        };
+        if (x > 0) edge(iabs(v - (int)__ldg(at - 1)));
+        if (y > 0) edge(iabs(v - (int)__ldg(at - pitch)));
+    }
+    sum = g.sum(sum);
+    grad = g.sum(grad);
+    grad_n = (int)g.sum((uint32_t)grad_n);
+    st.n = (int)g.sum((uint32_t)n);
+    st.edges = (int)g.sum((uint32_t)edges);
+    st.dark_grad = g.sum(dark);
+    st.dark_n = (int)g.sum((uint32_t)dark_n);
+    st.mn = g.low(mn);
+    st.mx = g.high(mx);
+    if (pp) residual = g.sum(residual);
     if (st.n) {
         st.mean = (double)sum / st.n;
         st.grad_avg = (double)grad / imax(1, grad_n);
@@ -594,19 +556,20 @@ __device__ __forceinline__ double aq_activity(const AqStats& st) {
 // block is chroma (the luma context), else nullptr
 // adjacency_out (luma blocks): the quiet-block-next-to-detail term, 0 when the scale is not
 // computed (perceptual_lambda_scale's adjacency_out, encoder_aq.cpp:410, :641)
-__device__ double aq_scale(const TrdArgs& A, const uint8_t* plane, int pitch, int w, int h, int x0, int y0, int bw, int bh,
-                           const uint8_t* pp, int ppitch, const uint8_t* luma, int lpitch, double* adjacency_out = nullptr) {
+// The team's threads all call it and all get the result.
+__device__ double aq_scale(const Team& g, const TrdArgs& A, const uint8_t* plane, int pitch, int w, int h, int x0, int y0,
+                           int bw, int bh, const uint8_t* pp, int ppitch, const uint8_t* luma, int lpitch, double* adjacency_out = nullptr) {
     const vc1cu_trd_cfg& c = A.cfg;
     if (adjacency_out) *adjacency_out = 0.0;
     if (!c.adaptive_quality || c.aq_strength <= 0.0) return 1.0;
-    const AqStats st = aq_stats(plane, pitch, w, h, x0, y0, bw, bh, pp, ppitch);
+    const AqStats st = aq_stats(g, plane, pitch, w, h, x0, y0, bw, bh, pp, ppitch);
     if (!st.n) return 1.0;
     const double range = (double)imax(0, st.mx - st.mn);
     const double contrast = dclamp((range - 64.0) / 144.0, 0.0, 1.0) * dclamp((st.grad_avg - 7.0) / 40.0, 0.0, 1.0);
     const double edge_density = dclamp((double)st.edges / imax(1, st.n / 3), 0.0, 1.0);
     const double motion = dclamp((st.residual_avg - 5.0) / 30.0, 0.0, 1.0);
     if (luma) {
-        const AqStats ly = aq_stats(luma, lpitch, A.P.W, A.P.H, x0 * 2, y0 * 2, bw * 2, bh * 2, nullptr, 0);
+        const AqStats ly = aq_stats(g, luma, lpitch, A.P.W, A.P.H, x0 * 2, y0 * 2, bw * 2, bh * 2, nullptr, 0);
         const double chroma_detail =
             dmax(dclamp((st.grad_avg - 1.5) / 11.0, 0.0, 1.0), dclamp((range - 6.0) / 48.0, 0.0, 1.0));
         const double luma_activity = aq_activity(ly);
@@ -622,22 +585,7 @@ __device__ double aq_scale(const TrdArgs& A, const uint8_t* plane, int pitch, in
                                                 0.08 * edge_density + 0.05 * motion);
         return dclamp(1.0 / (1.0 + protect), 0.24, 1.0);
     }
-    unsigned long long dark_grad = 0;
-    int dark_n = 0;
-    for (int y = 0; y < bh && y0 + y < h; ++y)
-        for (int x = 0; x < bw && x0 + x < w; ++x) {
-            const int px = x0 + x, py = y0 + y;
-            const int v = __ldg(plane + (size_t)py * pitch + px);
-            if (x > 0 && v >= 2 && v <= 112) {
-                dark_grad += (unsigned long long)iabs(v - (int)__ldg(plane + (size_t)py * pitch + px - 1));
-                ++dark_n;
-            }
-            if (y > 0 && v >= 2 && v <= 112) {
-                dark_grad += (unsigned long long)iabs(v - (int)__ldg(plane + (size_t)(py - 1) * pitch + px));
-                ++dark_n;
-            }
-        }
-    const double dark_avg = dark_n ? (double)dark_grad / dark_n : 0.0;
+    const double dark_avg = st.dark_n ? (double)st.dark_grad / st.dark_n : 0.0;
     const double dark_window = dclamp((118.0 - st.mean) / 96.0, 0.0, 1.0) * dclamp((st.mean - 1.0) / 13.0, 0.0, 1.0);
     const double dark_detail = dark_window * dclamp(dark_avg / 10.0, 0.0, 1.0);
     const double frame_mean = (w == A.P.W && h == A.P.H) ? A.frame_mean : st.mean;
@@ -648,25 +596,30 @@ __device__ double aq_scale(const TrdArgs& A, const uint8_t* plane, int pitch, in
     const int pad = 4;
     const int cx0 = imax(0, x0 - pad), cy0 = imax(0, y0 - pad);
     const int cx1 = imin(w, x0 + bw + pad), cy1 = imin(h, y0 + bh + pad);
-    unsigned long long ring_grad = 0;
+    uint32_t ring_grad = 0;
     int ring_n = 0, ring_edges = 0;
-    for (int py = cy0; py < cy1; ++py)
-        for (int px = cx0; px < cx1; ++px) {
-            if (px >= x0 && px < x0 + bw && py >= y0 && py < y0 + bh) continue;
-            const int v = __ldg(plane + (size_t)py * pitch + px);
-            if (px > cx0) {
-                const int d = iabs(v - (int)__ldg(plane + (size_t)py * pitch + px - 1));
-                ring_grad += d;
-                if (d >= 64) ++ring_edges;
-                ++ring_n;
-            }
-            if (py > cy0) {
-                const int d = iabs(v - (int)__ldg(plane + (size_t)(py - 1) * pitch + px));
-                ring_grad += d;
-                if (d >= 64) ++ring_edges;
-                ++ring_n;
-            }
+    const int rw = cx1 - cx0, rh = cy1 - cy0;
+    for (int i = g.lane; i < rw * rh; i += g.size) {
+        const int px = cx0 + i % rw, py = cy0 + i / rw;
+        if (px >= x0 && px < x0 + bw && py >= y0 && py < y0 + bh) continue;
+        const uint8_t* at = plane + (size_t)py * pitch + px;
+        const int v = __ldg(at);
+        if (px > cx0) {
+            const int d = iabs(v - (int)__ldg(at - 1));
+            ring_grad += (uint32_t)d;
+            if (d >= 64) ++ring_edges;
+            ++ring_n;
         }
+        if (py > cy0) {
+            const int d = iabs(v - (int)__ldg(at - pitch));
+            ring_grad += (uint32_t)d;
+            if (d >= 64) ++ring_edges;
+            ++ring_n;
+        }
+    }
+    ring_grad = g.sum(ring_grad);
+    ring_n = (int)g.sum((uint32_t)ring_n);
+    ring_edges = (int)g.sum((uint32_t)ring_edges);
     const double ring_grad_avg = ring_n ? (double)ring_grad / ring_n : 0.0;
     const double ring_edge_density = ring_n ? (double)ring_edges / ring_n : 0.0;
     const double context_activity = dclamp((ring_grad_avg - 10.0) / 36.0, 0.0, 1.0) +
@@ -701,68 +654,35 @@ __device__ __forceinline__ int ac_max_run(const TrdTables* T, int set, int level
 }
 __device__ __forceinline__ int esc3_level_bits(const DevParams& P) { return P.pq < 8 ? 11 : 8; }
 
-// trellis_rate_bits_for_set (encoder_transform.cpp:1811-1841)
-__device__ int rate_for_set(const DevParams& P, const TrdTables* T, int run, int level, bool last, int set) {
-    const int mag = iabs(level);
-    if (run < 0 || run > 63 || level == 0 || mag > trd_max_level(P)) return 1000000;
-    if (const int d = ac_direct(T, set, run, mag, last)) return d + 1;
-    const int esc = ent::kAcEscapeBits[set];
-    int best = 1000000;
-    const int level_delta = ac_max_level(T, set, run, last);
-    if (set != 3 && level_delta > 0 && mag > level_delta) {
-        if (const int b = ac_direct(T, set, run, mag - level_delta, last)) best = esc + 1 + b + 1;
-    }
-    const int run_delta = ac_max_run(T, set, mag, last);
-    if (run_delta >= 0 && run > run_delta) {
-        if (const int b = ac_direct(T, set, run - run_delta - 1, mag, last)) best = imin(best, esc + 2 + b + 1);
-    }
-    return imin(best, esc + 2 + 1 + 6 + 1 + esc3_level_bits(P));
-}
-
-// trellis_rate_bits (:1843-1857): the lower envelope of coding sets 1, 3, 5 (inter family) or
-// 0, 2, 4 (intra family)
-__device__ int rate_family(const DevParams& P, const TrdTables* T, int run, int level, bool last, bool intra) {
-    int bits = 1000000;
-    for (int s = intra ? 0 : 1; s <= 5; s += 2) bits = imin(bits, rate_for_set(P, T, run, level, last, s));
-    return bits;
-}
-
-// write_ac_coeff's length (encoder_entropy.cpp:246-302) with the Escape-3 length header state
-__device__ int ac_coeff_bits(const TrdArgs& A, int run, int level, bool last, bool& esc3_written) {
+// The length of one coefficient as write_ac_coeff (encoder_entropy.cpp:246-302) codes it, as a
+// function of the Escape-3 length header's state: the length where Escape 3 is not taken (0: it is,
+// whatever the state), and Escape 3's without the header. Escape 3 is taken when it is the shorter,
+// the header counted until one was written.
+struct CoeffBits {
+    int other, esc3;
+};
+__device__ CoeffBits ac_coeff_bits(const TrdArgs& A, int run, int level, bool last) {
     const DevParams& P = A.P;
-    const int set = A.cfg.coding_set;
-    const int mag = iabs(level);
-    const int esc = ent::kAcEscapeBits[set];
-    const int header = (P.pq < 8 || A.cfg.dquantfrm) ? 7 : 8;
-    auto esc3 = [&]() {
-        const int b = esc + 2 + 1 + (esc3_written ? 0 : header) + 6 + 1 + esc3_level_bits(P);
-        esc3_written = true;
-        return b;
-    };
-    if (!A.cfg.use_vlc) return esc3();
-    if (const int d = ac_direct(A.tab, set, run, mag, last)) return d + 1;
-    int best_bits = 1000000;
-    bool have = false;
+    const int set = A.cfg.coding_set, mag = iabs(level), esc = ent::kAcEscapeBits[set];
+    CoeffBits r{0, esc + 2 + 1 + 6 + 1 + esc3_level_bits(P)};
+    if (!A.cfg.use_vlc) return r;
+    if (const int d = ac_direct(A.tab, set, run, mag, last)) {
+        r.other = d + 1;
+        r.esc3 = 1000000;  // a direct code is always taken
+        return r;
+    }
     const int level_delta = ac_max_level(A.tab, set, run, last);
     if (set != 3 && level_delta > 0 && mag > level_delta) {
-        if (const int b = ac_direct(A.tab, set, run, mag - level_delta, last)) {
-            best_bits = esc + 1 + b + 1;
-            have = true;
-        }
+        if (const int b = ac_direct(A.tab, set, run, mag - level_delta, last)) r.other = esc + 1 + b + 1;
     }
     const int run_delta = ac_max_run(A.tab, set, mag, last);
     if (run_delta >= 0 && run > run_delta) {
         if (const int b = ac_direct(A.tab, set, run - run_delta - 1, mag, last)) {
             const int bits = esc + 2 + b + 1;
-            if (bits < best_bits) {
-                best_bits = bits;
-                have = true;
-            }
+            if (!r.other || bits < r.other) r.other = bits;
         }
     }
-    const int esc3_bits = esc + 2 + 1 + 6 + 1 + esc3_level_bits(P) + (esc3_written ? 0 : header);
-    if (have && best_bits < esc3_bits) return best_bits;
-    return esc3();
+    return r;
 }
 
 __device__ __forceinline__ const uint8_t* inter_scan(int t, int& n) {
@@ -771,24 +691,6 @@ __device__ __forceinline__ const uint8_t* inter_scan(int t, int& n) {
     if (t == 3) { n = 32; return ent::kInterScan4x8; }
     n = 16;
     return ent::kInterScan4x4;
-}
-
-// write_inter_scan (:1414-1432) of partition-local levels
-__device__ int inter_scan_bits(const TrdArgs& A, const int* q, int t, bool& esc3_written) {
-    int n;
-    const uint8_t* scan = inter_scan(t, n);
-    int last = -1;
-    for (int s = n - 1; s >= 0; --s)
-        if (q[scan[s]]) { last = s; break; }
-    if (last < 0) return 0;
-    int bits = 0, previous = -1;
-    for (int s = 0; s <= last; ++s) {
-        const int level = q[scan[s]];
-        if (!level) continue;
-        bits += ac_coeff_bits(A, s - previous - 1, level, s == last, esc3_written);
-        previous = s;
-    }
-    return bits;
 }
 
 __device__ __forceinline__ int tt_table(const DevParams& P) { return P.pq <= 4 ? 0 : (P.pq <= 12 ? 1 : 2); }
@@ -827,34 +729,11 @@ struct TParent {
     int16_t q[64];      // the partitions' levels in their sub-rectangles of the 8x8 grid
     double distortion;
     uint32_t bits;      // estimate_parent_payload_bits
-    uint8_t type, skip;
+    // the coefficients' bits alone: coded before any Escape-3 length header was written (esc0: one is
+    // written among them), and after
+    uint32_t coef0, coef1;
+    uint8_t type, skip, esc0;
 };
-
-__device__ __forceinline__ void load_part(const TParent& p, int t, int part, int* q) {
-    int ox, oy, bw, bh;
-    part_geometry(t, part, ox, oy, bw, bh);
-    for (int i = 0; i < 64; ++i) q[i] = 0;
-    for (int y = 0; y < bh; ++y)
-        for (int x = 0; x < bw; ++x) q[y * 8 + x] = p.q[(oy + y) * 8 + ox + x];
-}
-
-// estimate_parent_payload_bits (:1528-1543)
-__device__ uint32_t parent_payload_bits(const TrdArgs& A, const TParent& p) {
-    const int np = part_count(p.type);
-    const int allmask = (1 << np) - 1;
-    if (p.skip == allmask) return 0;
-    bool esc = false;
-    int bits = 0;
-    if (p.type == 4) bits += subblkpat_bits(A.P, p.skip);
-    else if (p.type == 2 || p.type == 3) bits += rect_subblkpat_bits(p.skip);
-    int q[64];
-    for (int part = 0; part < np; ++part) {
-        if (p.skip & (1 << (np - 1 - part))) continue;
-        load_part(p, p.type, part, q);
-        bits += inter_scan_bits(A, q, p.type, esc);
-    }
-    return (uint32_t)bits;
-}
 
 // estimate_ttblk_bits (:1545-1553)
 __device__ uint32_t parent_ttblk_bits(const DevParams& P, const TParent& p) {
@@ -865,209 +744,327 @@ __device__ uint32_t parent_ttblk_bits(const DevParams& P, const TParent& p) {
     return (uint32_t)bits;
 }
 
+// The grid index of partition `part`'s first coefficient, and the grid positions it covers.
+__device__ __forceinline__ int part_origin(int t, int part) {
+    return t == 2 ? 32 * part : (t == 3 ? 4 * part : (t == 4 ? 32 * (part >> 1) + 4 * (part & 1) : 0));
+}
+__device__ __forceinline__ uint64_t part_cells(int t, int part) {
+    return (t == 1 ? ~0ull : t == 2 ? 0xFFFFFFFFull : t == 3 ? 0x0F0F0F0F0F0F0F0Full : 0x0F0F0F0Full) << part_origin(t, part);
+}
+
+// ---- the forward transform (forward_transform_residual_part, :935-1045) -------------------------
+
+// One partition row of a block's residual (px: source minus prediction, zero outside the raster):
+// the vertical stage of row `a` and the outputs of its frequency, into the 8x8 grid c (8x8 output
+// transposed, rectangles row-major in their place).
+__device__ __forceinline__ void forward_row(const int16_t* px, int t, int part, int a, double* c) {
+    const int bh = (t == 2 || t == 4) ? 4 : 8, bw = (t == 3 || t == 4) ? 4 : 8, org = part_origin(t, part);
+    double row[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        double acc = 0.0;
+        if (x < bw)
+            for (int y = 0; y < bh; ++y)
+                acc = __dadd_rn(acc, __dmul_rn(bh == 8 ? c_k8[a][y] : c_k4[a][y], (double)px[org + y * 8 + x]));
+        row[x] = acc;
+    }
+    for (int b = 0; b < bw; ++b) {
+        double acc = 0.0;
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+            if (x < bw) acc = __dadd_rn(acc, __dmul_rn(row[x], bw == 8 ? c_k8[b][x] : c_k4[b][x]));
+        c[(t == 1 ? b * 8 + a : org + a * 8 + b)] = __dmul_rn(1024.0, acc);
+    }
+}
+
 // ---- trellis_quantize (:1873-2088) ---------------------------------------------------------
 
 // trellis_coeff_weight (:1859-1871)
 __device__ __forceinline__ double trellis_weight(int t, int index) {
-    const double e8[8] = {1152, 1156, 1168, 1156, 1152, 1156, 1168, 1156};
-    const double e4[4] = {1156, 1168, 1156, 1168};
-    const int row = index / 8, col = index & 7;
-    const bool x4 = t == 3 || t == 4, y4 = t == 2 || t == 4;
-    const double ex = x4 ? e4[col] : e8[col], ey = y4 ? e4[row] : e8[row];
+    const int row = index >> 3, col = index & 7;
+    auto e8 = [](int i) { return (i & 3) == 0 ? 1152.0 : ((i & 3) == 2 ? 1168.0 : 1156.0); };
+    auto e4 = [](int i) { return (i & 1) ? 1168.0 : 1156.0; };
+    const double ex = (t == 3 || t == 4) ? e4(col) : e8(col), ey = (t == 2 || t == 4) ? e4(row) : e8(row);
     return (ex * ey) / (1024.0 * 1024.0);
 }
 
-struct TState {
-    double distortion, score;
-    uint32_t bits;
-    int last_scan;
-    int from, level;  // the state of the previous position it extends, and this position's level
-};
+constexpr int kTrdThreads = 128;
 
-__device__ __forceinline__ bool tstate_less(const TState& a, const TState& b) {
-    if (a.score != b.score) return a.score < b.score;
-    if (a.bits != b.bits) return a.bits < b.bits;
-    return a.distortion < b.distortion;
+// One trellis's working memory: the successors of a step, the surviving states and, per scan
+// position, the state each survivor extends and the candidate it took there.
+template <int BEAM>
+struct TrellisMem {
+    static constexpr int kTeam = 4 * BEAM;  // four candidate lanes per state
+    uint64_t score[kTeam];
+    double dist[kTeam];
+    double sdist[BEAM];
+    uint32_t bits[kTeam], aux[kTeam], sbits[BEAM], saux[BEAM];
+    uint8_t bp[64 * BEAM];
+};
+constexpr int kTrellisBytes = (kTrdThreads / 16) * (int)sizeof(TrellisMem<4>);
+static_assert((kTrdThreads / 32) * (int)sizeof(TrellisMem<8>) <= kTrellisBytes + 1024, "trellis memory");
+
+// Candidate ci of a position whose scalar level is q0: 0, q0, one nearer zero, one farther (kept within
+// max_level); a candidate that repeats an earlier one, or that the search does not try, is absent.
+__device__ __forceinline__ int trellis_candidate(int q0, int ci, bool wide, int max_level, bool& present) {
+    const int sign = q0 > 0 ? 1 : -1;
+    const int v = ci == 0 ? 0 : (ci == 1 ? q0 : (ci == 2 ? q0 - sign : iclamp(q0 + sign, -max_level, max_level)));
+    present = ci == 0 || (q0 != 0 && (ci == 1 || (ci == 2 ? v != 0 : (wide && v != q0))));
+    return v;
 }
 
-// Levels q (partition-local 8-stride) of coefficients c for transform type t along scan[0..n); the
-// trellis decides positions first_scan..n-1 (1 for intra blocks, whose DC is coded apart, leaving
-// q[scan[0]] zero) with the rates of the intra or inter family. The beam's paths are kept as
-// back-pointers per scan position (the state each survivor extends, its level there).
-__device__ void trellis_quantize(const TrdArgs& A, const double* c, int t, double lambda_scale, int mquant, int* q,
-                                 const uint8_t* scan, int n, int first_scan, bool intra) {
+// Levels q of one partition's coefficients c (both at the partition's origin in the 8x8 grid), given
+// the scalar levels, along scan[0..n): positions first_scan.. (1 for intra blocks, whose DC is coded
+// apart), with the rates of the intra or inter family. A team of 4 x BEAM lanes: lane = state * 4 +
+// candidate computes one successor; survivors are the least of (score, bits, distortion), equal ones in
+// the order the reference makes them, found by ranking every successor against every other. A
+// position whose scalar level is zero has one successor per state and mostly keeps their order, which
+// costs one comparison with the next state instead. A survivor's exact rate (its last coefficient
+// coded as last) follows from the rate it carries and that coefficient's run and level.
+template <int BEAM>
+__device__ void trellis_team(const Team& g, const TrdArgs& A, const double* c, const int16_t* scalar, int t, double lambda_scale,
+                             int mquant, const uint8_t* scan, int n, int first_scan, bool intra, int16_t* q,
+                             TrellisMem<BEAM>& mem) {
+    constexpr int G = TrellisMem<BEAM>::kTeam;
     const DevParams& P = A.P;
-    const bool derived = mquant != P.pq;
+    const bool derived = mquant != P.pq, wide = A.cfg.trellis >= 2;
     const double qscale = (double)trd_double_quant(P, mquant, derived);
     const int max_level = trd_max_level(P);
-    int scalar[64];
-    for (int i = 0; i < 64; ++i) scalar[i] = 0;
-    for (int s = 0; s < n; ++s) scalar[scan[s]] = trd_squant(P, c[scan[s]], mquant, derived);
-    for (int i = 0; i < 64; ++i) q[i] = scalar[i];
-    if (A.cfg.trellis <= 0 || (A.cfg.hrd_enabled && mquant == 1)) return;
-    const int beam = A.cfg.trellis >= 2 ? 8 : 4;
     const double lambda = 0.15 * qscale * qscale * dclamp(lambda_scale, 0.20, 1.50);
-    uint16_t bp[64][8];  // back-pointer: from state (3 bits) | level + 4096 (13 bits)
-    TState states[8];
+    const uint8_t(*fam)[64][128] = A.tab->family[intra ? 1 : 0][P.pq < 8 ? 1 : 0];
+    const int si = g.lane >> 2, ci = g.lane & 3;
     int count = 1;
-    states[0] = TState{0.0, 0.0, 0u, first_scan - 1, -1, 0};
+    // the lane's state: aux = last position + 1 | run << 8 | level << 16 (clamped) | 1 << 24 of its last coefficient
+    double dist = 0.0;
+    uint32_t bits = 0, aux = (uint32_t)first_scan;
     for (int s = first_scan; s < n; ++s) {
         const int idx = scan[s];
         const int q0 = scalar[idx];
-        int cand[4], nc = 0;
-        auto add = [&](int v) {
-            v = iclamp(v, -max_level, max_level);
-            for (int i = 0; i < nc; ++i)
-                if (cand[i] == v) return;
-            cand[nc++] = v;
-        };
-        add(0);
-        if (q0 != 0) {
-            const int sign = q0 > 0 ? 1 : -1;
-            add(q0);
-            add(q0 - sign);
-            if (A.cfg.trellis >= 2) add(q0 + sign);
+        bool present;
+        const int level = trellis_candidate(q0, q0 ? ci : 0, wide, max_level, present);
+        const double e = c[idx] - (double)trd_dequant(P, level, mquant, derived);
+        const double nd = dist + e * e * trellis_weight(t, idx);
+        uint32_t nb = bits, na = aux;
+        if (level != 0) {
+            const int run = s - (int)(aux & 255), mag = imin(iabs(level), 127);
+            nb += __ldg(&fam[0][run][mag]);
+            na = (uint32_t)(s + 1) | ((uint32_t)run << 8) | ((uint32_t)mag << 16) | (1u << 24);
         }
-        double cd[4];
-        for (int ci = 0; ci < nc; ++ci) {
-            const double e = c[idx] - (double)trd_dequant(P, cand[ci], mquant, derived);
-            cd[ci] = e * e * trellis_weight(t, idx);
-        }
-        TState next[32];
-        int nn = 0;
-        for (int si = 0; si < count; ++si) {
-            const TState& st = states[si];
-            for (int ci = 0; ci < nc; ++ci) {
-                const int level = cand[ci];
-                TState ns = st;
-                ns.distortion += cd[ci];
-                ns.from = si;
-                ns.level = level;
-                if (level != 0) {
-                    const int rb = rate_family(P, A.tab, s - st.last_scan - 1, level, false, intra);
-                    if (rb >= 1000000) continue;
-                    ns.bits += (uint32_t)rb;
-                    ns.last_scan = s;
-                }
-                ns.score = ns.distortion + lambda * (double)ns.bits;
-                next[nn++] = ns;
+        const uint64_t score = (uint64_t)__double_as_longlong(nd + lambda * (double)nb);  // >= 0: ordered as integers
+        if (q0 == 0) {
+            const uint64_t ns = __shfl_down_sync(g.mask, score, 4, G);
+            const uint32_t nnb = __shfl_down_sync(g.mask, nb, 4, G);
+            const double nnd = __shfl_down_sync(g.mask, nd, 4, G);
+            const bool moves = si + 1 < count && (ns < score || (ns == score && (nnb < nb || (nnb == nb && nnd < nd))));
+            if (!__any_sync(g.mask, moves)) {
+                dist = nd;
+                if (ci == 0 && si < count) mem.bp[s * BEAM + si] = (uint8_t)(si << 2);
+                continue;
             }
         }
-        for (int i = 1; i < nn; ++i) {
-            const TState key = next[i];
-            int j = i;
-            while (j > 0 && tstate_less(key, next[j - 1])) {
-                next[j] = next[j - 1];
-                --j;
+        const bool valid = si < count && present && (q0 != 0 || ci == 0);
+        mem.score[g.lane] = valid ? score : ~0ull;
+        mem.dist[g.lane] = nd;
+        mem.bits[g.lane] = nb;
+        mem.aux[g.lane] = na;
+        const int made = __popc(__ballot_sync(g.mask, valid) & g.mask);
+        __syncwarp(g.mask);
+        int rank = 0;
+#pragma unroll 4
+        for (int j = 0; j < G; ++j) {
+            const uint64_t sj = mem.score[j];
+            bool less = sj < score;
+            if (sj == score && j != g.lane) {
+                const uint32_t bj = mem.bits[j];
+                const double dj = mem.dist[j];
+                less = bj != nb ? bj < nb : (dj != nd ? dj < nd : j < g.lane);
             }
-            next[j] = key;
+            rank += less ? 1 : 0;
         }
-        count = imin(nn, beam);
-        for (int i = 0; i < count; ++i) {
-            states[i] = next[i];
-            bp[s][i] = (uint16_t)((next[i].from << 13) | (next[i].level + 4096));
+        if (valid && rank < BEAM) {
+            mem.sdist[rank] = nd;
+            mem.sbits[rank] = nb;
+            mem.saux[rank] = na;
+            mem.bp[s * BEAM + rank] = (uint8_t)((si << 2) | ci);
+        }
+        __syncwarp(g.mask);
+        count = imin(made, BEAM);
+        if (si < count) {
+            dist = mem.sdist[si];
+            bits = mem.sbits[si];
+            aux = mem.saux[si];
         }
     }
-    // the exact rate of each survivor (its last coefficient coded as last), then the least D + lambda R
-    int best = 0;
-    double best_rd = __longlong_as_double(0x7ff0000000000000LL);  // +infinity
-    for (int si = 0; si < count; ++si) {
-        uint32_t bits = 0;
-        int next_pos = -1, next_level = 0;  // the coefficient after this one on the path (towards the end)
-        int j = si;
-        bool first = true;
+    // the exact rate of each survivor, then the least D + lambda R, the first of equal ones
+    uint32_t exact = bits;
+    if (aux >> 24) {
+        const int run = (int)((aux >> 8) & 255), mag = (int)((aux >> 16) & 255);
+        exact = bits - __ldg(&fam[0][run][mag]) + __ldg(&fam[1][run][mag]);
+    }
+    if (ci == 0) mem.score[si] = (uint64_t)__double_as_longlong(dist + lambda * (double)exact);
+    __syncwarp(g.mask);
+    if (g.lane == 0) {
+        int best = 0;
+        for (int i = 1; i < count; ++i)
+            if (mem.score[i] < mem.score[best]) best = i;
+        int j = best;
         for (int s = n - 1; s >= first_scan; --s) {
-            const int level = (int)(bp[s][j] & 0x1FFF) - 4096;
-            const int from = bp[s][j] >> 13;
-            if (level != 0) {
-                if (next_pos >= 0)
-                    bits += (uint32_t)rate_family(P, A.tab, next_pos - s - 1, next_level, first, intra);
-                if (next_pos >= 0) first = false;
-                next_pos = s;
-                next_level = level;
-            }
-            j = from;
-        }
-        if (next_pos >= 0) bits += (uint32_t)rate_family(P, A.tab, next_pos - first_scan, next_level, first, intra);
-        const double rd = states[si].distortion + lambda * (double)bits;
-        if (rd < best_rd) {
-            best = si;
-            best_rd = rd;
+            const int code = mem.bp[s * BEAM + j], idx = scan[s];
+            bool present;
+            q[idx] = (int16_t)trellis_candidate(scalar[idx], code & 3, wide, max_level, present);
+            j = code >> 2;
         }
     }
-    for (int i = 0; i < 64; ++i) q[i] = 0;
-    int j = best;
-    for (int s = n - 1; s >= first_scan; --s) {
-        const int level = (int)(bp[s][j] & 0x1FFF) - 4096;
-        if (level != 0) q[scan[s]] = level;
-        j = bp[s][j] >> 13;
-    }
+    __syncwarp(g.mask);
 }
 
-// ---- evaluate_transform_parent (:1555-1590) --------------------------------------------------
+// One macroblock's blocks and the search's working set.
+struct TrdShared {
+    double c[24][64];              // coefficients of (candidate type, parent)
+    alignas(16) uint8_t trellis[kTrellisBytes + 1024];
+    TParent pool[36];              // 24 candidate parents, 6 trellis macro parents, 6 trellis block parents
+    int16_t sq[24][64];            // scalar levels of (candidate type, parent)
+    int tmp[kTrdThreads / 8][64];  // the inverse transforms' first stage, one parent per eight threads
+    int16_t px[6][64];             // residual, zero outside the raster
+    uint8_t src[6][64], pred[6][64];
+    double lscale;                 // the macroblock's perceptual lambda scale
+    int list[4], count;            // candidate types
+    uint8_t need[6], macro_type;   // the block winners' types, the macroblock winner's
+    uint8_t jobs[48];              // trellis partitions: job * 4 + partition
+    int n_jobs;
+    int chosen[6];
+};
 
-__device__ void eval_parent(const TrdArgs& A, int mx, int my, int k, int t, bool allow_trellis, int mquant, TParent& out) {
-    const DevParams& P = A.P;
+// Visible columns / rows of block k.
+__device__ __forceinline__ int2 block_extent(const DevParams& P, int mx, int my, int k) {
     const bool chroma = k >= 4;
-    const uint8_t* sp = chroma ? (k == 4 ? A.src.u : A.src.v) : A.src.y;
-    const uint8_t* pp = chroma ? (k == 4 ? A.pred.u : A.pred.v) : A.pred.y;
-    const int spitch = chroma ? A.src.pitch_c : A.src.pitch_y, ppitch = chroma ? A.pred.pitch_c : A.pred.pitch_y;
-    const int w = chroma ? P.W / 2 : P.W, h = chroma ? P.H / 2 : P.H;
-    const int bx = chroma ? mx : mx * 2 + (k & 1), by = chroma ? my : my * 2 + ((k >> 1) & 1);
-    const bool derived = mquant != P.pq;
-    out.type = (uint8_t)t;
-    out.skip = 0;
-    for (int i = 0; i < 64; ++i) out.q[i] = 0;
-    int residual[64];
-    for (int i = 0; i < 64; ++i) residual[i] = 0;
-    const int np = part_count(t);
-    for (int part = 0; part < np; ++part) {
-        int ox, oy, bw, bh;
-        part_geometry(t, part, ox, oy, bw, bh);
-        const int x0 = bx * 8 + ox, y0 = by * 8 + oy;
-        int q[64];
-        for (int i = 0; i < 64; ++i) q[i] = 0;
-        // quantize_inter_part (:1087-1171): nothing to code for a partition outside the crop
-        if (!(x0 >= w || y0 >= h || x0 + bw <= 0 || y0 + bh <= 0)) {
-            double c[64];
-            trd_forward(sp, spitch, pp, ppitch, w, h, x0, y0, bw, bh, c);
-            if (allow_trellis && A.cfg.trellis > 0) {
-                const double ls = aq_scale(A, sp, spitch, w, h, x0, y0, bw, bh, pp, ppitch, chroma ? A.src.y : nullptr,
-                                           A.src.pitch_y);
-                int n;
-                const uint8_t* scan = inter_scan(t, n);
-                trellis_quantize(A, c, t, ls, mquant, q, scan, n, 0, false);
-            } else {
-                for (int y = 0; y < bh; ++y)
-                    for (int x = 0; x < bw; ++x) q[y * 8 + x] = trd_squant(P, c[y * 8 + x], mquant, derived);
-            }
-        }
-        for (int y = 0; y < bh; ++y)
-            for (int x = 0; x < bw; ++x) out.q[(oy + y) * 8 + ox + x] = (int16_t)q[y * 8 + x];
-        bool any = false;
-        for (int i = 0; i < 64; ++i) any |= q[i] != 0;
-        if (!any) {
-            out.skip |= (uint8_t)(1 << (np - 1 - part));
-            continue;
-        }
-        int r[64];
-        trd_inverse(P, t, q, mquant, A.cfg.dquantfrm != 0, r);  // the reference passes DQUANTFRM here
-        for (int y = 0; y < bh; ++y)
-            for (int x = 0; x < bw; ++x) residual[(oy + y) * 8 + ox + x] = r[y * 8 + x];
-    }
-    unsigned long long sse = 0;
-    for (int y = 0; y < 8 && by * 8 + y < h; ++y)
-        for (int x = 0; x < 8 && bx * 8 + x < w; ++x) {
-            const int px = bx * 8 + x, py = by * 8 + y;
-            const int recon = iclamp((int)__ldg(pp + (size_t)py * ppitch + px) + residual[y * 8 + x], 0, 255);
-            const int e = (int)__ldg(sp + (size_t)py * spitch + px) - recon;
-            sse += (unsigned long long)(e * e);
-        }
-    out.distortion = (double)sse;
-    out.bits = parent_payload_bits(A, out);
+    const int x0 = (chroma ? mx : mx * 2 + (k & 1)) * 8, y0 = (chroma ? my : my * 2 + ((k >> 1) & 1)) * 8;
+    return make_int2(iclamp((chroma ? P.W / 2 : P.W) - x0, 0, 8), iclamp((chroma ? P.H / 2 : P.H) - y0, 0, 8));
 }
 
-// An MbTransformDecision: parents by index into the warp's parent pool
+// The rest of evaluate_transform_parent (:1555-1590) of a parent whose levels are in p.q, by eight
+// threads (j = 0..7 of `mask`): inverse_partition (:1173-1274) with its DC-only shortcut, a row or
+// column each, the reconstruction SSE, and write_inter_scan's (:1414-1432) bits, eight scan slots
+// each. tmp: 64 words of the eight threads' own.
+__device__ void eval_octet(const TrdArgs& A, const TrdShared& sh, int j, unsigned mask, int k, int t, int mquant, int2 vis,
+                           TParent& p, int* tmp) {
+    const DevParams& P = A.P;
+    const bool derived = A.cfg.dquantfrm != 0;  // the reference passes DQUANTFRM here
+    const int np = part_count(t);
+    auto dq = [&](int i) { return trd_dequant(P, p.q[i], mquant, derived); };
+    uint32_t row = 0;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) row |= p.q[j * 8 + x] ? 1u << x : 0u;
+    const uint32_t lo = __reduce_or_sync(mask, j < 4 ? row << (8 * j) : 0u);
+    const uint32_t hi = __reduce_or_sync(mask, j >= 4 ? row << (8 * (j - 4)) : 0u);
+    const uint64_t cells = ((uint64_t)hi << 32) | lo;
+    int s[8], o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = dq(t == 1 ? i * 8 + j : j * 8 + i);
+    if (t <= 2) {
+        inv8(s, 1, o, 1, 4, 3, 0);
+    } else {
+        inv4(s, 1, o, 1, 4, 3);
+        inv4(s + 4, 1, o + 4, 1, 4, 3);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tmp[j * 8 + i] = o[i];
+    __syncwarp(mask);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = tmp[i * 8 + j];
+    if (t == 1 || t == 3) {
+        inv8(s, 1, o, 1, 64, 7, 1);
+    } else {
+        inv4(s, 1, o, 1, 64, 7);
+        inv4(s + 4, 1, o + 4, 1, 64, 7);
+    }
+    uint32_t sse = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // the column's upper and lower half lie in one partition each
+        const int part = t == 1 ? 0 : (t == 2 ? h : (t == 3 ? j >> 2 : 2 * h + (j >> 2)));
+        const int org = part_origin(t, part);
+        const uint64_t own = cells & part_cells(t, part);
+        const bool dc_only = own == (1ull << org);
+        int dc = 0;
+        if (dc_only) {
+            dc = dq(org);
+            dc = t <= 2 ? arshift(3 * dc + 1, 1) : arshift(17 * dc + 4, 3);
+            dc = t == 1 ? arshift(3 * dc + 16, 5) : (t == 3 ? arshift(12 * dc + 64, 7) : arshift(17 * dc + 64, 7));
+        }
+#pragma unroll
+        for (int i = 4 * h; i < 4 * h + 4; ++i) {
+            const int r = dc_only ? dc : (own ? o[i] : 0);
+            if (j < vis.x && i < vis.y) {
+                const int e = (int)sh.src[k][i * 8 + j] - iclamp((int)sh.pred[k][i * 8 + j] + r, 0, 255);
+                sse += (uint32_t)(e * e);
+            }
+        }
+    }
+    sse = __reduce_add_sync(mask, sse);
+    // the coded coefficients in scan order: slot = partition * n + scan position
+    int n;
+    const uint8_t* scan = inter_scan(t, n);
+    uint32_t slots = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int slot = 8 * j + i, part = slot / n;
+        slots |= ((cells >> (part_origin(t, part) + scan[slot - part * n])) & 1) ? 1u << i : 0u;
+    }
+    const uint32_t slo = __reduce_or_sync(mask, j < 4 ? slots << (8 * j) : 0u);
+    const uint32_t shi = __reduce_or_sync(mask, j >= 4 ? slots << (8 * (j - 4)) : 0u);
+    const uint64_t coded = ((uint64_t)shi << 32) | slo;
+    const int header = (P.pq < 8 || A.cfg.dquantfrm) ? 7 : 8;
+    auto bits_of = [&](int slot) {
+        const int part = slot / n;
+        const uint64_t in = coded & ((n == 64 ? ~0ull : (1ull << n) - 1) << (part * n));
+        const uint64_t before = in & ((1ull << slot) - 1);
+        const int prev = before ? 63 - __clzll((long long)before) : part * n - 1;
+        const bool last = (in >> slot) == 1;
+        return ac_coeff_bits(A, slot - prev - 1, p.q[part_origin(t, part) + scan[slot - part * n]], last);
+    };
+    uint32_t none = 0, after = 0;  // no header written yet / already written
+    int first = 64;                // the first coefficient that would write it
+    for (uint32_t m = slots; m; m &= m - 1) {
+        const int slot = 8 * j + __ffs(m) - 1;
+        const CoeffBits b = bits_of(slot);
+        if (b.other && b.other < b.esc3 + header) none += (uint32_t)b.other;
+        else if (first == 64) first = slot;
+        after += (uint32_t)((b.other && b.other < b.esc3) ? b.other : b.esc3);
+    }
+    first = __reduce_min_sync(mask, first);
+    if (first < 64) {
+        none = 0;
+        for (uint32_t m = slots; m; m &= m - 1) {
+            const int slot = 8 * j + __ffs(m) - 1;
+            const CoeffBits b = bits_of(slot);
+            none += (uint32_t)(slot < first ? b.other : slot == first ? b.esc3 + header
+                                                      : ((b.other && b.other < b.esc3) ? b.other : b.esc3));
+        }
+    }
+    none = __reduce_add_sync(mask, none);
+    after = __reduce_add_sync(mask, after);
+    if (j == 0) {
+        int skip = 0;
+        for (int part = 0; part < np; ++part)
+            if (!(cells & part_cells(t, part))) skip |= 1 << (np - 1 - part);
+        p.type = (uint8_t)t;
+        p.skip = (uint8_t)skip;
+        p.distortion = (double)sse;
+        p.coef0 = none;
+        p.coef1 = after;
+        p.esc0 = first < 64;
+        // estimate_parent_payload_bits (:1528-1543)
+        uint32_t bits = 0;
+        if (skip != (1 << np) - 1) {
+            if (t == 4) bits += (uint32_t)subblkpat_bits(P, skip);
+            else if (t == 2 || t == 3) bits += (uint32_t)rect_subblkpat_bits(skip);
+            bits += none;
+        }
+        p.bits = bits;
+    }
+}
+
+// An MbTransformDecision: parents by index into the parent pool
 struct TDec {
     int8_t parent[6];
     uint8_t type, level, cbp;
@@ -1093,202 +1090,304 @@ __device__ void refresh(const TrdArgs& A, TDec& d, const TParent* pool) {
     if (first >= 0 && d.level == 1) d.type = pool[d.parent[first]].type;
     d.bits = 0;
     if (!d.cbp) return;
-    int bits = ent::kPcbpBits[d.cbp];
+    uint32_t bits = ent::kPcbpBits[d.cbp];
     bool esc = false;
-    int q[64];
-    if (!A.cfg.variable_transforms) {
-        for (int k = 0; k < 6; ++k) {
-            if (!(d.cbp & (1 << (5 - k)))) continue;
-            load_part(pool[d.parent[k]], 1, 0, q);
-            bits += inter_scan_bits(A, q, 1, esc);
-        }
-        d.bits = (uint32_t)bits;
-        return;
-    }
     const TParent& fp = pool[d.parent[first]];
-    if (d.level == 0) bits += ttmb_macro_bits(P, d.type, fp.skip);
-    else if (d.level == 1) bits += ttmb_block_bits(P, fp.type, fp.skip);
+    if (A.cfg.variable_transforms) {
+        if (d.level == 0) bits += (uint32_t)ttmb_macro_bits(P, d.type, fp.skip);
+        else if (d.level == 1) bits += (uint32_t)ttmb_block_bits(P, fp.type, fp.skip);
+    }
     for (int k = 0; k < 6; ++k) {
         if (!(d.cbp & (1 << (5 - k)))) continue;
         const TParent& p = pool[d.parent[k]];
         const int t = p.type;
-        if (d.level == 1) {
-            if (k != first) bits += ttblk_bits(P, t, p.skip);
-            if (t == 4) bits += subblkpat_bits(P, p.skip);
-        } else if (d.level == 0) {
-            if (t == 4) bits += subblkpat_bits(P, p.skip);
-            else if ((t == 2 || t == 3) && k != first) bits += rect_subblkpat_bits(p.skip);
-        } else {
-            if (t == 4) bits += subblkpat_bits(P, p.skip);
-            else if (t == 2 || t == 3) bits += rect_subblkpat_bits(p.skip);
+        if (A.cfg.variable_transforms) {
+            if (d.level == 1) {
+                if (k != first) bits += (uint32_t)ttblk_bits(P, t, p.skip);
+                if (t == 4) bits += (uint32_t)subblkpat_bits(P, p.skip);
+            } else if (d.level == 0) {
+                if (t == 4) bits += (uint32_t)subblkpat_bits(P, p.skip);
+                else if ((t == 2 || t == 3) && k != first) bits += (uint32_t)rect_subblkpat_bits(p.skip);
+            } else {
+                if (t == 4) bits += (uint32_t)subblkpat_bits(P, p.skip);
+                else if (t == 2 || t == 3) bits += (uint32_t)rect_subblkpat_bits(p.skip);
+            }
         }
-        const int np = part_count(t);
-        for (int part = 0; part < np; ++part) {
-            if (p.skip & (1 << (np - 1 - part))) continue;
-            load_part(p, t, part, q);
-            bits += inter_scan_bits(A, q, t, esc);
-        }
+        bits += esc ? p.coef1 : p.coef0;
+        esc = esc || p.esc0;
     }
-    d.bits = (uint32_t)bits;
+    d.bits = bits;
 }
 
 __device__ __forceinline__ double rd_of(const TDec& d, double lambda) { return d.distortion + lambda * (double)d.bits; }
 
-constexpr int kTrdWarps = 4;
-constexpr int kTrdPool = 36;  // 24 candidate parents, 6 trellis macro parents, 6 trellis block parents
-
-__global__ void __launch_bounds__(32 * kTrdWarps) trd_kernel(const __grid_constant__ TrdArgs A) {
-    __shared__ TParent pool_all[kTrdWarps][kTrdPool];
-    __shared__ int list_all[kTrdWarps][8];  // [0..3] candidate types, [4] count, [5] macro type, [6..] scratch
-    __shared__ uint8_t need_all[kTrdWarps][6];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int item = blockIdx.x * kTrdWarps + warp;
+// The trellis of every listed partition (jobs[i] = job * 4 + partition; the job's parent, type and
+// coefficients by `job_of`), by teams of the block's threads.
+template <int BEAM, class F>
+__device__ __forceinline__ void trellis_jobs(const TrdArgs& A, TrdShared& sh, int mx, int my, int mquant, F job_of) {
+    constexpr int G = TrellisMem<BEAM>::kTeam;
+    const int tid = threadIdx.x, team = tid / G, lane = tid & 31;
+    const Team g{G == 32 ? 0xffffffffu : 0xffffu << (lane & 16), tid % G, G};
+    TrellisMem<BEAM>& mem = reinterpret_cast<TrellisMem<BEAM>*>(sh.trellis)[team];
     const DevParams& P = A.P;
-    if (item >= (A.mb_list ? A.n_list : P.mbw * P.mbh)) return;
+    for (int i = team; i < sh.n_jobs; i += kTrdThreads / G) {
+        const int job = sh.jobs[i] >> 2, part = sh.jobs[i] & 3;
+        int k, t, cand, out;
+        job_of(job, k, t, cand, out);
+        int ox, oy, bw, bh;
+        part_geometry(t, part, ox, oy, bw, bh);
+        const bool chroma = k >= 4;
+        const int x0 = (chroma ? mx : mx * 2 + (k & 1)) * 8 + ox, y0 = (chroma ? my : my * 2 + ((k >> 1) & 1)) * 8 + oy;
+        const uint8_t* sp = chroma ? (k == 4 ? A.src.u : A.src.v) : A.src.y;
+        const uint8_t* pp = chroma ? (k == 4 ? A.pred.u : A.pred.v) : A.pred.y;
+        const int w = chroma ? P.W / 2 : P.W, h = chroma ? P.H / 2 : P.H;
+        const int org = part_origin(t, part);
+        double ls = 1.0;
+        if (x0 < w && y0 < h)
+            ls = aq_scale(g, A, sp, chroma ? A.src.pitch_c : A.src.pitch_y, w, h, x0, y0, bw, bh, pp,
+                          chroma ? A.pred.pitch_c : A.pred.pitch_y, chroma ? A.src.y : nullptr, A.src.pitch_y);
+        int n;
+        const uint8_t* scan = inter_scan(t, n);
+        trellis_team<BEAM>(g, A, sh.c[cand] + org, sh.sq[cand] + org, t, ls, mquant, scan, n, 0, false, sh.pool[out].q + org, mem);
+    }
+}
+
+__global__ void __launch_bounds__(kTrdThreads) trd_kernel(const __grid_constant__ TrdArgs A) {
+    __shared__ TrdShared sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int item = blockIdx.x;
+    const DevParams& P = A.P;
     const int mb = A.mb_list ? A.mb_list[item] : item;
-    TParent* pool = pool_all[warp];
-    int* list = list_all[warp];
-    uint8_t* need = need_all[warp];
     const int mx = mb % P.mbw, my = mb / P.mbw;
     const int mquant = (A.mquant && A.mquant[mb] >= 1) ? (int)A.mquant[mb] : P.pq;
     const vc1cu_trd_cfg& cfg = A.cfg;
-    // ---- the candidate list ----
-    if (!cfg.variable_transforms || cfg.frame_type) {
-        if (lane == 0) {
-            list[0] = cfg.variable_transforms ? cfg.frame_type : 1;
-            list[4] = 1;
-        }
-    } else {
-        // transform_metrics (transform_residual_metrics.h:29-61), each lane half a row
-        const int py = lane >> 1, px0 = (lane & 1) * 8;
-        uint32_t sad = 0, hedge = 0, vedge = 0, grad = 0;
-        const int y = my * 16 + py;
-        if (y < P.H) {
-            auto R = [&](int xx, int yy) {
-                return (int)A.src.y[(size_t)yy * A.src.pitch_y + xx] - (int)A.pred.y[(size_t)yy * A.pred.pitch_y + xx];
-            };
-            for (int px = px0; px < px0 + 8 && mx * 16 + px < P.W; ++px) {
-                const int x = mx * 16 + px;
-                const int r = R(x, y);
-                sad += (uint32_t)iabs(r);
-                if ((py & 7) == 4) hedge += (uint32_t)iabs(r - R(x, y - 1));
-                if ((px & 7) == 4) vedge += (uint32_t)iabs(r - R(x - 1, y));
-                if (px > 0) grad += (uint32_t)iabs(r - R(x - 1, y));
-                if (py > 0) grad += (uint32_t)iabs(r - R(x, y - 1));
-            }
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            sad += __shfl_xor_sync(0xffffffffu, sad, o);
-            hedge += __shfl_xor_sync(0xffffffffu, hedge, o);
-            vedge += __shfl_xor_sync(0xffffffffu, vedge, o);
-            grad += __shfl_xor_sync(0xffffffffu, grad, o);
-        }
-        if (lane == 0) {
-            const uint64_t S = sad, HE = hedge, VE = vedge, G = grad, lim = (uint64_t)(64 * mquant);
-            int l[4] = {1, 1, 1, 1}, count = 0;
-            const bool split_x = mx == P.mbw - 1 && (P.W & 15) != 0, split_y = my == P.mbh - 1 && (P.H & 15) != 0;
-            if (split_x && split_y) {
-                l[count++] = 4;
-            } else if (split_x || split_y) {
-                l[count++] = split_x ? 3 : 2;
-                if (S > lim && G > S * 2) l[count++] = 4;
-            } else {
-                l[count++] = 1;
-                if (S > lim) {
-                    if (HE * 5 > VE * 6) l[count++] = 2;
-                    else if (VE * 5 > HE * 6) l[count++] = 3;
-                    else { l[count++] = 2; l[count++] = 3; }
-                    if (count < 4 && G > S * 2) l[count++] = 4;
-                }
-            }
-            for (int i = 0; i < 4; ++i) list[i] = l[i];
-            list[4] = count;
-        }
-    }
-    __syncwarp();
-    const int count = list[4];
     // candidates whose decision is final at once: the 8x8-only and frame-level forms (with trellis)
     const bool direct = !cfg.variable_transforms || cfg.frame_type;
-    const bool scalar_search = cfg.trellis > 0;
-    // ---- every candidate's six parents, one per lane ----
-    if (lane < count * 6) {
-        const int i = lane / 6, k = lane % 6;
-        eval_parent(A, mx, my, k, list[i], direct ? true : !scalar_search, mquant, pool[i * 6 + k]);
+    const bool trellis = cfg.trellis > 0 && !(cfg.hrd_enabled && mquant == 1);  // else its levels are the scalar ones
+    // ---- the macroblock's blocks ----
+    for (int i = tid; i < 384; i += kTrdThreads) {
+        const int k = i >> 6, x = i & 7, y = (i >> 3) & 7;
+        const bool chroma = k >= 4;
+        const int2 vis = block_extent(P, mx, my, k);
+        const int gx = (chroma ? mx : mx * 2 + (k & 1)) * 8 + x, gy = (chroma ? my : my * 2 + ((k >> 1) & 1)) * 8 + y;
+        int a = 0, b = 0;
+        if (x < vis.x && y < vis.y) {
+            a = __ldg((chroma ? (k == 4 ? A.src.u : A.src.v) : A.src.y) + (size_t)gy * (chroma ? A.src.pitch_c : A.src.pitch_y) + gx);
+            b = __ldg((chroma ? (k == 4 ? A.pred.u : A.pred.v) : A.pred.y) + (size_t)gy * (chroma ? A.pred.pitch_c : A.pred.pitch_y) + gx);
+        }
+        sh.src[k][i & 63] = (uint8_t)a;
+        sh.pred[k][i & 63] = (uint8_t)b;
+        sh.px[k][i & 63] = (int16_t)(a - b);
     }
-    __syncwarp();
+    __syncthreads();
+    // ---- the candidate list, and beside it the macroblock's lambda scale ----
+    if (warp == 0) {
+        if (direct) {
+            if (lane == 0) {
+                sh.list[0] = cfg.variable_transforms ? cfg.frame_type : 1;
+                sh.count = 1;
+            }
+        } else {
+            // transform_metrics (transform_residual_metrics.h:29-61), each lane half a row
+            const int py = lane >> 1, px0 = (lane & 1) * 8;
+            uint32_t sad = 0, hedge = 0, vedge = 0, grad = 0;
+            if (my * 16 + py < P.H) {
+                auto R = [&](int x, int y) { return (int)sh.px[(y >> 3) * 2 + (x >> 3)][(y & 7) * 8 + (x & 7)]; };
+                for (int px = px0; px < px0 + 8 && mx * 16 + px < P.W; ++px) {
+                    const int r = R(px, py);
+                    sad += (uint32_t)iabs(r);
+                    if ((py & 7) == 4) hedge += (uint32_t)iabs(r - R(px, py - 1));
+                    if ((px & 7) == 4) vedge += (uint32_t)iabs(r - R(px - 1, py));
+                    if (px > 0) grad += (uint32_t)iabs(r - R(px - 1, py));
+                    if (py > 0) grad += (uint32_t)iabs(r - R(px, py - 1));
+                }
+            }
+            sad = __reduce_add_sync(0xffffffffu, sad);
+            hedge = __reduce_add_sync(0xffffffffu, hedge);
+            vedge = __reduce_add_sync(0xffffffffu, vedge);
+            grad = __reduce_add_sync(0xffffffffu, grad);
+            if (lane == 0) {
+                const uint64_t S = sad, HE = hedge, VE = vedge, GR = grad, lim = (uint64_t)(64 * mquant);
+                int l[4] = {1, 1, 1, 1}, count = 0;
+                const bool split_x = mx == P.mbw - 1 && (P.W & 15) != 0, split_y = my == P.mbh - 1 && (P.H & 15) != 0;
+                if (split_x && split_y) {
+                    l[count++] = 4;
+                } else if (split_x || split_y) {
+                    l[count++] = split_x ? 3 : 2;
+                    if (S > lim && GR > S * 2) l[count++] = 4;
+                } else {
+                    l[count++] = 1;
+                    if (S > lim) {
+                        if (HE * 5 > VE * 6) l[count++] = 2;
+                        else if (VE * 5 > HE * 6) l[count++] = 3;
+                        else { l[count++] = 2; l[count++] = 3; }
+                        if (count < 4 && GR > S * 2) l[count++] = 4;
+                    }
+                }
+                for (int i = 0; i < 4; ++i) sh.list[i] = l[i];
+                sh.count = count;
+            }
+        }
+    } else if (warp == 1 && !direct) {
+        const Team g{0xffffffffu, lane, 32};
+        const double ls = aq_scale(g, A, A.src.y, A.src.pitch_y, P.W, P.H, mx * 16, my * 16, 16, 16, A.pred.y, A.pred.pitch_y,
+                                   nullptr, 0);
+        if (lane == 0) sh.lscale = ls;
+    }
+    __syncthreads();
+    const int count = sh.count, parents = 6 * count;
+    // ---- every candidate's six parents: coefficients, scalar levels ----
+    {
+        int base = 0;
+        for (int i = 0; i < count; ++i) {
+            const int t = sh.list[i], per = xform_threads(t), bh = (t == 2 || t == 4) ? 4 : 8;
+            // the first thread of a type follows the last of the one before it
+            for (int task = (tid - base) & (kTrdThreads - 1); task < 6 * per; task += kTrdThreads) {
+                const int k = task / per, sub = task - k * per;
+                forward_row(sh.px[k], t, sub / bh, sub % bh, sh.c[i * 6 + k]);
+            }
+            base += 6 * per;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < parents * 64; i += kTrdThreads) {
+        const int v = trd_squant(P, sh.c[i >> 6][i & 63], mquant, mquant != P.pq);
+        sh.sq[i >> 6][i & 63] = (int16_t)v;
+        sh.pool[i >> 6].q[i & 63] = (int16_t)v;
+    }
+    if (tid == 0) {
+        sh.n_jobs = 0;
+        if (direct && trellis)
+            for (int k = 0; k < 6; ++k)
+                for (int part = 0; part < part_count(sh.list[0]); ++part) sh.jobs[sh.n_jobs++] = (uint8_t)(k * 4 + part);
+    }
+    __syncthreads();
+    if (direct && trellis) {
+        auto job_of = [&](int job, int& k, int& t, int& cand, int& out) {
+            k = cand = out = job;
+            t = sh.list[0];
+        };
+        if (cfg.trellis >= 2) trellis_jobs<8>(A, sh, mx, my, mquant, job_of);
+        else trellis_jobs<4>(A, sh, mx, my, mquant, job_of);
+        __syncthreads();
+    }
+    const int octet = tid >> 3, oj = tid & 7;
+    const unsigned omask = 0xffu << (lane & 24);
+    for (int i = octet; i < parents; i += kTrdThreads / 8)
+        eval_octet(A, sh, oj, omask, i % 6, sh.list[i / 6], mquant, block_extent(P, mx, my, i % 6), sh.pool[i], sh.tmp[octet]);
+    __syncthreads();
+    // ---- the macroblock- and block-level winners ----
     TDec macro{}, block{};
     double lambda = 0.0;
-    if (lane == 0) {
+    if (warp == 0) {
         if (direct) {
-            for (int k = 0; k < 6; ++k) macro.parent[k] = (int8_t)k;
-            macro.type = (uint8_t)list[0];
-            macro.level = cfg.variable_transforms ? 2 : 0;
-            refresh(A, macro, pool);
-        } else {
-            TDec cand[4];
-            for (int i = 0; i < count; ++i) {
-                for (int k = 0; k < 6; ++k) cand[i].parent[k] = (int8_t)(i * 6 + k);
-                cand[i].type = (uint8_t)list[i];
-                cand[i].level = 0;
-                refresh(A, cand[i], pool);
+            if (lane == 0) {
+                for (int k = 0; k < 6; ++k) macro.parent[k] = (int8_t)k;
+                macro.type = (uint8_t)sh.list[0];
+                macro.level = cfg.variable_transforms ? 2 : 0;
+                refresh(A, macro, sh.pool);
             }
-            const double mb_lscale = aq_scale(A, A.src.y, A.src.pitch_y, P.W, P.H, mx * 16, my * 16, 16, 16, A.pred.y,
-                                              A.pred.pitch_y, nullptr, 0);
-            lambda = 0.75 * (double)(2 * mquant) * (double)(2 * mquant) * mb_lscale;
+        } else {
+            lambda = 0.75 * (double)(2 * mquant) * (double)(2 * mquant) * sh.lscale;
+            // a candidate per lane; the first of the least
+            TDec cand{};
+            double rd = __longlong_as_double(0x7ff0000000000000LL);
+            if (lane < count) {
+                for (int k = 0; k < 6; ++k) cand.parent[k] = (int8_t)(lane * 6 + k);
+                cand.type = (uint8_t)sh.list[lane];
+                cand.level = 0;
+                refresh(A, cand, sh.pool);
+                rd = rd_of(cand, lambda);
+            }
             int best_i = 0;
-            double best_rd = rd_of(cand[0], lambda);
+            double best_rd = __shfl_sync(0xffffffffu, rd, 0);
             for (int i = 1; i < count; ++i) {
-                const double r = rd_of(cand[i], lambda);
+                const double r = __shfl_sync(0xffffffffu, rd, i);
                 if (r < best_rd) {
                     best_rd = r;
                     best_i = i;
                 }
             }
-            block = cand[0];
-            block.level = 1;
-            for (int k = 0; k < 6; ++k) {
-                int bi = 0;
+            // a parent block per lane
+            int bi = 0;
+            if (lane < 6) {
                 auto prd = [&](const TParent& p) {
                     return p.distortion + lambda * (double)(p.bits + parent_ttblk_bits(P, p));
                 };
-                double brd = prd(pool[cand[0].parent[k]]);
+                double brd = prd(sh.pool[lane]);
                 for (int i = 1; i < count; ++i) {
-                    const double r = prd(pool[cand[i].parent[k]]);
+                    const double r = prd(sh.pool[i * 6 + lane]);
                     if (r < brd) {
                         brd = r;
                         bi = i;
                     }
                 }
-                block.parent[k] = cand[bi].parent[k];
             }
-            refresh(A, block, pool);
-            macro = cand[best_i];
-            list[5] = macro.type;
-            for (int k = 0; k < 6; ++k) need[k] = pool[block.parent[k]].type;
+            for (int k = 0; k < 6; ++k) block.parent[k] = (int8_t)(__shfl_sync(0xffffffffu, bi, k) * 6 + k);
+            // the winner's estimate from its lane, the block decision's on lane 0
+            macro.distortion = __shfl_sync(0xffffffffu, cand.distortion, best_i);
+            macro.bits = __shfl_sync(0xffffffffu, cand.bits, best_i);
+            macro.cbp = (uint8_t)__shfl_sync(0xffffffffu, (int)cand.cbp, best_i);
+            macro.type = (uint8_t)__shfl_sync(0xffffffffu, (int)cand.type, best_i);
+            if (lane == 0) {
+                for (int k = 0; k < 6; ++k) macro.parent[k] = (int8_t)(best_i * 6 + k);
+                macro.level = 0;
+                block.type = (uint8_t)sh.list[0];
+                block.level = 1;
+                refresh(A, block, sh.pool);
+                sh.macro_type = macro.type;
+                int n = 0;
+                for (int job = 0; job < 12; ++job) {
+                    const int k = job % 6, t = job < 6 ? macro.type : sh.pool[block.parent[k]].type;
+                    if (job >= 6) sh.need[k] = (uint8_t)t;
+                    if (job >= 6 && t == macro.type) continue;
+                    for (int part = 0; part < part_count(t); ++part) sh.jobs[n++] = (uint8_t)(job * 4 + part);
+                }
+                sh.n_jobs = n;
+            }
         }
     }
-    __syncwarp();
     // ---- trellis re-evaluation of the macroblock winner and of the block winners of other types ----
     if (!direct && cfg.trellis > 0) {
-        const int mt = list[5];
-        if (lane < 6) eval_parent(A, mx, my, lane, mt, true, mquant, pool[24 + lane]);
-        else if (lane < 12 && need[lane - 6] != mt) eval_parent(A, mx, my, lane - 6, need[lane - 6], true, mquant, pool[30 + lane - 6]);
-        __syncwarp();
-        if (lane == 0) {
-            const uint8_t mtype = macro.type;
+        __syncthreads();
+        auto job_of = [&](int job, int& k, int& t, int& cand, int& out) {
+            k = job % 6;
+            t = job < 6 ? sh.macro_type : sh.need[k];
+            int i = 0;
+            while (i < 3 && sh.list[i] != t) ++i;
+            cand = i * 6 + k;
+            out = 24 + job;
+        };
+        if (!trellis) {
+            for (int i = tid; i < 12 * 64; i += kTrdThreads) {
+                int k, t, cand, out;
+                job_of(i >> 6, k, t, cand, out);
+                sh.pool[out].q[i & 63] = sh.sq[cand][i & 63];
+            }
+        } else if (cfg.trellis >= 2) {
+            trellis_jobs<8>(A, sh, mx, my, mquant, job_of);
+        } else {
+            trellis_jobs<4>(A, sh, mx, my, mquant, job_of);
+        }
+        __syncthreads();
+        if (octet < 12) {
+            int k, t, cand, out;
+            job_of(octet, k, t, cand, out);
+            if (octet < 6 || t != sh.macro_type)
+                eval_octet(A, sh, oj, omask, k, t, mquant, block_extent(P, mx, my, k), sh.pool[out], sh.tmp[octet]);
+        }
+        __syncthreads();
+        if (tid == 0) {
             for (int k = 0; k < 6; ++k) macro.parent[k] = (int8_t)(24 + k);
             macro.level = 0;
-            refresh(A, macro, pool);
-            for (int k = 0; k < 6; ++k) block.parent[k] = (int8_t)(need[k] == mtype ? 24 + k : 30 + k);
+            refresh(A, macro, sh.pool);
+            for (int k = 0; k < 6; ++k) block.parent[k] = (int8_t)(sh.need[k] == sh.macro_type ? 24 + k : 30 + k);
             block.level = 1;
-            refresh(A, block, pool);
+            refresh(A, block, sh.pool);
         }
     }
-    __syncwarp();
     // ---- the signaling decision and the outputs ----
-    __shared__ int chosen_all[kTrdWarps][6];
-    if (lane == 0) {
+    if (tid == 0) {
         TDec d = macro;
         if (!direct && cfg.extended_transform_signaling && rd_of(block, lambda) < rd_of(macro, lambda) * 0.9999) d = block;
         vc1cu_tdecision o{};
@@ -1298,19 +1397,18 @@ __global__ void __launch_bounds__(32 * kTrdWarps) trd_kernel(const __grid_consta
         o.estimated_bits = d.bits;
         o.distortion = d.distortion;
         for (int k = 0; k < 6; ++k) {
-            const TParent& p = pool[d.parent[k]];
+            const TParent& p = sh.pool[d.parent[k]];
             o.parent_type[k] = p.type;
             o.skip_mask[k] = p.skip;
             o.parent_bits[k] = p.bits;
             o.parent_distortion[k] = p.distortion;
-            chosen_all[warp][k] = d.parent[k];
+            sh.chosen[k] = d.parent[k];
         }
         A.out[item] = o;
     }
-    __syncwarp();
+    __syncthreads();
     if (A.levels)
-        for (int i = lane; i < 6 * 64; i += 32)
-            A.levels[(size_t)item * 384 + i] = pool[chosen_all[warp][i >> 6]].q[i & 63];
+        for (int i = tid; i < 6 * 64; i += kTrdThreads) A.levels[(size_t)item * 384 + i] = sh.pool[sh.chosen[i >> 6]].q[i & 63];
 }
 
 // ---- I-picture intra reconstruction (reconstruct_i_signed_padded, encoder_encode.cpp:814-887) ----
@@ -1375,63 +1473,84 @@ __device__ __forceinline__ int intra_mq(const IntraArgs& A, int mb) {
     return (A.mquant && A.mquant[mb] >= 1) ? (int)A.mquant[mb] : A.P.pq;
 }
 
-// One thread per (MB, block): forward_transform (:672-795; samples outside the source read the
+// One block of threads per MB: forward_transform (:672-795; samples outside the source read the
 // pad value, 0 luma / 128 chroma, minus 128), the AC levels of quantize_ac (:2090-2144: scalar, or
 // the trellis along the intra scan from position 1 with the intra-family rates and the perceptual
 // lambda scale of the block, chroma weighed against the intra source's luma) and
-// choose_dc_for_mean of the padded block mean.
-__global__ void intra_fwd_kernel(const __grid_constant__ IntraArgs A) {
+// choose_dc_for_mean of the padded block mean. The stages are the transform RD's: one transform row
+// and one coefficient per thread, sixteen (32) threads per trellis. One thread per block took 0.5 ms
+// per 720p picture with the trellis.
+__global__ void __launch_bounds__(kTrdThreads) intra_fwd_kernel(const __grid_constant__ IntraArgs A) {
+    __shared__ double c[6][64];
+    __shared__ int16_t px[6][64], sq[6][64], lv[6][64];
+    __shared__ unsigned sums[6];
+    __shared__ alignas(16) uint8_t trellis_mem[kTrellisBytes + 1024];
     const DevParams& P = A.P;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.mbw * P.mbh * 6) return;
-    const int mb = i / 6, k = i % 6, mx = mb % P.mbw, my = mb / P.mbw;
-    const bool chroma = k >= 4;
-    const uint8_t* p = chroma ? (k == 4 ? A.u : A.v) : A.y;
-    const int pitch = chroma ? A.pitch_c : A.pitch_y, w = chroma ? A.sw / 2 : A.sw, h = chroma ? A.sh / 2 : A.sh;
-    const int bx = chroma ? mx : mx * 2 + (k & 1), by = chroma ? my : my * 2 + ((k >> 1) & 1);
-    const int x0 = bx * 8, y0 = by * 8, pad = chroma ? 128 : 0;
+    const int tid = threadIdx.x, lane = tid & 31, mb = blockIdx.x, mx = mb % P.mbw, my = mb / P.mbw;
     const int mq = intra_mq(A, mb);
-    const bool derived = A.derived && A.derived[mb];
-    int r[8][8];
-    unsigned sum = 0;
-    for (int y = 0; y < 8; ++y)
-        for (int x = 0; x < 8; ++x) {
-            const int sx = x0 + x, sy = y0 + y;
-            const int v = (sx < w && sy < h) ? (int)__ldg(p + (size_t)sy * pitch + sx) : pad;
-            sum += (unsigned)v;
-            r[y][x] = v - 128;
-        }
-    double tmp[8][8];
-    for (int a = 0; a < 8; ++a)
-        for (int x = 0; x < 8; ++x) {
-            double acc = 0.0;
-            for (int y = 0; y < 8; ++y) acc = __dadd_rn(acc, __dmul_rn(c_k8[a][y], (double)r[y][x]));
-            tmp[a][x] = acc;
-        }
-    int16_t* q = A.q + (size_t)i * 64;
-    q[0] = 0;
     const bool trellis = A.trd.cfg.trellis > 0 && !(A.trd.cfg.hrd_enabled && mq == 1);
-    double c[64];
-    for (int a = 0; a < 8; ++a)
-        for (int b = 0; b < 8; ++b) {
-            if (!a && !b) continue;
-            double acc = 0.0;
-            for (int x = 0; x < 8; ++x) acc = __dadd_rn(acc, __dmul_rn(tmp[a][x], c_k8[b][x]));
-            c[b * 8 + a] = __dmul_rn(1024.0, acc);  // c[row*8+col] = xform[col][row]
-            if (!trellis) q[b * 8 + a] = (int16_t)trd_squant(P, c[b * 8 + a], mq, derived);
-        }
-    if (trellis) {
-        c[0] = 0.0;  // the DC stays out of the trellis (first_scan 1)
-        // the luma context is read as a coded-width raster (stats(*luma_context, width, height, ...)):
-        // an edge source of a cropped picture is a padded-width raster read at the coded width
-        const int lpitch = A.sw == P.W ? A.pitch_y : P.W;
-        const double ls = aq_scale(A.trd, p, pitch, w, h, x0, y0, 8, 8, nullptr, 0, chroma ? A.y : nullptr, lpitch);
-        int lv[64];
-        trellis_quantize(A.trd, c, 1, ls, mq, lv, ent::kIntraScan, 64, 1, !chroma);
-        for (int j = 1; j < 64; ++j) q[j] = (int16_t)lv[j];
+    // the scalar levels the trellis starts from take its own rule for the half step
+    const bool derived = trellis ? mq != P.pq : (A.derived && A.derived[mb]);
+    if (tid < 6) sums[tid] = 0;
+    __syncthreads();
+    for (int i = tid; i < 384; i += kTrdThreads) {
+        const int k = i >> 6;
+        const bool chroma = k >= 4;
+        const uint8_t* p = chroma ? (k == 4 ? A.u : A.v) : A.y;
+        const int pitch = chroma ? A.pitch_c : A.pitch_y, w = chroma ? A.sw / 2 : A.sw, h = chroma ? A.sh / 2 : A.sh;
+        const int sx = (chroma ? mx : mx * 2 + (k & 1)) * 8 + (i & 7), sy = (chroma ? my : my * 2 + ((k >> 1) & 1)) * 8 + ((i >> 3) & 7);
+        const int v = (sx < w && sy < h) ? (int)__ldg(p + (size_t)sy * pitch + sx) : (chroma ? 128 : 0);
+        px[k][i & 63] = (int16_t)(v - 128);
+        const unsigned s = __reduce_add_sync(0xffffffffu, (unsigned)v);  // a warp's 32 samples lie in one block
+        if (lane == 0) atomicAdd(&sums[k], s);
     }
-    const int gw = chroma ? P.mbw : P.mbw * 2;
-    A.dc[chroma ? k - 3 : 0][by * gw + bx] = intra_dc_for_mean((int)((sum + 32u) / 64u), mq, 128);
+    __syncthreads();
+    if (tid < 48) forward_row(px[tid >> 3], 1, 0, tid & 7, c[tid >> 3]);
+    __syncthreads();
+    for (int i = tid; i < 384; i += kTrdThreads) {
+        const int k = i >> 6, j = i & 63;
+        const int v = j ? trd_squant(P, c[k][j], mq, derived) : 0;
+        if (!j) c[k][0] = 0.0;  // the DC stays out of the trellis (first_scan 1)
+        sq[k][j] = (int16_t)v;
+        lv[k][j] = (int16_t)v;
+    }
+    __syncthreads();
+    if (trellis) {
+        auto block = [&](const Team& g, int k, auto& mem, auto run) {
+            const bool chroma = k >= 4;
+            const uint8_t* p = chroma ? (k == 4 ? A.u : A.v) : A.y;
+            const int x0 = (chroma ? mx : mx * 2 + (k & 1)) * 8, y0 = (chroma ? my : my * 2 + ((k >> 1) & 1)) * 8;
+            // the luma context is read as a coded-width raster (stats(*luma_context, width, height, ...)):
+            // an edge source of a cropped picture is a padded-width raster read at the coded width
+            const int lpitch = A.sw == P.W ? A.pitch_y : P.W;
+            const double ls = aq_scale(g, A.trd, p, chroma ? A.pitch_c : A.pitch_y, chroma ? A.sw / 2 : A.sw,
+                                       chroma ? A.sh / 2 : A.sh, x0, y0, 8, 8, nullptr, 0, chroma ? A.y : nullptr, lpitch);
+            run(g, k, ls, !chroma, mem);
+        };
+        if (A.trd.cfg.trellis >= 2) {
+            TrellisMem<8>& mem = reinterpret_cast<TrellisMem<8>*>(trellis_mem)[tid / 32];
+            for (int k = tid / 32; k < 6; k += kTrdThreads / 32)
+                block(Team{0xffffffffu, lane, 32}, k, mem, [&](const Team& g, int kk, double ls, bool intra, TrellisMem<8>& m) {
+                    trellis_team<8>(g, A.trd, c[kk], sq[kk], 1, ls, mq, ent::kIntraScan, 64, 1, intra, lv[kk], m);
+                });
+        } else {
+            TrellisMem<4>& mem = reinterpret_cast<TrellisMem<4>*>(trellis_mem)[tid / 16];
+            const int k = tid / 16;
+            if (k < 6)
+                block(Team{0xffffu << (lane & 16), tid & 15, 16}, k, mem,
+                      [&](const Team& g, int kk, double ls, bool intra, TrellisMem<4>& m) {
+                          trellis_team<4>(g, A.trd, c[kk], sq[kk], 1, ls, mq, ent::kIntraScan, 64, 1, intra, lv[kk], m);
+                      });
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < 384; i += kTrdThreads) A.q[(size_t)mb * 384 + i] = lv[i >> 6][i & 63];
+    if (tid < 6) {
+        const bool chroma = tid >= 4;
+        const int bx = chroma ? mx : mx * 2 + (tid & 1), by = chroma ? my : my * 2 + ((tid >> 1) & 1);
+        const int gw = chroma ? P.mbw : P.mbw * 2;
+        A.dc[chroma ? tid - 3 : 0][by * gw + bx] = intra_dc_for_mean((int)((sums[tid] + 32u) / 64u), mq, 128);
+    }
 }
 
 // predict_dc_dquant + clamp_dc_target_for_diff (encoder_entropy.cpp:549-571, :426-432) along the
@@ -1539,27 +1658,36 @@ __global__ void edge_source_kernel(const __grid_constant__ EdgeArgs E) {
 
 // The DQUANT search's per-macroblock inputs (choose_dquant_transform_mb, encoder_aq.cpp:318-336):
 // the perceptual lambda scale of the MB's luma against its prediction with its adjacency term,
-// and the bright-detail-on-dark test of the source MB. One thread per MB.
-__global__ void dquant_stats_kernel(const __grid_constant__ TrdArgs A, double* lscale, double* adjacency, uint8_t* bright) {
+// and the bright-detail-on-dark test of the source MB. One warp per MB.
+__global__ void __launch_bounds__(128) dquant_stats_kernel(const __grid_constant__ TrdArgs A, double* lscale,
+                                                           double* adjacency, uint8_t* bright) {
     const DevParams& P = A.P;
-    const int mb = blockIdx.x * blockDim.x + threadIdx.x;
+    const int mb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (mb >= P.mbw * P.mbh) return;
+    const Team g{0xffffffffu, (int)(threadIdx.x & 31), 32};
     const int x0 = (mb % P.mbw) * 16, y0 = (mb / P.mbw) * 16;
     double adj = 0.0;
-    lscale[mb] = aq_scale(A, A.src.y, A.src.pitch_y, P.W, P.H, x0, y0, 16, 16, A.pred.y, A.pred.pitch_y, nullptr, 0, &adj);
-    adjacency[mb] = adj;
-    unsigned long long sum = 0;
-    int n = 0, hi = 0, lo = 0;
-    for (int y = 0; y < 16 && y0 + y < P.H; ++y)
-        for (int x = 0; x < 16 && x0 + x < P.W; ++x) {
-            const int v = A.src.y[(size_t)(y0 + y) * A.src.pitch_y + x0 + x];
-            sum += (unsigned long long)v;
-            ++n;
-            hi += v >= 180;
-            lo += v <= 48;
-        }
-    const double mean = n ? (double)sum / n : 128.0;
-    bright[mb] = (n && mean < 90.0 && hi >= imax(2, n / 32) && lo >= n / 2) ? 1 : 0;
+    const double ls = aq_scale(g, A, A.src.y, A.src.pitch_y, P.W, P.H, x0, y0, 16, 16, A.pred.y, A.pred.pitch_y, nullptr, 0, &adj);
+    uint32_t sum = 0, n = 0, hi = 0, lo = 0;
+    for (int i = g.lane; i < 256; i += 32) {
+        const int x = x0 + (i & 15), y = y0 + (i >> 4);
+        if (x >= P.W || y >= P.H) continue;
+        const int v = A.src.y[(size_t)y * A.src.pitch_y + x];
+        sum += (uint32_t)v;
+        ++n;
+        hi += v >= 180;
+        lo += v <= 48;
+    }
+    sum = g.sum(sum);
+    n = g.sum(n);
+    hi = g.sum(hi);
+    lo = g.sum(lo);
+    if (g.lane == 0) {
+        lscale[mb] = ls;
+        adjacency[mb] = adj;
+        const double mean = n ? (double)sum / (int)n : 128.0;
+        bright[mb] = (n && mean < 90.0 && (int)hi >= imax(2, (int)n / 32) && lo >= n / 2) ? 1 : 0;
+    }
 }
 
 // mean of the source luma plane (cached_luma_mean, encoder_aq.cpp:506-545): one block's partial sums
@@ -1572,6 +1700,12 @@ __global__ void luma_sum_kernel(const uint8_t* y, int pitch, int W, int H, unsig
 }
 
 }  // namespace
+
+// The escape lengths on the host (ent::kAcEscapeBits lives in constant memory here).
+static int ent_escape_bits(int set) {
+    constexpr uint8_t bits[8] = {9, 9, 7, 9, 7, 7, 7, 7};
+    return bits[set];
+}
 
 // The dense rate tables from the code lengths (host side).
 size_t trd_tables_bytes() { return sizeof(TrdTables); }
@@ -1586,6 +1720,34 @@ void trd_fill_tables(void* host) {
         if (level > t.max_level[set][last][run]) t.max_level[set][last][run] = (uint8_t)level;
         if (run > t.max_run[set][last][level]) t.max_run[set][last][level] = (int8_t)run;
     }
+    // trellis_rate_bits_for_set (encoder_transform.cpp:1811-1841)
+    auto direct = [&](int set, int run, int level, int last) {
+        return run < 0 || run > 63 || level < 0 || level > 63 ? 0 : (int)t.ac_bits[set][last][run][level];
+    };
+    auto rate = [&](int run, int mag, int last, int set, int level_bits) {
+        if (const int d = direct(set, run, mag, last)) return d + 1;
+        const int esc = ent_escape_bits(set);
+        int best = 1000000;
+        const int level_delta = t.max_level[set][last][run];
+        if (set != 3 && level_delta > 0 && mag > level_delta)
+            if (const int b = direct(set, run, mag - level_delta, last)) best = esc + 1 + b + 1;
+        const int run_delta = mag < 64 ? t.max_run[set][last][mag] : -1;
+        if (run_delta >= 0 && run > run_delta)
+            if (const int b = direct(set, run - run_delta - 1, mag, last)) best = std::min(best, esc + 2 + b + 1);
+        return std::min(best, esc + 2 + 1 + 6 + 1 + level_bits);
+    };
+    // trellis_rate_bits (:1843-1857): the lower envelope of coding sets 1, 3, 5 (inter family) or 0, 2, 4
+    // (intra family)
+    for (int intra = 0; intra < 2; ++intra)
+        for (int fine = 0; fine < 2; ++fine)
+            for (int last = 0; last < 2; ++last)
+                for (int run = 0; run < 64; ++run)
+                    for (int mag = 1; mag < 128; ++mag) {
+                        int bits = 1000000;
+                        for (int set = intra ? 0 : 1; set <= 5; set += 2)
+                            bits = std::min(bits, rate(run, mag, last, set, fine ? 11 : 8));
+                        t.family[intra][fine][last][run][mag] = (uint8_t)bits;
+                    }
 }
 
 // The source luma mean the perceptual lambda scale reads (0 when the scale is off).
@@ -1623,7 +1785,7 @@ cudaError_t launch_trd(const DevParams& P, const DevFrame& src, const DevFrame& 
     a.n_list = n_list;
     const int items = mb_list ? n_list : P.mbw * P.mbh;
     if (items <= 0) return cudaSuccess;
-    trd_kernel<<<(items + kTrdWarps - 1) / kTrdWarps, 32 * kTrdWarps, 0, s>>>(a);
+    trd_kernel<<<items, kTrdThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -1644,7 +1806,7 @@ cudaError_t launch_dquant_stats(const DevParams& P, const DevFrame& src, const D
     a.frame_mean = frame_mean;
     const int mbs = P.mbw * P.mbh;
     if (mbs <= 0) return cudaSuccess;
-    dquant_stats_kernel<<<(mbs + 127) / 128, 128, 0, s>>>(a, lscale, adjacency, bright);
+    dquant_stats_kernel<<<(mbs + 3) / 4, 128, 0, s>>>(a, lscale, adjacency, bright);
     return cudaGetLastError();
 }
 
@@ -1742,7 +1904,7 @@ cudaError_t launch_intra_recon(const DevParams& P, const DevFrame& src, int over
         if ((e = frame_mean_for(sp, sf, cfg, d_sum, s, A.trd.frame_mean)) != cudaSuccess) return e;
     }
     const unsigned blocks = (unsigned)((mbs * 6 + 127) / 128);
-    intra_fwd_kernel<<<blocks, 128, 0, s>>>(A);
+    intra_fwd_kernel<<<(unsigned)mbs, kTrdThreads, 0, s>>>(A);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     intra_dc_kernel<<<3, 256, 0, s>>>(A);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
