@@ -325,6 +325,57 @@ __device__ __forceinline__ uint64_t key_cost(uint64_t k) {
     return c == 0xFFFFFull ? kBad : c;
 }
 
+// 16 bytes at any address as four little-endian words: aligned word loads that each hold at least
+// one of the bytes, and funnel shifts.
+__device__ __forceinline__ void gload16(const uint8_t* p, uint32_t r[4]) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
+    const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
+    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+    const uint32_t w4 = sh ? __ldg(w + 4) : 0u;
+    r[0] = __funnelshift_r(w0, w1, sh);
+    r[1] = __funnelshift_r(w1, w2, sh);
+    r[2] = __funnelshift_r(w2, w3, sh);
+    r[3] = __funnelshift_r(w3, w4, sh);
+}
+
+// The bytes 0, 4, 8, 12 of 16, packed.
+__device__ __forceinline__ uint32_t gpick4(const uint32_t r[4]) {
+    return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+}
+
+// This thread's share (the block's threads together: all) of a whole-frame SAD at displacement
+// (dx, dy) over the sampled rows r0 .. r1 - 1 (row r samples line r * st, columns 0, st, 2 st ..), with
+// clamped sampling of the reference. A thread takes 16-pixel chunks with packed byte SADs; chunks
+// that the clamping touches, the ragged last one and the strides above 4 go sample by sample.
+__device__ __forceinline__ uint32_t frame_sad_part(const uint8_t* cur, int cpitch, const uint8_t* ref, int rpitch, int W, int H,
+                                                   int dx, int dy, int st, int r0, int r1) {
+    const int chunks = (W + 15) >> 4, items = (r1 - r0) * chunks;
+    uint32_t acc = 0;
+    for (int t = threadIdx.x; t < items; t += blockDim.x) {
+        const int r = t / chunks, x = (t - r * chunks) << 4, y = (r0 + r) * st;
+        const uint8_t* cp = cur + (size_t)y * cpitch;
+        const uint8_t* rp = ref + (size_t)iclamp(y + dy, 0, H - 1) * rpitch;
+        if (st <= 4 && x + 16 <= W && x + dx >= 0 && x + dx + 16 <= W) {
+            uint32_t a[4], b[4];
+            gload16(cp + x, a);
+            gload16(rp + x + dx, b);
+            if (st == 4) {
+                acc += __vsadu4(gpick4(a), gpick4(b));
+            } else if (st == 2) {
+                acc += __vsadu4(__byte_perm(a[0], a[1], 0x6420), __byte_perm(b[0], b[1], 0x6420)) +
+                       __vsadu4(__byte_perm(a[2], a[3], 0x6420), __byte_perm(b[2], b[3], 0x6420));
+            } else {
+                acc += __vsadu4(a[0], b[0]) + __vsadu4(a[1], b[1]) + __vsadu4(a[2], b[2]) + __vsadu4(a[3], b[3]);
+            }
+        } else {
+            // x is a multiple of 16, so of every stride: the chunk's samples start at x
+            for (int i = 0; i < 16 && x + i < W; i += st)
+                acc += (uint32_t)iabs((int)__ldg(cp + x + i) - (int)__ldg(rp + iclamp(x + i + dx, 0, W - 1)));
+        }
+    }
+    return acc;
+}
+
 __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) {

@@ -287,27 +287,7 @@ __device__ void gfold(GState& s, int stage) {
     }
 }
 
-// 16 bytes at any address as four little-endian words: aligned word loads that each hold at least
-// one of the bytes, and funnel shifts.
-__device__ __forceinline__ void gload16(const uint8_t* p, uint32_t r[4]) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
-    const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3) * 8;
-    const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
-    const uint32_t w4 = sh ? __ldg(w + 4) : 0u;
-    r[0] = __funnelshift_r(w0, w1, sh);
-    r[1] = __funnelshift_r(w1, w2, sh);
-    r[2] = __funnelshift_r(w2, w3, sh);
-    r[3] = __funnelshift_r(w3, w4, sh);
-}
-
-// The bytes 0, ST, 2 ST .. of 16, packed (four for ST 4, eight for ST 2).
-__device__ __forceinline__ uint32_t gpick4(const uint32_t r[4]) {
-    return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
-}
-
-// frame_sad of every candidate of every search: grid (slab, candidate slot, search). A thread takes
-// 16-pixel chunks of the sampled rows with packed byte SADs; chunks that the clamped sampling
-// touches, the ragged last one and the strides above 4 go sample by sample.
+// frame_sad of every candidate of every search: grid (slab, candidate slot, search).
 // Two 1080p searches at range 32 (8 launches, the folds included): 277 us, against 363 us for the
 // scoring alone with one sample per load.
 __global__ void __launch_bounds__(kGThreads) gsad_kernel(GState* states, int W, int H, int rows_per_slab, int stage) {
@@ -317,31 +297,7 @@ __global__ void __launch_bounds__(kGThreads) gsad_kernel(GState* states, int W, 
     const int nrows = (H + st - 1) / st, r0 = blockIdx.x * rows_per_slab, r1 = imin(nrows, r0 + rows_per_slab);
     const int2 c = ci < s.n ? s.cand[ci] : make_int2(kGEmpty, 0);
     if (c.x != kGEmpty && r0 < r1) {
-        const int chunks = (W + 15) >> 4, items = (r1 - r0) * chunks;
-        const DevFrame &cf = s.in.cur, &rf = s.in.ref;
-        uint32_t acc = 0;  // at most (64 rows x 16384 samples / 256 threads) x 255
-        for (int t = threadIdx.x; t < items; t += kGThreads) {
-            const int r = t / chunks, x = (t - r * chunks) << 4, y = (r0 + r) * st;
-            const uint8_t* cp = cf.y + (size_t)y * cf.pitch_y;
-            const uint8_t* rp = rf.y + (size_t)iclamp(y + c.y, 0, H - 1) * rf.pitch_y;
-            if (st <= 4 && x + 16 <= W && x + c.x >= 0 && x + c.x + 16 <= W) {
-                uint32_t a[4], b[4];
-                gload16(cp + x, a);
-                gload16(rp + x + c.x, b);
-                if (st == 4) {
-                    acc += __vsadu4(gpick4(a), gpick4(b));
-                } else if (st == 2) {
-                    acc += __vsadu4(__byte_perm(a[0], a[1], 0x6420), __byte_perm(b[0], b[1], 0x6420)) +
-                           __vsadu4(__byte_perm(a[2], a[3], 0x6420), __byte_perm(b[2], b[3], 0x6420));
-                } else {
-                    acc += __vsadu4(a[0], b[0]) + __vsadu4(a[1], b[1]) + __vsadu4(a[2], b[2]) + __vsadu4(a[3], b[3]);
-                }
-            } else {
-                // x is a multiple of 16, so of every stride: the chunk's samples start at x
-                for (int i = 0; i < 16 && x + i < W; i += st)
-                    acc += (uint32_t)iabs((int)__ldg(cp + x + i) - (int)__ldg(rp + iclamp(x + i + c.x, 0, W - 1)));
-            }
-        }
+        const uint32_t acc = frame_sad_part(s.in.cur.y, s.in.cur.pitch_y, s.in.ref.y, s.in.ref.pitch_y, W, H, c.x, c.y, st, r0, r1);
         const uint64_t sum = warp_sum_u64(acc);
         __shared__ unsigned long long part[kGThreads / 32];
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;

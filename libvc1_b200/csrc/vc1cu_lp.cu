@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "vc1cu_common.cuh"
 #include "vc1cu_lp.cuh"
 
 namespace vc1cu {
@@ -185,18 +186,12 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
 //     samples): every displacement in [-R16, R16]^2, R16 = min(16, ceil(range / 16));
 //  B  1/4 resolution: the 7x7 displacements about 4x A's, within +-ceil(range / 4);
 //  C  full resolution, frame SAD at stride 2: the 5x5 vectors about 4x B's, within +-range.
-// Clamped reference sampling at every level; one block per candidate.
+// Clamped reference sampling at every level; one block per candidate and slab of rows. The winner
+// of a finished stage is found again by each block of the next (a minimum over at most 1,089 costs).
+// One block per candidate left the chip to 49 and 25 blocks: 0.82 ms per 1080p pair in stages B and C
+// and the pick, 0.06 now.
 __device__ __forceinline__ int hint_r16(const LpGeom& g) { return min(16, (g.range + 15) / 16); }
 __device__ __forceinline__ int hint_na(const LpGeom& g) { return (2 * hint_r16(g) + 1) * (2 * hint_r16(g) + 1); }
-
-// (cost, |dx|+|dy|, dy, dx) lexicographic order.
-__device__ __forceinline__ bool hint_less(unsigned long long ca, int ax, int ay, unsigned long long cb, int bx, int by) {
-    if (ca != cb) return ca < cb;
-    const int ma = abs(ax) + abs(ay), mb = abs(bx) + abs(by);
-    if (ma != mb) return ma < mb;
-    if (ay != by) return ay < by;
-    return ax < bx;
-}
 
 __device__ __forceinline__ int2 vec_a(const LpGeom& g, int i) {
     const int R = hint_r16(g), n = 2 * R + 1;
@@ -210,32 +205,48 @@ __device__ __forceinline__ int2 vec_c(const LpGeom& g, int2 b, int k) {
     return make_int2(min(max(4 * b.x + k % 5 - 2, -g.range), g.range), min(max(4 * b.y + k / 5 - 2, -g.range), g.range));
 }
 
+// Index of the least of n costs by (cost, |dx|+|dy|, dy, dx), vec(i) the i-th vector (each component
+// within +-1024), on every thread of a block of 256. The cost is compared first, then the rest.
+template <class V>
+__device__ int best_of(const unsigned long long* cost, int n, V vec, unsigned long long* red) {
+    auto least = [&](unsigned long long v) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long w = __shfl_xor_sync(FULLM, v, o);
+            v = w < v ? w : v;
+        }
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        v = red[0];
+        for (int k = 1; k < 8; ++k) v = red[k] < v ? red[k] : v;
+        return v;
+    };
+    unsigned long long mine = ~0ull;
+    for (int i = threadIdx.x; i < n; i += 256) {
+        const unsigned long long c = __ldcg(cost + i);
+        mine = c < mine ? c : mine;
+    }
+    const unsigned long long c0 = least(mine);
+    mine = ~0ull;
+    for (int i = threadIdx.x; i < n; i += 256)
+        if (__ldcg(cost + i) == c0) {
+            const int2 v = vec(i);
+            const unsigned long long k = ((unsigned long long)(abs(v.x) + abs(v.y)) << 48) |
+                                         ((unsigned long long)(v.y + 2048) << 32) | ((unsigned long long)(v.x + 2048) << 16) |
+                                         (unsigned long long)i;
+            mine = k < mine ? k : mine;
+        }
+    return (int)(least(mine) & 0xFFFF);
+}
 // The winners of the finished stages (cost layout: A's, then B's 49, then C's 25).
-__device__ int2 best_a(const unsigned long long* cost, const LpGeom& g) {
-    unsigned long long bc = ~0ull;
-    int2 b = make_int2(0, 0);
-    for (int i = 0; i < hint_na(g); ++i) {
-        const int2 v = vec_a(g, i);
-        if (hint_less(cost[i], v.x, v.y, bc, b.x, b.y)) {
-            bc = cost[i];
-            b = v;
-        }
-    }
-    return b;
+__device__ int2 best_a(const unsigned long long* cost, const LpGeom& g, unsigned long long* red) {
+    return vec_a(g, best_of(cost, hint_na(g), [&](int i) { return vec_a(g, i); }, red));
 }
-__device__ int2 best_b(const unsigned long long* cost, const LpGeom& g, int2 a) {
-    const unsigned long long* cb = cost + hint_na(g);
-    unsigned long long bc = ~0ull;
-    int2 b = make_int2(0, 0);
-    for (int k = 0; k < 49; ++k) {
-        const int2 v = vec_b(g, a, k);
-        if (hint_less(cb[k], v.x, v.y, bc, b.x, b.y)) {
-            bc = cb[k];
-            b = v;
-        }
-    }
-    return b;
+__device__ int2 best_b(const unsigned long long* cost, const LpGeom& g, int2 a, unsigned long long* red) {
+    return vec_b(g, a, best_of(cost + hint_na(g), 49, [&](int i) { return vec_b(g, a, i); }, red));
 }
+constexpr int kHintSlab = 32;  // sampled rows per block of stages B and C and of the frame SAD
 
 // 1/16-resolution pictures: the rounded mean of each macroblock's 4x4 quarter-res samples.
 __global__ void lp_down16_kernel(const uint8_t* cur4, const uint8_t* ref4, LpGeom g, uint8_t* cur16, uint8_t* ref16) {
@@ -267,68 +278,39 @@ __global__ void lp_hint_a_kernel(const uint8_t* cur16, const uint8_t* ref16, LpG
     if (threadIdx.x == 0) cost[blockIdx.x] = s;
 }
 
-__global__ void lp_hint_b_kernel(const uint8_t* cur4, const uint8_t* ref4, LpGeom g, unsigned long long* cost) {
-    __shared__ unsigned long long red[8];
-    __shared__ int2 a;
-    if (threadIdx.x == 0) a = best_a(cost, g);
-    __syncthreads();
-    const int2 v = vec_b(g, a, blockIdx.x);
-    unsigned long long s = 0;
-    for (int i = threadIdx.x; i < g.W4 * g.H4; i += blockDim.x) {
-        const int x = i % g.W4, y = i / g.W4;
-        const int rx = min(max(x + v.x, 0), g.W4 - 1), ry = min(max(y + v.y, 0), g.H4 - 1);
-        s += (unsigned)abs((int)cur4[i] - (int)ref4[ry * g.W4 + rx]);
-    }
-    s = block_sum_u64(s, red);
-    if (threadIdx.x == 0) cost[hint_na(g) + blockIdx.x] = s;
+__global__ void __launch_bounds__(256) lp_hint_b_kernel(const uint8_t* cur4, const uint8_t* ref4, LpGeom g,
+                                                        unsigned long long* cost) {
+    __shared__ unsigned long long red[8], sums[8];
+    const int2 v = vec_b(g, best_a(cost, g, red), blockIdx.x);
+    const int r0 = blockIdx.y * kHintSlab, r1 = min(g.H4, r0 + kHintSlab);
+    const unsigned long long s = block_sum_u64(frame_sad_part(cur4, g.W4, ref4, g.W4, g.W4, g.H4, v.x, v.y, 1, r0, r1), sums);
+    if (threadIdx.x == 0) atomicAdd(&cost[hint_na(g) + blockIdx.x], s);
 }
 
-__global__ void lp_hint_c_kernel(const uint8_t* cur, int cp, const uint8_t* ref, int rp, LpGeom g,
-                                 unsigned long long* cost) {
-    __shared__ unsigned long long red[8];
-    __shared__ int2 b;
-    if (threadIdx.x == 0) b = best_b(cost, g, best_a(cost, g));
-    __syncthreads();
-    const int2 v = vec_c(g, b, blockIdx.x);
-    const int sw = (g.W + 1) / 2, sh = (g.H + 1) / 2;
-    unsigned long long s = 0;
-    for (int i = threadIdx.x; i < sw * sh; i += blockDim.x) {
-        const int x = 2 * (i % sw), y = 2 * (i / sw);
-        const int rx = min(max(x + v.x, 0), g.W - 1), ry = min(max(y + v.y, 0), g.H - 1);
-        s += (unsigned)abs((int)cur[(size_t)y * cp + x] - (int)ref[(size_t)ry * rp + rx]);
-    }
-    s = block_sum_u64(s, red);
-    if (threadIdx.x == 0) cost[hint_na(g) + 49 + blockIdx.x] = s;
+__global__ void __launch_bounds__(256) lp_hint_c_kernel(const uint8_t* cur, int cp, const uint8_t* ref, int rp, LpGeom g,
+                                                        unsigned long long* cost) {
+    __shared__ unsigned long long red[8], sums[8];
+    const int2 v = vec_c(g, best_b(cost, g, best_a(cost, g, red), red), blockIdx.x);
+    const int r0 = blockIdx.y * kHintSlab, r1 = min((g.H + 1) / 2, r0 + kHintSlab);
+    const unsigned long long s = block_sum_u64(frame_sad_part(cur, cp, ref, rp, g.W, g.H, v.x, v.y, 2, r0, r1), sums);
+    if (threadIdx.x == 0) atomicAdd(&cost[hint_na(g) + 49 + blockIdx.x], s);
 }
 
-__global__ void lp_pick_kernel(const unsigned long long* cost, LpGeom g, int2* hint) {
-    const int2 b = best_b(cost, g, best_a(cost, g));
-    const unsigned long long* cc = cost + hint_na(g) + 49;
-    unsigned long long bc = ~0ull;
-    int2 best = make_int2(0, 0);
-    for (int k = 0; k < 25; ++k) {
-        const int2 v = vec_c(g, b, k);
-        if (hint_less(cc[k], v.x, v.y, bc, best.x, best.y)) {
-            bc = cc[k];
-            best = v;
-        }
-    }
-    *hint = best;
+__global__ void __launch_bounds__(256) lp_pick_kernel(const unsigned long long* cost, LpGeom g, int2* hint) {
+    __shared__ unsigned long long red[8];
+    const int2 b = best_b(cost, g, best_a(cost, g, red), red);
+    const int k = best_of(cost + hint_na(g) + 49, 25, [&](int i) { return vec_c(g, b, i); }, red);
+    if (threadIdx.x == 0) *hint = vec_c(g, b, k);
 }
 
 // The full-resolution frame SAD at the hint (stride 1, clamped sampling): the analysis pass's
 // global_full_sad when the hint stands in for the global search. `sad` is zeroed by the launcher.
-__global__ void lp_hint_sad_kernel(const uint8_t* cur, int cp, const uint8_t* ref, int rp, LpGeom g, const int2* hint,
-                                   unsigned long long* sad) {
+__global__ void __launch_bounds__(256) lp_hint_sad_kernel(const uint8_t* cur, int cp, const uint8_t* ref, int rp, LpGeom g,
+                                                          const int2* hint, unsigned long long* sad) {
     __shared__ unsigned long long red[8];
     const int2 h = *hint;
-    unsigned long long s = 0;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < (long)g.W * g.H; i += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % g.W), y = (int)(i / g.W);
-        const int rx = min(max(x + h.x, 0), g.W - 1), ry = min(max(y + h.y, 0), g.H - 1);
-        s += (unsigned)abs((int)cur[(size_t)y * cp + x] - (int)ref[(size_t)ry * rp + rx]);
-    }
-    s = block_sum_u64(s, red);
+    const int r0 = blockIdx.x * kHintSlab, r1 = min(g.H, r0 + kHintSlab);
+    const unsigned long long s = block_sum_u64(frame_sad_part(cur, cp, ref, rp, g.W, g.H, h.x, h.y, 1, r0, r1), red);
     if (threadIdx.x == 0) atomicAdd(sad, s);
 }
 
@@ -364,6 +346,17 @@ __global__ void lp_feat_kernel(const uint8_t* ref, int rp, LpGeom g, const uint8
     x0[2 * (size_t)i + 1] = hi;
 }
 
+// 16 bytes from global to shared memory without a register round trip, or 16 zero bytes (!on). All of
+// a thread's copies are in flight at once; operand_wait() completes them and makes them visible to the
+// tensor cores' proxy. Staged through registers a tile's loads came in groups of a few.
+__device__ __forceinline__ void copy16(uint8_t* dst, const void* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void operand_wait() {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    fence_async_smem();
+}
+
 // ---- the convolutions on the tensor cores --------------------------------------------------
 
 // One CTA (4 warps = the 128 tensor-memory lanes) per 128-sample row segment, persistent over
@@ -396,6 +389,11 @@ __global__ void __launch_bounds__(128) lp_conv_kernel(const __grid_constant__ Lp
     constexpr uint32_t idesc = idesc_bf16(128, 32, false, false);
     uint32_t phase = 0;
     bool ok = true;
+    float db[DGRAD ? 32 : 1];
+    if (DGRAD) {
+#pragma unroll
+        for (int c = 0; c < (DGRAD ? 32 : 1); ++c) db[c] = 0.0f;
+    }
     const uint4* X = static_cast<const uint4*>(a.x);
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const int seg = t % segs, row = (t / segs) % a.H4, f = t / (segs * a.H4);
@@ -404,12 +402,10 @@ __global__ void __launch_bounds__(128) lp_conv_kernel(const __grid_constant__ Lp
         for (int i = tid; i < 3 * kHaloW * CH; i += 128) {
             const int j = i % CH, p = (i / CH) % kHaloW, r = i / (CH * kHaloW);
             const int xx = x0 - 1 + p, yy = row - 1 + r;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (xx >= 0 && xx < a.W4 && yy >= 0 && yy < a.H4)
-                v = __ldg(X + (((size_t)f * a.H4 + yy) * a.W4 + xx) * CH + j);
-            *reinterpret_cast<uint4*>(sA + ((j * 3 + r) * kHaloW + p) * 16) = v;
+            const bool on = xx >= 0 && xx < a.W4 && yy >= 0 && yy < a.H4;
+            copy16(sA + ((j * 3 + r) * kHaloW + p) * 16, on ? X + (((size_t)f * a.H4 + yy) * a.W4 + xx) * CH + j : X, on);
         }
-        fence_async_smem();
+        operand_wait();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
@@ -456,18 +452,15 @@ __global__ void __launch_bounds__(128) lp_conv_kernel(const __grid_constant__ Lp
                     const float g1 = bf16_hi(mw[c / 2]) > 0.0f ? v[c + 1] : 0.0f;
                     w[c / 2] = pack_bf16x2(g0, g1);
                 }
-                // the input layer's bias gradient: the stored (rounded) values, summed over the warp
+                // the input layer's bias gradient: the stored (rounded) values, summed by each lane
+                // over its tiles and by the warp once at the end (160 shuffles and 32 atomic adds per
+                // tile took three quarters of the kernel: 0.50 ms per layer at 4 x 1080p, against
+                // 0.14 for the forward pass)
+                if (valid) {
 #pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    float s0 = valid ? bf16_lo(w[c / 2]) : 0.0f, s1 = valid ? bf16_hi(w[c / 2]) : 0.0f;
-#pragma unroll
-                    for (int o = 16; o; o >>= 1) {
-                        s0 += __shfl_xor_sync(FULLM, s0, o);
-                        s1 += __shfl_xor_sync(FULLM, s1, o);
-                    }
-                    if (lane == 0) {
-                        atomicAdd(a.dbias + c, s0);
-                        atomicAdd(a.dbias + c + 1, s1);
+                    for (int c = 0; c < 32; c += 2) {
+                        db[c] += bf16_lo(w[c / 2]);
+                        db[c + 1] += bf16_hi(w[c / 2]);
                     }
                 }
             }
@@ -481,6 +474,15 @@ __global__ void __launch_bounds__(128) lp_conv_kernel(const __grid_constant__ Lp
         }
         tc_fence_before();
         __syncthreads();
+    }
+    if (DGRAD) {
+#pragma unroll
+        for (int c = 0; c < (DGRAD ? 32 : 1); ++c) {
+            float v = db[c];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULLM, v, o);
+            if (lane == 0) atomicAdd(a.dbias + c, v);
+        }
     }
     __syncthreads();
     tc_fence_after();
@@ -524,19 +526,16 @@ __global__ void __launch_bounds__(128) lp_wgrad_kernel(const __grid_constant__ L
             const int tap = g / CH, j = g % CH, ty = tap / 3, tx = tap % 3;
             const int p = x0 + 8 * kg + r;
             const int xx = p + tx - 1, yy = row + ty - 1;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (p < a.W4 && xx >= 0 && xx < a.W4 && yy >= 0 && yy < a.H4)
-                v = __ldg(X + (((size_t)f * a.H4 + yy) * a.W4 + xx) * CH + j);
-            *reinterpret_cast<uint4*>(sA + ((kg * GP + g) * 8 + r) * 16) = v;
+            const bool on = p < a.W4 && xx >= 0 && xx < a.W4 && yy >= 0 && yy < a.H4;
+            copy16(sA + ((kg * GP + g) * 8 + r) * 16, on ? X + (((size_t)f * a.H4 + yy) * a.W4 + xx) * CH + j : X, on);
         }
         for (int i = tid; i < KG * 4 * 8; i += 128) {
             const int r = i % 8, j = (i / 8) % 4, kg = i / 32;
             const int p = x0 + 8 * kg + r;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (p < a.W4) v = __ldg(DZ + (((size_t)f * a.H4 + row) * a.W4 + p) * 4 + j);
-            *reinterpret_cast<uint4*>(sB + ((kg * 4 + j) * 8 + r) * 16) = v;
+            const bool on = p < a.W4;
+            copy16(sB + ((kg * 4 + j) * 8 + r) * 16, on ? DZ + (((size_t)f * a.H4 + row) * a.W4 + p) * 4 + j : DZ, on);
         }
-        fence_async_smem();
+        operand_wait();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
@@ -737,14 +736,15 @@ cudaError_t lp_launch_hint(const uint8_t* cur, int cur_pitch, const uint8_t* ref
     uint8_t* ref16 = const_cast<uint8_t*>(ref4) + (size_t)g.W4 * g.H4;
     lp_down16_kernel<<<(g.mbw * g.mbh + 255) / 256, 256, 0, s>>>(cur4, ref4, g, cur16, ref16);
     lp_hint_a_kernel<<<na, 256, 0, s>>>(cur16, ref16, g, scratch);
-    lp_hint_b_kernel<<<49, 256, 0, s>>>(cur4, ref4, g, scratch);
-    lp_hint_c_kernel<<<25, 256, 0, s>>>(cur, cur_pitch, ref, ref_pitch, g, scratch);
-    lp_pick_kernel<<<1, 1, 0, s>>>(scratch, g, hint);
-    cudaError_t e = cudaMemsetAsync(hint_sad, 0, sizeof(unsigned long long), s);
+    cudaError_t e = cudaMemsetAsync(scratch + na, 0, (49 + 25) * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
-    const long px = (long)g.W * g.H;
-    lp_hint_sad_kernel<<<(int)std::min<long>((px + 255) / 256, 1184L), 256, 0, s>>>(cur, cur_pitch, ref, ref_pitch, g,
-                                                                                  hint, hint_sad);
+    auto slabs = [](int rows) { return (unsigned)((rows + kHintSlab - 1) / kHintSlab); };
+    lp_hint_b_kernel<<<dim3(49, slabs(g.H4)), 256, 0, s>>>(cur4, ref4, g, scratch);
+    lp_hint_c_kernel<<<dim3(25, slabs((g.H + 1) / 2)), 256, 0, s>>>(cur, cur_pitch, ref, ref_pitch, g, scratch);
+    lp_pick_kernel<<<1, 256, 0, s>>>(scratch, g, hint);
+    e = cudaMemsetAsync(hint_sad, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    lp_hint_sad_kernel<<<slabs(g.H), 256, 0, s>>>(cur, cur_pitch, ref, ref_pitch, g, hint, hint_sad);
     return cudaGetLastError();
 }
 
