@@ -41,6 +41,7 @@ cudaError_t launch_learned_merge(const DevResult& dst, const DevResult& src, con
 cudaError_t launch_subpel_planes(const uint8_t* ref, int pitch, int W, int H, int rnd, int bilinear, uint32_t phase_mask,
                                  uint8_t* out, int opitch, int border, long long stride, cudaStream_t s);
 int warp_bytes_for_host(const WinCfg& wc);
+int umh_offsets(int range);
 struct GState;
 struct GIn;
 size_t gstate_bytes();
@@ -973,6 +974,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     }
     // window / bitset geometry
     WinCfg wc;
+    wc.offs = any_unseeded && !learned && P.me_algorithm == 0 && P.range > 0 ? umh_offsets(P.local_range) : 0;
     if (learned) {
         wc.rw = kLearnRw;
     } else if (any_unseeded) {

@@ -104,7 +104,9 @@ struct SpecBlk;
 struct WarpMem {
     SPtr<uint8_t> cur;          // 16x16 current MB (zero outside the visible raster)
     SPtr<uint8_t> win;          // reference window
+    SPtr<uint64_t> list;        // the refinement's candidate list; the search's finalists
     SPtr<uint64_t> list_satd;   // SATD of the shortlist
+    SPtr<uint32_t> offs;        // the UMH stages' candidate offsets
     SPtr<int2> batch;           // scratch MV batch
     SPtr<uint64_t> batch_cost;
     SPtr<uint64_t> top;         // umh_early's results
@@ -426,7 +428,7 @@ struct MbCtx {
     int gpitch;
     int subpel, fast_subpel, subpel_range, me_quality, mvrange, mant_bits, lam_s;
     uint64_t lam_m;
-    uint32_t batch, cost, satd;  // the warp's shortlist buffers
+    uint32_t batch, cost, satd, list;  // the warp's shortlist buffers
     const uint8_t* sp;           // the pass's prediction planes (nullptr: none)
     int sp_pitch, sp_border;
     long long sp_stride;
@@ -523,10 +525,17 @@ __device__ __forceinline__ uint32_t sp_load4(const uint8_t* p) {
 // Offset in the pass's prediction planes of vector mv's prediction of the bw x bh block at
 // (bx, by), or -1 where the planes do not hold all of it.
 __device__ __forceinline__ long long plane_offset(const MbCtx& c, int2 mv, int bx, int by, int bw, int bh) {
-    const int ix = floor_div4(mv.x), iy = floor_div4(mv.y), hm = mv.x - 4 * ix, vm = mv.y - 4 * iy;
+    const int ix = mv.x >> 2, iy = mv.y >> 2, hm = mv.x & 3, vm = mv.y & 3;  // floor_div4 and its remainder
     const int b = c.sp_border, sx = bx + ix, sy = by + iy;
     if (!c.sp || sx < -b || sx + bw > c.g.W + b || sy < -b || sy + bh > c.g.H + b) return -1;
-    return (long long)(vm * 4 + hm) * c.sp_stride + (long long)(sy + b) * c.sp_pitch + (sx + b);
+    return (long long)((unsigned long long)(uint32_t)(vm * 4 + hm) * (uint32_t)c.sp_stride + (uint32_t)((sy + b) * c.sp_pitch + sx + b));
+}
+
+// Whether vector mv may reach hidden padding at all: false only where hidden_padding (with or without
+// its chroma test) is false, from each test's largest reach.
+__device__ __forceinline__ bool near_padding(const ScoreGeo& g, int bx, int by, int bw, int bh, int2 mv) {
+    return ((g.pads & 1) && bx + bw + 1 + (mv.x >> 2) >= g.vw) || ((g.pads & 2) && by + bh + 1 + (mv.y >> 2) >= g.vh) ||
+           ((g.pads & 4) && (bx >> 1) + 9 + (mv.x >> 3) >= g.cvw) || ((g.pads & 8) && (by >> 1) + 9 + (mv.y >> 3) >= g.cvh);
 }
 
 // The bytes of an 8-byte (4-byte) group of which the first n are visible (n <= 0: none).
@@ -558,36 +567,30 @@ __device__ __noinline__ uint32_t sad_interpolated(uint32_t ctx, int mvx, int mvy
     return __reduce_add_sync(FULL, part);
 }
 
-// SAD of n <= 32 candidates of block (bx,by,bw,bh) (bw = bh in {8,16}) under the CPU law, written
-// to out[]. One out-of-line copy serves every call site. Lane i works out candidate i's legality
-// and address once; the block's 8-pixel row segments lie across 32 (16x16) or 8 (8x8) lanes, whose
-// current pixels stay in registers, and the segments of several candidates are loaded from the
-// prediction planes before any is summed: the routine is bound by the latency of those loads, not
-// by their number. Two SADs share a word in the warp sum (a 16x16 SAD is below 2^16). With the
-// keyed list and the word-wise minima below, a refinement takes 16 K clocks against 43 K for one
-// candidate at a time and selections by shuffles of whole structures (CIF, one macroblock alone).
-// GROUP: the 16x16 candidates whose rows are in flight together (registers bound it: nine, a whole
-// stencil, in the wide-register builds; five under the seeded builds' 128 registers).
+// SAD of the vectors that lanes i < n hold, for block (bx,by,bw,bh) (bw = bh in {8,16}) under the CPU
+// law: kSadBadCode for an illegal one. One out-of-line copy serves every call site. Lane i works out
+// vector i's legality and address once; the block's 8-pixel row segments lie across 32 (16x16) or 8
+// (8x8) lanes, whose current pixels stay in registers, and the segments of several vectors are
+// loaded from the prediction planes before any is summed: the routine is bound by the latency of
+// those loads, not by their number. Two SADs share a word in the warp sum (a 16x16 SAD is below 2^16).
+// GROUP: the 16x16 vectors whose rows are in flight together (registers bound it: nine, a whole
+// stencil, in the unseeded builds; five under the seeded builds' 128 registers).
+constexpr uint32_t kSadBadCode = 0x1FFFF;
 template <int GROUP>
-__device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int n, int bx, int by,
-                                            int bw, int bh, int mode, uint32_t out_off) {
+__device__ __noinline__ uint32_t sad_lanes_core(uint32_t ctx, int mvx, int mvy, int n, int bx, int by, int bw, int bh, int mode) {
     const MbCtx& c = mbctx(ctx);
     const int lane = threadIdx.x & 31;
-    const int2* mvs = reinterpret_cast<const int2*>(g_smem + mvs_off);
-    uint64_t* out = reinterpret_cast<uint64_t*>(g_smem + out_off);
     const int aw = imax(0, imin(bw, c.g.W - bx)), ah = imax(0, imin(bh, c.g.H - by));
-    const int2 mv = lane < n ? mvs[lane] : make_int2(0, 0);
-    bool bad = false;
-    long long off = -1;
-    if (lane < n) {
+    const int2 mv = make_int2(mvx, mvy);
+    bool bad = lane < n && mode_bilinear(mode) && ((mv.x | mv.y) & 1);
+    if (__any_sync(FULL, lane < n && near_padding(c.g, bx, by, bw, bh, mv))) {
         const DevParams P = geo_params(c.g);
-        bad = hidden_padding(P, bx, by, bw, bh, mv.x, mv.y, mode, chroma_gate(bx, by, bw, bh)) ||
-              (mode_bilinear(mode) && ((mv.x | mv.y) & 1));
-        if (!bad) off = plane_offset(c, mv, bx, by, bw, bh);
+        bad = bad || (lane < n && hidden_padding(P, bx, by, bw, bh, mv.x, mv.y, mode, chroma_gate(bx, by, bw, bh)));
     }
+    const long long off = lane < n && !bad ? plane_offset(c, mv, bx, by, bw, bh) : -1;
     const unsigned planes = __ballot_sync(FULL, off >= 0);
     const int cx = bx - c.x0, cy = by - c.y0;
-    uint32_t mine = 0;  // lane i: candidate i's SAD
+    uint32_t mine = 0;
     if (bw == 16) {
         const int r = lane >> 1, c0 = (lane & 1) * 8, vis = r < ah ? aw - c0 : 0;
         const uint32_t m0 = vis_mask(vis), m1 = vis_mask(vis - 4);
@@ -648,7 +651,7 @@ __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int 
             if (k >= 0 && k < 12) mine = k < 4 ? (t0 & 0xffffu) : (k < 8 ? (t0 >> 16) : t1);
         }
     }
-    // the candidates beyond the planes
+    // the vectors beyond the planes
     unsigned rest = __ballot_sync(FULL, lane < n && !bad) & ~planes;
     while (rest) {
         const int i = __ffs(rest) - 1;
@@ -656,8 +659,7 @@ __device__ __noinline__ void sad_batch_core(uint32_t ctx, uint32_t mvs_off, int 
         const uint32_t v = sad_interpolated(ctx, __shfl_sync(FULL, mv.x, i), __shfl_sync(FULL, mv.y, i), bx, by, bw, bh, mode);
         if (lane == i) mine = v;
     }
-    if (lane < n) out[lane] = bad ? kBad : (uint64_t)mine;
-    __syncwarp();
+    return bad ? kSadBadCode : mine;
 }
 
 // Four rows of a 4x4 tile's prediction as words, where the planes do not hold the block.
@@ -741,11 +743,18 @@ __device__ __noinline__ void satd_batch_core(uint32_t ctx, uint32_t mvs_off, int
     __syncwarp();
 }
 
+__device__ __forceinline__ uint32_t sad_lanes(const Mb& m, int2 mv, int n, int bx, int by, int bw, int bh, int mode) {
+    return m.wide ? sad_lanes_core<9>(m.sm.ctx.off, mv.x, mv.y, n, bx, by, bw, bh, mode)
+                  : sad_lanes_core<5>(m.sm.ctx.off, mv.x, mv.y, n, bx, by, bw, bh, mode);
+}
+__device__ __forceinline__ uint64_t sad_of_code(uint32_t c) { return c == kSadBadCode ? kBad : (uint64_t)c; }
+
 // mvs and out point into the warp's shared-memory buffers.
 __device__ __forceinline__ void sad_batch(const DevParams& P, const Mb& m, const int2* mvs, int n, int bx, int by, int bw,
                                           int bh, int mode, uint64_t* out) {
-    if (m.wide) sad_batch_core<9>(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
-    else sad_batch_core<5>(m.sm.ctx.off, soff(mvs), n, bx, by, bw, bh, mode, soff(out));
+    const uint32_t c = sad_lanes(m, m.lane < n ? mvs[m.lane] : make_int2(0, 0), n, bx, by, bw, bh, mode);
+    if (m.lane < n) out[m.lane] = sad_of_code(c);
+    __syncwarp();
 }
 
 __device__ __forceinline__ void satd_batch(const DevParams& P, const Mb& m, const int2* mvs, int n, int bx, int by, int bw,
@@ -773,6 +782,19 @@ __device__ __forceinline__ uint64_t warp_min_key(uint64_t k) {
     const uint32_t h = __reduce_min_sync(FULL, (uint32_t)(k >> 32));
     const uint32_t l = __reduce_min_sync(FULL, (uint32_t)(k >> 32) == h ? (uint32_t)k : 0xffffffffu);
     return ((uint64_t)h << 32) | l;
+}
+
+// A candidate of the integer search as one key: (cost, |dx| + |dy|, dy, dx), each component within
+// +-256. kIllegal (kBad) is the largest cost; legal ones are below 2^17, sampled ones rescaled.
+constexpr uint32_t kIllegal = 0xFFFFF;
+__device__ __forceinline__ uint64_t search_key(uint32_t cost, int dx, int dy) {
+    return ((uint64_t)cost << 32) | ((uint32_t)(iabs(dx) + iabs(dy)) << 18) | ((uint32_t)(dy + 256) << 9) | (uint32_t)(dx + 256);
+}
+__device__ __forceinline__ int search_dx(uint64_t k) { return (int)((uint32_t)k & 511) - 256; }
+__device__ __forceinline__ int search_dy(uint64_t k) { return (int)(((uint32_t)k >> 9) & 511) - 256; }
+__device__ __forceinline__ uint64_t search_cost(uint64_t k) {
+    const uint32_t c = (uint32_t)(k >> 32);
+    return c >= kIllegal ? kBad : c;
 }
 
 struct Top4 {
@@ -814,22 +836,24 @@ __device__ __forceinline__ void top4_merge(Top4& t, uint64_t key) {
 
 // What scoring the macroblock's integer candidates reads, in registers.
 struct SearchGeo {
-    uint32_t win, cur, cur2, cur4;
-    int wp, wx0, wy0, wh, x0, y0, xl, yl, W, H, gpitch;
+    uint32_t base0, cur, cur2, cur4;  // base0: shared offset of the block at (0, 0) in the window
+    int wp, x0, y0, xl, yl, W, H, gpitch;
+    int dx0, dx1, dy0, dy1;  // the displacements whose block lies in the window
     const uint8_t* gref;
     int aw, ah;  // the columns and rows inside the raster
     __device__ __forceinline__ explicit SearchGeo(uint32_t ctx) {
         const MbCtx& c = mbctx(ctx);
-        win = c.win_off;
         cur = c.cur_off >> 2;
         cur2 = c.cur2_off >> 2;
         cur4 = c.cur4_off >> 2;
         wp = c.wp;
-        wx0 = c.wx0;
-        wy0 = c.wy0;
-        wh = c.wh;
         x0 = c.x0;
         y0 = c.y0;
+        base0 = c.win_off + (uint32_t)((c.y0 - c.wy0) * c.wp + (c.x0 - c.wx0));
+        dx0 = c.wx0 - c.x0;
+        dx1 = dx0 + c.wp - 16;
+        dy0 = c.wy0 - c.y0;
+        dy1 = dy0 + c.wh - 16;
         xl = c.xl;
         yl = c.yl;
         W = c.g.W;
@@ -840,18 +864,13 @@ struct SearchGeo {
         ah = c.ah;
     }
     // the candidate's block lies in the window
-    __device__ __forceinline__ bool staged(int dx, int dy) const {
-        const int rx = x0 + dx - wx0, ry = y0 + dy - wy0;
-        return rx >= 0 && ry >= 0 && rx + 16 <= wp && ry + 16 <= wh;
-    }
+    __device__ __forceinline__ bool staged(int dx, int dy) const { return dx >= dx0 && dx <= dx1 && dy >= dy0 && dy <= dy1; }
     // the candidate's block lies in the frame
     __device__ __forceinline__ bool inside(int dx, int dy) const {
         const int x = x0 + dx, y = y0 + dy;
         return aw == 16 && x >= 0 && y >= 0 && x + 16 <= W && y + ah <= H;
     }
-    __device__ __forceinline__ uint32_t base(int dx, int dy) const {
-        return win + (uint32_t)((y0 + dy - wy0) * wp + (x0 + dx - wx0));
-    }
+    __device__ __forceinline__ uint32_t base(int dx, int dy) const { return base0 + (uint32_t)(dy * wp + dx); }
 };
 
 // Packed SAD of the sampled rows r0 .. r0 + nr - 1 (those inside the raster) of a candidate, its
@@ -891,7 +910,6 @@ __device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, 
 // lanes share, each scoring its part of the rows. Every lane calls it with its candidate; !on
 // scores nothing. FAR: candidates may lie beyond the window (long-range vectors), where blocks
 // inside the frame are scored from it.
-constexpr uint32_t kIllegal = 0xFFFFF;
 template <int STRIDE, bool FAR = false>
 __device__ __forceinline__ uint32_t shared_cost(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
     const int part = (threadIdx.x & 31) & ((1 << sh) - 1), nr = (16 / STRIDE) >> sh;
@@ -910,11 +928,11 @@ __device__ __forceinline__ uint32_t shared_cost(uint32_t ctx, const SearchGeo& g
     if (sh > 2) s += __shfl_xor_sync(FULL, s, 4);
     return legal ? s : kIllegal;
 }
-// int_key of it; UINT64_MAX where !on.
+// search_key of it; UINT64_MAX where !on.
 template <int STRIDE>
 __device__ __forceinline__ uint64_t shared_key(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
     const uint32_t c = shared_cost<STRIDE>(ctx, g, on, dx, dy, sh);
-    return on ? int_key(c, dx, dy) : UINT64_MAX;
+    return on ? search_key(c, dx, dy) : UINT64_MAX;
 }
 
 // The four least keys of the sparse lattice over the whole window (:1865-1870, range >= 8), one
@@ -986,8 +1004,8 @@ __device__ __forceinline__ bool match_good(uint64_t sad, uint64_t pixels) {
 // stride-4 grid and the square about its best; and, on a very poor match (local ranges up to 32),
 // the stride-2 grid and the square about its best. Their least full-resolution keys.
 __device__ __forceinline__ uint64_t rescue_around(uint32_t ctx, uint64_t k, int r, int range) {
-    const int xlo = imax(-range, key_dx(k) - r), xhi = imin(range, key_dx(k) + r);
-    const int ylo = imax(-range, key_dy(k) - r), yhi = imin(range, key_dy(k) + r);
+    const int xlo = imax(-range, search_dx(k) - r), xhi = imin(range, search_dx(k) + r);
+    const int ylo = imax(-range, search_dy(k) - r), yhi = imin(range, search_dy(k) + r);
     return box_min(ctx, xlo, ylo, xhi - xlo + 1, yhi - ylo + 1, 1, 1, range, false);
 }
 __device__ __noinline__ uint64_t rescue_coarse(uint32_t ctx, int range) {
@@ -1014,14 +1032,14 @@ __device__ __noinline__ uint64_t umh_early(uint32_t ctx, uint32_t top_off, int g
     Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
     if (range >= 8) t = umh_lattice(ctx, g, range);
     const int i = lane >> 3;
-    const int dx = i == 1 ? iclamp(gdx, -range, range) : (i == 2 && range >= 8 ? key_dx(t.a) : 0);
-    const int dy = i == 1 ? iclamp(gdy, -range, range) : (i == 2 && range >= 8 ? key_dy(t.a) : 0);
+    const int dx = i == 1 ? iclamp(gdx, -range, range) : (i == 2 && range >= 8 ? search_dx(t.a) : 0);
+    const int dy = i == 1 ? iclamp(gdy, -range, range) : (i == 2 && range >= 8 ? search_dy(t.a) : 0);
     uint64_t best = warp_min_key(shared_key<1>(ctx, g, i < 3, dx, dy, 3));
     uint64_t coarse = UINT64_MAX, dense = UINT64_MAX;
-    if (!match_good(key_cost(best), (uint64_t)pixels)) {
+    if (!match_good(search_cost(best), (uint64_t)pixels)) {
         coarse = rescue_coarse(ctx, range);
         if (coarse < best) best = coarse;
-        if (dense_wanted(key_cost(best), (uint64_t)pixels, range)) {
+        if (dense_wanted(search_cost(best), (uint64_t)pixels, range)) {
             dense = rescue_dense(ctx, range);
             if (dense < best) best = dense;
         }
@@ -1036,62 +1054,98 @@ __device__ __noinline__ uint64_t umh_early(uint32_t ctx, uint32_t top_off, int g
         top[5] = dense;
     }
     __syncwarp();
-    return key_cost(best);
+    return search_cost(best);
 }
 
-// The search after the wavefront wait: seeds in seeds[0..ns), umh_early's results in top[]. The
-// result's key.
-__device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint32_t top_off, int ns, int range, int pixels) {
+// The candidate offsets of the search's stages, a launch constant: the 5x5 square, the uneven cross,
+// the hexagon rings, the small hexagon and the closing diamond, packed (dy + 512) << 16 | (dx + 512).
+struct UmhStages {
+    int cs, nh, nv, hs, nr;
+    __host__ __device__ explicit UmhStages(int range) {
+        cs = range >= 96 ? 8 : (range >= 32 ? 4 : 2);
+        nh = range / cs;
+        nv = imin(range, imax(8, range / 2)) / cs;
+        hs = range >= 96 ? 8 : (range >= 24 ? 4 : 2);
+        nr = range / hs;
+    }
+    __host__ __device__ int cross() const { return 25; }
+    __host__ __device__ int rings() const { return 25 + 2 * (nh + nv); }
+    __host__ __device__ int hexagon() const { return rings() + 6 * nr; }
+    __host__ __device__ int total() const { return hexagon() + 10; }
+    __device__ uint32_t offset(int i) const {
+        int dx = 0, dy = 0;
+        if (i < 25) {  // (:1855-1859)
+            dx = i % 5 - 2;
+            dy = i / 5 - 2;
+        } else if (i < rings()) {  // (:1875-1884)
+            const int k = i - 25, j = k < 2 * nh ? k : k - 2 * nh, d = cs * (j / 2 + 1);
+            (k < 2 * nh ? dx : dy) = (j & 1) ? d : -d;
+        } else if (i < hexagon()) {  // (:1889-1897)
+            const int k = i - rings(), r = hs * (k / 6 + 1), h = (r + 1) / 2, q = k % 6;
+            dx = q < 2 ? (q ? r : -r) : ((q & 1) ? h : -h);
+            dy = q < 2 ? 0 : (q < 4 ? -r : r);
+        } else {  // (-2,0) (2,0) (-1,-2) (1,-2) (-1,2) (1,2) (:1902-1908), (-1,0) (1,0) (0,-1) (0,1) (:1909-1913)
+            const int k = i - hexagon(), q = k - 6;
+            if (k < 6) {
+                dx = k < 2 ? (k ? 2 : -2) : ((k & 1) ? 1 : -1);
+                dy = k < 2 ? 0 : (k < 4 ? -2 : 2);
+            } else {
+                dx = q < 2 ? (q ? 1 : -1) : 0;
+                dy = q < 2 ? 0 : (q == 3 ? 1 : -1);
+            }
+        }
+        return ((uint32_t)(dy + 512) << 16) | (uint32_t)(dx + 512);
+    }
+};
+
+// The search after the wavefront wait: seeds in seeds[0..ns), umh_early's results in top[], the
+// stages' offsets in offs[]; fin: room for 36 words. The result's key. The small hexagon is scored
+// together with the closing diamond about the same centre, which stands once the hexagon has not
+// moved (its keys count only then).
+__device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint32_t top_off, uint32_t offs_off, uint32_t fin_off,
+                                          int ns, int range, int pixels) {
     const SearchGeo g(ctx);
+    const UmhStages st(range);
     const int lane = threadIdx.x & 31;
     const int2* seeds = reinterpret_cast<const int2*>(g_smem + seeds_off);
+    const uint32_t* offs = reinterpret_cast<const uint32_t*>(g_smem + offs_off);
     // Each lane keeps the four least of the keys it scored; a stage only needs the least of all.
     Top4 own{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
     uint64_t best = UINT64_MAX;
-    const int cs = range >= 96 ? 8 : (range >= 32 ? 4 : 2);
-    const int nh = range / cs, nv = imin(range, imax(8, range / 2)) / cs;
-    const int hs = range >= 96 ? 8 : (range >= 24 ? 4 : 2);
-    enum { kSeeds, kSquare, kCross, kRings, kHexagon, kDiamond, kDone };
+    enum { kSeeds, kSquare, kCross, kRings, kHexagon, kDiamond };
     int stage = kSeeds, iter = 0;
 #pragma unroll 1
-    while (stage != kDone) {
+    for (;;) {
         // the stage's centre is the least candidate before it
-        const int cx = key_dx(best), cy = key_dy(best);
-        uint64_t least = UINT64_MAX;
-        const int n = stage == kSeeds ? ns : stage == kSquare ? 25 : stage == kCross ? 2 * (nh + nv)
-                    : stage == kRings ? 6 * (range / hs) : stage == kHexagon ? 6 : 4;
+        const int cx = search_dx(best), cy = search_dy(best);
+        const int first = stage == kCross ? st.cross() : stage == kRings ? st.rings() : stage == kHexagon ? st.hexagon()
+                        : stage == kDiamond ? st.hexagon() + 6 : 0;
+        const int n = stage == kSeeds ? ns : stage == kSquare ? 25 : stage == kCross ? st.rings() - st.cross()
+                    : stage == kRings ? st.hexagon() - st.rings() : stage == kHexagon ? 10 : 4;
+        uint64_t least = UINT64_MAX, diamond = UINT64_MAX;
 #pragma unroll 1
         for (int base = 0; base < n;) {
             const int rem = n - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : 2);
-            const int i = base + (lane >> sh);
-            int dx = cx, dy = cy;
+            const int i = base + (lane >> sh), at = imin(i, n - 1);
+            int dx, dy;
             if (stage == kSeeds) {  // predictor, zero, global, then A and C where they exist (:1843-1850)
-                const int2 v = seeds[imin(i, ns - 1)];
+                const int2 v = seeds[at];
                 dx = v.x;
                 dy = v.y;
-            } else if (stage == kSquare) {  // 5x5 around the best (:1855-1859)
-                dx += i % 5 - 2;
-                dy += i / 5 - 2;
-            } else if (stage == kCross) {  // uneven cross (:1875-1884)
-                const int j = i < 2 * nh ? i : i - 2 * nh, d = cs * (j / 2 + 1);
-                if (i < 2 * nh) dx += (j & 1) ? d : -d;
-                else dy += (j & 1) ? d : -d;
-            } else if (stage == kRings) {  // multi-hexagon rings (:1889-1897)
-                const int r = hs * (i / 6 + 1), h = (r + 1) / 2, q = i % 6;
-                dx += q < 2 ? (q ? r : -r) : ((q & 1) ? h : -h);
-                dy += q < 2 ? 0 : (q < 4 ? -r : r);
-            } else if (stage == kHexagon) {  // small hexagon, repeated (:1902-1908)
-                dx += i < 2 ? (i ? 2 : -2) : ((i & 1) ? 1 : -1);
-                dy += i < 2 ? 0 : (i < 4 ? -2 : 2);
-            } else {  // closing diamond (:1909-1913)
-                dx += i < 2 ? (i ? 1 : -1) : 0;
-                dy += i < 2 ? 0 : (i == 3 ? 1 : -1);
+            } else {
+                const uint32_t o = offs[first + at];
+                dx = cx + (int)(o & 0xffff) - 512;
+                dy = cy + (int)(o >> 16) - 512;
             }
             dx = iclamp(dx, -range, range);
             dy = iclamp(dy, -range, range);
             const uint64_t k = shared_key<2>(ctx, g, i < n, dx, dy, sh);
-            least = k < least ? k : least;
-            top4_insert(own, k);
+            if (stage == kHexagon && i >= 6) {
+                diamond = k;
+            } else {
+                least = k < least ? k : least;
+                top4_insert(own, k);
+            }
             base += 32 >> sh;
         }
         if (stage == kSquare && range >= 8 && lane < 4) {  // the lattice comes after the square
@@ -1101,31 +1155,54 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
         }
         least = warp_min_key(least);
         if (least < best) best = least;
-        if (stage != kHexagon || ++iter == 32 || (key_dx(best) == cx && key_dy(best) == cy)) ++stage;
+        if (stage < kHexagon) {
+            ++stage;
+        } else if (stage == kHexagon) {
+            if (search_dx(best) == cx && search_dy(best) == cy) {
+                top4_insert(own, diamond);
+                break;
+            }
+            if (++iter == 32) stage = kDiamond;  // the last hexagon moved: the diamond about its end
+        } else {
+            break;
+        }
     }
     const Top4 t = top4_gather(own);
-    // full-resolution 3x3 about the four finalists (:1929-1952)
-    uint64_t fk = UINT64_MAX;
+    // full-resolution 3x3 about the four finalists (:1929-1952), each vector once
     const int nf = 9 * ((t.a != UINT64_MAX) + (t.b != UINT64_MAX) + (t.c != UINT64_MAX) + (t.d != UINT64_MAX));
+    uint32_t* fin = reinterpret_cast<uint32_t*>(g_smem + fin_off);
+    int nd = 0;
 #pragma unroll 1
-    for (int base = 0; base < nf;) {
-        const int rem = nf - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : (rem > 4 ? 2 : 3));
-        const int i = base + (lane >> sh), f = i / 9, q = i % 9;
+    for (int base = 0; base < nf; base += 32) {
+        const int i = base + lane, f = i / 9, q = i - 9 * f;
         const uint64_t c = f == 0 ? t.a : (f == 1 ? t.b : (f == 2 ? t.c : t.d));
-        const uint64_t k = shared_key<1>(ctx, g, i < nf, iclamp(key_dx(c) + q % 3 - 1, -range, range),
-                                         iclamp(key_dy(c) + q / 3 - 1, -range, range), sh);
+        const int dx = iclamp(search_dx(c) + q % 3 - 1, -range, range), dy = iclamp(search_dy(c) + q / 3 - 1, -range, range);
+        auto covered = [&](uint64_t k) { return iabs(dx - search_dx(k)) <= 1 && iabs(dy - search_dy(k)) <= 1; };
+        const bool fresh = i < nf && !(f > 0 && covered(t.a)) && !(f > 1 && covered(t.b)) && !(f > 2 && covered(t.c));
+        const unsigned fm = __ballot_sync(FULL, fresh);
+        if (fresh) fin[nd + __popc(fm & ((1u << lane) - 1))] = ((uint32_t)(dy + 512) << 16) | (uint32_t)(dx + 512);
+        nd += __popc(fm);
+    }
+    __syncwarp();
+    uint64_t fk = UINT64_MAX;
+#pragma unroll 1
+    for (int base = 0; base < nd;) {
+        const int rem = nd - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : (rem > 4 ? 2 : 3));
+        const int i = base + (lane >> sh);
+        const uint32_t o = fin[imin(i, nd - 1)];
+        const uint64_t k = shared_key<1>(ctx, g, i < nd, (int)(o & 0xffff) - 512, (int)(o >> 16) - 512, sh);
         fk = k < fk ? k : fk;
         base += 32 >> sh;
     }
     fk = warp_min_key(fk);
     // bounded rescue on a poor match (:1958-2020)
     const uint64_t px = (uint64_t)pixels;
-    if (range > 0 && !match_good(key_cost(fk), px)) {
+    if (range > 0 && !match_good(search_cost(fk), px)) {
         const uint64_t* top = reinterpret_cast<const uint64_t*>(g_smem + top_off);
         uint64_t k = top[4];
         if (k == UINT64_MAX) k = rescue_coarse(ctx, range);
         if (k < fk) fk = k;
-        if (dense_wanted(key_cost(fk), px, range)) {
+        if (dense_wanted(search_cost(fk), px, range)) {
             k = top[5];
             if (k == UINT64_MAX) k = rescue_dense(ctx, range);
             if (k < fk) fk = k;
@@ -1142,8 +1219,9 @@ __device__ IntRes umh(const DevParams& P, const Mb& m, const PInfo& pi, int gdx,
                                          : make_int2(round_qpel_to_pixel(v.x), round_qpel_to_pixel(v.y));
     }
     __syncwarp();
-    const uint64_t fk = umh_core(m.sm.ctx.off, soff(m.sm.batch), soff(m.sm.top), ns, range, (int)pixels);
-    return IntRes{key_dx(fk), key_dy(fk), key_cost(fk)};
+    const uint64_t fk = umh_core(m.sm.ctx.off, soff(m.sm.batch), soff(m.sm.top), m.sm.offs.off, m.sm.list.off, ns, range,
+                                 (int)pixels);
+    return IntRes{search_dx(fk), search_dy(fk), search_cost(fk)};
 }
 
 // integer_motion_diamond, encoder_motion_diamond.cpp:13-73
@@ -1518,76 +1596,48 @@ static_assert(sizeof(SpecBlk) <= kSpecBlkBytes, "SpecBlk layout");
 
 __device__ __forceinline__ int make_even(int v) { return !(v & 1) ? v : (v > 0 ? v - 1 : v + 1); }
 
-// ---- the refinement's candidate list, held across the warp's lanes -------------------------
+// ---- the refinement's candidate list ---------------------------------------------------------
 //
-// Lane j < n holds list entry j as one key: (SAD, |x| + |y|, y, x), the reference's (sad, tie_less)
-// order, with the vector recoverable from it. Entries are distinct vectors; their order is
-// immaterial because every selection over them uses a total order, so membership tests are warp
-// votes and minima two 32-bit warp reductions. A SAD is below 2^16 or kBad (the largest code);
-// components lie within +-4096 and +-1024.
-constexpr uint32_t kSadBadCode = 0x1FFFF;
-
+// An entry is one key: (SAD, |x| + |y|, y, x), the reference's (sad, tie_less) order, with the vector
+// recoverable from it. The entries (distinct vectors) stand in shared memory in any order, because
+// every selection over them uses a total order; a stencil's keys are in its lanes' registers, so a
+// membership test is a few broadcast loads and a minimum two 32-bit warp reductions. A SAD is below
+// 2^16 or kBad (the largest code); components lie within +-4096 and +-1024.
 __device__ __forceinline__ uint32_t mv_id(int2 v) { return ((uint32_t)(v.y + 2048) << 14) | (uint32_t)(v.x + 8192); }
 __device__ __forceinline__ int2 id_mv(uint32_t id) { return make_int2((int)(id & 0x3FFF) - 8192, (int)((id >> 14) & 0xFFF) - 2048); }
-__device__ __forceinline__ uint64_t sad_key(uint64_t sad, int2 v) {
-    const uint64_t c = sad >= kBad ? kSadBadCode : (uint32_t)sad;
-    return (c << 40) | ((uint64_t)(iabs(v.x) + iabs(v.y)) << 26) | mv_id(v);
+__device__ __forceinline__ uint64_t code_key(uint32_t code, int2 v) {
+    return ((uint64_t)code << 40) | ((uint64_t)(iabs(v.x) + iabs(v.y)) << 26) | mv_id(v);
 }
-__device__ __forceinline__ uint64_t key_sad(uint64_t k) {
-    const uint32_t c = (uint32_t)(k >> 40);
-    return c == kSadBadCode ? kBad : c;
-}
+__device__ __forceinline__ uint64_t sad_key(uint64_t sad, int2 v) { return code_key(sad >= kBad ? kSadBadCode : (uint32_t)sad, v); }
+__device__ __forceinline__ uint64_t key_sad(uint64_t k) { return sad_of_code((uint32_t)(k >> 40)); }
 __device__ __forceinline__ int2 sad_key_mv(uint64_t k) { return id_mv((uint32_t)k & 0x3FFFFFFu); }
 
-struct RegList {
-    int n;         // warp-uniform entry count (<= 32)
-    uint64_t key;  // this lane's entry (UINT64_MAX: none)
-};
-
-// Adds the candidates that lanes i < nb hold in `c` and the list lacks, in lane order, and
-// scores the new ones with the CPU law in one batch (the `add` lambda, :3324-3337). Returns whether
-// this lane's entry is one of the nb candidates.
-__device__ __forceinline__ bool reg_add(const DevParams& P, const Mb& m, RegList& L, int2 c, int nb, int bx, int by,
-                                        int bw, int bh, int mode) {
+// Adds the vectors that lanes i < nb hold in `c` and the list lacks (n entries so far), scored with
+// the CPU law (the `add` lambda, :3324-3337; hidden padding costs BAD). Returns the lane's key
+// (UINT64_MAX for lanes >= nb). Listed vectors are scored again with the rest: a lane costs nothing.
+__device__ __forceinline__ uint64_t list_add(const Mb& m, int& n, int2 c, int nb, int bx, int by, int bw, int bh, int mode) {
     const bool act = m.lane < nb;
-    const uint32_t id = mv_id(c), own = m.lane < L.n ? (uint32_t)L.key & 0x3FFFFFFu : 0xffffffffu;
-    bool listed = false, among = false;
-#pragma unroll 3
-    for (int i = 0; i < nb; ++i) {
-        const bool same = own == __shfl_sync(FULL, id, i);
-        const bool hit = __any_sync(FULL, same);
-        among |= same;
-        if (m.lane == i) listed = hit;
-    }
-    const unsigned amask = (nb >= 32) ? FULL : ((1u << nb) - 1);
+    const uint32_t id = mv_id(c);
+    const uint32_t code = sad_lanes(m, c, nb, bx, by, bw, bh, mode);
+    int at = -1;
+#pragma unroll 4
+    for (int e = 0; e < n; ++e)
+        if (((uint32_t)m.sm.list[e] & 0x3FFFFFFu) == id) at = e;
+    const uint64_t key = act ? (at >= 0 ? m.sm.list[at] : code_key(code, c)) : UINT64_MAX;
     bool first = false;
-    if (act) first = (__ffs(__match_any_sync(amask, id)) - 1) == m.lane;
-    const bool fresh = act && !listed && first;
+    if (act) first = (__ffs(__match_any_sync((1u << nb) - 1, id)) - 1) == m.lane;
+    const bool fresh = first && at < 0;
     const unsigned fm = __ballot_sync(FULL, fresh);
-    const int nn = __popc(fm);
-    if (!nn) return among;
-    if (fresh) m.sm.batch[__popc(fm & ((1u << m.lane) - 1))] = c;
+    if (fresh) m.sm.list[n + __popc(fm & ((1u << m.lane) - 1))] = key;
+    n += __popc(fm);
     __syncwarp();
-    sad_batch(P, m, m.sm.batch, nn, bx, by, bw, bh, mode, m.sm.batch_cost);  // hidden padding costs BAD
-    if (m.lane >= L.n && m.lane < L.n + nn) {
-        L.key = sad_key(m.sm.batch_cost[m.lane - L.n], m.sm.batch[m.lane - L.n]);
-        among = true;
-    }
-    L.n += nn;
-    __syncwarp();
-    return among;
+    return key;
 }
 
-// The least entry among the lanes with `in`, folded into `best` by the same order.
-__device__ __forceinline__ void reg_update_min(const RegList& L, bool in, uint64_t& best) {
-    const uint64_t k = warp_min_key(in ? L.key : UINT64_MAX);
+// The least of the lanes' keys, folded into `best`.
+__device__ __forceinline__ void fold_least(uint64_t key, uint64_t& best) {
+    const uint64_t k = warp_min_key(key);
     if (k < best) best = k;
-}
-
-// Key of the listed vector v (warp-uniform; it must be listed).
-__device__ __forceinline__ uint64_t reg_find(const RegList& L, int lane, int2 v) {
-    const unsigned hit = __ballot_sync(FULL, lane < L.n && ((uint32_t)L.key & 0x3FFFFFFu) == mv_id(v));
-    return __shfl_sync(FULL, L.key, __ffs(hit) - 1);
 }
 
 // refine_motion_integer_only, encoder_motion.cpp:3247-3269
@@ -1631,14 +1681,16 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
         seed = make_int2(0, 0);
         known = UINT64_MAX;
     }
-    RegList L{0, UINT64_MAX};
+    int n = 0;
+    uint64_t best_key;
     if (known != UINT64_MAX) {
-        L.n = 1;
-        if (m.lane == 0) L.key = sad_key(known, seed);
+        n = 1;
+        best_key = sad_key(known, seed);
+        if (m.lane == 0) m.sm.list[0] = best_key;
+        __syncwarp();
     } else {
-        reg_add(P, m, L, seed, 1, bx, by, bw, bh, emode);
+        best_key = __shfl_sync(FULL, list_add(m, n, seed, 1, bx, by, bw, bh, emode), 0);
     }
-    uint64_t best_key = __shfl_sync(FULL, L.key, 0);
     int2 best = seed;
     auto fix = [&](int2 v) {
         v.x = iclamp(v.x, xmin, xmax);
@@ -1649,7 +1701,7 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
     // one stencil stage: gen(i) for i < np, clamped, scored and folded into (cost, best)
     auto stage = [&](int np, auto gen) {
         const int2 c = m.lane < np ? fix(gen(m.lane)) : make_int2(0, 0);
-        reg_update_min(L, reg_add(P, m, L, c, np, bx, by, bw, bh, emode), best_key);
+        fold_least(list_add(m, n, c, np, bx, by, bw, bh, emode), best_key);
         best = sad_key_mv(best_key);
     };
     // the two candidates beside an axis move: (c.x, c.y -/+ d) or (c.x -/+ d, c.y)
@@ -1725,17 +1777,17 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
     seed.x = iclamp(seed.x, xmin, xmax);
     seed.y = iclamp(seed.y, ymin, ymax);
     if (hp) { seed.x = make_even(seed.x); seed.y = make_even(seed.y); }
-    RegList L{0, UINT64_MAX};
+    int n = 0;
     const bool seed_hidden = hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, mode, cg);
-    // add(seed, known)
+    // add(seed, known); an unknown seed is scored with the first stencil, which holds it
+    uint64_t half_key = UINT64_MAX;
     if (known != UINT64_MAX) {
-        L.n = 1;
-        if (m.lane == 0) L.key = sad_key(seed_hidden ? kBad : known, seed);
-    } else {
-        reg_add(P, m, L, seed, 1, bx, by, bw, bh, mode);
+        n = 1;
+        half_key = sad_key(seed_hidden ? kBad : known, seed);
+        if (m.lane == 0) m.sm.list[0] = half_key;
+        __syncwarp();
     }
-    if (seed_hidden) reg_add(P, m, L, make_int2(0, 0), 1, bx, by, bw, bh, mode);
-    uint64_t half_key = __shfl_sync(FULL, L.key, 0);
+    if (seed_hidden) list_add(m, n, make_int2(0, 0), 1, bx, by, bw, bh, mode);
     int2 half_best = seed;
     const bool fast = P.fast_subpel;
     auto clampmv = [&](int x, int y) {
@@ -1749,7 +1801,7 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
         const int2 c = fast ? (i == 0 ? seed : i == 1 ? clampmv(seed.x - 2, seed.y) : i == 2 ? clampmv(seed.x + 2, seed.y)
                                              : i == 3 ? clampmv(seed.x, seed.y - 2) : clampmv(seed.x, seed.y + 2))
                             : clampmv(seed.x + (i % 3 - 1) * 2, seed.y + (i / 3 - 1) * 2);
-        reg_update_min(L, reg_add(P, m, L, c, nb, bx, by, bw, bh, mode), half_key);
+        fold_least(list_add(m, n, c, nb, bx, by, bw, bh, mode), half_key);
         half_best = sad_key_mv(half_key);
     }
     if (fast && !(half_best.x == seed.x && half_best.y == seed.y)) {
@@ -1766,7 +1818,7 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
         }
         if (hp) { c.x = make_even(c.x); c.y = make_even(c.y); }
         if (nd) {
-            reg_update_min(L, reg_add(P, m, L, c, nd, bx, by, bw, bh, mode), half_key);
+            fold_least(list_add(m, n, c, nd, bx, by, bw, bh, mode), half_key);
             half_best = sad_key_mv(half_key);
         }
     }
@@ -1777,36 +1829,33 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
                          : i == 2 ? make_int2(iclamp(qc.x + 1, xmin, xmax), qc.y)
                          : i == 3 ? make_int2(qc.x, iclamp(qc.y - 1, ymin, ymax))
                                   : make_int2(qc.x, iclamp(qc.y + 1, ymin, ymax));
-            const bool in = reg_add(P, m, L, c, 5, bx, by, bw, bh, mode);
-            uint64_t qkey = reg_find(L, m.lane, qc);
-            reg_update_min(L, in, qkey);
+            uint64_t qkey = UINT64_MAX;
+            fold_least(list_add(m, n, c, 5, bx, by, bw, bh, mode), qkey);
             const int2 qbmv = sad_key_mv(qkey);
             const int dx = qbmv.x - qc.x, dy = qbmv.y - qc.y;
             if (dx && !dy) {
-                reg_add(P, m, L, make_int2(qbmv.x, iclamp(qc.y + (i ? 1 : -1), ymin, ymax)), 2, bx, by, bw, bh, mode);
+                list_add(m, n, make_int2(qbmv.x, iclamp(qc.y + (i ? 1 : -1), ymin, ymax)), 2, bx, by, bw, bh, mode);
             } else if (dy && !dx) {
-                reg_add(P, m, L, make_int2(iclamp(qc.x + (i ? 1 : -1), xmin, xmax), qbmv.y), 2, bx, by, bw, bh, mode);
+                list_add(m, n, make_int2(iclamp(qc.x + (i ? 1 : -1), xmin, xmax), qbmv.y), 2, bx, by, bw, bh, mode);
             }
         } else {
             const int2 hbv = half_best;
-            reg_add(P, m, L, make_int2(iclamp(hbv.x + i % 3 - 1, xmin, xmax), iclamp(hbv.y + i / 3 - 1, ymin, ymax)), 9,
+            list_add(m, n, make_int2(iclamp(hbv.x + i % 3 - 1, xmin, xmax), iclamp(hbv.y + i / 3 - 1, ymin, ymax)), 9,
                     bx, by, bw, bh, mode);
         }
     }
     // sort by (sad, tie_less), keep 8 / 4 (:3445-3456): each entry ranks itself among all, read
     // from shared memory (broadcast loads)
     const int keep = fast ? 4 : 8;
-    m.sm.batch_cost[m.lane] = L.key;
-    __syncwarp();
+    const uint64_t key = m.lane < n ? m.sm.list[m.lane] : UINT64_MAX;
     int rank = 0;
 #pragma unroll 4
-    for (int k = 0; k < L.n; ++k) rank += m.sm.batch_cost[k] < L.key ? 1 : 0;
-    const uint64_t screen = key_sad(warp_min_key(L.key));
-    const int nk = imin(L.n, keep);
-    __syncwarp();
-    if (m.lane < L.n && rank < nk) {
-        m.sm.batch[rank] = sad_key_mv(L.key);
-        m.sm.batch_cost[rank] = key_sad(L.key);
+    for (int k = 0; k < n; ++k) rank += m.sm.list[k] < key ? 1 : 0;
+    const uint64_t screen = key_sad(warp_min_key(key));
+    const int nk = imin(n, keep);
+    if (m.lane < n && rank < nk) {
+        m.sm.batch[rank] = sad_key_mv(key);
+        m.sm.batch_cost[rank] = key_sad(key);
     }
     __syncwarp();
     sl.direct = 0;
@@ -1932,6 +1981,7 @@ __device__ void publish_ctx(const DevParams& P, const Mb& m) {
         r.batch = m.sm.batch.off;
         r.cost = m.sm.batch_cost.off;
         r.satd = m.sm.list_satd.off;
+        r.list = m.sm.list.off;
         r.sp = m.d->sp_planes;
         r.sp_pitch = m.d->sp_pitch;
         r.sp_border = m.d->sp_border;
@@ -1974,6 +2024,7 @@ __device__ __forceinline__ void ref_unpack(uint32_t ctx, DevParams& P, Mb& m) {
     m.sm.batch.off = r.batch;
     m.sm.batch_cost.off = r.cost;
     m.sm.list_satd.off = r.satd;
+    m.sm.list.off = r.list;
 }
 
 // DR: the launch runs the default refinement (me_quality SATD, the full stencils); fixing those
@@ -2337,6 +2388,8 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
         return q;
     };
     s.list_satd.off = take(8 * kListCap);
+    s.list.off = take(8 * 32);
+    s.offs.off = take(4 * (uint32_t)wc.offs);
     s.batch_cost.off = take(8 * 32);
     s.top.off = take(8 * 8);
     s.batch.off = take(8 * 32);
@@ -2361,12 +2414,13 @@ __device__ void carve(WarpMem& s, uint32_t base, const WinCfg& wc) {
 
 __host__ __device__ inline int warp_bytes_for(const WinCfg& wc) {
     auto r = [](int b) { return (b + 15) & ~15; };
-    return r(8 * kListCap) + r(8 * 32) + r(64) + r(8 * 32) + r(128) + r(64) + r(32) + r(32) +
+    return r(8 * kListCap) + r(8 * 32) + r(4 * wc.offs) + r(8 * 32) + r(64) + r(8 * 32) + r(128) + r(64) + r(32) + r(32) +
            r(128) + r(16) + 3 * r(8 * 40) + r(kSpecBlkBytes * 5) + r(kMbCtxBytes) + r(256) + r(8) + 128 +
            r(wc.wp * wc.wh + 32);
 }
 
 int warp_bytes_for_host(const WinCfg& wc) { return warp_bytes_for(wc); }
+int umh_offsets(int range) { return UmhStages(range).total(); }
 
 // 16 bytes from global to shared memory without a register round trip (cp.async; both
 // addresses 16-byte aligned). The copy lands by the next window_wait().
@@ -2556,6 +2610,11 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
     if (wc.tma && m.lane == 0) tma_bar_init(sh_addr(m.sm.tma_bar.get()));
     __syncwarp();
     const int range = P0.range, local_range = P0.local_range;  // one search configuration per launch
+    if ((KIND & kCoreUnseededOnly) && wc.offs) {
+        const UmhStages st(local_range);
+        for (int i = m.lane; i < st.total(); i += 32) m.sm.offs[i] = st.offset(i);
+        __syncwarp();
+    }
     for (;;) {
         unsigned item = 0;
         if (m.lane == 0) item = atomicAdd(&st->queue, 1u);

@@ -99,6 +99,7 @@ struct WinCfg {
     int rw;        // window radius in integer pixels around its centre MV
     int wh;        // window height = 16 + 2*rw + 3
     int wp;        // window row pitch = width: wh + 15 rounded up to 16 (16-byte-aligned origin)
+    int offs;      // words of the UMH stages' offset table (0: no UMH search)
     int warp_bytes;
     int tma;       // 1: windows wholly inside the picture are staged by one TMA tensor copy
 };
