@@ -130,10 +130,8 @@ __host__ __device__ inline int round_qpel_to_pixel(int q) { return q >= 0 ? (q +
 
 // Vc1Encoder::modular_component_distance / modular_mv_distance, encoder_motion.cpp:1298-1310
 __device__ inline int modular_component_distance(int a, int b, int range) {
-    int d = a - b;
-    const int span = range * 2;
-    d = ((d + range) % span + span) % span - range;
-    return iabs(d);
+    const int span = range * 2;  // a power of two: the residue modulo span is a mask
+    return iabs(((a - b + range) & (span - 1)) - range);
 }
 // mvrange_x_qpel {256,512,2048,4096} / mvrange_y_qpel {128,256,512,1024} (:1263-1271)
 __device__ __forceinline__ int mvrange_xq(int r) { return r < 2 ? (256 << r) : (2048 << (r - 2)); }

@@ -567,6 +567,16 @@ __device__ __noinline__ uint32_t sad_interpolated(uint32_t ctx, int mvx, int mvy
     return __reduce_add_sync(FULL, part);
 }
 
+// hidden_padding, out of line (each of its several call sites took 60-100 instructions), and only
+// where the vector may reach the padding.
+__device__ __noinline__ bool hidden_ool(uint32_t ctx, int bx, int by, int bw, int bh, int mvx, int mvy, int mode, bool chroma) {
+    const DevParams P = geo_params(mbctx(ctx).g);
+    return hidden_padding(P, bx, by, bw, bh, mvx, mvy, mode, chroma);
+}
+__device__ __forceinline__ bool hidden_near(uint32_t ctx, int bx, int by, int bw, int bh, int2 mv, int mode, bool chroma) {
+    return near_padding(mbctx(ctx).g, bx, by, bw, bh, mv) && hidden_ool(ctx, bx, by, bw, bh, mv.x, mv.y, mode, chroma);
+}
+
 // SAD of the vectors that lanes i < n hold, for block (bx,by,bw,bh) (bw = bh in {8,16}) under the CPU
 // law: kSadBadCode for an illegal one. One out-of-line copy serves every call site. Lane i works out
 // vector i's legality and address once; the block's 8-pixel row segments lie across 32 (16x16) or 8
@@ -583,10 +593,7 @@ __device__ __noinline__ uint32_t sad_lanes_core(uint32_t ctx, int mvx, int mvy, 
     const int aw = imax(0, imin(bw, c.g.W - bx)), ah = imax(0, imin(bh, c.g.H - by));
     const int2 mv = make_int2(mvx, mvy);
     bool bad = lane < n && mode_bilinear(mode) && ((mv.x | mv.y) & 1);
-    if (__any_sync(FULL, lane < n && near_padding(c.g, bx, by, bw, bh, mv))) {
-        const DevParams P = geo_params(c.g);
-        bad = bad || (lane < n && hidden_padding(P, bx, by, bw, bh, mv.x, mv.y, mode, chroma_gate(bx, by, bw, bh)));
-    }
+    bad = bad || (lane < n && hidden_near(ctx, bx, by, bw, bh, mv, mode, chroma_gate(bx, by, bw, bh)));
     const long long off = lane < n && !bad ? plane_offset(c, mv, bx, by, bw, bh) : -1;
     const unsigned planes = __ballot_sync(FULL, off >= 0);
     const int cx = bx - c.x0, cy = by - c.y0;
@@ -773,7 +780,7 @@ __device__ __forceinline__ void satd_batch(const DevParams& P, const Mb& m, cons
 // search, so it is written for its latency: stages of few candidates spread each one's rows over
 // several lanes, and the neighbour-independent lattice is scored before the wait (umh_lattice).
 // A CIF picture alone (clocks per macroblock after the wait): 28 K with the stages' candidates one
-// per lane, first-visit bitsets and a top-8 list in shared memory, 16 K now (and 6 K before the
+// per lane, first-visit bitsets and a top-8 list in shared memory, 15 K now (and 6 K before the
 // wait for the lattice); a 720p B picture's two passes at range 64, 9.3 -> 4.5 ms with the
 // refinement below.
 
@@ -834,94 +841,74 @@ __device__ __forceinline__ void top4_merge(Top4& t, uint64_t key) {
     }
 }
 
-// What scoring the macroblock's integer candidates reads, in registers.
-struct SearchGeo {
-    uint32_t base0, cur, cur2, cur4;  // base0: shared offset of the block at (0, 0) in the window
-    int wp, x0, y0, xl, yl, W, H, gpitch;
-    int dx0, dx1, dy0, dy1;  // the displacements whose block lies in the window
-    const uint8_t* gref;
-    int aw, ah;  // the columns and rows inside the raster
-    __device__ __forceinline__ explicit SearchGeo(uint32_t ctx) {
-        const MbCtx& c = mbctx(ctx);
-        cur = c.cur_off >> 2;
-        cur2 = c.cur2_off >> 2;
-        cur4 = c.cur4_off >> 2;
-        wp = c.wp;
-        x0 = c.x0;
-        y0 = c.y0;
-        base0 = c.win_off + (uint32_t)((c.y0 - c.wy0) * c.wp + (c.x0 - c.wx0));
-        dx0 = c.wx0 - c.x0;
-        dx1 = dx0 + c.wp - 16;
-        dy0 = c.wy0 - c.y0;
-        dy1 = dy0 + c.wh - 16;
-        xl = c.xl;
-        yl = c.yl;
-        W = c.g.W;
-        H = c.g.H;
-        gref = c.gref;
-        gpitch = c.gpitch;
-        aw = c.aw;
-        ah = c.ah;
-    }
-    // the candidate's block lies in the window
-    __device__ __forceinline__ bool staged(int dx, int dy) const { return dx >= dx0 && dx <= dx1 && dy >= dy0 && dy <= dy1; }
-    // the candidate's block lies in the frame
-    __device__ __forceinline__ bool inside(int dx, int dy) const {
-        const int x = x0 + dx, y = y0 + dy;
-        return aw == 16 && x >= 0 && y >= 0 && x + 16 <= W && y + ah <= H;
-    }
-    __device__ __forceinline__ uint32_t base(int dx, int dy) const { return base0 + (uint32_t)(dy * wp + dx); }
-};
-
-// Packed SAD of the sampled rows r0 .. r0 + nr - 1 (those inside the raster) of a candidate, its
-// rows staged in the window (at shared offset base) or, GLOBAL, read from the frame (at ref). The
-// current macroblock is zero outside the raster, so its columns there only need the reference's
-// bytes masked away: a bottom row of half macroblocks (1080 lines) runs like any other, where byte
-// loops made it the tail of every 1080p wavefront (120 macroblocks one behind the other).
-template <int STRIDE, bool GLOBAL>
-__device__ __forceinline__ uint32_t sad_rows(const SearchGeo& g, uint32_t base, const uint8_t* ref, int r0, int nr) {
-    uint32_t acc = 0;
-    const int end = imin(r0 + nr, (g.ah + STRIDE - 1) / STRIDE);
-    const bool ragged = g.aw < 16;
-#pragma unroll 2
-    for (int r = r0; r < end; ++r) {
-        uint32_t v[4];
-        if (GLOBAL) glob_load16(ref + (size_t)(r * STRIDE) * g.gpitch, v);
-        else win_load16(base + (uint32_t)(r * STRIDE * g.wp), v);
-        if (ragged) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] &= vis_mask(g.aw - 4 * i);
-        }
-        if (STRIDE == 1) {
-            acc += __vsadu4(v[0], g_smem32[g.cur + r * 4]) + __vsadu4(v[1], g_smem32[g.cur + r * 4 + 1]) +
-                   __vsadu4(v[2], g_smem32[g.cur + r * 4 + 2]) + __vsadu4(v[3], g_smem32[g.cur + r * 4 + 3]);
-        } else if (STRIDE == 2) {
-            acc += __vsadu4(__byte_perm(v[0], v[1], 0x6420), g_smem32[g.cur2 + r * 4]) +
-                   __vsadu4(__byte_perm(v[2], v[3], 0x6420), g_smem32[g.cur2 + r * 4 + 1]);
-        } else {
-            const uint32_t e = __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
-            acc += __vsadu4(e, g_smem32[g.cur4 + 4 * r]);
-        }
-    }
-    return acc;
-}
-
 // Cost (mb_sad at the given stride; kIllegal for kBad) of the candidate that 2^sh neighbouring
 // lanes share, each scoring its part of the rows. Every lane calls it with its candidate; !on
-// scores nothing. FAR: candidates may lie beyond the window (long-range vectors), where blocks
-// inside the frame are scored from it.
-template <int STRIDE, bool FAR = false>
-__device__ __forceinline__ uint32_t shared_cost(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
-    const int part = (threadIdx.x & 31) & ((1 << sh) - 1), nr = (16 / STRIDE) >> sh;
-    const bool legal = dx <= g.xl && dy <= g.yl;
+// scores nothing. One out-of-line copy serves every stage: a search stage is one warp's chain of
+// instructions, most of them fetched anew each time (above 10 KB of code a lone warp issues one per
+// 3 to 6 clocks, measured), so what counts is how few there are. Sampled rows are packed before
+// they are compared (a stride-2 row: 5 loads, 4 shifts, 2 permutes, 2 byte SADs). Clocks of a
+// 32-candidate stage: 2.2 K with every stride's row compared in full under masks, 1.4 K so; a CIF
+// picture's search pass 1.12 -> 1.01 ms. Blocks beyond the window (long-range vectors, shrunken
+// windows) are scored from the frame.
+__device__ __noinline__ uint32_t shared_cost(uint32_t ctx, int dx, int dy, int flags) {
+    // flags: stride | sh << 4 | on << 8
+    const MbCtx& c = mbctx(ctx);
+    const int stride = flags & 15, sh = (flags >> 4) & 15, ls = stride == 1 ? 0 : (stride == 2 ? 1 : 2);
+    const int part = (threadIdx.x & 31) & ((1 << sh) - 1), nr = (16 >> ls) >> sh;
+    const bool legal = dx <= c.xl && dy <= c.yl;
+    const int rx = c.x0 + dx - c.wx0, ry = c.y0 + dy - c.wy0;
+    const bool staged = rx >= 0 && ry >= 0 && rx + 16 <= c.wp && ry + 16 <= c.wh;
     uint32_t s = 0;
-    if (on && legal) {
-        if (!FAR && g.staged(dx, dy))
-            s = sad_rows<STRIDE, false>(g, g.base(dx, dy), nullptr, part * nr, nr) * (STRIDE * STRIDE);
-        else if (FAR && g.inside(dx, dy))
-            s = sad_rows<STRIDE, true>(g, 0, g.gref + (size_t)(g.y0 + dy) * g.gpitch + g.x0 + dx, part * nr, nr) * (STRIDE * STRIDE);
-        else if (part == 0)
-            s = (uint32_t)mb_sad_core(ctx, dx, dy, STRIDE);
+    if ((flags >> 8) && legal) {
+        if (staged) {
+            const int r0 = part * nr, r1 = imin(r0 + nr, (c.ah + stride - 1) >> ls);
+            const int step = c.wp << ls;
+            uint32_t at = c.win_off + (uint32_t)(ry * c.wp + rx + r0 * step);
+            // the staged macroblock is 0 right of the raster: the window's bytes there are masked
+            if (stride == 2) {
+                uint32_t cur = (c.cur2_off >> 3) + 2 * r0;
+                const int vis = (c.aw + 1) >> 1;
+                const uint32_t k0 = vis_mask(vis), k1 = vis_mask(vis - 4);
+#pragma unroll 4
+                for (int r = r0; r < r1; ++r) {
+                    uint32_t v[4];
+                    win_load16(at, v);
+                    const uint2 w = reinterpret_cast<const uint2*>(g_smem)[cur];
+                    s += __vsadu4(__byte_perm(v[0], v[1], 0x6420) & k0, w.x);
+                    s += __vsadu4(__byte_perm(v[2], v[3], 0x6420) & k1, w.y);
+                    at += (uint32_t)step;
+                    cur += 2;
+                }
+            } else if (stride == 1) {
+                uint32_t cur = (c.cur_off >> 4) + r0;
+                const uint32_t k0 = vis_mask(c.aw), k1 = vis_mask(c.aw - 4), k2 = vis_mask(c.aw - 8), k3 = vis_mask(c.aw - 12);
+#pragma unroll 4
+                for (int r = r0; r < r1; ++r) {
+                    uint32_t v[4];
+                    win_load16(at, v);
+                    const uint4 w = reinterpret_cast<const uint4*>(g_smem)[cur];
+                    s += __vsadu4(v[0] & k0, w.x) + __vsadu4(v[1] & k1, w.y);
+                    s += __vsadu4(v[2] & k2, w.z) + __vsadu4(v[3] & k3, w.w);
+                    at += (uint32_t)step;
+                    ++cur;
+                }
+            } else {
+                uint32_t cur = (c.cur4_off >> 2) + 4 * r0;
+                const uint32_t k0 = vis_mask((c.aw + 3) >> 2);
+#pragma unroll 2
+                for (int r = r0; r < r1; ++r) {
+                    uint32_t v[4];
+                    win_load16(at, v);
+                    const uint32_t e = __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
+                    s += __vsadu4(e & k0, g_smem32[cur]);
+                    at += (uint32_t)step;
+                    cur += 4;
+                }
+            }
+            s <<= 2 * ls;
+        } else if (part == 0) {
+            s = (uint32_t)mb_sad_core(ctx, dx, dy, stride);
+        }
     }
     if (sh > 0) s += __shfl_xor_sync(FULL, s, 1);
     if (sh > 1) s += __shfl_xor_sync(FULL, s, 2);
@@ -929,15 +916,14 @@ __device__ __forceinline__ uint32_t shared_cost(uint32_t ctx, const SearchGeo& g
     return legal ? s : kIllegal;
 }
 // search_key of it; UINT64_MAX where !on.
-template <int STRIDE>
-__device__ __forceinline__ uint64_t shared_key(uint32_t ctx, const SearchGeo& g, bool on, int dx, int dy, int sh) {
-    const uint32_t c = shared_cost<STRIDE>(ctx, g, on, dx, dy, sh);
+__device__ __forceinline__ uint64_t shared_key(uint32_t ctx, int stride, bool on, int dx, int dy, int sh) {
+    const uint32_t c = shared_cost(ctx, dx, dy, stride | (sh << 4) | (on ? 256 : 0));
     return on ? search_key(c, dx, dy) : UINT64_MAX;
 }
 
 // The four least keys of the sparse lattice over the whole window (:1865-1870, range >= 8), one
 // candidate per lane.
-__device__ __forceinline__ Top4 umh_lattice(uint32_t ctx, const SearchGeo& g, int range) {
+__device__ __forceinline__ Top4 umh_lattice(uint32_t ctx, int range) {
     const int lane = threadIdx.x & 31;
     const int L = (2 * range) / 8 + 1;
     // the far edges repeat the lattice's last row and column when its step divides the window
@@ -956,7 +942,7 @@ __device__ __forceinline__ Top4 umh_lattice(uint32_t ctx, const SearchGeo& g, in
             dx = (j & 1) ? d : range;
             dy = (j & 1) ? range : d;
         }
-        top4_merge(t, shared_key<2>(ctx, g, i < n, dx, dy, 0));
+        top4_merge(t, shared_key(ctx, 2, i < n, dx, dy, 0));
     }
     return t;
 }
@@ -965,7 +951,6 @@ __device__ __forceinline__ Top4 umh_lattice(uint32_t ctx, const SearchGeo& g, in
 // column and row at +range): the full_resolution / stride-2 / stride-4 scans of the rescue.
 __device__ __noinline__ uint64_t box_min(uint32_t ctx, int bx, int by, int nx, int ny, int step, int stride, int range,
                                          bool edges) {
-    const SearchGeo g(ctx);
     const int lane = threadIdx.x & 31;
     const int n0 = nx * ny, n = n0 + (edges ? 2 * nx : 0);
     uint64_t best = UINT64_MAX;
@@ -982,10 +967,7 @@ __device__ __noinline__ uint64_t box_min(uint32_t ctx, int bx, int by, int nx, i
             dx = (j & 1) ? d : range;
             dy = (j & 1) ? range : d;
         }
-        uint64_t k;
-        if (stride == 1) k = shared_key<1>(ctx, g, i < n, dx, dy, 0);
-        else if (stride == 2) k = shared_key<2>(ctx, g, i < n, dx, dy, 0);
-        else k = shared_key<4>(ctx, g, i < n, dx, dy, 0);
+        const uint64_t k = shared_key(ctx, stride, i < n, dx, dy, 0);
         best = k < best ? k : best;
     }
     return warp_min_key(best);
@@ -1027,14 +1009,13 @@ __device__ __forceinline__ bool dense_wanted(uint64_t cost, uint64_t pixels, int
 // and then find the rescue done; the others have spent idle time on it. Returns the least full
 // resolution cost seen.
 __device__ __noinline__ uint64_t umh_early(uint32_t ctx, uint32_t top_off, int gdx, int gdy, int range, int pixels) {
-    const SearchGeo g(ctx);
     const int lane = threadIdx.x & 31;
     Top4 t{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
-    if (range >= 8) t = umh_lattice(ctx, g, range);
+    if (range >= 8) t = umh_lattice(ctx, range);
     const int i = lane >> 3;
     const int dx = i == 1 ? iclamp(gdx, -range, range) : (i == 2 && range >= 8 ? search_dx(t.a) : 0);
     const int dy = i == 1 ? iclamp(gdy, -range, range) : (i == 2 && range >= 8 ? search_dy(t.a) : 0);
-    uint64_t best = warp_min_key(shared_key<1>(ctx, g, i < 3, dx, dy, 3));
+    uint64_t best = warp_min_key(shared_key(ctx, 1, i < 3, dx, dy, 3));
     uint64_t coarse = UINT64_MAX, dense = UINT64_MAX;
     if (!match_good(search_cost(best), (uint64_t)pixels)) {
         coarse = rescue_coarse(ctx, range);
@@ -1072,6 +1053,18 @@ struct UmhStages {
     __host__ __device__ int rings() const { return 25 + 2 * (nh + nv); }
     __host__ __device__ int hexagon() const { return rings() + 6 * nr; }
     __host__ __device__ int total() const { return hexagon() + 10; }
+    // The table's words: six headers (a stage's first word | its count << 16; two unused words), the
+    // offsets, and the seeds of the current macroblock as offsets from zero.
+    static constexpr int kHead = 8, kSeeds = 8;
+    __host__ __device__ int words() const { return kHead + total() + kSeeds; }
+    __host__ __device__ int seeds() const { return kHead + total(); }
+    __device__ uint32_t word(int i) const {
+        if (i >= kHead + total()) return 0;
+        if (i >= kHead) return offset(i - kHead);
+        const int first = i == 2 ? cross() : i == 3 ? rings() : i == 4 ? hexagon() : i == 5 ? hexagon() + 6 : 0;
+        const int n = i == 1 ? 25 : i == 2 ? rings() - cross() : i == 3 ? hexagon() - rings() : i == 4 ? 10 : 4;
+        return (uint32_t)(kHead + first) | ((uint32_t)n << 16);
+    }
     __device__ uint32_t offset(int i) const {
         int dx = 0, dy = 0;
         if (i < 25) {  // (:1855-1859)
@@ -1098,48 +1091,36 @@ struct UmhStages {
     }
 };
 
-// The search after the wavefront wait: seeds in seeds[0..ns), umh_early's results in top[], the
-// stages' offsets in offs[]; fin: room for 36 words. The result's key. The small hexagon is scored
+// The search after the wavefront wait: umh_early's results in top[], the stages' offsets (the seeds
+// are stage 0) in offs[]; fin: room for 36 words. The result's key. The small hexagon is scored
 // together with the closing diamond about the same centre, which stands once the hexagon has not
 // moved (its keys count only then).
-__device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint32_t top_off, uint32_t offs_off, uint32_t fin_off,
-                                          int ns, int range, int pixels) {
-    const SearchGeo g(ctx);
-    const UmhStages st(range);
+__device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t top_off, uint32_t offs_off, uint32_t fin_off, int range,
+                                          int pixels) {
     const int lane = threadIdx.x & 31;
-    const int2* seeds = reinterpret_cast<const int2*>(g_smem + seeds_off);
     const uint32_t* offs = reinterpret_cast<const uint32_t*>(g_smem + offs_off);
     // Each lane keeps the four least of the keys it scored; a stage only needs the least of all.
     Top4 own{UINT64_MAX, UINT64_MAX, UINT64_MAX, UINT64_MAX};
     uint64_t best = UINT64_MAX;
     enum { kSeeds, kSquare, kCross, kRings, kHexagon, kDiamond };
-    int stage = kSeeds, iter = 0;
+    int stage = kSeeds, iter = 0, cx = 0, cy = 0;
 #pragma unroll 1
     for (;;) {
-        // the stage's centre is the least candidate before it
-        const int cx = search_dx(best), cy = search_dy(best);
-        const int first = stage == kCross ? st.cross() : stage == kRings ? st.rings() : stage == kHexagon ? st.hexagon()
-                        : stage == kDiamond ? st.hexagon() + 6 : 0;
-        const int n = stage == kSeeds ? ns : stage == kSquare ? 25 : stage == kCross ? st.rings() - st.cross()
-                    : stage == kRings ? st.hexagon() - st.rings() : stage == kHexagon ? 10 : 4;
+        // the stage's centre (cx, cy) is the least candidate before it; predictor, zero, global, then A
+        // and C where they exist are the seeds (:1843-1850)
+        const uint32_t head = offs[stage];
+        const int n = (int)(head >> 16);
+        const uint32_t* list = offs + (head & 0xffff);
         uint64_t least = UINT64_MAX, diamond = UINT64_MAX;
 #pragma unroll 1
         for (int base = 0; base < n;) {
             const int rem = n - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : 2);
-            const int i = base + (lane >> sh), at = imin(i, n - 1);
-            int dx, dy;
-            if (stage == kSeeds) {  // predictor, zero, global, then A and C where they exist (:1843-1850)
-                const int2 v = seeds[at];
-                dx = v.x;
-                dy = v.y;
-            } else {
-                const uint32_t o = offs[first + at];
-                dx = cx + (int)(o & 0xffff) - 512;
-                dy = cy + (int)(o >> 16) - 512;
-            }
+            const int i = base + (lane >> sh);
+            const uint32_t o = list[imin(i, n - 1)];
+            int dx = cx + (int)(o & 0xffff) - 512, dy = cy + (int)(o >> 16) - 512;
             dx = iclamp(dx, -range, range);
             dy = iclamp(dy, -range, range);
-            const uint64_t k = shared_key<2>(ctx, g, i < n, dx, dy, sh);
+            const uint64_t k = shared_key(ctx, 2, i < n, dx, dy, sh);
             if (stage == kHexagon && i >= 6) {
                 diamond = k;
             } else {
@@ -1166,19 +1147,24 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
         } else {
             break;
         }
+        cx = search_dx(best);
+        cy = search_dy(best);
     }
     const Top4 t = top4_gather(own);
     // full-resolution 3x3 about the four finalists (:1929-1952), each vector once
     const int nf = 9 * ((t.a != UINT64_MAX) + (t.b != UINT64_MAX) + (t.c != UINT64_MAX) + (t.d != UINT64_MAX));
+    const int xa = search_dx(t.a), ya = search_dy(t.a), xb = search_dx(t.b), yb = search_dy(t.b);
+    const int xc = search_dx(t.c), yc = search_dy(t.c), xd = search_dx(t.d), yd = search_dy(t.d);
     uint32_t* fin = reinterpret_cast<uint32_t*>(g_smem + fin_off);
     int nd = 0;
 #pragma unroll 1
     for (int base = 0; base < nf; base += 32) {
-        const int i = base + lane, f = i / 9, q = i - 9 * f;
-        const uint64_t c = f == 0 ? t.a : (f == 1 ? t.b : (f == 2 ? t.c : t.d));
-        const int dx = iclamp(search_dx(c) + q % 3 - 1, -range, range), dy = iclamp(search_dy(c) + q / 3 - 1, -range, range);
-        auto covered = [&](uint64_t k) { return iabs(dx - search_dx(k)) <= 1 && iabs(dy - search_dy(k)) <= 1; };
-        const bool fresh = i < nf && !(f > 0 && covered(t.a)) && !(f > 1 && covered(t.b)) && !(f > 2 && covered(t.c));
+        const int i = base + lane, f = i / 9, q = i - 9 * f, qy = q / 3;
+        const int dx = iclamp((f == 0 ? xa : (f == 1 ? xb : (f == 2 ? xc : xd))) + q - 3 * qy - 1, -range, range);
+        const int dy = iclamp((f == 0 ? ya : (f == 1 ? yb : (f == 2 ? yc : yd))) + qy - 1, -range, range);
+        auto covered = [&](int x, int y) { return ((unsigned)(dx - x + 1) <= 2u) & ((unsigned)(dy - y + 1) <= 2u); };
+        const bool dup = ((f > 0) & covered(xa, ya)) | ((f > 1) & covered(xb, yb)) | ((f > 2) & covered(xc, yc));
+        const bool fresh = (i < nf) & !dup;
         const unsigned fm = __ballot_sync(FULL, fresh);
         if (fresh) fin[nd + __popc(fm & ((1u << lane) - 1))] = ((uint32_t)(dy + 512) << 16) | (uint32_t)(dx + 512);
         nd += __popc(fm);
@@ -1190,7 +1176,7 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
         const int rem = nd - base, sh = rem > 16 ? 0 : (rem > 8 ? 1 : (rem > 4 ? 2 : 3));
         const int i = base + (lane >> sh);
         const uint32_t o = fin[imin(i, nd - 1)];
-        const uint64_t k = shared_key<1>(ctx, g, i < nd, (int)(o & 0xffff) - 512, (int)(o >> 16) - 512, sh);
+        const uint64_t k = shared_key(ctx, 1, i < nd, (int)(o & 0xffff) - 512, (int)(o >> 16) - 512, sh);
         fk = k < fk ? k : fk;
         base += 32 >> sh;
     }
@@ -1212,15 +1198,19 @@ __device__ __noinline__ uint64_t umh_core(uint32_t ctx, uint32_t seeds_off, uint
 }
 
 __device__ IntRes umh(const DevParams& P, const Mb& m, const PInfo& pi, int gdx, int gdy, int range, uint64_t pixels) {
+    // the predictor, zero, the global vector, then A and C where they exist
     const int ns = 3 + (pi.a_valid ? 1 : 0) + (pi.c_valid ? 1 : 0);
+    const uint32_t first = m.sm.offs[0] & 0xffff;
     if (m.lane < ns) {
         const int2 v = m.lane == 0 ? pi.pre : ((m.lane == 3 && pi.a_valid) ? pi.a : pi.c);
-        m.sm.batch[m.lane] = m.lane == 1 ? make_int2(0, 0) : m.lane == 2 ? make_int2(gdx, gdy)
-                                         : make_int2(round_qpel_to_pixel(v.x), round_qpel_to_pixel(v.y));
+        const int dx = m.lane == 1 ? 0 : (m.lane == 2 ? gdx : round_qpel_to_pixel(v.x));
+        const int dy = m.lane == 1 ? 0 : (m.lane == 2 ? gdy : round_qpel_to_pixel(v.y));
+        m.sm.offs[first + m.lane] = ((uint32_t)(iclamp(dy, -range, range) + 512) << 16) | (uint32_t)(iclamp(dx, -range, range) + 512);
     }
     __syncwarp();
-    const uint64_t fk = umh_core(m.sm.ctx.off, soff(m.sm.batch), soff(m.sm.top), m.sm.offs.off, m.sm.list.off, ns, range,
-                                 (int)pixels);
+    if (m.lane == 0) m.sm.offs[0] = first | ((uint32_t)ns << 16);
+    __syncwarp();
+    const uint64_t fk = umh_core(m.sm.ctx.off, soff(m.sm.top), m.sm.offs.off, m.sm.list.off, range, (int)pixels);
     return IntRes{search_dx(fk), search_dy(fk), search_cost(fk)};
 }
 
@@ -1324,7 +1314,6 @@ __device__ __forceinline__ int2 lr_prop_offset(int l) {
 __device__ IntRes lr_propagated(const DevParams& P, const Mb& m, const DevResult& o, int range) {
     IntRes best{0, 0, UINT64_MAX};
     const Bounds b = bounds_px(range);
-    const SearchGeo g(m.sm.ctx.off);
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
         const int nx = m.mx + (k == 0 || k == 2 ? -1 : (k == 3 ? 1 : 0)), ny = m.my - (k == 0 ? 0 : 1);
@@ -1337,7 +1326,7 @@ __device__ IntRes lr_propagated(const DevParams& P, const Mb& m, const DevResult
         const int i = m.lane >> 1;
         const int2 of = lr_prop_offset(imin(i, 12));
         int dx = iclamp(cx + of.x, b.xmin, b.xmax), dy = iclamp(cy + of.y, b.ymin, b.ymax);
-        const uint32_t c = shared_cost<1, true>(m.sm.ctx.off, g, i < 13, dx, dy, 1);
+        const uint32_t c = shared_cost(m.sm.ctx.off, dx, dy, 1 | (1 << 4) | (i < 13 ? 256 : 0));
         const uint64_t key = i < 13 ? ((uint64_t)c << 32) | ((uint64_t)(iabs(dx) + iabs(dy)) << 5) | (uint64_t)i : UINT64_MAX;
         const uint64_t least = warp_min_key(key);
         const int src = 2 * (int)(least & 31);
@@ -1400,13 +1389,12 @@ __device__ __forceinline__ uint32_t sig_distance(uint64_t a, uint64_t b) {
 // wavefront step for macroblocks whose content entered the picture.
 __device__ __noinline__ IntRes lr_nearest(uint32_t ctx, const PassDesc* dp, int W, int H, int range, uint64_t pixels) {
     const PassDesc& d = *dp;
-    const SearchGeo g(ctx);
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, bx0 = mbctx(ctx).x0, by0 = mbctx(ctx).y0;
     const Bounds b = bounds_px(range);
-    const uint64_t want = warp_signature(d.cur, W, H, g.x0, g.y0, lane);
+    const uint64_t want = warp_signature(d.cur, W, H, bx0, by0, lane);
     // the cells whose offset lies within the bounds
-    const int c0 = imax(0, (g.x0 + b.xmin + 7) >> 3), c1 = imin(d.lr_nx - 1, (g.x0 + b.xmax) >> 3);
-    const int r0 = imax(0, (g.y0 + b.ymin + 7) >> 3), r1 = imin(d.lr_ny - 1, (g.y0 + b.ymax) >> 3);
+    const int c0 = imax(0, (bx0 + b.xmin + 7) >> 3), c1 = imin(d.lr_nx - 1, (bx0 + b.xmax) >> 3);
+    const int r0 = imax(0, (by0 + b.ymin + 7) >> 3), r1 = imin(d.lr_ny - 1, (by0 + b.ymax) >> 3);
     const int nc = c1 - c0 + 1;
     uint64_t top = UINT64_MAX, bound = UINT64_MAX;  // lane j < 16: the j-th least key
     int cx = c0 + lane, cy = r0;
@@ -1421,7 +1409,7 @@ __device__ __noinline__ IntRes lr_nearest(uint32_t ctx, const PassDesc* dp, int 
             }
             key[u] = UINT64_MAX;
             if (cy <= r1) {
-                const int dx = cx * 8 - g.x0, dy = cy * 8 - g.y0, i = cy * d.lr_nx + cx;
+                const int dx = cx * 8 - bx0, dy = cy * 8 - by0, i = cy * d.lr_nx + cx;
                 if (!(iabs(dx) <= 32 && iabs(dy) <= 32) && IDX_OK(d.lr_sig != nullptr, kSiteSignature, i))
                     key[u] = ((uint64_t)sig_distance(want, __ldg(&d.lr_sig[i])) << 36) |
                              ((uint64_t)(iabs(dx) + iabs(dy)) << 24) | ((uint64_t)(dy + 2048) << 12) | (uint64_t)(dx + 2048);
@@ -1451,13 +1439,13 @@ __device__ __noinline__ IntRes lr_nearest(uint32_t ctx, const PassDesc* dp, int 
         const bool on = lane < 25;
         // 5x5 at step 4, stride 2: the first least SAD in scan order
         int dx = iclamp(cdx - 8 + 4 * (lane % 5), b.xmin, b.xmax), dy = iclamp(cdy - 8 + 4 * (lane / 5), b.ymin, b.ymax);
-        uint32_t c = shared_cost<2, true>(ctx, g, on, dx, dy, 0);
+        uint32_t c = shared_cost(ctx, dx, dy, 2 | (on ? 256 : 0));
         uint64_t least = warp_min_key(on ? ((uint64_t)c << 32) | (uint64_t)lane : UINT64_MAX);
         const int sx = __shfl_sync(FULL, dx, (int)(least & 31)), sy = __shfl_sync(FULL, dy, (int)(least & 31));
         // 5x5 full search around it: least (sad, |d|), first in scan order
         dx = iclamp(sx + lane % 5 - 2, b.xmin, b.xmax);
         dy = iclamp(sy + lane / 5 - 2, b.ymin, b.ymax);
-        c = shared_cost<1, true>(ctx, g, on, dx, dy, 0);
+        c = shared_cost(ctx, dx, dy, 1 | (on ? 256 : 0));
         least = warp_min_key(on ? ((uint64_t)c << 32) | ((uint64_t)(iabs(dx) + iabs(dy)) << 5) | (uint64_t)lane : UINT64_MAX);
         dx = __shfl_sync(FULL, dx, (int)(least & 31));
         dy = __shfl_sync(FULL, dy, (int)(least & 31));
@@ -1650,7 +1638,7 @@ __device__ RefineOut refine_integer_only(const DevParams& P, const Mb& m, int bx
         return iclamp(nr * 4, lo, hi / 4 * 4);
     };
     int2 integer = make_int2(snap(seed.x, qb.xmin, qb.xmax), snap(seed.y, qb.ymin, qb.ymax));
-    if (hidden_padding(P, bx, by, bw, bh, integer.x, integer.y, mode, chroma_gate(bx, by, bw, bh))) integer = make_int2(0, 0);
+    if (hidden_near(m.sm.ctx.off, bx, by, bw, bh, integer, mode, chroma_gate(bx, by, bw, bh))) integer = make_int2(0, 0);
     uint64_t s;
     if (integer.x == seed.x && integer.y == seed.y && known != UINT64_MAX) {
         s = known;
@@ -1677,7 +1665,7 @@ __device__ __forceinline__ RefineOut refine_sad_only(const DevParams& P, const M
     seed.x = iclamp(seed.x, xmin, xmax);
     seed.y = iclamp(seed.y, ymin, ymax);
     if (hp) { seed.x = make_even(seed.x); seed.y = make_even(seed.y); }
-    if (hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, emode, chroma_gate(bx, by, bw, bh))) {
+    if (hidden_near(m.sm.ctx.off, bx, by, bw, bh, seed, emode, chroma_gate(bx, by, bw, bh))) {
         seed = make_int2(0, 0);
         known = UINT64_MAX;
     }
@@ -1778,7 +1766,7 @@ __device__ __forceinline__ Shortlist refine_prepare(const DevParams& P, const Mb
     seed.y = iclamp(seed.y, ymin, ymax);
     if (hp) { seed.x = make_even(seed.x); seed.y = make_even(seed.y); }
     int n = 0;
-    const bool seed_hidden = hidden_padding(P, bx, by, bw, bh, seed.x, seed.y, mode, cg);
+    const bool seed_hidden = hidden_near(m.sm.ctx.off, bx, by, bw, bh, seed, mode, cg);
     // add(seed, known); an unknown seed is scored with the first stencil, which holds it
     uint64_t half_key = UINT64_MAX;
     if (known != UINT64_MAX) {
@@ -1884,6 +1872,13 @@ __device__ __forceinline__ int warp_argmin(bool in, unsigned __int128 key, uint6
     return __ffs(__ballot_sync(FULL, in)) - 1;
 }
 
+// score_key, one copy of its 128-bit arithmetic.
+__device__ __noinline__ unsigned __int128 score_key_ool(int mant_bits, uint64_t lam_m, int lam_s, uint64_t sad, uint32_t rate) {
+    DevParams P{};
+    P.mant_bits = mant_bits;
+    return score_key(P, lam_m, lam_s, sad, rate);
+}
+
 // The rest of refine_motion_block_staged (encoder_motion.cpp:3458-3535) given the predictor.
 // Lane i < nk holds shortlist entry i; both selections are warp reductions.
 __device__ RefineOut refine_select(const DevParams& P, const Mb& m, const Shortlist& sl, int bx, int by, int bw, int bh,
@@ -1904,7 +1899,7 @@ __device__ RefineOut refine_select(const DevParams& P, const Mb& m, const Shortl
             ++rate;
         }
         rate += mv_rate_bits(P, mv, pred, mode, more);
-        key = score_key(P, m.lam_m, m.lam_s, sad, rate);
+        key = score_key_ool(P.mant_bits, m.lam_m, m.lam_s, sad, rate);
     }
     const int rw = warp_argmin(valid, key, order);  // the rate winner (:3477-3488)
     if (P.me_quality == 1) {
@@ -1931,7 +1926,7 @@ __device__ RefineOut refine_select(const DevParams& P, const Mb& m, const Shortl
     }
     // the final order (:3526-3531): eligible first, then (score, satd, sad, tie_less); of equal
     // scores the lesser SATD is found first
-    if (valid) key = score_key(P, m.lam_m, m.lam_s, satd, rate);
+    if (valid) key = score_key_ool(P.mant_bits, m.lam_m, m.lam_s, satd, rate);
     const bool in = em ? elig : valid;
     const uint32_t sc = satd >= kBad ? 0xffffffffu : (uint32_t)satd;
     int best = warp_argmin(in, key, ((uint64_t)sc << 32));
@@ -2420,7 +2415,7 @@ __host__ __device__ inline int warp_bytes_for(const WinCfg& wc) {
 }
 
 int warp_bytes_for_host(const WinCfg& wc) { return warp_bytes_for(wc); }
-int umh_offsets(int range) { return UmhStages(range).total(); }
+int umh_offsets(int range) { return UmhStages(range).words(); }
 
 // 16 bytes from global to shared memory without a register round trip (cp.async; both
 // addresses 16-byte aligned). The copy lands by the next window_wait().
@@ -2489,6 +2484,14 @@ __device__ __forceinline__ void window_wait(Mb& m, LaunchStatus* st, uint32_t co
     __syncwarp();
 }
 
+// 16 window bytes from a row's clamped columns gx .. gx + 15.
+__device__ __noinline__ void stage_edge_chunk(uint8_t* dst, const uint8_t* row, int gx, int W) {
+    uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i >> 2] |= (uint32_t)__ldg(row + iclamp(gx + i, 0, W - 1)) << (8 * (i & 3));
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Stages the reference window around MV (cdx, cdy) integer pixels: rows wy0 .. wy0+wh-1,
 // columns from the 16-byte-aligned wx0. Chunks inside the raster are asynchronous 16-byte
 // copies (all of a lane's in flight at once) that land at the next window_wait(); edge
@@ -2510,7 +2513,7 @@ __device__ void load_window(const DevParams& P, Mb& m, const DevFrame& ref, int 
     }
     const int cpr = m.wp >> 4;
     const int total = m.wh * cpr;
-#pragma unroll 4
+#pragma unroll 1
     for (int j = m.lane; j < total; j += 32) {
         const int r = j / cpr, c = j - r * cpr;
         const int gy = iclamp(m.wy0 + r, 0, P.H - 1), gx = m.wx0 + 16 * c;
@@ -2520,15 +2523,7 @@ __device__ void load_window(const DevParams& P, Mb& m, const DevFrame& ref, int 
         if (gx >= 0 && gx + 16 <= P.W) {
             cp_async16(dst, row + gx);
         } else {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                uint32_t x = 0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) x |= (uint32_t)__ldg(row + iclamp(gx + 4 * k + i, 0, P.W - 1)) << (8 * i);
-                w[k] = x;
-            }
-            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            stage_edge_chunk(dst, row, gx, P.W);
         }
     }
 }
@@ -2612,7 +2607,7 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
     const int range = P0.range, local_range = P0.local_range;  // one search configuration per launch
     if ((KIND & kCoreUnseededOnly) && wc.offs) {
         const UmhStages st(local_range);
-        for (int i = m.lane; i < st.total(); i += 32) m.sm.offs[i] = st.offset(i);
+        for (int i = m.lane; i < st.words(); i += 32) m.sm.offs[i] = i ? st.word(i) : (uint32_t)st.seeds();
         __syncwarp();
     }
     for (;;) {
@@ -2715,10 +2710,11 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 const RefineOut og = refine_select_ool<kDR>(m.sm.ctx.off, sl, m.x0, m.y0, 16, 16, one_mode, pig, true);
                 spec_result_save(m, 0, pig, og);
                 one_g = og.mv;
-                if (hidden_padding(P, m.x0, m.y0, 16, 16, one_g.x, one_g.y, one_mode, true)) one_g = make_int2(0, 0);
+                if (hidden_near(m.sm.ctx.off, m.x0, m.y0, 16, 16, one_g, one_mode, true)) one_g = make_int2(0, 0);
                 if (spec4) {
                     if (m.lane < 4) cur4g[m.lane] = one_g;
                     __syncwarp();
+#pragma unroll 1
                     for (int k = 0; k < 4; ++k) {
                         const int bx = m.x0 + (k & 1) * 8, by = m.y0 + ((k >> 1) & 1) * 8;
                         const PInfo pi4g = predictor_4mv(P, fg, m.mx, m.my, k);
@@ -2868,7 +2864,7 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                                     true, im.cost);
             }
             PHASE_MARK(8);
-            if (hidden_padding(P, m.x0, m.y0, 16, 16, one.mv.x, one.mv.y, one_mode, true)) {
+            if (hidden_near(m.sm.ctx.off, m.x0, m.y0, 16, 16, one.mv, one_mode, true)) {
                 if (m.lane == 0) m.sm.batch[31] = make_int2(0, 0);
                 __syncwarp();
                 sad_batch(P, m, m.sm.batch + 31, 1, m.x0, m.y0, 16, 16, one_mode, m.sm.batch_cost + 31);
@@ -2889,6 +2885,7 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 uint64_t four_sad = 0, four_screen = 0, extra_bits = 1;
                 const Bounds qb = bounds_qpel(range);
                 const bool hit = spec4 && one.mv.x == one_g.x && one.mv.y == one_g.y;
+#pragma unroll 1
                 for (int k = 0; k < 4; ++k) {
                     const PInfo pi4 = predictor_4mv(P, field, m.mx, m.my, k);
                     const int bx = m.x0 + (k & 1) * 8, by = m.y0 + ((k >> 1) & 1) * 8;
