@@ -834,6 +834,9 @@ void same_search_config(const DevParams& a, const DevParams& b) {
 // The autotuner's cache key of a launch: raster, ranges, algorithm and the instantiation.
 std::vector<int> tune_key(const DevParams& P, int kind) { return {P.W, P.H, P.range, P.local_range, P.me_algorithm, kind}; }
 
+// The macroblocks of one wavefront step, at most.
+int front_of(int mbw, int mbh) { return std::min((mbw + 1) / 2, mbh); }
+
 // per_pass: null, or n parameter blocks (pictures of different sizes in one kCoreMulti launch).
 int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, int n, bool globals_ready = false,
                  const PassExtra* extra = nullptr, const vc1cu_params* per_pass = nullptr,
@@ -1020,17 +1023,42 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     // windows so large that a second 4-warp block cannot fit: the wide-register build costs no occupancy
     if (!(kind & kCoreSeededOnly) && 2 * 4 * (size_t)wc.warp_bytes > (size_t)c->max_smem_sm) kind |= kCoreWide;
     const void* kern = core_kernel(kind);
+    // The macroblocks in flight (one per warp). A wavefront step occupies `front` of them; the others
+    // wait, and run the part of theirs that needs no neighbour on the schedulers the front is on. So a
+    // launch holds what hides that part and no more. 1080p pictures, range 64 (one block per SM): one
+    // picture (front 60) 5.2 ms with 4 warps per SM and 5.4 with 7, 10 pictures 7.4 with 4 and 7.1 with
+    // 5, 16 pictures 10.5 with 4 and 9.3 with 7: one warp per front macroblock, at least 4. Range 32,
+    // in blocks of 4: 8 pictures 5.7 ms with 1 block per SM and 6.2 with 3, 16 8.1 and 8.6, 24 11.6 with
+    // 1 and 9.7 with 2. Seeded passes need more (speculation behind the seeds): three passes per picture,
+    // 1 picture 3.35 ms with 1 block and 3.75 with 4, 3 6.5 with 1 and 6.2 with 2, 6 10.0 with 2 and 9.3
+    // with 3. Pictures of uneven sizes (a front that varies) and passes that do not wait keep as many
+    // as fit: 5.6 ms, against 5.8 with 1 block.
+    int blocks = 0;  // per SM; 0: as many as fit
+    bool waits = !multi && !learned;
+    for (int i = 0; i < n; ++i) waits &= !h[i].no_wait;
+    if (waits) {
+        long front = 0;
+        for (int i = 0; i < n; ++i) front += front_of(h[i].geom.mbw, h[i].geom.mbh);
+        const long sms = c->sm_count;
+        if (kind & kCoreWide) {
+            while (warps < 8 && warps * sms < front && (size_t)(warps + 1) * wc.warp_bytes <= (size_t)c->max_smem) ++warps;
+            smem = (size_t)warps * wc.warp_bytes;
+        } else if (any_unseeded) {
+            blocks = (int)std::max(1L, (front + 2 * sms) / (4 * sms));
+        } else {
+            blocks = (int)std::max(1L, (5 * front + 12 * sms - 1) / (12 * sms));
+        }
+    }
     // a launch shape chosen by vc1cu_autotune for this raster, search configuration and instantiation
-    int tuned_blocks = 0;
     {
         c->last_tune_key = tune_key(P, kind);
         auto t = c->tuned.find(c->last_tune_key);
         if (c->tune_force.first) {
             warps = c->tune_force.first;
-            tuned_blocks = c->tune_force.second;
+            blocks = c->tune_force.second;
         } else if (t != c->tuned.end()) {
             warps = t->second.first;
-            tuned_blocks = t->second.second;
+            blocks = t->second.second;
         }
         // a wider block of unseeded passes: their windows shrink until `warps` of them fit; a
         // candidate outside its window reads the frame in global memory, at the same result
@@ -1129,7 +1157,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     int per_sm = 0;
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem), "occupancy");
     per_sm = std::max(per_sm, 1);
-    if (tuned_blocks > 0) per_sm = std::min(per_sm, tuned_blocks);
+    if (blocks > 0) per_sm = std::min(per_sm, blocks);
     long items = 0;
     for (int i = 0; i < n; ++i) items += (long)h[i].geom.mbw * h[i].geom.mbh;
     const long need = (items + warps - 1) / warps;
@@ -1242,7 +1270,7 @@ std::vector<std::vector<int>> plan_launches(vc1cu_ctx* c, const vc1cu_params* p,
         for (int i = 0; i < n; ++i)
             if (level[i] == l && passes[i].seed_slot >= 0) {
                 const vc1cu_params& g = per_pass ? per_pass[i] : *p;
-                front += std::min(((g.width + 15) / 16 + 1) / 2, (g.height + 15) / 16);
+                front += front_of((g.width + 15) / 16, (g.height + 15) / 16);
             }
         const bool merge = per_pass || front <= (long)kMergeFront * c->sm_count;
         std::vector<int> keys;
@@ -2316,7 +2344,7 @@ int vc1cu_autotune(vc1cu_ctx* c, const vc1cu_params* params, const vc1cu_pass* p
             std::vector<int> key;
             // warps (macroblocks) per block and blocks per SM (0: as many as fit); shapes that do not fit
             // the launch's instantiation or shared memory are skipped
-            const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
+            const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {4, 3}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
                                                   {5, 1}, {6, 1}, {7, 1}, {8, 1}};
             for (const auto& s : shapes) {
                 c->tune_force = s;

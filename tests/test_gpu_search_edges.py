@@ -59,3 +59,22 @@ def test_largest_local_range(ctx, oracle):
     with pytest.raises(Vc1cuError) as e:
         ctx.analyze_p_core(make_params(50, 36, search_range=191, local_search_range=191), 1, 0, MV_QPEL, False)
     assert e.value.code == 6
+
+
+@pytest.mark.parametrize("rng", [32, 64])
+@pytest.mark.parametrize("n", [1, 64, 119])
+def test_launch_shapes(ctx, oracle, rng, n):
+    """n equal pairs in one call: the fronts of few, of more and of twice as many macroblocks as four
+    warps per SM hold, each with its own blocks per SM or warps per block."""
+    w, h = 320, 336
+    cur, ref = _frames("moved", w, h, rng)
+    p = make_params(w, h, search_range=rng, local_search_range=rng)
+    ctx.upload_frame(0, *ref)
+    ctx.upload_frame(1, *cur)
+    ctx.core_passes(p, [(1, 0, MV_QPEL, 0, -1, k) for k in range(n)])
+    ctx.core_passes(p, [(1, 0, MV_MIXED, 1, k, n + k) for k in range(n)])
+    want = oracle.analyze_p_core(p, cur, ref, MV_QPEL, False)
+    mixed = oracle.analyze_p_core(p, cur, ref, MV_MIXED, True, seed=want.mvs, seed_distant=want)
+    for k in range(n):
+        assert ctx.read_result(p, k).equal(want) == [], k
+        assert ctx.read_result(p, n + k).equal(mixed) == [], k
