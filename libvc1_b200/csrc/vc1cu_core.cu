@@ -596,9 +596,15 @@ __device__ __noinline__ uint32_t sad_lanes_core(uint32_t ctx, int mvx, int mvy, 
     bad = bad || (lane < n && hidden_near(ctx, bx, by, bw, bh, mv, mode, chroma_gate(bx, by, bw, bh)));
     const long long off = lane < n && !bad ? plane_offset(c, mv, bx, by, bw, bh) : -1;
     const unsigned planes = __ballot_sync(FULL, off >= 0);
+    // Candidates outside the planes read the first one inside, and a short batch reads one again
+    // (their sums are not used): no load stands behind a test, so a group's loads are all in flight
+    // together. 1080p, unseeded pass 5.16 -> 4.86 ms, three seeded passes 3.35 -> 3.29; with a test
+    // per candidate, even one that is the same for the warp, 5.12 and 3.39.
+    const long long first = __shfl_sync(FULL, off, (__ffs(planes) - 1) & 31), at = off >= 0 ? off : first;
     const int cx = bx - c.x0, cy = by - c.y0;
     uint32_t mine = 0;
-    if (bw == 16) {
+    if (!planes) {
+    } else if (bw == 16) {
         const int r = lane >> 1, c0 = (lane & 1) * 8, vis = r < ah ? aw - c0 : 0;
         const uint32_t m0 = vis_mask(vis), m1 = vis_mask(vis - 4);
         const uint32_t cw = (c.cur_off + (uint32_t)((cy + r) * 16 + cx + c0)) >> 2;
@@ -606,18 +612,12 @@ __device__ __noinline__ uint32_t sad_lanes_core(uint32_t ctx, int mvx, int mvy, 
         const uint8_t* seg = c.sp + (long long)r * c.sp_pitch + c0;
 #pragma unroll 1
         for (int base = 0; base < n; base += GROUP) {
-            uint32_t part[GROUP + 1];
+            uint32_t part[GROUP + 1], lo[GROUP], hi[GROUP];
             part[GROUP] = 0;
 #pragma unroll
-            for (int u = 0; u < GROUP; ++u) {
-                part[u] = 0;
-                const long long o = __shfl_sync(FULL, off, (base + u) & 31);
-                if (base + u < n && o >= 0) {
-                    uint32_t lo, hi;
-                    sp_load8(seg + o, lo, hi);
-                    part[u] = __vsadu4(lo & m0, a0) + __vsadu4(hi & m1, a1);
-                }
-            }
+            for (int u = 0; u < GROUP; ++u) sp_load8(seg + __shfl_sync(FULL, at, (base + u) & 31), lo[u], hi[u]);
+#pragma unroll
+            for (int u = 0; u < GROUP; ++u) part[u] = __vsadu4(lo[u] & m0, a0) + __vsadu4(hi[u] & m1, a1);
 #pragma unroll
             for (int u = 0; u < GROUP; u += 2) {
                 const uint32_t two = __reduce_add_sync(FULL, part[u] | (part[u + 1] << 16));
@@ -633,19 +633,11 @@ __device__ __noinline__ uint32_t sad_lanes_core(uint32_t ctx, int mvx, int mvy, 
         const uint8_t* seg = c.sp + (long long)r * c.sp_pitch;
 #pragma unroll 1
         for (int base = 0; base < n; base += 12) {
-            uint32_t part[4];
-            part[3] = 0;
+            uint32_t part[3], lo[3], hi[3];
 #pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                part[u] = 0;
-                const int ci = base + 4 * u + g;
-                const long long o = __shfl_sync(FULL, off, ci & 31);
-                if (ci < n && o >= 0) {
-                    uint32_t lo, hi;
-                    sp_load8(seg + o, lo, hi);
-                    part[u] = __vsadu4(lo & m0, a0) + __vsadu4(hi & m1, a1);
-                }
-            }
+            for (int u = 0; u < 3; ++u) sp_load8(seg + __shfl_sync(FULL, at, (base + 4 * u + g) & 31), lo[u], hi[u]);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) part[u] = __vsadu4(lo[u] & m0, a0) + __vsadu4(hi[u] & m1, a1);
             uint32_t s0 = part[0] | (part[1] << 16), s1 = part[2];
 #pragma unroll
             for (int o = 4; o; o >>= 1) {
@@ -2323,7 +2315,10 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void fence_acquire() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+}
 
 // Waits (bounded) until each lane's flag equals epoch (a macroblock of this launch was
 // published; a lane with a null flag waits for nothing). The flags are polled with relaxed
@@ -2339,8 +2334,11 @@ __device__ bool wait_flags(const uint32_t* flag, uint32_t epoch, LaunchStatus* s
     for (long it = 0; it < limit; ++it) {
         if (!mine) mine = ld_relaxed(flag) == epoch;
         if (__all_sync(FULL, mine)) {
-            // the observing lanes acquire; the warp barrier orders the other lanes' reads after it
-            fence_acquire();
+            // the observing lanes acquire, by loading their flags once more (a fence would also wait
+            // for the warp's earlier stores: some 900 clocks on every step of the wavefront; 1080p
+            // unseeded pass 4.86 -> 4.74 ms, P-intra pass 1.14 -> 1.03); the warp barrier orders the
+            // other lanes' reads after it
+            if (flag) ld_acquire(flag);
             __syncwarp();
             return true;
         }
@@ -2348,7 +2346,7 @@ __device__ bool wait_flags(const uint32_t* flag, uint32_t epoch, LaunchStatus* s
             const int ab = __shfl_sync(FULL, (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&st->abort)), 0);
             if (ab) return false;
         }
-        __nanosleep(64);
+        __nanosleep(20);
     }
     const unsigned waiting = __ballot_sync(FULL, !mine);
     if ((threadIdx.x & 31) == 0) {
@@ -2898,6 +2896,11 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                         // same seeds, same shortlist, same predictor: the parked result
                         r = sb.res;
                         have = true;
+                    } else if (hit && pi4.pre.x == sb.pi.pre.x && pi4.pre.y == sb.pi.pre.y) {
+                        // the same seeds, so the same shortlist; only A or C differs
+                        const Shortlist sk = shortlist_restore(m, k + 1);
+                        r = refine_select_ool<kDR>(m.sm.ctx.off, sk, bx, by, 8, 8, VC1CU_MV_MIXED, pi4, true);
+                        have = true;
                     } else if (hit) {
                         // the parked seed search covered every slot but the predictor's
                         put_4mv_seeds(P, m, one.mv, pi4.pre, qb);
@@ -2961,12 +2964,10 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 }
             }
             const uint64_t temporal = chosen;
-            double ratio = -1.0;
+            uint64_t intra_rate = 0;
             if (allow_intra) {
                 // P-intra decision (:396-414)
-                const uint64_t intra_rate = (uint64_t)llround(__dmul_rn(lambda, 72.0));
-                ratio = temporal_screen > 0 ? __ddiv_rn((double)(intra_sad + intra_rate), (double)temporal_screen)
-                                            : __longlong_as_double(0x7ff0000000000000ll);
+                intra_rate = (uint64_t)llround(__dmul_rn(lambda, 72.0));
                 if (intra_sad + intra_rate < (uint64_t)llround(__dmul_rn((double)temporal_screen, P.inter_intra_threshold))) {
                     intra = 1;
                     use4 = 0;
@@ -2977,8 +2978,8 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
             }
             bool moved = false, frac = false;
             for (int k = 0; k < 4; ++k) {
-                moved |= out4[k].x != 0 || out4[k].y != 0;
-                frac |= (out4[k].x % 8) != 0 || (out4[k].y % 8) != 0;
+                moved |= (out4[k].x | out4[k].y) != 0;
+                frac |= ((out4[k].x | out4[k].y) & 7) != 0;
             }
             // what the neighbours read, then the flag, then the rest (which only later launches read)
             if (m.lane == 0) {
@@ -2989,6 +2990,10 @@ __global__ void __launch_bounds__((KIND & kCoreWide) ? 256 : 128,
                 b4[0] = make_int4(out4[0].x, out4[0].y, out4[1].x, out4[1].y);
                 b4[1] = make_int4(out4[2].x, out4[2].y, out4[3].x, out4[3].y);
                 if (code != P.withhold) st_release(&o.done[m.pos], epoch);
+                double ratio = -1.0;
+                if (allow_intra)
+                    ratio = temporal_screen > 0 ? __ddiv_rn((double)(intra_sad + intra_rate), (double)temporal_screen)
+                                                : __longlong_as_double(0x7ff0000000000000ll);
                 o.use4[m.pos] = use4;
                 o.screen[m.pos] = temporal_screen;
                 o.ratio[m.pos] = ratio;
