@@ -162,3 +162,20 @@ def test_b_prediction_matches_reference_fixture(ctx, oracle, i):
     co, lv = ctx.forward_quant(p, 1, 5, 15)
     eco, elv = oracle.forward_quant(p, cur, pred, 15)
     assert np.array_equal(co.view(np.uint64), eco.view(np.uint64)) and np.array_equal(lv, elv)
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (16, 80), (80, 16), (18, 34), (34, 2080)])
+def test_decision_walk_edges(ctx, oracle, w, h):
+    """One row or column of macroblocks, partial ones, and more rows than one lane group each."""
+    clip = synth.generate(w, h, 3, 11 + w, n_objects=2, obj_min=8, obj_max=12)
+    p = make_params(w, h, search_range=8, local_search_range=8, pqindex=5)
+    for k in range(3):
+        ctx.upload_frame(k, *clip.frame(k))
+    rng = np.random.default_rng(w * h)
+    mbs = ((w + 15) // 16) * ((h + 15) // 16)
+    amv = rng.integers(-40, 41, (mbs, 2)).astype(np.int32)
+    a4 = (rng.random(mbs) < 0.2).astype(np.uint8)
+    for mode in (MV_QPEL, MV_HPEL_BILINEAR):
+        g = ctx.analyze_b_picture(p, 1, 0, 2, amv, a4, 1, 2, mode)
+        e = oracle.analyze_b(p, clip.frame(1), clip.frame(0), clip.frame(2), amv, a4, 1, 2, mode)
+        assert g.equal(e) == [], mode
