@@ -217,8 +217,7 @@ int vc1cu_measure_int32_peak(vc1cu_ctx* ctx, double* ops_per_second);
 int vc1cu_measure_fp64_peak(vc1cu_ctx* ctx, double* flops_per_second);
 /* The index-checked build of this library (libvc1cu_checked.so, compiled with
  * -DVC1CU_INDEX_CHECK) tests every guarded access of the analysis kernels against its buffer
- * (search window, stage key array, first-visit bitset, neighbour, candidate and signature
- * tables, work items, window staging), counts violations and skips them. This returns the count
+ * (search window, neighbour, candidate and signature tables, work items, window staging), counts violations and skips them. This returns the count
  * and the first violation (site << 40 | index, sites as in vc1cu_core.cu's IndexSite) since the
  * last reset, process-wide; with reset != 0 it clears them. Other builds return
  * VC1CU_ERR_UNSUPPORTED. */
@@ -307,9 +306,10 @@ int vc1cu_analyze_p_core(vc1cu_ctx* ctx, const vc1cu_params* p, int cur_id, int 
                          const vc1cu_panalysis* seed_distant, vc1cu_panalysis* out);
 
 /*
- * Device-resident batch form. Every pass in the batch is independent of the others; all
- * of them run in ONE persistent launch fed by a macroblock-row work queue (wavefront
- * order inside each picture). Results stay on the device in result slot out_slot
+ * Device-resident batch form. A pass may be seeded by another pass of the batch. The passes run
+ * in one persistent launch per step of that chain and code path (unseeded or seeded, MV mode,
+ * P-intra; few seeded passes of one step share a launch), each fed by a work queue in wavefront
+ * order inside each picture. Results stay on the device in result slot out_slot
  * (0 <= slot < 4096); a seeded pass names the slot of its seed. Asynchronous on the
  * context's stream; vc1cu_synchronize waits for it.
  */
@@ -325,12 +325,13 @@ typedef struct vc1cu_pass {
 
 int vc1cu_core_passes(vc1cu_ctx* ctx, const vc1cu_params* p, const vc1cu_pass* passes, int n);
 /*
- * Passes over pictures of different sizes (many clips) in ONE persistent launch: params holds one
+ * Passes over pictures of different sizes (many clips), one persistent launch for all unseeded
+ * passes and one for each step of seeded ones (with and without P-intra): params holds one
  * parameter block per pass (its raster, display crop, PQINDEX, rounding control); the search
  * configuration (ranges, algorithm, quality, sub-pel and long-range settings, thresholds) must be
  * the same in all of them. A pass may be seeded by another pass of the same call (a picture's
- * seed pass, mode passes and final pass together), as in vc1cu_core_passes. The work queue
- * interleaves every pass's wavefront, so no picture waits for another. Asynchronous.
+ * seed pass, mode passes and final pass together), as in vc1cu_core_passes. A launch's work
+ * queue interleaves its passes' wavefronts, so no picture waits for another. Asynchronous.
  */
 int vc1cu_core_passes_multi(vc1cu_ctx* ctx, const vc1cu_params* params, const vc1cu_pass* passes, int n);
 
@@ -352,12 +353,13 @@ int vc1cu_graph_launch(vc1cu_ctx* ctx, int graph_id);
 int vc1cu_graph_destroy(vc1cu_ctx* ctx, int graph_id);
 
 /*
- * Launch-shape autotuner (no counterpart in the reference): runs the given passes as one launch
+ * Launch-shape autotuner (no counterpart in the reference): runs the given passes' launches
  * (per_pass_params: params holds one block per pass, as vc1cu_core_passes_multi; else one block)
- * under several shapes of the persistent core kernel - macroblocks (warps) per block 1..4 and
- * blocks per SM - and keeps the fastest for this raster, search configuration and kernel
+ * under several shapes of the persistent core kernel - macroblocks (warps) per block and blocks
+ * per SM - and keeps each launch's fastest for its raster, search configuration and kernel
  * instantiation; later launches of that key use it. The passes' result slots are overwritten.
- * Synchronous; *warps, *blocks (0 = as many as fit) and *ms (one launch) may be NULL.
+ * Synchronous; *warps, *blocks (0 = as many as fit) of the longest launch and *ms (all launches,
+ * one pass over them) may be NULL.
  */
 int vc1cu_autotune(vc1cu_ctx* ctx, const vc1cu_params* params, const vc1cu_pass* passes, int n, int per_pass_params,
                    int* warps, int* blocks, double* ms);

@@ -819,7 +819,7 @@ struct PassExtra {
     const DevResult* nb = nullptr;  // no-wait pass: read the neighbours from this finished field
 };
 
-// The search configuration every pass of one launch shares (the kernel's window, bitsets and
+// The search configuration every pass of one launch shares (the kernel's window, offset table and
 // instantiation depend on it); the picture geometry, rounding control and quantiser may differ.
 void same_search_config(const DevParams& a, const DevParams& b) {
     if (a.range != b.range || a.local_range != b.local_range || a.me_algorithm != b.me_algorithm ||
@@ -975,7 +975,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
             c->counters.kernel_launches++;
         }
     }
-    // window / bitset geometry
+    // window geometry
     WinCfg wc;
     wc.offs = any_unseeded && !learned && P.me_algorithm == 0 && P.range > 0 ? umh_offsets(P.local_range) : 0;
     if (learned) {
@@ -1237,9 +1237,9 @@ void check_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
 }
 
 // Wavefront fronts (macroblocks of one step, at most) of up to this many macroblocks per SM run
-// seeded passes of different modes as one launch. A seeded launch holds 16 warps per SM and every
-// step of its chain waits for one macroblock's latency: passes that leave warps idle cost one chain
-// together instead of one each, and more of them pay for the larger code of several modes.
+// seeded passes of different modes as one launch. Every step of its chain waits for one macroblock's
+// latency: passes that leave warps idle cost one chain together instead of one each, and more of them
+// pay for the larger code of several modes.
 constexpr int kMergeFront = VC1CU_MERGE_FRONT;
 
 // The launches of a call's passes, in order, as index lists. A pass seeded by another pass of the

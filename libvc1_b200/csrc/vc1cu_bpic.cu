@@ -194,7 +194,7 @@ __device__ __forceinline__ BIn b_load(const BDesc& d, int pos, int role) {
 // last four columns of each row), a row's next inputs are loaded a step ahead, and everything that
 // no decision reads (the intra ratio, the counts) follows in one parallel pass. One 720p picture
 // (168 steps): 0.65 ms with one thread per macroblock and the vectors read back from global memory,
-// 0.44 now; sixteen 1080p decisions (254 steps): 1.16 -> 0.72.
+// 0.44 now; fourteen 1080p decisions (254 steps): 1.16 -> 0.72.
 constexpr int kDecideThreads = 512;
 __global__ void __launch_bounds__(kDecideThreads) b_decide_kernel(const __grid_constant__ DevParams P, const BDesc* descs) {
     const BDesc d = descs[blockIdx.x];
