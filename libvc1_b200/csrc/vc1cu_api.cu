@@ -1196,7 +1196,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     }
     {
         Timer tm(c, kTotals);
-        totals_kernel<<<n, 256, 0, c->stream>>>(P, c->d_passes, n);
+        totals_kernel<<<n, kTotalsThreads, 0, c->stream>>>(P, c->d_passes, n);
         ck(cudaGetLastError(), "totals_kernel launch");
         tm.stop(1);
     }
@@ -4185,7 +4185,7 @@ int vc1cu_lp_analyze(vc1cu_lp* n, const vc1cu_params* p, const vc1cu_lp_pass* pa
         ck(cudaMemcpyAsync(c->d_passes, hp, sizeof(PassDesc) * count, cudaMemcpyHostToDevice, c->stream),
            "cudaMemcpyAsync(pass descriptors)");
         staging_mark(c);
-        totals_kernel<<<count, 256, 0, c->stream>>>(learned[0].geom, c->d_passes, count);
+        totals_kernel<<<count, kTotalsThreads, 0, c->stream>>>(learned[0].geom, c->d_passes, count);
         ck(cudaGetLastError(), "totals_kernel launch");
         return VC1CU_OK;
     });

@@ -75,6 +75,7 @@ struct alignas(64) PassDesc {
                                  // launch's parameter block)
 };
 constexpr int kLearnK = 4;       // candidates per macroblock of a learned pass
+constexpr int kTotalsThreads = 1024;  // of totals_kernel
 constexpr int kLearnRw = 8;      // window radius of a learned pass around its best candidate
 
 // core_pass_kernel instantiations, as flags: each flag compiles out code that the launch's
