@@ -296,21 +296,24 @@ __global__ void __launch_bounds__(kGThreads) gsad_kernel(GState* states, int W, 
     const int st = gstage_stride(s.in.range, stage);
     const int nrows = (H + st - 1) / st, r0 = blockIdx.x * rows_per_slab, r1 = imin(nrows, r0 + rows_per_slab);
     const int2 c = ci < s.n ? s.cand[ci] : make_int2(kGEmpty, 0);
-    if (c.x != kGEmpty && r0 < r1) {
+    const bool scored = c.x != kGEmpty && r0 < r1;
+    __shared__ unsigned long long part[kGThreads / 32];
+    if (scored) {
         const uint32_t acc = frame_sad_part(s.in.cur.y, s.in.cur.pitch_y, s.in.ref.y, s.in.ref.pitch_y, W, H, c.x, c.y, st, r0, r1);
         const uint64_t sum = warp_sum_u64(acc);
-        __shared__ unsigned long long part[kGThreads / 32];
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
+    }
+    // Every warp has read its slot before the block counts as finished, an empty slot's too: the last
+    // block rewrites the slots.
+    __syncthreads();
+    // the last block of this search to arrive sees every block's cost and folds the stage
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        if (scored) {
             unsigned long long t = 0;
             for (int w = 0; w < kGThreads / 32; ++w) t += part[w];
             atomicAdd(&s.cost[ci], t);
         }
-    }
-    // the last block of this search to arrive sees every block's cost and folds the stage
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
         __threadfence();
         last = atomicAdd(&s.arrived, 1) == (int)(gridDim.x * gridDim.y) - 1;
         __threadfence();
