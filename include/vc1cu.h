@@ -346,6 +346,10 @@ int vc1cu_core_passes_multi(vc1cu_ctx* ctx, const vc1cu_params* params, const vc
  * (the work-item tables and slots are built outside captures); calls that wait for the device
  * (reads, synchronous calls) fail inside a capture and close it. Core passes in a graph clear their
  * macroblock done flags at every replay.
+ * Other calls may come between a capture and its replays, larger ones too: a workspace of the context
+ * that one of them outgrows stays allocated until the graphs that use it are destroyed. A replay is
+ * refused (VC1CU_ERR_STATE) once a frame or result slot of the graph has had another size since the
+ * capture. A network (vc1cu_lp_create) whose calls were captured must outlive the graph.
  */
 int vc1cu_graph_begin(vc1cu_ctx* ctx);
 int vc1cu_graph_end(vc1cu_ctx* ctx, int* graph_id);

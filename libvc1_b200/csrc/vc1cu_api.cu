@@ -20,6 +20,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -364,11 +365,30 @@ struct vc1cu_ctx {
     bool capturing = false;
     std::vector<void*> capture_hold;
     std::vector<int> capture_results, capture_bresults, capture_frames;
+    // A graph's nodes hold addresses. What captured work uses is recorded: the context's buffers
+    // (bufs: one that a later call outgrows is kept until the last graph using it is destroyed) and
+    // the slots with the buffer and size each had (slots: a replay is refused once one has another).
+    enum SlotKind { kFrameSlot, kResultSlot, kBSlot };
+    struct SlotState {
+        const void* d;
+        int a, b;  // a frame's width and height, a result's macroblocks
+        bool operator!=(const SlotState& o) const { return d != o.d || a != o.a || b != o.b; }
+    };
+    struct GraphUse {
+        std::set<const void*> bufs;
+        std::map<std::pair<int, int>, SlotState> slots;  // (kind, id)
+    } capture_use;
+    struct Retired {
+        void* p;
+        bool host;  // pinned host memory
+    };
+    std::vector<Retired> retired;
     struct Graph {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
         std::vector<void*> hold;
         std::vector<int> results, bresults, frames;
+        GraphUse use;
     };
     std::map<int, Graph> graphs;
     int graph_next = 1;
@@ -394,13 +414,43 @@ struct vc1cu_ctx {
 
 namespace {
 
-void* ensure(void*& p, size_t& cap, size_t bytes, const char* what) {
-    if (cap >= bytes && p) return p;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    ck(cudaMalloc(&p, bytes), what);
-    cap = bytes;
+// Notes that the work being captured uses the context's buffer p.
+void captured_use(vc1cu_ctx* c, const void* p) {
+    if (c->capturing && p) c->capture_use.bufs.insert(p);
+}
+// Notes the buffer and size of a slot that captured work uses (the last of a slot that one capture
+// builds anew).
+void captured_slot(vc1cu_ctx* c, vc1cu_ctx::SlotKind kind, int id, const void* d, int a, int b = 0) {
+    if (!c->capturing) return;
+    captured_use(c, d);
+    c->capture_use.slots[{kind, id}] = vc1cu_ctx::SlotState{d, a, b};
+}
+// Frees a buffer of the context, once no graph and no open capture uses it.
+void release(vc1cu_ctx* c, void* p, bool host = false) {
+    if (!p) return;
+    bool used = c->capture_use.bufs.count(p) != 0;
+    for (const auto& g : c->graphs) used = used || g.second.use.bufs.count(p) != 0;
+    if (used) c->retired.push_back({p, host});
+    else if (host) cudaFreeHost(p);
+    else cudaFree(p);
+}
+// After a graph or a capture went: frees what only it used.
+void release_retired(vc1cu_ctx* c) {
+    std::vector<vc1cu_ctx::Retired> r;
+    r.swap(c->retired);
+    for (const auto& x : r) release(c, x.p, x.host);
+}
+
+void* ensure(vc1cu_ctx* c, void*& p, size_t& cap, size_t bytes, const char* what) {
+    if (cap < bytes || !p) {
+        void* old = p;
+        p = nullptr;
+        cap = 0;
+        release(c, old);
+        ck(cudaMalloc(&p, bytes), what);
+        cap = bytes;
+    }
+    captured_use(c, p);
     return p;
 }
 
@@ -561,15 +611,19 @@ FrameSlot& frame_slot(vc1cu_ctx* c, int id) {
     c->used_frames.push_back(id);
     auto it = c->frames.find(id);
     if (it == c->frames.end() || !it->second.valid) throw Fail{VC1CU_ERR_STATE, "frame slot " + std::to_string(id) + " was never uploaded"};
+    captured_slot(c, vc1cu_ctx::kFrameSlot, id, it->second.d, it->second.w, it->second.h);
     return it->second;
 }
 
 ResultSlot& result_slot(vc1cu_ctx* c, int id, int mbs, bool create) {
     if (create) c->dirty_results.push_back(id);  // create: the caller writes the slot
     auto& s = c->results[id];
-    if (s.valid && s.mbs == mbs) return s;
+    if (s.valid && s.mbs == mbs) {
+        captured_slot(c, vc1cu_ctx::kResultSlot, id, s.d, mbs);
+        return s;
+    }
     if (!create) throw Fail{VC1CU_ERR_STATE, "result slot " + std::to_string(id) + " holds no result of this size"};
-    if (s.d) cudaFree(s.d);
+    release(c, s.d);
     s = ResultSlot{};
     const size_t n = (size_t)mbs;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -599,6 +653,7 @@ ResultSlot& result_slot(vc1cu_ctx* c, int id, int mbs, bool create) {
     s.r.itotals = (unsigned long long*)take(40);
     s.mbs = mbs;
     s.valid = true;
+    captured_slot(c, vc1cu_ctx::kResultSlot, id, s.d, mbs);
     return s;
 }
 
@@ -610,7 +665,7 @@ FrameSlot& alloc_frame(vc1cu_ctx* c, int id, int w, int h, bool by_upload = fals
     const int py = (w + 15) & ~15, pc = (w / 2 + 15) & ~15;
     const size_t bytes = (size_t)py * h + 2 * (size_t)pc * (h / 2);
     if (!f.d || f.cap < bytes) {
-        if (f.d) cudaFree(f.d);
+        release(c, f.d);
         f.d = nullptr;
         f.cap = 0;
         void* d = nullptr;
@@ -623,6 +678,7 @@ FrameSlot& alloc_frame(vc1cu_ctx* c, int id, int w, int h, bool by_upload = fals
     f.pitch_y = py;
     f.pitch_c = pc;
     f.valid = true;
+    if (!by_upload) captured_slot(c, vc1cu_ctx::kFrameSlot, id, f.d, w, h);
     return f;
 }
 
@@ -640,7 +696,7 @@ uint8_t* cache_frame(vc1cu_ctx* c, const uint8_t* data, int w, int h) {
         if (s.age < slot->age) slot = &s;
     }
     void* d = slot->d;
-    ensure(d, slot->cap, bytes, "cudaMalloc(cached frame)");
+    ensure(c, d, slot->cap, bytes, "cudaMalloc(cached frame)");
     slot->d = static_cast<uint8_t*>(d);
     ck(cudaMemcpyAsync(slot->d, data, bytes, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(frame)");
     slot->host = data;
@@ -752,7 +808,7 @@ void staging_mark(vc1cu_ctx* c) {
 
 int score_common(vc1cu_ctx* c, const DevParams& P, const ScoreArgs& a, const vc1cu_mv* cands, size_t n, uint64_t* costs) {
     const size_t cb = n * sizeof(int2), ob = n * sizeof(unsigned long long);
-    ensure(c->d_scratch, c->scratch_cap, cb + ob + 256, "cudaMalloc(candidates)");
+    ensure(c, c->d_scratch, c->scratch_cap, cb + ob + 256, "cudaMalloc(candidates)");
     int2* dc = static_cast<int2*>(c->d_scratch);
     unsigned long long* dout = reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(c->d_scratch) + ((cb + 255) & ~size_t(255)));
     const auto t0 = std::chrono::steady_clock::now();
@@ -784,7 +840,7 @@ struct GSearches {
 
 GSearches global_searches(vc1cu_ctx* c, int n) {
     if (c->gstates_cap < n) {
-        if (c->d_gstates) cudaFree(c->d_gstates);
+        release(c, c->d_gstates);
         c->d_gstates = nullptr;
         c->gstates_cap = 0;
         void* d = nullptr;
@@ -792,6 +848,7 @@ GSearches global_searches(vc1cu_ctx* c, int n) {
         c->d_gstates = static_cast<GState*>(d);
         c->gstates_cap = n;
     }
+    captured_use(c, c->d_gstates);
     GSearches g;
     g.n = n;
     g.h = static_cast<uint8_t*>(staging(c, gin_bytes() * n));
@@ -963,7 +1020,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         for (size_t k = 0; k < unseeded.size(); ++k)
             per = std::max(per, sizeof(uint64_t) * (size_t)((h[unseeded[k]].geom.W + 7) / 8) *
                                     (size_t)((h[unseeded[k]].geom.H + 7) / 8));
-        uint64_t* base = static_cast<uint64_t*>(ensure(c->d_lr, c->lr_cap, per * unseeded.size(), "cudaMalloc(long-range index)"));
+        uint64_t* base = static_cast<uint64_t*>(ensure(c, c->d_lr, c->lr_cap, per * unseeded.size(), "cudaMalloc(long-range index)"));
         for (size_t k = 0; k < unseeded.size(); ++k) {
             PassDesc& d = h[unseeded[k]];
             const int nx = (d.geom.W + 7) / 8, ny = (d.geom.H + 7) / 8;
@@ -1118,7 +1175,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         }
         if (c->capturing && c->sp_cap < total)
             throw Fail{VC1CU_ERR_STATE, "run this launch once before capturing it (sub-pel plane pool too small)"};
-        uint8_t* pool = static_cast<uint8_t*>(ensure(c->d_sp, c->sp_cap, total, "cudaMalloc(sub-pel planes)"));
+        uint8_t* pool = static_cast<uint8_t*>(ensure(c, c->d_sp, c->sp_cap, total, "cudaMalloc(sub-pel planes)"));
         // timed with the core passes: the planes carry part of their interpolation work
         Timer tm(c, kCoreAux);
         for (const auto& k : keys)
@@ -1138,7 +1195,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
     // pass descriptors, ordered on the context stream after any launch still reading the
     // previous ones
     if (c->passes_cap < n) {
-        if (c->d_passes) cudaFree(c->d_passes);
+        release(c, c->d_passes);
         c->d_passes = nullptr;
         c->passes_cap = 0;
         void* d = nullptr;
@@ -1146,6 +1203,7 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
         c->d_passes = static_cast<PassDesc*>(d);
         c->passes_cap = n;
     }
+    captured_use(c, c->d_passes);
     {
         void* hp = staging(c, sizeof(PassDesc) * n);
         std::memcpy(hp, h.data(), sizeof(PassDesc) * n);
@@ -1367,7 +1425,7 @@ int launch_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
             }
             if (!copies.empty()) {
                 const size_t cb = sizeof(GlobalCopy) * copies.size();
-                void* dcp = ensure(c->d_gcopy, c->gcopy_cap, cb, "cudaMalloc(global copies)");
+                void* dcp = ensure(c, c->d_gcopy, c->gcopy_cap, cb, "cudaMalloc(global copies)");
                 void* hc = staging(c, cb);
                 std::memcpy(hc, copies.data(), cb);
                 ck(cudaMemcpyAsync(dcp, hc, cb, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(global copies)");
@@ -1431,6 +1489,8 @@ void abort_capture(vc1cu_ctx* c) {
     c->capture_results.clear();
     c->capture_bresults.clear();
     c->capture_frames.clear();
+    c->capture_use = vc1cu_ctx::GraphUse{};
+    release_retired(c);
 }
 
 // Orders the read stream after the work that last wrote a slot (after everything enqueued so far
@@ -1545,9 +1605,10 @@ BSlot& bresult_slot(vc1cu_ctx* c, int id, int mbs) {
     auto& s = c->bresults[id];
     if (s.d && s.mbs == mbs) {
         s.valid = true;
+        captured_slot(c, vc1cu_ctx::kBSlot, id, s.d, mbs);
         return s;
     }
-    if (s.d) cudaFree(s.d);
+    release(c, s.d);
     s = BSlot{};
     const size_t n = (size_t)mbs;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -1573,6 +1634,7 @@ BSlot& bresult_slot(vc1cu_ctx* c, int id, int mbs) {
     s.r.totals = (double*)take(16);
     s.mbs = mbs;
     s.valid = true;
+    captured_slot(c, vc1cu_ctx::kBSlot, id, s.d, mbs);
     return s;
 }
 
@@ -1646,7 +1708,7 @@ void launch_b(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_bpass* b, int n, 
         h[i].out = o.r;
     }
     if (c->bdescs_cap < n) {
-        if (c->d_bdescs) cudaFree(c->d_bdescs);
+        release(c, c->d_bdescs);
         c->d_bdescs = nullptr;
         c->bdescs_cap = 0;
         void* d = nullptr;
@@ -1654,6 +1716,7 @@ void launch_b(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_bpass* b, int n, 
         c->d_bdescs = static_cast<BDesc*>(d);
         c->bdescs_cap = n;
     }
+    captured_use(c, c->d_bdescs);
     void* hp = staging(c, sizeof(BDesc) * n);
     std::memcpy(hp, h.data(), sizeof(BDesc) * n);
     ck(cudaMemcpyAsync(c->d_bdescs, hp, sizeof(BDesc) * n, cudaMemcpyHostToDevice, c->stream), "cudaMemcpyAsync(B descriptors)");
@@ -1716,16 +1779,17 @@ void ic_enqueue(vc1cu_ctx* c, const DevParams& P, const std::vector<IcJob>& jobs
     t.n = n;
     if (!n) return;
     const size_t sb = ic_scratch_bytes(), db = (ic_desc_bytes() + 15) & ~size_t(15);
-    uint8_t* scratch = static_cast<uint8_t*>(ensure(c->d_ic, c->ic_cap, sb * n, "cudaMalloc(intensity scratch)"));
-    void* ddesc = ensure(c->d_icdesc, c->icdesc_cap, db * n, "cudaMalloc(intensity descriptors)");
+    uint8_t* scratch = static_cast<uint8_t*>(ensure(c, c->d_ic, c->ic_cap, sb * n, "cudaMalloc(intensity scratch)"));
+    void* ddesc = ensure(c, c->d_icdesc, c->icdesc_cap, db * n, "cudaMalloc(intensity descriptors)");
     if (t.cap < kIcHostBytes * n) {
         if (t.done) ck(cudaEventSynchronize(t.done), "cudaEventSynchronize(intensity)");
-        if (t.h) cudaFreeHost(t.h);
+        release(c, t.h, true);
         t.h = nullptr;
         t.cap = 0;
         ck(cudaMallocHost(&t.h, kIcHostBytes * n), "cudaMallocHost(intensity results)");
         t.cap = kIcHostBytes * n;
     }
+    captured_use(c, t.h);
     if (!t.done) ck(cudaEventCreateWithFlags(&t.done, cudaEventDisableTiming), "cudaEventCreate(intensity)");
     uint8_t* hp = static_cast<uint8_t*>(staging(c, db * n));
     for (int i = 0; i < n; ++i) ic_fill_desc(hp + db * i, jobs[i].cur, jobs[i].ref, jobs[i].mvs, scratch + sb * i);
@@ -1984,6 +2048,9 @@ int vc1cu_close(vc1cu_ctx* c) {
         cudaGraphDestroy(kv.second.g);
         for (void* h : kv.second.hold) cudaFreeHost(h);
     }
+    c->graphs.clear();
+    c->capture_use = vc1cu_ctx::GraphUse{};
+    release_retired(c);
     for (auto& kv : c->items) cudaFree(kv.second.first);
     if (c->h_read) cudaFreeHost(c->h_read);
     for (auto& b : c->staging_ring) {
@@ -2181,7 +2248,7 @@ int vc1cu_synth_frames(vc1cu_ctx* c, const vc1cu_synth_cfg* cfg, int first, int 
         const size_t nterms = (size_t)((s.width + 1) / 2) * ((s.height + 1) / 2);
         const size_t args_bytes = (sizeof(SynthArgs) + 255) & ~size_t(255);
         uint8_t* d = static_cast<uint8_t*>(
-            ensure(c->d_synth, c->synth_cap, args_bytes + 256 + nterms * sizeof(double), "cudaMalloc(synth)"));
+            ensure(c, c->d_synth, c->synth_cap, args_bytes + 256 + nterms * sizeof(double), "cudaMalloc(synth)"));
         SynthArgs* da = reinterpret_cast<SynthArgs*>(d);
         double* d_ms = reinterpret_cast<double*>(d + args_bytes);
         double* d_terms = reinterpret_cast<double*>(d + args_bytes + 256);
@@ -2258,6 +2325,7 @@ int vc1cu_graph_begin(vc1cu_ctx* c) {
         c->capture_results.clear();
         c->capture_bresults.clear();
         c->capture_frames.clear();
+        c->capture_use = vc1cu_ctx::GraphUse{};
         return VC1CU_OK;
     });
 }
@@ -2269,15 +2337,18 @@ int vc1cu_graph_end(vc1cu_ctx* c, int* graph_id) {
         stamp_written(c);
         vc1cu_ctx::Graph g;
         c->capturing = false;
-        ck(cudaStreamEndCapture(c->stream, &g.g), "cudaStreamEndCapture");
+        const cudaError_t ended = cudaStreamEndCapture(c->stream, &g.g);
         g.hold.swap(c->capture_hold);
         g.results.swap(c->capture_results);
         g.bresults.swap(c->capture_bresults);
         g.frames.swap(c->capture_frames);
-        const cudaError_t e = cudaGraphInstantiate(&g.exec, g.g, 0);
+        std::swap(g.use, c->capture_use);
+        const cudaError_t e = ended != cudaSuccess ? ended : cudaGraphInstantiate(&g.exec, g.g, 0);
         if (e != cudaSuccess) {
-            cudaGraphDestroy(g.g);
+            if (g.g) cudaGraphDestroy(g.g);
             for (void* h : g.hold) cudaFreeHost(h);
+            release_retired(c);
+            ck(ended, "cudaStreamEndCapture");
             throw Fail{VC1CU_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)};
         }
         const int id = c->graph_next++;
@@ -2292,6 +2363,22 @@ int vc1cu_graph_launch(vc1cu_ctx* c, int graph_id) {
         auto it = c->graphs.find(graph_id);
         if (it == c->graphs.end()) throw Fail{VC1CU_ERR_ARG, "unknown graph id"};
         if (c->capturing) throw Fail{VC1CU_ERR_STATE, "a capture is open on this context"};
+        for (const auto& u : it->second.use.slots) {
+            const int id = u.first.second;
+            vc1cu_ctx::SlotState now{nullptr, 0, 0};
+            if (u.first.first == vc1cu_ctx::kFrameSlot) {
+                const FrameSlot& f = c->frames[id];
+                now = {f.d, f.w, f.h};
+            } else if (u.first.first == vc1cu_ctx::kResultSlot) {
+                const ResultSlot& r = c->results[id];
+                now = {r.d, r.mbs, 0};
+            } else {
+                const BSlot& b = c->bresults[id];
+                now = {b.d, b.mbs, 0};
+            }
+            if (now != u.second)
+                throw Fail{VC1CU_ERR_STATE, "slot " + std::to_string(id) + " of the graph has had another size since its capture"};
+        }
         // frames the graph reads may have uploads in flight on the upload stream
         for (int id : it->second.frames) {
             auto f = c->frames.find(id);
@@ -2316,6 +2403,7 @@ int vc1cu_graph_destroy(vc1cu_ctx* c, int graph_id) {
         cudaGraphDestroy(it->second.g);
         for (void* h : it->second.hold) cudaFreeHost(h);
         c->graphs.erase(it);
+        release_retired(c);
         return VC1CU_OK;
     });
 }
@@ -2489,6 +2577,7 @@ int vc1cu_b_predict(vc1cu_ctx* c, const vc1cu_params* p, int bslot, int cur_id, 
         FrameSlot& fo = alloc_frame(c, pred_id, P.W, P.H);
         const DevFrame o = fo.view();
         const BSlot& b = it->second;
+        captured_slot(c, vc1cu_ctx::kBSlot, bslot, b.d, b.mbs);
         Timer tm(c, kMc);
         ck(launch_b_mc(P, cur, past, fut, b.r.modes, b.r.fmv, b.r.bmv, b.mode, (uint8_t*)o.y, (uint8_t*)o.u, (uint8_t*)o.v,
                        fo.pitch_y, fo.pitch_c, c->stream),
@@ -2750,7 +2839,7 @@ int vc1cu_fast_transform_types(vc1cu_ctx* c, const vc1cu_params* p, int src_id, 
         if (fs.w != P.W || fs.h != P.H || fp.w != P.W || fp.h != P.H)
             throw Fail{VC1CU_ERR_ARG, "frame size does not match the configuration"};
         const size_t mbs = (size_t)P.mbw * P.mbh;
-        uint8_t* d = static_cast<uint8_t*>(ensure(c->d_btypes, c->btypes_cap, std::max<size_t>(mbs * 6, 256), "cudaMalloc(types)"));
+        uint8_t* d = static_cast<uint8_t*>(ensure(c, c->d_btypes, c->btypes_cap, std::max<size_t>(mbs * 6, 256), "cudaMalloc(types)"));
         Timer tm(c, kXform);
         launch_fast_tt(P, fs.view(), fp.view(), d, c->stream);
         ck(cudaGetLastError(), "transform type launch");
@@ -2797,7 +2886,7 @@ int vc1cu_choose_transform(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_trd_
         trd_tables(c);
         auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
         const size_t b_sum = 256, b_mq = al(mbs), b_out = al(mbs * sizeof(vc1cu_tdecision)), b_lv = al(mbs * 384 * 2);
-        uint8_t* base = static_cast<uint8_t*>(ensure(c->d_trd, c->trd_cap, b_sum + b_mq + b_out + b_lv,
+        uint8_t* base = static_cast<uint8_t*>(ensure(c, c->d_trd, c->trd_cap, b_sum + b_mq + b_out + b_lv,
                                                      "cudaMalloc(transform RD buffers)"));
         auto* d_sum = reinterpret_cast<unsigned long long*>(base);
         uint8_t* d_mq = base + b_sum;
@@ -2849,7 +2938,7 @@ int vc1cu_choose_dquant(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_trd_cfg
                      b_lv = levels ? al((size_t)mbs * 768) : 0, b_stat = al(8 * (size_t)mbs);
         const size_t round_bytes = b_mq + b_list + b_out + b_lv;
         uint8_t* base = static_cast<uint8_t*>(
-            ensure(c->d_dq, c->dq_cap, 256 + kDqRounds * round_bytes + 2 * b_stat + al(mbs), "cudaMalloc(DQUANT search)"));
+            ensure(c, c->d_dq, c->dq_cap, 256 + kDqRounds * round_bytes + 2 * b_stat + al(mbs), "cudaMalloc(DQUANT search)"));
         auto* d_sum = reinterpret_cast<unsigned long long*>(base);
         auto rb_at = [&](int r) { return base + 256 + (size_t)r * round_bytes; };
         auto* d_lscale = reinterpret_cast<double*>(base + 256 + kDqRounds * round_bytes);
@@ -3044,7 +3133,7 @@ static int p_mv_mode_index(int mode, int pq, bool secondary) {
 // The mode decision's device buffer: 7 counters, the sampled MB list, their decisions.
 constexpr int kModeRdSamples = 32;
 static uint8_t* mrd_buffer(vc1cu_ctx* c) {
-    return static_cast<uint8_t*>(ensure(c->d_mrd, c->mrd_cap, 256 + 256 + kModeRdSamples * sizeof(vc1cu_tdecision),
+    return static_cast<uint8_t*>(ensure(c, c->d_mrd, c->mrd_cap, 256 + 256 + kModeRdSamples * sizeof(vc1cu_tdecision),
                                         "cudaMalloc(mode decision buffers)"));
 }
 
@@ -3374,7 +3463,7 @@ static int loop_filter_p(vc1cu_ctx* c, const vc1cu_params* p, int frame_id, cons
             if (cbp[i] > 15 || !(tt[i] == 0 || tt[i] == 3 || tt[i] == 6 || tt[i] == 7))
                 throw Fail{VC1CU_ERR_ARG, "block patterns are 4-bit and transform kinds 0, 3, 6 or 7"};
         const size_t bm = 32 * mbs, al = (bm + 255) & ~size_t(255);
-        uint8_t* d = static_cast<uint8_t*>(ensure(c->d_lf, c->lf_cap, al + 13 * mbs + 256, "cudaMalloc(loop filter metadata)"));
+        uint8_t* d = static_cast<uint8_t*>(ensure(c, c->d_lf, c->lf_cap, al + 13 * mbs + 256, "cudaMalloc(loop filter metadata)"));
         ck(cudaMemcpyAsync(d, block_mvs, bm, cudaMemcpyHostToDevice, c->stream), "upload block vectors");
         ck(cudaMemcpyAsync(d + al, cbp, 6 * mbs, cudaMemcpyHostToDevice, c->stream), "upload block patterns");
         ck(cudaMemcpyAsync(d + al + 6 * mbs, tt, 6 * mbs, cudaMemcpyHostToDevice, c->stream), "upload transform kinds");
@@ -3411,7 +3500,7 @@ static void intra_recon(vc1cu_ctx* c, const DevParams& P, const vc1cu_trd_cfg& c
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t b_scr = al(intra_scratch_bytes(P)), b_edge = al(mbs * 256 * 3 / 2), b_map = al(mbs);
     uint8_t* base = static_cast<uint8_t*>(
-        ensure(c->d_intra, c->intra_cap, b_scr + b_edge + 3 * b_map, "cudaMalloc(intra reconstruction)"));
+        ensure(c, c->d_intra, c->intra_cap, b_scr + b_edge + 3 * b_map, "cudaMalloc(intra reconstruction)"));
     uint8_t* d_flags = base + b_scr + b_edge;
     uint8_t* d_mq = d_flags + b_map;
     uint8_t* d_der = d_mq + b_map;
@@ -3487,7 +3576,7 @@ int vc1cu_choose_i_overlap(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_trd_
         auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
         const size_t ny = mbs * 256, nc = mbs * 64, b_rec = al(4 * (ny + 2 * nc)), b_sse = al(8 * mbs);
         uint8_t* base = static_cast<uint8_t*>(
-            ensure(c->d_iovl, c->iovl_cap, 3 * b_rec + 3 * b_sse + al(mbs) + 256, "cudaMalloc(overlap plan)"));
+            ensure(c, c->d_iovl, c->iovl_cap, 3 * b_rec + 3 * b_sse + al(mbs) + 256, "cudaMalloc(overlap plan)"));
         auto rec = [&](int k, int pl) {
             int32_t* r = reinterpret_cast<int32_t*>(base + (size_t)k * b_rec);
             return pl == 0 ? r : (pl == 1 ? r + ny : r + ny + nc);
@@ -3560,7 +3649,7 @@ int vc1cu_choose_i_overlap(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_trd_
 // The per-macroblock byte map of an overlap call on the device (stream-ordered after any launch
 // still reading the previous one).
 static const uint8_t* upload_mb_map(vc1cu_ctx* c, const uint8_t* map, size_t mbs) {
-    uint8_t* d = static_cast<uint8_t*>(ensure(c->d_ovl, c->ovl_cap, mbs, "cudaMalloc(macroblock map)"));
+    uint8_t* d = static_cast<uint8_t*>(ensure(c, c->d_ovl, c->ovl_cap, mbs, "cudaMalloc(macroblock map)"));
     ck(cudaMemcpyAsync(d, map, mbs, cudaMemcpyHostToDevice, c->stream), "upload macroblock map");
     return d;
 }
@@ -3628,7 +3717,7 @@ static int reconstruct(vc1cu_ctx* c, const vc1cu_params* p, int pred_id, const i
             for (int i = 0; i < mbs; ++i)
                 if (mquant[i] < 1 || mquant[i] > 31) throw Fail{VC1CU_ERR_ARG, "MQUANT must be 1..31"};
         // block types, then the per-MB MQUANT and derived flags (8 bytes per MB in all)
-        uint8_t* dt = static_cast<uint8_t*>(ensure(c->d_btypes, c->btypes_cap, (size_t)mbs * 8, "cudaMalloc(block types)"));
+        uint8_t* dt = static_cast<uint8_t*>(ensure(c, c->d_btypes, c->btypes_cap, (size_t)mbs * 8, "cudaMalloc(block types)"));
         ck(cudaMemcpyAsync(dt, block_types, (size_t)mbs * 6, cudaMemcpyHostToDevice, c->stream), "upload block types");
         uint8_t* dmq = dt + (size_t)mbs * 6;
         uint8_t* dder = dmq + mbs;
@@ -3688,7 +3777,7 @@ int vc1cu_forward_quant(vc1cu_ctx* c, const vc1cu_params* p, int src_id, int pre
         for (int t = 0; t < 4; ++t) nt += (type_mask >> t) & 1;
         const size_t n = (size_t)nt * P.mbw * P.mbh * 6 * 64;
         const size_t cb = n * 8, lb = n * 2;
-        ensure(c->d_scratch, c->scratch_cap, cb + lb + 256, "cudaMalloc(transform output)");
+        ensure(c, c->d_scratch, c->scratch_cap, cb + lb + 256, "cudaMalloc(transform output)");
         double* dco = static_cast<double*>(c->d_scratch);
         int16_t* dlv = reinterpret_cast<int16_t*>(static_cast<uint8_t*>(c->d_scratch) + ((cb + 255) & ~size_t(255)));
         FrameSlot& fs = frame_slot(c, src_id);
