@@ -806,6 +806,15 @@ void staging_mark(vc1cu_ctx* c) {
     ck(cudaEventRecord(c->staging_ring[c->staging_cur].done, c->stream), "cudaEventRecord(staging)");
 }
 
+// A caller's host array as the source of an upload: itself, or inside a capture a copy that the graph
+// keeps (its replays read it again, when the caller's array may have changed or gone).
+const void* upload_source(vc1cu_ctx* c, const void* host, size_t bytes) {
+    if (!c->capturing) return host;
+    void* h = staging(c, bytes);
+    std::memcpy(h, host, bytes);
+    return h;
+}
+
 int score_common(vc1cu_ctx* c, const DevParams& P, const ScoreArgs& a, const vc1cu_mv* cands, size_t n, uint64_t* costs) {
     const size_t cb = n * sizeof(int2), ob = n * sizeof(unsigned long long);
     ensure(c, c->d_scratch, c->scratch_cap, cb + ob + 256, "cudaMalloc(candidates)");
@@ -3650,7 +3659,7 @@ int vc1cu_choose_i_overlap(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_trd_
 // still reading the previous one).
 static const uint8_t* upload_mb_map(vc1cu_ctx* c, const uint8_t* map, size_t mbs) {
     uint8_t* d = static_cast<uint8_t*>(ensure(c, c->d_ovl, c->ovl_cap, mbs, "cudaMalloc(macroblock map)"));
-    ck(cudaMemcpyAsync(d, map, mbs, cudaMemcpyHostToDevice, c->stream), "upload macroblock map");
+    ck(cudaMemcpyAsync(d, upload_source(c, map, mbs), mbs, cudaMemcpyHostToDevice, c->stream), "upload macroblock map");
     return d;
 }
 
@@ -3718,7 +3727,8 @@ static int reconstruct(vc1cu_ctx* c, const vc1cu_params* p, int pred_id, const i
                 if (mquant[i] < 1 || mquant[i] > 31) throw Fail{VC1CU_ERR_ARG, "MQUANT must be 1..31"};
         // block types, then the per-MB MQUANT and derived flags (8 bytes per MB in all)
         uint8_t* dt = static_cast<uint8_t*>(ensure(c, c->d_btypes, c->btypes_cap, (size_t)mbs * 8, "cudaMalloc(block types)"));
-        ck(cudaMemcpyAsync(dt, block_types, (size_t)mbs * 6, cudaMemcpyHostToDevice, c->stream), "upload block types");
+        const void* types = upload_source(c, block_types, (size_t)mbs * 6);
+        ck(cudaMemcpyAsync(dt, types, (size_t)mbs * 6, cudaMemcpyHostToDevice, c->stream), "upload block types");
         uint8_t* dmq = dt + (size_t)mbs * 6;
         uint8_t* dder = dmq + mbs;
         if (mquant) ck(cudaMemcpyAsync(dmq, mquant, (size_t)mbs, cudaMemcpyHostToDevice, c->stream), "upload MQUANT");

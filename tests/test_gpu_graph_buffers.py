@@ -4,6 +4,7 @@ A graph's nodes hold the addresses of the context's buffers (search states, pass
 descriptors, prediction planes, signature indexes). A later, larger call replaces them; the replay
 must still write what the recorded calls wrote. A slot that has had another size since is refused.
 """
+import numpy as np
 import pytest
 
 from libvc1_b200 import synth
@@ -96,5 +97,41 @@ def test_replay_refused_after_a_slot_changed_size(own, slot):
         _upload(c, 96, 64, 3, 20)
         c.core_passes(p, [(22, 20, MV_QPEL, 0, -1, 5)])
         assert c.read_result(p, 5).equal(want) == []
+    finally:
+        c.graph_destroy(g)
+
+
+def test_replay_keeps_the_recorded_host_arrays(own):
+    """The host arrays of captured calls may change or go after the capture."""
+    torch = pytest.importorskip("torch")
+    c = own
+    w, h, mbs = 96, 64, 24
+    p = make_params(w, h, search_range=8, local_search_range=8, pqindex=4)
+    _upload(c, w, h, 5, 0)
+    lv = torch.empty((4, mbs, 6, 64), dtype=torch.int16, device="cuda")
+    c.forward_quant_device(p, 1, 0, 15, 0, lv.data_ptr())
+    signed = [torch.arange(n, dtype=torch.int32, device="cuda") % 255 for n in (w * h, w * h // 4, w * h // 4)]
+    torch.cuda.synchronize()
+    rng = np.random.default_rng(1)
+    types = rng.integers(1, 5, (mbs, 6)).astype(np.uint8)
+    mask = rng.integers(0, 2, mbs).astype(np.uint8)
+
+    def calls():
+        c.reconstruct(p, 0, lv.data_ptr(), 15, types, 3)
+        c.store_signed(p, *[s.data_ptr() for s in signed], 0, 3, mask)
+
+    calls()
+    want = c.download_frame(3, w, h)
+    c.graph_begin()
+    calls()
+    g = c.graph_end()
+    try:
+        types[:] = 5 - types
+        mask[:] = 1 - mask
+        calls()
+        assert any(not np.array_equal(a, b) for a, b in zip(c.download_frame(3, w, h), want))
+        c.graph_launch(g)
+        for a, b in zip(c.download_frame(3, w, h), want):
+            assert np.array_equal(a, b)
     finally:
         c.graph_destroy(g)
