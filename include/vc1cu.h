@@ -910,9 +910,10 @@ int vc1cu_lp_analyze(vc1cu_lp* net, const vc1cu_params* p, const vc1cu_lp_pass* 
  * Limits: 1 <= n <= 16 pictures per call and 0 <= range <= 32; larger requests are
  * rejected with VC1CU_ERR_ARG. The search state lives in one fixed device array of
  * 134,784 bytes that every GPU loading this library holds until the process exits. All
- * calls on one device share that array: two calls whose GPU work can overlap (issued on
- * different streams, or from threads that do not order them) race on it and give wrong
- * results; calls issued in order on one stream are safe, and devices are independent.
+ * calls on one device share that array, so their work runs one after another, in the order of the
+ * calls, whatever streams and threads they come from; devices are independent. Calls recorded
+ * into a CUDA graph are not ordered by this: replays whose GPU work can overlap another call's or
+ * another replay's race on the array, and the caller must order them.
  * Each call resets the state it reads, so nothing carries over from an earlier call.
  *
  * width and height may be odd (any coding size up to 16384); pitch >= width.

@@ -613,8 +613,9 @@ def global_motion_noalloc(cur_ptrs, ref_ptrs, pitch: int, width: int, height: in
     device address the caller already owns (luma planes, int32[2n] and uint64[n] outputs),
     and the search state lives in a fixed array inside the library (at most 16 pictures
     per call, search_range 0..32). Enqueued on `stream` (a cudaStream_t handle); the
-    results are ready once that stream is synchronised. Calls on one device must not
-    overlap on the GPU: they share that array.
+    results are ready once that stream is synchronised. Calls on one device share that
+    array and run one after another on the GPU; replays of captured calls are the caller's
+    to order.
     """
     L = load_library()
     n = len(cur_ptrs)

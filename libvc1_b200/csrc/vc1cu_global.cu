@@ -17,9 +17,12 @@
 // only on insertion) does depend on the order and is replayed by one warp, entry per lane.
 // Folding on one thread, with the lists in global memory, took 0.87 ms of a CIF search, 2.3 ms of two
 // at 1080p; folded here it is within the scoring launches' time.
+#include <cuda.h>  // CUcontext (cuCtxGetId is reached through the runtime's entry point)
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <map>
+#include <mutex>
 
 #include "vc1cu_core.cuh"
 
@@ -373,7 +376,7 @@ void init_gin(GIn* h, const DevFrame& cur, const DevFrame& ref, int range, int* 
 // the device or is not permitted. For them the search state of up to
 // kNoAllocMaxPictures pictures lives in this fixed array, which every GPU that loads the
 // library holds until the process exits (16 states of 8,424 bytes: 134,784 bytes).
-// Every call shares it.
+// Every call shares it; calls are ordered on the device, one after another.
 constexpr int kNoAllocMaxPictures = 16;
 static __device__ __align__(256) GState g_noalloc_states[kNoAllocMaxPictures];
 static_assert(sizeof(GState) * kNoAllocMaxPictures == 134784, "the size the interface documents");
@@ -401,6 +404,38 @@ __global__ void noalloc_init_kernel(GState* states, const __grid_constant__ NoAl
 }  // namespace vc1cu
 
 namespace {
+
+// The order of the calls that share a context's array: each call's work waits for the event after the
+// work of the call before it, whatever streams and threads they come from. One event per context (its
+// id is never given again, so an event that went with its context is not used).
+std::mutex& noalloc_mutex() {
+    static std::mutex* m = new std::mutex;  // not destroyed: calls may come from exit handlers
+    return *m;
+}
+
+cudaError_t noalloc_event(cudaEvent_t* e) {
+    using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+    static CtxGetIdFn ctx_id = []() -> CtxGetIdFn {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<CtxGetIdFn>(p);
+    }();
+    static auto* events = new std::map<unsigned long long, cudaEvent_t>;
+    unsigned long long id = 0;
+    if (!ctx_id || ctx_id(nullptr, &id) != CUDA_SUCCESS) return cudaErrorDeviceUninitialized;
+    cudaEvent_t& ev = (*events)[id];
+    if (!ev) {
+        const cudaError_t rc = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (rc != cudaSuccess) {
+            events->erase(id);
+            return rc;
+        }
+    }
+    *e = ev;
+    return cudaSuccess;
+}
 
 int noalloc_fail(char* err, size_t err_len, int code, const char* msg) {
     if (err && err_len) std::snprintf(err, err_len, "%s", msg);
@@ -445,11 +480,26 @@ extern "C" int vc1cu_global_motion_noalloc(const uint8_t* const* cur_y, const ui
                             e != cudaSuccess ? cudaGetErrorString(e) : "cudaGetSymbolAddress returned null");
     GState* states = static_cast<GState*>(ptr);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // a captured call is ordered by whoever replays it
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
+    std::lock_guard<std::mutex> lock(noalloc_mutex());
+    cudaEvent_t after = nullptr;
+    if (capture == cudaStreamCaptureStatusNone) {
+        e = noalloc_event(&after);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, after, 0);
+        if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
+    }
     noalloc_init_kernel<<<1, 32, 0, s>>>(states, a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
     run_global_search(states, nullptr, n, range, width, height, s);
     e = cudaGetLastError();
+    if (after) {
+        const cudaError_t r = cudaEventRecord(after, s);
+        if (e == cudaSuccess) e = r;
+    }
     if (e != cudaSuccess) return noalloc_fail(err, err_len, VC1CU_ERR_CUDA, cudaGetErrorString(e));
     return VC1CU_OK;
 }

@@ -5,6 +5,7 @@
 // rewritten to emu::shared and EMU_LAUNCH (see test_global_search_blocks.py).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 #include <ucontext.h>
@@ -61,6 +62,7 @@ inline dim3 grid_dim, block_dim;
 inline const std::function<void()>* body = nullptr;
 inline Order order = kInOrder;
 inline std::string fault;
+inline std::vector<std::string> trace;  // launches ("launch <stream>"), and what the test's stubs add
 
 inline void yield(Thread::State s) {
     Thread* t = cur;
@@ -143,8 +145,10 @@ inline Thread* pick(std::vector<Block>& blocks) {
 
 struct Cfg {
     dim3 grid, block;
-    Cfg(dim3 g, dim3 b, size_t = 0, cudaStream_t = nullptr) : grid(g), block(b) {}
+    cudaStream_t stream;
+    Cfg(dim3 g, dim3 b, size_t = 0, cudaStream_t s = nullptr) : grid(g), block(b), stream(s) {}
     void run(const std::function<void()>& f) const {
+        trace.push_back("launch " + std::to_string(reinterpret_cast<uintptr_t>(stream)));
         if (!fault.empty()) return;
         constexpr size_t kStack = 64 << 10;
         const size_t per = block.x, n = (size_t)grid.x * grid.y * grid.z;

@@ -5,6 +5,9 @@ the stage has read. So no warp may still have its candidate to read once its blo
 finished, however late that warp runs: the order "late warps" lets the first warp of each block run
 ahead and holds the rest of a finished block back until nothing else can advance. The kernels'
 source itself is compiled (emulation/cuda_blocks.h); the results are the oracle's.
+
+The allocation-free form keeps its state in one array per device: a call's work has to wait for the
+work of the call before it, whatever their streams.
 """
 import ctypes as C
 import os
@@ -27,6 +30,49 @@ extern "C" int emulate(const uint8_t* cur, const uint8_t* ref, int w, int h, int
     const int rc = vc1cu_global_motion_noalloc(&cur, &ref, w, w, h, range, 1, dxdy, (uint64_t*)sad, nullptr, why, cap);
     if (!emu::fault.empty()) std::snprintf(why, cap, "%s", emu::fault.c_str());
     return rc ? rc : (emu::fault.empty() ? 0 : -1);
+}
+static bool g_capturing;
+static std::string num(const void* p) { return std::to_string(reinterpret_cast<uintptr_t>(p)); }
+// One call per stream; the launches, event records and waits that they make, one per line.
+extern "C" int emulate_calls(const uint8_t* a, const uint8_t* b, int w, int h, const uintptr_t* streams, int n,
+                             int capturing, char* out, size_t cap) {
+    emu::order = emu::kInOrder;
+    emu::fault.clear();
+    emu::trace.clear();
+    g_capturing = capturing != 0;
+    int dxdy[2], rc = 0;
+    uint64_t sad;
+    for (int i = 0; i < n && !rc; ++i)
+        rc = vc1cu_global_motion_noalloc(&a, &b, w, w, h, 1, 1, dxdy, &sad, reinterpret_cast<void*>(streams[i]), out, cap);
+    std::string t;
+    for (const auto& l : emu::trace) t += l + "\n";
+    std::snprintf(out, cap, "%s", t.c_str());
+    g_capturing = false;
+    return rc;
+}
+static CUresult fake_ctx_id(CUcontext, unsigned long long* id) { *id = 7; return CUDA_SUCCESS; }
+extern "C" cudaError_t cudaGetDriverEntryPoint(const char*, void** fn, unsigned long long,
+                                               cudaDriverEntryPointQueryResult* q) {
+    *fn = reinterpret_cast<void*>(&fake_ctx_id);
+    if (q) *q = cudaDriverEntryPointSuccess;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* c) {
+    *c = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    static uintptr_t next = 100;
+    *e = reinterpret_cast<cudaEvent_t>(next++);
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    emu::trace.push_back("wait " + num(s) + " " + num(e));
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    emu::trace.push_back("record " + num(s) + " " + num(e));
+    return cudaSuccess;
 }
 extern "C" cudaError_t cudaGetLastError() { return cudaSuccess; }
 extern "C" const char* cudaGetErrorString(cudaError_t) { return "emulated"; }
@@ -55,6 +101,16 @@ def search(tmp_path_factory):
                          C.byref(sad), why, C.c_size_t(256))
         return rc, why.value.decode(), (dxdy[0], dxdy[1], sad.value)
 
+    def calls(pic, streams, capturing=False):
+        h, w = pic.shape
+        out = C.create_string_buffer(1 << 16)
+        ptr = pic.ctypes.data_as(C.c_void_p)
+        rc = lib.emulate_calls(ptr, ptr, w, h, (C.c_size_t * len(streams))(*streams), len(streams), int(capturing), out,
+                               C.c_size_t(1 << 16))
+        assert rc == 0, out.value
+        return out.value.decode().split("\n")[:-1]
+
+    run.calls = calls
     return run
 
 
@@ -74,3 +130,22 @@ def test_stage_fold_waits_for_every_warp(search, oracle, rng, dx, dy, order):
     rc, why, got = search(cur, ref, rng, ["in order", "late warps"].index(order))
     assert rc == 0, why
     assert got == tuple(int(v) for v in want)
+
+
+def test_calls_that_share_the_array_run_in_order(search):
+    pic = np.zeros((16, 16), np.uint8)
+    done = []  # (stream, event) of the last record
+    first = True
+    for line in search.calls(pic, [1, 2, 2, 3]):
+        what, *v = line.split()
+        if what == "record":
+            done, first = [v[0], v[1]], True
+        elif what == "wait":
+            assert not done or v[1] == done[1]
+            done = []
+        else:  # a call's first launch comes after the wait for the last call's record
+            assert not first or not done, line
+            first = False
+    assert done  # the last call left its record
+    # a captured call takes no part: an event outside its capture would end the capture
+    assert {line.split()[0] for line in search.calls(pic, [1, 2], capturing=True)} == {"launch"}
