@@ -360,8 +360,10 @@ int vc1cu_graph_destroy(vc1cu_ctx* ctx, int graph_id);
  * Launch-shape autotuner (no counterpart in the reference): runs the given passes' launches
  * (per_pass_params: params holds one block per pass, as vc1cu_core_passes_multi; else one block)
  * under several shapes of the persistent core kernel - macroblocks (warps) per block and blocks
- * per SM - and keeps each launch's fastest for its raster, search configuration and kernel
- * instantiation; later launches of that key use it. The passes' result slots are overwritten.
+ * per SM - and keeps each launch's fastest. Later launches use it that have the same search
+ * configuration, kernel instantiation and MV modes and as many passes of each raster (launches of
+ * this call that agree in these take the shape that is fastest for them together); other launches,
+ * of more or fewer passes, keep the library's own choice. The passes' result slots are overwritten.
  * Synchronous; *warps, *blocks (0 = as many as fit) of the longest launch and *ms (all launches,
  * one pass over them) may be NULL.
  */

@@ -28,6 +28,7 @@
 #include "vc1cu_core.cuh"
 #include "vc1cu_lp.cuh"
 #include "vc1cu_synth.cuh"
+#include "vc1cu_tune.cuh"
 
 namespace vc1cu {
 // kernels and drivers of the other translation units
@@ -392,8 +393,8 @@ struct vc1cu_ctx {
     };
     std::map<int, Graph> graphs;
     int graph_next = 1;
-    // launch shapes chosen by vc1cu_autotune: key (W, H, range, local range, instantiation) ->
-    // (warps per block, blocks per SM; 0 = the occupancy limit)
+    // launch shapes chosen by vc1cu_autotune: tune_key -> (warps per block, blocks per SM; 0 = the
+    // occupancy limit)
     std::map<std::vector<int>, std::pair<int, int>> tuned;
     std::pair<int, int> tune_force{0, 0};  // a shape under trial (vc1cu_autotune), (0, 0) otherwise
     std::vector<int> last_tune_key;        // the key of the last core launch
@@ -897,9 +898,6 @@ void same_search_config(const DevParams& a, const DevParams& b) {
                                   "quality, sub-pel and long-range settings, thresholds)"};
 }
 
-// The autotuner's cache key of a launch: raster, ranges, algorithm and the instantiation.
-std::vector<int> tune_key(const DevParams& P, int kind) { return {P.W, P.H, P.range, P.local_range, P.me_algorithm, kind}; }
-
 // The macroblocks of one wavefront step, at most.
 int front_of(int mbw, int mbh) { return std::min((mbw + 1) / 2, mbh); }
 
@@ -1115,9 +1113,11 @@ int launch_group(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes, 
             blocks = (int)std::max(1L, (5 * front + 12 * sms - 1) / (12 * sms));
         }
     }
-    // a launch shape chosen by vc1cu_autotune for this raster, search configuration and instantiation
-    {
-        c->last_tune_key = tune_key(P, kind);
+    // a shape chosen by vc1cu_autotune for such launches
+    if (c->tune_force.first || !c->tuned.empty()) {
+        std::vector<TunePass> tp(n);
+        for (int i = 0; i < n; ++i) tp[i] = TunePass{h[i].geom.W, h[i].geom.H, h[i].mode, h[i].allow_intra};
+        c->last_tune_key = tune_key(P.range, P.local_range, P.me_algorithm, kind, tp);
         auto t = c->tuned.find(c->last_tune_key);
         if (c->tune_force.first) {
             warps = c->tune_force.first;
@@ -2424,9 +2424,21 @@ int vc1cu_autotune(vc1cu_ctx* c, const vc1cu_params* params, const vc1cu_pass* p
         if (c->capturing) throw Fail{VC1CU_ERR_STATE, "cannot tune during a capture"};
         const vc1cu_params* pp = per_pass_params ? params : nullptr;
         check_passes(c, params, passes, n, pp);
-        cudaEvent_t a = take_event(c), b = take_event(c);
-        double total = 0.0, longest = -1.0;
-        std::pair<int, int> shown{0, 0};
+        // warps (macroblocks) per block and blocks per SM (0: as many as fit); shapes that do not fit
+        // the launch's instantiation or shared memory are skipped
+        const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {4, 3}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
+                                              {5, 1}, {6, 1}, {7, 1}, {8, 1}};
+        struct Events {
+            vc1cu_ctx* c;
+            cudaEvent_t a, b;
+            explicit Events(vc1cu_ctx* cc) : c(cc), a(take_event(cc)), b(take_event(cc)) {}
+            ~Events() {
+                c->tune_force = {0, 0};
+                c->event_pool.push_back(a);
+                c->event_pool.push_back(b);
+            }
+        } ev(c);
+        std::vector<TuneTrial> trials;
         // each of the call's launches in turn (a later one reads the seeds an earlier one leaves)
         for (const std::vector<int>& g : plan_launches(c, params, passes, n, pp)) {
             std::vector<vc1cu_pass> q;
@@ -2436,54 +2448,40 @@ int vc1cu_autotune(vc1cu_ctx* c, const vc1cu_params* params, const vc1cu_pass* p
                 if (pp) gp.push_back(pp[i]);
             }
             auto run = [&]() { launch_group(c, params, q.data(), (int)q.size(), false, nullptr, pp ? gp.data() : nullptr); };
-            double best = -1.0;
-            std::pair<int, int> best_shape{0, 0};
-            std::vector<int> key;
-            // warps (macroblocks) per block and blocks per SM (0: as many as fit); shapes that do not fit
-            // the launch's instantiation or shared memory are skipped
-            const std::pair<int, int> shapes[] = {{4, 0}, {4, 1}, {4, 2}, {4, 3}, {2, 0}, {2, 2}, {1, 0}, {1, 4}, {3, 0},
-                                                  {5, 1}, {6, 1}, {7, 1}, {8, 1}};
+            TuneTrial trial;
             for (const auto& s : shapes) {
                 c->tune_force = s;
+                float ms = -1.f;
                 try {
                     run();  // warm-up (and the shape's work-item table)
-                    ck(cudaEventRecord(a, c->stream), "cudaEventRecord");
+                    ck(cudaEventRecord(ev.a, c->stream), "cudaEventRecord");
                     run();
                     run();
-                    ck(cudaEventRecord(b, c->stream), "cudaEventRecord");
+                    ck(cudaEventRecord(ev.b, c->stream), "cudaEventRecord");
                     check_status(c);
+                    ck(cudaEventElapsedTime(&ms, ev.a, ev.b), "cudaEventElapsedTime");
                 } catch (const Fail& f) {
-                    if (f.code != VC1CU_ERR_ARG) {  // a shape that does not fit is skipped, anything else fails
-                        c->tune_force = {0, 0};
-                        c->event_pool.push_back(a);
-                        c->event_pool.push_back(b);
-                        throw;
-                    }
-                    continue;
+                    if (f.code != VC1CU_ERR_ARG) throw;  // a shape that does not fit is skipped
                 }
-                float ms = 0.f;
-                ck(cudaEventElapsedTime(&ms, a, b), "cudaEventElapsedTime");
-                key = c->last_tune_key;
-                if (best < 0.0 || ms < best) {
-                    best = ms;
-                    best_shape = s;
-                }
+                trial.ms.push_back(ms / 2.0);
             }
-            c->tune_force = {0, 0};
-            if (best < 0.0) {
-                c->event_pool.push_back(a);
-                c->event_pool.push_back(b);
-                throw Fail{VC1CU_ERR_UNSUPPORTED, "no launch shape fits"};
-            }
-            c->tuned[key] = best_shape;
-            total += best / 2.0;
-            if (best > longest) {
-                longest = best;
-                shown = best_shape;
+            trial.key = c->last_tune_key;
+            trials.push_back(trial);
+        }
+        const auto choice = tune_choice(trials);
+        for (const auto& k : choice)
+            if (k.second < 0) throw Fail{VC1CU_ERR_UNSUPPORTED, "no launch shape fits"};
+        double total = 0.0, longest = -1.0;
+        std::pair<int, int> shown{0, 0};
+        for (const TuneTrial& t : trials) {
+            const int s = choice.at(t.key);
+            c->tuned[t.key] = shapes[s];
+            total += t.ms[s];
+            if (t.ms[s] > longest) {
+                longest = t.ms[s];
+                shown = shapes[s];
             }
         }
-        c->event_pool.push_back(a);
-        c->event_pool.push_back(b);
         if (warps_out) *warps_out = shown.first;
         if (blocks_out) *blocks_out = shown.second;
         if (ms_out) *ms_out = total;
