@@ -1298,7 +1298,7 @@ void check_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
         for (int j = 0; j < n; ++j)
             if (passes[j].out_slot == passes[i].seed_slot) s = j;
         if (s < 0) result_slot(c, passes[i].seed_slot, geom[i].mbw * geom[i].mbh, false);
-        else if (geom[s].mbw != geom[i].mbw || geom[s].mbh != geom[i].mbh)
+        else if (geom[s].mbw * geom[s].mbh != geom[i].mbw * geom[i].mbh)  // as result_slot tests it
             throw Fail{VC1CU_ERR_ARG, "a pass's seed is a pass over another raster"};
     }
 }
