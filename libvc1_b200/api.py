@@ -331,8 +331,9 @@ class CudaComputeContext:
         self._check(self._L.vc1cu_core_passes(self._h, C.byref(params), arr, len(passes)))
 
     def core_passes_multi(self, params_list, passes):
-        """Passes over pictures of different sizes in one launch: params_list[i] is pass i's
-        parameter block; passes as for core_passes."""
+        """Passes over pictures of different sizes, one launch per step of their seed chain (and one each
+        for the passes with and without P-intra): params_list[i] is pass i's parameter block; passes
+        as for core_passes."""
         arr = (Pass * len(passes))(*[Pass(*p) for p in passes])
         pp = (Params * len(params_list))(*params_list)
         self._check(self._L.vc1cu_core_passes_multi(self._h, pp, arr, len(passes)))

@@ -1306,7 +1306,10 @@ void check_passes(vc1cu_ctx* c, const vc1cu_params* p, const vc1cu_pass* passes,
 // Wavefront fronts (macroblocks of one step, at most) of up to this many macroblocks per SM run
 // seeded passes of different modes as one launch. Every step of its chain waits for one macroblock's
 // latency: passes that leave warps idle cost one chain together instead of one each, and more of them
-// pay for the larger code of several modes.
+// pay for the larger code of several modes. Three modes of n equal pictures, one launch against one per
+// mode (ms): 1080p n = 1 (1.2 per SM) 3.4 / 5.8, 6 (7.3) 9.3 / 9.6, 8 (9.7) 10.7 / 10.7, 12 (14.6) 13.9 /
+// 12.5, 20 (24) 20.8 / 14.9; 720p 8 (6.5) 5.6 / 6.1, 12 (9.7) 6.9 / 6.9, 16 (13) 8.2 / 7.7; CIF 1 (0.2) 0.83
+// / 1.42, 32 (7.1) 2.4 / 2.6, 64 (14) 3.6 / 3.3. The two meet near 9.7 at every size.
 constexpr int kMergeFront = VC1CU_MERGE_FRONT;
 
 // The launches of a call's passes, in order, as index lists. A pass seeded by another pass of the

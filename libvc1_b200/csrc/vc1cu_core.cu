@@ -3,7 +3,7 @@
 //
 // Execution model (sm_100a):
 //   * persistent grid; each warp owns one macroblock at a time, taken from a global work
-//     queue that interleaves the pictures of the batch in raster order, so every
+//     queue that interleaves the pictures of the batch in wavefront order, so every
 //     dependency of an item was handed out before it;
 //   * the raster-order dependency of the reference (left, top-left, top, top-right MVs of
 //     the same pass, encoder_motion.cpp:1312-1466) is a wavefront: a warp waits on the
@@ -137,10 +137,6 @@ struct Mb {
     uint32_t tma_phase;    // parity of the window mbarrier's next phase
     bool tma_pending;      // a TMA window copy is in flight
 };
-
-__device__ __forceinline__ bool win_inside(const Mb& m, int xa, int ya, int xb, int yb) {
-    return xa >= m.wx0 && ya >= m.wy0 && xb < m.wx0 + m.wp && yb < m.wy0 + m.wh;
-}
 
 // SAD of one row segment of n <= 8 visible pixels against the current block at shared
 // byte offset `cur`: the same predictions as predict_row<8> (sx = px + floor(xq/4) ...),
@@ -2322,8 +2318,8 @@ __device__ __forceinline__ void ld_acquire(const uint32_t* p) {
 
 // Waits (bounded) until each lane's flag equals epoch (a macroblock of this launch was
 // published; a lane with a null flag waits for nothing). The flags are polled with relaxed
-// loads, all lanes at once, and one acquire fence follows the last poll, so a poll costs
-// no L1 invalidation. Every lane calls it. After 2^log2_limit polls it gives up: it raises
+// loads, all lanes at once, and loaded once more with acquire semantics after the last poll, so
+// a poll costs no L1 invalidation. Every lane calls it. After 2^log2_limit polls it gives up: it raises
 // the launch's error and abort flags and returns false (a wait that sees the abort flag
 // returns false at once).
 // code: the waiting work item, recorded (with the lanes still waiting) by the first wait

@@ -119,7 +119,7 @@ struct LaunchStatus {
     unsigned int queue;
     unsigned int timeouts;
     unsigned int tcode;  // 1 + the work item of the first wait that gave up (0: none)
-    unsigned int tmask;  // its lanes still waiting (lanes 0-3: left, top-left, top, top-right; lane 0: seed)
+    unsigned int tmask;  // its lanes still waiting (lanes 0-3: left, top-left, top, top-right); 0x100: the window copy
 };
 
 // A pass that reuses another pass's whole-frame search (same picture pair) takes its result.
